@@ -76,6 +76,21 @@ struct DevBuf {
     size_t cap = 0;
 };
 
+// A frame's descriptors on their way to the device: its draws, then its jobs,
+// built in place and copied as one.  Small ones go through ordinary memory
+// (the runtime copies them out before the call returns); from RF_UPLOAD_PIN
+// bytes on through a ring of page-locked buffers, each free again when the
+// copy that reads it is done -- from ordinary memory such a copy would hold
+// the host until the stream reaches it.
+constexpr size_t RF_UPLOAD_PIN = 16384;
+constexpr uint32_t RF_UPLOAD_RING = 3;
+struct UploadBuf {
+    char *p = nullptr;  // page-locked
+    size_t cap = 0;
+    cudaEvent_t copied = nullptr;
+    bool pending = false;
+};
+
 // An instantiated launch sequence and the frame shape it was captured for.
 struct GraphKey {
     uint64_t v[13];
@@ -152,7 +167,16 @@ struct rf_ctx {
     rf_stats host_acc{};
     rf_stats taken{};
     char last_error[1024] = {0};  // the failing call (as written) and the CUDA message
-    std::vector<DrawDev> hdraws;
+    // Descriptors of the frame being built: ndraws draws in hdraws (the
+    // upload buffer), the jobs in hjobs, which follow the draws there.
+    UploadBuf uploads[RF_UPLOAD_RING];
+    uint32_t upload_at = 0;
+    std::vector<char> small_upload;
+    UploadBuf *upload = nullptr;  // the ring's buffer in use (nullptr: small_upload)
+    DrawDev *hdraws = nullptr;
+    size_t ndraws = 0;
+    bool any_cull = false;  // a draw asks for object culling
+    int kind = 0;           // the shader kind of every draw, or RF_K_ANY
     std::vector<JobDev> hjobs;
     // stage timing
     bool timing = false;
@@ -253,6 +277,46 @@ rf_status sync_all(rf_ctx *ctx) {
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->up) CK(cudaStreamSynchronize(ctx->up));
     if (ctx->down) CK(cudaStreamSynchronize(ctx->down));
+    return RF_OK;
+}
+
+// Byte offset of the jobs behind n draws.
+size_t jobs_at(size_t n) { return (n * sizeof(DrawDev) + 255) & ~(size_t)255; }
+
+// Room for the descriptors of up to ndraws draws and njobs jobs.
+rf_status upload_begin(rf_ctx *ctx, size_t ndraws, size_t njobs) {
+    const size_t bytes = jobs_at(ndraws) + njobs * sizeof(JobDev);
+    if (bytes < RF_UPLOAD_PIN) {
+        if (ctx->small_upload.size() < RF_UPLOAD_PIN) ctx->small_upload.resize(RF_UPLOAD_PIN);
+        ctx->upload = nullptr;
+        ctx->hdraws = reinterpret_cast<DrawDev *>(ctx->small_upload.data());
+        return RF_OK;
+    }
+    UploadBuf &u = ctx->uploads[ctx->upload_at++ % RF_UPLOAD_RING];
+    if (u.pending) CK(cudaEventSynchronize(u.copied));
+    u.pending = false;
+    if (u.cap < bytes) {
+        if (u.p) CK(cudaFreeHost(u.p));
+        u.p = nullptr;
+        u.cap = 0;
+        CK(cudaMallocHost(&u.p, bytes + bytes / 4));
+        u.cap = bytes + bytes / 4;
+        if (!u.copied) CK(cudaEventCreateWithFlags(&u.copied, cudaEventDisableTiming));
+    }
+    ctx->upload = &u;
+    ctx->hdraws = reinterpret_cast<DrawDev *>(u.p);
+    return RF_OK;
+}
+
+// Queues the copy of the built descriptors to ctx->draws.
+rf_status upload_queue(rf_ctx *ctx) {
+    const size_t at = jobs_at(ctx->ndraws), n = ctx->hjobs.size() * sizeof(JobDev);
+    memcpy(reinterpret_cast<char *>(ctx->hdraws) + at, ctx->hjobs.data(), n);
+    CK(cudaMemcpyAsync(ctx->draws.p, ctx->hdraws, at + n, cudaMemcpyHostToDevice, ctx->stream));
+    if (ctx->upload) {
+        CK(cudaEventRecord(ctx->upload->copied, ctx->stream));
+        ctx->upload->pending = true;
+    }
     return RF_OK;
 }
 
@@ -375,11 +439,23 @@ uint64_t layout_masks(std::vector<JobDev> &hj) {
 // Nothing is queued on the GPU and no state changes on failure.
 rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<JobHost> &host,
                      uint64_t &nv_out, uint64_t &nt_out) {
-    auto &hd = ctx->hdraws;
     auto &hj = ctx->hjobs;
-    hd.clear();
     hj.clear();
     ctx->async_meshes.clear();
+    size_t most = 0;
+    for (uint32_t k = 0; k < nin; ++k) most += in[k].draws ? in[k].ndraws : 0u;
+    rf_status us = upload_begin(ctx, most, nin);
+    if (us) return us;
+    DrawDev *hd = ctx->hdraws;
+    size_t nd = 0;
+    ctx->any_cull = false;
+    // The objects of the draw before (instances share their mesh and
+    // texture, and a frame may have 10^5 of them).
+    rf_mesh mesh_h = 0;
+    Mesh *mesh = nullptr;
+    rf_texture tex_h = 0;
+    Texture *tex = nullptr;
+    int kind = 0;
     host.assign(nin, JobHost{});
     uint64_t nv = 0, nt = 0;
     uint64_t tiles = 0, mask_words = 0;
@@ -387,20 +463,26 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
     for (uint32_t k = 0; k < nin; ++k) {
         const JobIn &ji = in[k];
         if (!ji.vp || !flags_ok(ji.fl) || !ji.tg || (ji.ndraws && !ji.draws)) return RF_ERR_BAD_ARG;
-        const size_t d0 = hd.size();
+        const size_t d0 = nd;
         const uint64_t nt0 = nt, nv0 = nv;
+        const int kind0 = kind;
+        bool culls = false;
         for (uint32_t i = 0; i < ji.ndraws; ++i) {
             const rf_draw &dr = ji.draws[i];
-            auto mit = ctx->res->meshes.find(dr.mesh);
-            if (mit == ctx->res->meshes.end()) return RF_ERR_BAD_HANDLE;
-            Mesh &m = mit->second;
+            if (!mesh || dr.mesh != mesh_h) {
+                auto mit = ctx->res->meshes.find(dr.mesh);
+                if (mit == ctx->res->meshes.end()) return RF_ERR_BAD_HANDLE;
+                mesh_h = dr.mesh;
+                mesh = &mit->second;
+            }
+            Mesh &m = *mesh;
             if (m.lines) return RF_ERR_BAD_ARG;  // line meshes render with rf_render_lines
             if (m.async && !ctx->shared_res &&
                 (ctx->async_meshes.empty() || ctx->async_meshes.back() != &m))
                 ctx->async_meshes.push_back(&m);
             if (dr.shader < RF_SHADER_FLAT || dr.shader > RF_SHADER_GOURAUD_SRGB) return RF_ERR_BAD_ARG;
             if (m.nattr != nattr_for(dr.shader)) return RF_ERR_BAD_ARG;
-            DrawDev d{};
+            DrawDev &d = hd[nd];
             d.verts = m.verts;
             d.idx = m.idx;
             d.nverts = m.nverts;
@@ -411,15 +493,21 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
             d.shader = dr.shader;
             d.sampler = (int32_t)dr.uniforms.sampler;
             d.flat_rgba = dr.uniforms.flat_rgba;
+            d.tex = nullptr;
+            d.tw = d.th = 0;
             if (dr.shader == RF_SHADER_TEXTURED || dr.shader == RF_SHADER_TEX_GOURAUD) {
-                auto tit = ctx->res->textures.find(dr.uniforms.texture);
-                if (tit == ctx->res->textures.end()) return RF_ERR_BAD_HANDLE;
+                if (!tex || dr.uniforms.texture != tex_h) {
+                    auto tit = ctx->res->textures.find(dr.uniforms.texture);
+                    if (tit == ctx->res->textures.end()) return RF_ERR_BAD_HANDLE;
+                    tex_h = dr.uniforms.texture;
+                    tex = &tit->second;
+                }
                 if (d.sampler < RF_SAMPLER_REPEAT_POT || d.sampler > RF_SAMPLER_ONCE) return RF_ERR_BAD_ARG;
-                if (d.sampler == RF_SAMPLER_REPEAT_POT && (!is_pot(tit->second.w) || !is_pot(tit->second.h)))
+                if (d.sampler == RF_SAMPLER_REPEAT_POT && (!is_pot(tex->w) || !is_pot(tex->h)))
                     return RF_ERR_NON_POT_TEXTURE;
-                d.tex = tit->second.texels;
-                d.tw = tit->second.w;
-                d.th = tit->second.h;
+                d.tex = tex->texels;
+                d.tw = tex->w;
+                d.th = tex->h;
             }
             d.vert_base = (uint32_t)nv;
             d.tri_base = (uint32_t)nt;
@@ -432,7 +520,9 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
             nv += m.nverts;
             nt += m.ntri;
             if (nv > 0xFFFFFFF0ull || nt > 0x7FFFFFF0ull) return RF_ERR_BAD_ARG;
-            hd.push_back(d);
+            culls = culls || d.flags != 0;
+            kind = nd == 0 || kind == d.shader ? d.shader : (int)RF_K_ANY;
+            ++nd;
         }
         JobHost &h = host[k];
         h.calls = ji.ndraws;
@@ -440,11 +530,13 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
         h.verts_i = nv - nv0;
         if (nt == nt0 || nv == nv0) {
             // Nothing to draw: a pending clear stays pending for the next read.
-            hd.resize(d0);
+            nd = d0;
+            kind = kind0;
             nt = nt0;
             nv = nv0;
             continue;
         }
+        ctx->any_cull = ctx->any_cull || culls;
         const Target &tg = *ji.tg;
         JobDev J{};
         J.color = tg.color;
@@ -475,6 +567,8 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
         hj.push_back(J);
     }
     layout_masks(hj);
+    ctx->ndraws = nd;
+    ctx->kind = kind;
     nv_out = nv;
     nt_out = nt;
     return RF_OK;
@@ -559,7 +653,6 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     if (st) return st;
     uint64_t nv = 0, nt = 0;
     if ((st = build_jobs(ctx, in, nin, host, nv, nt))) return st;
-    auto &hd = ctx->hdraws;
     auto &hj = ctx->hjobs;
     for (const JobHost &h : host) {
         ctx->host_acc.calls += h.calls;
@@ -574,7 +667,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     {
         uint64_t px = 0;
         for (const JobDev &J : hj) px += (uint64_t)J.w * J.h;
-        const uint64_t key[5] = {hd.size(), nj, nv, nt, px};
+        const uint64_t key[5] = {ctx->ndraws, nj, nv, nt, px};
         if ((st = tune_tile(ctx, key, TW, tuned))) return st;
         if (TW != ctx->tile_w && (st = retile(hj, TW))) return st;
     }
@@ -582,10 +675,9 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     const JobDev &JL = hj.back();
     const uint32_t ntiles = JL.tile_base + JL.tiles_x * JL.tiles_y;
     const size_t mask_words = JL.sum_base + (size_t)JL.tiles_x * JL.tiles_y * JL.sum_words;  // masks + summaries
-    const uint32_t ndraws = (uint32_t)hd.size();
+    const uint32_t ndraws = (uint32_t)ctx->ndraws;
 
-    if ((st = ensure(ctx, ctx->draws, hd.size() * sizeof(DrawDev)))) return st;
-    if ((st = ensure(ctx, ctx->jobs, hj.size() * sizeof(JobDev)))) return st;
+    if ((st = ensure(ctx, ctx->draws, jobs_at(ndraws) + hj.size() * sizeof(JobDev)))) return st;
     if (per_job && (st = ensure(ctx, ctx->jstats, hj.size() * sizeof(StatsDev)))) return st;
     if ((st = ensure(ctx, ctx->cpos, nv * sizeof(float4)))) return st;
     if ((st = ensure(ctx, ctx->coc, nv))) return st;
@@ -617,12 +709,8 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     if ((st = ensure(ctx, ctx->rows, ctx->rows_cap * 4))) return st;
 
     cudaStream_t s = ctx->stream;
-    int kind = hd[0].shader;
-    bool any_cull = false;
-    for (const DrawDev &d : hd) {
-        if (d.shader != kind) kind = RF_K_ANY;
-        any_cull = any_cull || (d.flags & RF_DRAW_CULL_BBOX);
-    }
+    const int kind = ctx->kind;
+    const bool any_cull = ctx->any_cull;
     bool fast = true;
     for (const JobDev &J : hj)
         fast = fast && J.depth && J.depth_test == RF_DEPTH_LESS && J.color_write && J.depth_write;
@@ -640,8 +728,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     // Per-frame parameters travel as data (draws, jobs); the launch sequence
     // below depends only on the sizes, so it is replayed as a CUDA graph when
     // a frame of the same shape comes again.
-    CK(cudaMemcpyAsync(ctx->draws.p, hd.data(), hd.size() * sizeof(DrawDev), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->jobs.p, hj.data(), hj.size() * sizeof(JobDev), cudaMemcpyHostToDevice, s));
+    if ((st = upload_queue(ctx))) return st;
 
     std::vector<cudaEvent_t> ev;
     if (ctx->timing) {
@@ -659,7 +746,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     uint32_t *counters = P<uint32_t>(ctx->counters);
     StatsDev *kst = per_job ? P<StatsDev>(ctx->jstats) : P<StatsDev>(ctx->stats);
     const DrawDev *dd = P<DrawDev>(ctx->draws);
-    const JobDev *jd = P<JobDev>(ctx->jobs);
+    const JobDev *jd = reinterpret_cast<const JobDev *>(P<char>(ctx->draws) + jobs_at(ndraws));
     auto enqueue = [&](bool marks) -> rf_status {
         auto mark = [&](int i) -> cudaError_t { return marks ? cudaEventRecord(ev[i], s) : cudaSuccess; };
         CK(cudaMemsetAsync(ctx->mask.p, 0, mask_words * 4, s));
@@ -734,7 +821,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         CK(cudaStreamSynchronize(s));
         // The setup pass's draws and jobs count clipped triangles, in the
         // sorted order (draw by draw, as the keys lead with the draw).
-        std::vector<DrawDev> vd = hd;
+        std::vector<DrawDev> vd(ctx->hdraws, ctx->hdraws + ndraws);
         std::vector<JobDev> vj = hj;
         uint64_t np = 0;
         for (uint32_t d = 0; d < ndraws; ++d) {
@@ -1052,6 +1139,10 @@ rf_status rf_ctx_destroy(rf_ctx *ctx) {
                       &ctx->rowtot, &ctx->clipq, &ctx->rows, &ctx->rprims, &ctx->live, &ctx->marks, &ctx->items, &ctx->jstats, &ctx->lrec, &ctx->lmask,
                       &ctx->perm, &ctx->ptri, &ctx->nout, &ctx->dsort, &ctx->vdraws, &ctx->vjobs,
                       &ctx->vtoff, &ctx->vtcnt};
+    for (UploadBuf &u : ctx->uploads) {
+        if (u.p) cudaFreeHost(u.p);
+        if (u.copied) cudaEventDestroy(u.copied);
+    }
     if (ctx->nout_host) cudaFreeHost(ctx->nout_host);
     if (ctx->rows_need_host) cudaFreeHost(ctx->rows_need_host);
     if (ctx->rows_evt) cudaEventDestroy(ctx->rows_evt);
