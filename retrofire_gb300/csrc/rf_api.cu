@@ -93,7 +93,7 @@ struct UploadBuf {
 
 // An instantiated launch sequence and the frame shape it was captured for.
 struct GraphKey {
-    uint64_t v[13];
+    uint64_t v[13 + RF_MAX_GROUPS];
     bool operator==(const GraphKey &o) const { return memcmp(v, o.v, sizeof v) == 0; }
 };
 struct GraphEntry {
@@ -139,7 +139,7 @@ struct rf_ctx {
     std::unordered_map<uint64_t, Target> targets;
     // per-frame scratch
     DevBuf draws, jobs, cpos, coc, tcnt, toff, tpoly, pool, prims, mask, scan, counters, stats;
-    DevBuf rowtot, rows, rprims, live, marks, items, jstats, clipq;
+    DevBuf rowtot, rows, rprims, live, marks, items, jstats, clipq, segs, list;
     DevBuf lrec, lmask;  // line pass
     // depth-sorted frames: sorted order, source triangles, per-draw counts,
     // sort scratch, the setup pass's draws / jobs, the raster's unit arrays
@@ -158,8 +158,8 @@ struct rf_ctx {
     uint32_t last_tile_w = 0;
     // Row-record capacity (words): grown when a frame asked for more, which
     // the library learns from an asynchronous read-back of the total.
-    uint64_t rows_cap = 0;
-    unsigned long long *rows_need_host = nullptr;  // pinned
+    uint64_t rows_cap = 0, list_cap = 0;           // (list_cap: entries of the triangle lists, likewise)
+    unsigned long long *rows_need_host = nullptr;  // pinned: row words, list entries
     cudaEvent_t rows_evt = nullptr;
     bool rows_evt_pending = false;
     // stats: host-side counts + device-accumulated counts, and what was
@@ -178,6 +178,11 @@ struct rf_ctx {
     bool any_cull = false;  // a draw asks for object culling
     int kind = 0;           // the shader kind of every draw, or RF_K_ANY
     std::vector<JobDev> hjobs;
+    std::vector<RasterGroup> groups;
+    // Frames of several raster groups: the second launches on a side stream,
+    // forked and joined by events (lazily made).
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_fork = nullptr, side_join = nullptr;
     // stage timing
     bool timing = false;
     std::vector<cudaEvent_t> ev_free;
@@ -419,8 +424,11 @@ void graphs_drop(rf_ctx *ctx) {
     ctx->gcache.clear();
 }
 
+constexpr uint64_t RF_LIST_PIECE = 16;  // (see layout_masks)
+
 // Word offsets of every job's tile masks and, after all of them, of the
-// tiles' summary words (one bit per mask word); returns the words in all.
+// tiles' summary words (one bit per mask word), and the pieces of the tiles'
+// triangle lists; returns the words in all.
 uint64_t layout_masks(std::vector<JobDev> &hj) {
     uint64_t w = 0;
     for (JobDev &J : hj) {
@@ -432,7 +440,65 @@ uint64_t layout_masks(std::vector<JobDev> &hj) {
         J.sum_base = w;
         w += (uint64_t)J.tiles_x * J.tiles_y * J.sum_words;
     }
+    // The pieces of the tiles' triangle lists: one warp builds one, 32 entries
+    // a step, so the tiles of a mesh far larger than its target come in
+    // several.  RF_LIST_PIECE triangles per tile and piece: the 64-scene
+    // batch's heaviest lists took 0.4 ms in one piece, and pieces of less
+    // than a step's entries cost the 500 k-triangle grid 10 us.
+    uint64_t base = 0;
+    for (JobDev &at : hj) {
+        JobDev &J = hj[at.nth];
+        const uint64_t t = std::max<uint64_t>(1, (uint64_t)J.tiles_x * J.tiles_y);
+        const uint32_t n = (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>(J.sum_words, (J.ntri + RF_LIST_PIECE * t - 1) / (RF_LIST_PIECE * t)));
+        J.seg_words = (J.sum_words + n - 1) / n;
+        J.nseg = J.seg_words ? (J.sum_words + J.seg_words - 1) / J.seg_words : 1u;
+        J.seg_base = at.nth_seg = base;
+        base += t * J.nseg;
+    }
     return w;
+}
+
+// The raster groups present (J.group: kind and context, then the group's
+// index among them), and the order the jobs' tiles are laid out in: by group.
+void group_jobs(rf_ctx *ctx) {
+    auto &hj = ctx->hjobs;
+    auto &gr = ctx->groups;
+    gr.clear();
+    uint32_t seen = 0;
+    for (const JobDev &J : hj) seen |= 1u << J.group;
+    uint32_t dense[RF_MAX_GROUPS];
+    for (uint32_t g = 0; g < RF_MAX_GROUPS; ++g)
+        if (seen & (1u << g)) {
+            dense[g] = (uint32_t)gr.size();
+            gr.push_back(RasterGroup{(int32_t)(g / 2), g % 2 == 0, 0u, 0u});
+        }
+    for (JobDev &J : hj) J.group = dense[J.group];
+    uint32_t n = 0;
+    for (uint32_t g = 0; g < gr.size(); ++g)
+        for (size_t j = 0; j < hj.size(); ++j)
+            if (hj[j].group == g) hj[n++].nth = (uint32_t)j;
+}
+
+// Tile and mask fields of every job, and the groups' tile ranges, for tile
+// width TW.
+rf_status layout_tiles(std::vector<JobDev> &hj, std::vector<RasterGroup> &gr, uint32_t TW) {
+    uint64_t tiles = 0;
+    for (RasterGroup &g : gr) g.ntiles = 0;
+    for (JobDev &at : hj) {
+        JobDev &J = hj[at.nth];
+        J.tiles_x = (J.w + TW - 1) / TW;
+        J.tiles_y = (J.h + RF_TILE_H - 1) / RF_TILE_H;
+        J.tile_base = at.nth_tile = (uint32_t)tiles;
+        RasterGroup &g = gr[J.group];
+        if (g.ntiles == 0) g.tile0 = J.tile_base;
+        J.group_tile = g.tile0;
+        g.ntiles += J.tiles_x * J.tiles_y;
+        tiles += (uint64_t)J.tiles_x * J.tiles_y;
+        if (tiles > RF_MAX_TILES) return RF_ERR_BAD_ARG;
+    }
+    layout_masks(hj);
+    return RF_OK;
 }
 
 // Validates every draw of every job and fills ctx->hdraws / ctx->hjobs.
@@ -455,17 +521,17 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
     Mesh *mesh = nullptr;
     rf_texture tex_h = 0;
     Texture *tex = nullptr;
-    int kind = 0;
+    int frame_kind = RF_K_ANY;
     host.assign(nin, JobHost{});
     uint64_t nv = 0, nt = 0;
-    uint64_t tiles = 0, mask_words = 0;
+    uint64_t tiles = 0;
     const uint32_t TW = ctx->tile_w;
     for (uint32_t k = 0; k < nin; ++k) {
         const JobIn &ji = in[k];
         if (!ji.vp || !flags_ok(ji.fl) || !ji.tg || (ji.ndraws && !ji.draws)) return RF_ERR_BAD_ARG;
         const size_t d0 = nd;
         const uint64_t nt0 = nt, nv0 = nv;
-        const int kind0 = kind;
+        int kind = RF_K_ANY;  // of every draw of the job
         bool culls = false;
         for (uint32_t i = 0; i < ji.ndraws; ++i) {
             const rf_draw &dr = ji.draws[i];
@@ -517,11 +583,11 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
             d.src_tri_base = (uint32_t)nt;
             d.bbox = m.bbox;
             memcpy(d.mvp, dr.uniforms.mvp, sizeof d.mvp);
+            kind = i == 0 || kind == dr.shader ? dr.shader : (int)RF_K_ANY;
             nv += m.nverts;
             nt += m.ntri;
             if (nv > 0xFFFFFFF0ull || nt > 0x7FFFFFF0ull) return RF_ERR_BAD_ARG;
             culls = culls || d.flags != 0;
-            kind = nd == 0 || kind == d.shader ? d.shader : (int)RF_K_ANY;
             ++nd;
         }
         JobHost &h = host[k];
@@ -531,12 +597,12 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
         if (nt == nt0 || nv == nv0) {
             // Nothing to draw: a pending clear stays pending for the next read.
             nd = d0;
-            kind = kind0;
             nt = nt0;
             nv = nv0;
             continue;
         }
         ctx->any_cull = ctx->any_cull || culls;
+        frame_kind = hj.empty() || frame_kind == kind ? kind : (int)RF_K_ANY;
         const Target &tg = *ji.tg;
         JobDev J{};
         J.color = tg.color;
@@ -550,44 +616,27 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
         J.face_cull = ji.fl->face_cull;
         J.tiles_x = (tg.w + TW - 1) / TW;
         J.tiles_y = (tg.h + RF_TILE_H - 1) / RF_TILE_H;
-        J.tile_base = (uint32_t)tiles;
         J.tri_base = (uint32_t)nt0;
         J.ntri = (uint32_t)(nt - nt0);
         J.mask_words = (J.ntri + 31) / 32;
-        J.mask_base = mask_words;
         J.clear_flags = tg.clear_flags;
         J.clear_px = tg.clear_px;
         J.clear_z = tg.clear_z;
         J.depth_sort = ji.fl->depth_sort;
+        const bool fast = J.depth && J.depth_test == RF_DEPTH_LESS && J.color_write && J.depth_write;
+        J.group = (uint32_t)(kind * 2 + (fast ? 0 : 1));  // (made dense by group_jobs)
         memcpy(J.vp, ji.vp, sizeof J.vp);
         tiles += (uint64_t)J.tiles_x * J.tiles_y;
-        mask_words += (uint64_t)J.tiles_x * J.tiles_y * J.mask_words;
         if (tiles > RF_MAX_TILES) return RF_ERR_BAD_ARG;
         h.slot = (int32_t)hj.size();
         hj.push_back(J);
     }
-    layout_masks(hj);
+    group_jobs(ctx);
+    layout_tiles(hj, ctx->groups, TW);
     ctx->ndraws = nd;
-    ctx->kind = kind;
+    ctx->kind = frame_kind;
     nv_out = nv;
     nt_out = nt;
-    return RF_OK;
-}
-
-// Tile fields of every job for tile width TW (the jobs were built for
-// another width).
-rf_status retile(std::vector<JobDev> &hj, uint32_t TW) {
-    uint64_t tiles = 0, mask_words = 0;
-    for (JobDev &J : hj) {
-        J.tiles_x = (J.w + TW - 1) / TW;
-        J.tiles_y = (J.h + RF_TILE_H - 1) / RF_TILE_H;
-        J.tile_base = (uint32_t)tiles;
-        J.mask_base = mask_words;
-        tiles += (uint64_t)J.tiles_x * J.tiles_y;
-        mask_words += (uint64_t)J.tiles_x * J.tiles_y * J.mask_words;
-        if (tiles > RF_MAX_TILES) return RF_ERR_BAD_ARG;
-    }
-    layout_masks(hj);
     return RF_OK;
 }
 
@@ -669,11 +718,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         for (const JobDev &J : hj) px += (uint64_t)J.w * J.h;
         const uint64_t key[5] = {ctx->ndraws, nj, nv, nt, px};
         if ((st = tune_tile(ctx, key, TW, tuned))) return st;
-        if (TW != ctx->tile_w && (st = retile(hj, TW))) return st;
+        if (TW != ctx->tile_w && (st = layout_tiles(hj, ctx->groups, TW))) return st;
     }
     ctx->last_tile_w = TW;
     const JobDev &JL = hj.back();
-    const uint32_t ntiles = JL.tile_base + JL.tiles_x * JL.tiles_y;
+    const JobDev &JT = hj[JL.nth];  // the last one's tiles
+    const uint32_t ntiles = JT.tile_base + JT.tiles_x * JT.tiles_y;
     const size_t mask_words = JL.sum_base + (size_t)JL.tiles_x * JL.tiles_y * JL.sum_words;  // masks + summaries
     const uint32_t ndraws = (uint32_t)ctx->ndraws;
 
@@ -690,30 +740,62 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     if ((st = ensure(ctx, ctx->prims, (size_t)nt * RF_MAX_FAN * sizeof(PrimRec)))) return st;
     if ((st = ensure(ctx, ctx->mask, mask_words * 4))) return st;
     if ((st = ensure(ctx, ctx->scan, rfk::scan_scratch_words((uint32_t)nt) * 4))) return st;
-    if ((st = ensure(ctx, ctx->rowtot, 8))) return st;
+    if ((st = ensure(ctx, ctx->rowtot, 16))) return st;
     if ((st = ensure(ctx, ctx->rprims, (size_t)nt * RF_MAX_FAN * sizeof(RasterPrim)))) return st;
     if ((st = ensure(ctx, ctx->live, (size_t)nt * RF_MAX_FAN * 12))) return st;  // three lists
     if ((st = ensure(ctx, ctx->marks, 8))) return st;
     if ((st = ensure(ctx, ctx->items, (size_t)ntiles * (RF_SPLIT_K + 1) * 4))) return st;
     if (!ctx->rows_need_host) {
-        CK(cudaMallocHost(&ctx->rows_need_host, sizeof(unsigned long long)));
+        CK(cudaMallocHost(&ctx->rows_need_host, 2 * sizeof(unsigned long long)));
         CK(cudaEventCreateWithFlags(&ctx->rows_evt, cudaEventDisableTiming));
     }
     if (ctx->rows_evt_pending && cudaEventQuery(ctx->rows_evt) == cudaSuccess) {
         const uint64_t need = *ctx->rows_need_host;
         if (need > ctx->rows_cap) ctx->rows_cap = need + need / 4;
+        const uint64_t lneed = ctx->rows_need_host[1];
+        if (lneed > ctx->list_cap) ctx->list_cap = lneed + lneed / 4;
         ctx->rows_evt_pending = false;
     }
     if (ctx->rows_cap == 0) ctx->rows_cap = std::max<uint64_t>((uint64_t)nt * 160u, 1u << 22);
     if (ctx->rows_cap > 0xFFFF0000ull) ctx->rows_cap = 0xFFFF0000ull;  // 32-bit record offsets
     if ((st = ensure(ctx, ctx->rows, ctx->rows_cap * 4))) return st;
+    ctx->list_cap = std::max<uint64_t>(ctx->list_cap, std::max<uint64_t>((uint64_t)nt * 4u, 1u << 20));
+    ctx->list_cap = std::min<uint64_t>(ctx->list_cap, 0xFFFF0000ull);  // 32-bit piece offsets
+    if ((st = ensure(ctx, ctx->list, ctx->list_cap * 8))) return st;
+    auto pieces = [&](const std::vector<JobDev> &j) {
+        const JobDev &last = j[j.back().nth];
+        return (uint32_t)(last.seg_base + (uint64_t)last.tiles_x * last.tiles_y * last.nseg);
+    };
+    if ((st = ensure(ctx, ctx->segs, (size_t)pieces(hj) * 8))) return st;
 
     cudaStream_t s = ctx->stream;
     const int kind = ctx->kind;
     const bool any_cull = ctx->any_cull;
-    bool fast = true;
-    for (const JobDev &J : hj)
-        fast = fast && J.depth && J.depth_test == RF_DEPTH_LESS && J.color_write && J.depth_write;
+    const uint32_t ng = (uint32_t)ctx->groups.size();
+    if (ng > 1 && !ctx->side) {
+        CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ctx->side_join, cudaEventDisableTiming));
+    }
+    // The raster pass, its groups on two streams so that one group's last
+    // tiles overlap the other's first.
+    auto raster = [&](const JobDev *jobs, const DrawDev *draws, const uint32_t *tcnt, const uint32_t *toff,
+                      uint32_t *counters, StatsDev *stats) -> rf_status {
+        const cudaStream_t st2[2] = {ctx->stream, ctx->side};
+        if (ng > 1) {
+            CK(cudaEventRecord(ctx->side_fork, ctx->stream));
+            CK(cudaStreamWaitEvent(ctx->side, ctx->side_fork, 0));
+        }
+        CK(rfk::launch_raster(TW, ctx->groups.data(), ng, jobs, nj, draws, P<PrimRec>(ctx->prims),
+                              P<RasterPrim>(ctx->rprims), P<uint32_t>(ctx->rows), tcnt, toff, P<uint32_t>(ctx->mask),
+                              P<uint2>(ctx->segs), P<uint2>(ctx->list), ntiles, P<uint32_t>(ctx->items), counters, stats, ctx->warps, ctx->nsm, st2,
+                              ng > 1 ? 2u : 1u));
+        if (ng > 1) {
+            CK(cudaEventRecord(ctx->side_join, ctx->side));
+            CK(cudaStreamWaitEvent(ctx->stream, ctx->side_join, 0));
+        }
+        return RF_OK;
+    };
 
     // Asynchronous uploads of the meshes read and read-backs of the targets
     // written must finish first.
@@ -770,13 +852,13 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
                              P<uint32_t>(ctx->rows), ctx->rows_cap, P<RasterPrim>(ctx->rprims),
                              P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
                              kst, counters, ctx->nsm, s, nullptr, nullptr, kind));
-        CK(rfk::launch_items(jd, nj, P<uint32_t>(ctx->mask), ntiles, P<unsigned long long>(ctx->marks),
-                             (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, s));
+        CK(rfk::launch_lists(jd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(hj), P<uint32_t>(ctx->toff),
+                             P<uint32_t>(ctx->tcnt), P<RasterPrim>(ctx->rprims), P<unsigned long long>(ctx->marks),
+                             (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, P<uint2>(ctx->segs),
+                             P<uint2>(ctx->list), P<unsigned long long>(ctx->rowtot) + 1, ctx->list_cap, s));
         CK(mark(RF_STAGE_RASTER));
-        CK(rfk::launch_raster(TW, kind, fast, jd, nj, dd, P<PrimRec>(ctx->prims),
-                              P<RasterPrim>(ctx->rprims), P<uint32_t>(ctx->rows), P<uint32_t>(ctx->tcnt),
-                              P<uint32_t>(ctx->toff), P<uint32_t>(ctx->mask), ntiles, P<uint32_t>(ctx->items),
-                              counters + RF_CNT_ITEMS, counters + RF_CNT_QUEUE, kst, ctx->warps, ctx->nsm, s));
+        rf_status st2 = raster(jd, dd, P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->toff), counters, kst);
+        if (st2) return st2;
         CK(mark(RF_STAGE_N));
         if (per_job) CK(rfk::launch_stats_fold(kst, nj, P<StatsDev>(ctx->stats), s));
         return RF_OK;
@@ -852,6 +934,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
             return st2;
         if ((st2 = ensure(ctx, ctx->vtoff, (size_t)std::max<uint32_t>(n32, 1) * 4))) return st2;
         if ((st2 = ensure(ctx, ctx->vtcnt, (size_t)std::max<uint32_t>(n32, 1) * 4))) return st2;
+        if ((st2 = ensure(ctx, ctx->segs, (size_t)pieces(vj) * 8))) return st2;
         if ((st2 = ensure(ctx, ctx->vdraws, vd.size() * sizeof(DrawDev)))) return st2;
         if ((st2 = ensure(ctx, ctx->vjobs, vj.size() * sizeof(JobDev)))) return st2;
         CK(cudaMemcpyAsync(ctx->vdraws.p, vd.data(), vd.size() * sizeof(DrawDev), cudaMemcpyHostToDevice, s));
@@ -871,13 +954,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
                              P<uint32_t>(ctx->rows), ctx->rows_cap, P<RasterPrim>(ctx->rprims),
                              P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
                              kst, counters, ctx->nsm, s, P<uint32_t>(ctx->perm), P<uint32_t>(ctx->ptri), kind));
-        CK(rfk::launch_items(vjd, nj, P<uint32_t>(ctx->mask), ntiles, P<unsigned long long>(ctx->marks),
-                             (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, s));
+        CK(rfk::launch_lists(vjd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(vj), P<uint32_t>(ctx->vtoff),
+                             P<uint32_t>(ctx->vtcnt), P<RasterPrim>(ctx->rprims), P<unsigned long long>(ctx->marks),
+                             (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, P<uint2>(ctx->segs),
+                             P<uint2>(ctx->list), P<unsigned long long>(ctx->rowtot) + 1, ctx->list_cap, s));
         CK(mark(RF_STAGE_RASTER));
-        CK(rfk::launch_raster(TW, kind, fast, vjd, nj, vdd, P<PrimRec>(ctx->prims), P<RasterPrim>(ctx->rprims),
-                              P<uint32_t>(ctx->rows), P<uint32_t>(ctx->vtcnt), P<uint32_t>(ctx->vtoff),
-                              P<uint32_t>(ctx->mask), ntiles, P<uint32_t>(ctx->items), counters + RF_CNT_ITEMS,
-                              counters + RF_CNT_QUEUE, kst, ctx->warps, ctx->nsm, s));
+        if ((st2 = raster(vjd, vdd, P<uint32_t>(ctx->vtcnt), P<uint32_t>(ctx->vtoff), counters, kst))) return st2;
         CK(mark(RF_STAGE_N));
         if (per_job) CK(rfk::launch_stats_fold(kst, nj, P<StatsDev>(ctx->stats), s));
         // draw counts, sort keys, per digit pass a histogram, a scan of 1 or 3
@@ -894,10 +976,11 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     } else if (ctx->graphs && !ctx->timing) {
         GraphKey key{};
         const uint64_t kv[] = {ctx->gen, ndraws, nj, nv, nt, ntiles, mask_words, TW, ctx->warps,
-                               (uint64_t)(kind + 16) | (any_cull ? 0x100u : 0u), fast ? 1u : 0u,
-                               per_job ? 1u : 0u, ctx->rows_cap};
-        static_assert(sizeof kv == sizeof key.v, "graph key size");
+                               (uint64_t)(kind + 16) | (any_cull ? 0x100u : 0u), per_job ? 1u : 0u, ctx->rows_cap, ctx->list_cap};
+        static_assert(sizeof kv + RF_MAX_GROUPS * 8 == sizeof key.v, "graph key size");
         memcpy(key.v, kv, sizeof kv);
+        for (const RasterGroup &g : ctx->groups)  // (a group's slot is never 0: it has tiles)
+            key.v[13 + g.kind * 2 + (g.fast ? 0 : 1)] = g.ntiles;
         GraphEntry *hit = nullptr;
         for (GraphEntry &g : ctx->gcache)
             if (g.key == key) hit = &g;
@@ -936,12 +1019,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         tuned->pending = true;
     }
     // vertex, clip (2), setup, bin (3: 8- and 16-lane groups, then warps),
-    // work list, raster (+ the stats fold; a depth-sorted frame adds the
+    // work list, raster (one launch a group; + the stats fold; a depth-sorted frame adds the
     // scan of the fan counts, 3 launches or 1 for one block, and its sort)
     const uint64_t scan_kernels = sorted ? (nt <= RF_SCAN_BLOCK_ITEMS ? 1 : 3) : 0;
-    ctx->kernels += 9 + scan_kernels + (per_job ? 1 : 0) + (any_cull ? 1 : 0) + sort_kernels;
+    ctx->kernels += 8 + ng + scan_kernels + (per_job ? 1 : 0) + (any_cull ? 1 : 0) + sort_kernels;
     if (!ctx->rows_evt_pending) {
-        CK(cudaMemcpyAsync(ctx->rows_need_host, ctx->rowtot.p, 8, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(ctx->rows_need_host, ctx->rowtot.p, 16, cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(ctx->rows_evt, s));
         ctx->rows_evt_pending = true;
     }
@@ -1128,6 +1211,9 @@ rf_status rf_ctx_destroy(rf_ctx *ctx) {
     for (auto &kv : ctx->targets) { cudaFree(kv.second.color); cudaFree(kv.second.depth); drop_async(kv.second); }
     if (ctx->up) cudaStreamDestroy(ctx->up);
     if (ctx->down) cudaStreamDestroy(ctx->down);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->side_fork) cudaEventDestroy(ctx->side_fork);
+    if (ctx->side_join) cudaEventDestroy(ctx->side_join);
     graphs_drop(ctx);
     for (TuneState &t : ctx->tunes) {
         if (t.e0) cudaEventDestroy(t.e0);
@@ -1136,7 +1222,7 @@ rf_status rf_ctx_destroy(rf_ctx *ctx) {
     DevBuf *bufs[] = {&ctx->draws, &ctx->jobs, &ctx->cpos, &ctx->coc, &ctx->tcnt, &ctx->toff,
                       &ctx->tpoly, &ctx->pool, &ctx->prims, &ctx->mask, &ctx->scan,
                       &ctx->counters, &ctx->stats,
-                      &ctx->rowtot, &ctx->clipq, &ctx->rows, &ctx->rprims, &ctx->live, &ctx->marks, &ctx->items, &ctx->jstats, &ctx->lrec, &ctx->lmask,
+                      &ctx->rowtot, &ctx->clipq, &ctx->rows, &ctx->rprims, &ctx->live, &ctx->marks, &ctx->items, &ctx->segs, &ctx->list, &ctx->jstats, &ctx->lrec, &ctx->lmask,
                       &ctx->perm, &ctx->ptri, &ctx->nout, &ctx->dsort, &ctx->vdraws, &ctx->vjobs,
                       &ctx->vtoff, &ctx->vtcnt};
     for (UploadBuf &u : ctx->uploads) {

@@ -14,6 +14,8 @@
 //   prim[p]  PrimRec  triangle setup: two ScanlineIter starts (raster.rs:248-302)
 //   mask     u32      per tile, one bit per input triangle of the job that
 //                     touches the tile; bit order = submission order
+//   list     uint2    the tiles' set bits as triangle entries (RF_ENT_*), in
+//                     submission order, a piece per (tile, segment)
 #ifndef RF_INTERNAL_CUH
 #define RF_INTERNAL_CUH
 
@@ -61,7 +63,15 @@ struct JobDev {
     float clear_z;
     uint32_t sum_words;       // summary words per tile: bit b of word s = mask word 32 s + b is nonzero
     int32_t depth_sort;       // Context::depth_sort: 0 none, 1 front to back, 2 back to front
+    uint32_t group;           // raster group (rf_kernels.cuh RasterGroup) and its first tile
+    uint32_t group_tile;
+    // Not of this job, but the tile layout's directory: the job whose tiles
+    // (and list pieces) come nth when laid out by group, and where they start.
+    uint32_t nth, nth_tile;
+    uint64_t nth_seg;
     uint64_t sum_base;        // word offset of the job's tile-0 summary (after every job's masks)
+    uint32_t nseg, seg_words; // a tile's triangle list comes in nseg pieces of seg_words summary words
+    uint64_t seg_base;        // first piece of the job's tile 0
     float vp[16];             // Mat4<Ndc, Screen>
 };
 
@@ -144,12 +154,16 @@ struct RasterPrim {
     uint32_t stride;  // words per row record (1 + 2 NC)
     uint32_t y0, c0;  // upper half: rows y0 .. y0+c0-1, records 0 .. c0-1
     uint32_t y1, c1;  // lower half: rows y1 .. y1+c1-1, records c0 .. c0+c1-1
-    float dvdx[2][RF_NC];
     float zmax;       // >= the depth of every fragment it writes into the target
                       // (+inf when unknown): a tile whose current depths are all
                       // >= zmax cannot pass any of them under the Less test
     uint32_t pad_[2];
+    float dvdx[2][RF_NC];
 };
+// The rasteriser loads the fields before dvdx as three 16-byte words.
+static_assert(offsetof(RasterPrim, stride) == 16 && offsetof(RasterPrim, c1) == 32 &&
+                  offsetof(RasterPrim, zmax) == 36 && offsetof(RasterPrim, dvdx) == 48 && sizeof(RasterPrim) % 16 == 0,
+              "RasterPrim layout");
 
 // One line after clipping and to_screen (raster.rs:121-173): it steps
 // along x (wide) or y, n pixels from `begin`; the other coordinate of

@@ -10,7 +10,8 @@
 //   k_bin        scanline walk: stats (frags.i, oob),  raster.rs:80-114, target.rs:259-264
 //                row records, tile binning, one warp
 //                per live triangle
-//   k_tile_items the rasteriser's work list            (scheduling only)
+//   k_tile_lists the tiles' triangle lists and the     (scheduling only)
+//                rasteriser's work list
 //   k_raster     per-tile span fill, depth test,       raster.rs:60-69, target.rs:163-198
 //                fragment shading, pixel packing       (rf_raster.cuh)
 //   k_fill       Frame::clear without a later render   front/src/lib.rs:103-120
@@ -68,7 +69,6 @@ __global__ void k_vertex(const DrawDev *__restrict__ draws, uint32_t nd, uint32_
     if (blockIdx.x == 0) {  // the frame's counters, for the kernels after this one
         if (counters && threadIdx.x == 0) {
             counters[RF_CNT_POOL] = 0;
-            counters[RF_CNT_QUEUE] = 0;
             counters[RF_CNT_LIVE] = 0;
             counters[RF_CNT_LIVE_SMALL] = 0;
             counters[RF_CNT_LIVE_MID] = 0;
@@ -76,6 +76,7 @@ __global__ void k_vertex(const DrawDev *__restrict__ draws, uint32_t nd, uint32_
             counters[RF_CNT_CLIPQ] = 0;
             *marks = 0;
         }
+        if (counters && threadIdx.x <= 2 * RF_MAX_GROUPS) counters[RF_CNT_QUEUE_G + threadIdx.x] = 0;  // .. LISTOVF
     }
     // Warp-uniform loop (the draw lookup is shared by the warp's lanes).
     for (uint32_t wbase = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); wbase < nv_total;
@@ -696,9 +697,8 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd,
                         uint32_t *__restrict__ live, uint32_t *__restrict__ live_n,
                         uint32_t *__restrict__ live_small, uint32_t *__restrict__ live_small_n,
                         uint32_t *__restrict__ live_mid, uint32_t *__restrict__ live_mid_n,
-                        uint32_t *__restrict__ extra, StatsDev *__restrict__ stats,
+                        StatsDev *__restrict__ stats,
                         const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ptri) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *extra = 0;  // the work list's counter
     // Each thread builds its record in shared memory; the warp then writes
     // the records out with coalesced 16-byte stores.  Only triangles that
     // pass the face-cull test get a record, and their indices are appended
@@ -1512,46 +1512,169 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
     warp_add_u64(marks, acc_marks, true);
 }
 
-// The rasteriser's work list.  A tile walks its triangles serially, so the
-// tiles that take longest should start first, and a tile far more crowded
-// than the rest (the horizon of a scene of many small objects) would close
-// the pass alone: such a tile is split into RF_SPLIT_K items, one per slice
-// of RF_TILE_H / RF_SPLIT_K rows, walked by different warps (each pixel
-// still sees its triangles in order: a row belongs to one slice).  The list
-// is items[ntiles ..) -- the heavy tiles and the slices of the crowded ones,
-// in no particular order -- then items[0 .. ntiles) -- every tile in index
-// order, RF_ITEM_SKIP where the tile went to the first part.
+// The tiles' triangle lists and the rasteriser's work list, one warp per
+// piece of a tile's list.
 //
-// k_tile_items: one warp per tile.  Its nonzero mask words (the set bits
-// of its summary words) stand for its triangle count: at most the count,
-// about it where the tile's triangles are scattered through the submission
-// order; where most words are nonzero the bits are counted instead.  A
-// crowded tile is one whose count exceeds twice the frame's marks per
-// resident warp: its walk alone would outlast two warps' fair shares of
-// the pass, so splitting it shortens the pass.
+// List: the mask's set bits in order -- per 32 summary words their nonzero
+// mask words, 32 at a time, one a lane; then those words' bits, 32 triangles
+// at a time, one a lane, each finding its word by the prefix counts.  The
+// rasteriser's warps used to walk the masks themselves, at 16 warps per SM
+// and a quarter of their time; here the same steps run at full occupancy.
+//
+// Work list: a tile walks its triangles serially, so the tiles that take
+// longest should start first, and a tile far more crowded than the rest (the
+// horizon of a scene of many small objects) would close the pass alone: such
+// a tile is split into RF_SPLIT_K items, one per slice of RF_TILE_H /
+// RF_SPLIT_K rows, walked by different warps (each pixel still sees its
+// triangles in order: a row belongs to one slice).  The list is the heavy
+// tiles and the slices of the crowded ones, in no particular order, then
+// every tile in index order, RF_ITEM_SKIP where the tile went to the first
+// part.  A tile's nonzero mask words (the set bits of its summary words)
+// stand for its triangle count: at most the count, about it where the tile's
+// triangles are scattered through the submission order; where most words are
+// nonzero the bits are counted instead.  A crowded tile is one whose count
+// exceeds twice the frame's marks per resident warp: its walk alone would
+// outlast two warps' fair shares of the pass, so splitting it shortens the
+// pass.
 #define RF_SPLIT_MIN 64u  // a tile with fewer binned triangles is never split
 #define RF_HEAVY_MIN 16u  // ... nor taken early
-__global__ void __launch_bounds__(256)
-k_tile_items(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__restrict__ mask,
-             uint32_t ntiles, const unsigned long long *__restrict__ marks, uint32_t slots,
-             uint32_t *__restrict__ items, uint32_t *__restrict__ extra) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (tile >= ntiles) return;
-    const uint32_t ji = upper_index(nj, tile, [&](uint32_t i) { return jobs[i].tile_base; });
-    const JobDev &J = jobs[ji];
-    const uint32_t lt = tile - J.tile_base;
+#define RF_LIST_WARPS 8u
+namespace {
+// Position of the r-th set bit of v (r >= 1, at most popc(v)): halving
+// search on popcounts.
+__device__ __forceinline__ uint32_t nth_bit(uint32_t v, uint32_t r) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (uint32_t w = 16; w >= 1; w >>= 1) {
+        const uint32_t c = __popc(v & ((1u << w) - 1u));
+        if (c < r) {
+            r -= c;
+            v >>= w;
+            pos += w;
+        }
+    }
+    return pos;
+}
+__device__ __forceinline__ uint32_t warp_incl(uint32_t v, uint32_t lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= (uint32_t)o) v += y;
+    }
+    return v;
+}
+// The lane whose bits hold the k-th of all (incl: the lanes' inclusive
+// counts; every lane calls).
+__device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t k) {
+    uint32_t L = 0;
+#pragma unroll
+    for (uint32_t step = 16; step >= 1; step >>= 1) {
+        const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, L + step - 1u);
+        if (v <= k) L += step;
+    }
+    return L & 31u;
+}
+}  // namespace
+
+__global__ void __launch_bounds__(RF_LIST_WARPS * 32)
+k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__restrict__ mask,
+             uint32_t ntiles, uint32_t npieces, const uint32_t *__restrict__ toff,
+             const uint32_t *__restrict__ tcnt, const RasterPrim *__restrict__ rprims,
+             const unsigned long long *__restrict__ marks, uint32_t slots, uint32_t *__restrict__ items,
+             uint32_t *__restrict__ extras, uint2 *__restrict__ segs, uint2 *__restrict__ list,
+             unsigned long long *__restrict__ cursor, unsigned long long cap, uint32_t *__restrict__ ovf) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t piece = blockIdx.x * RF_LIST_WARPS + w;
+    __shared__ unsigned long long place[RF_LIST_WARPS];
+    const bool have = piece < npieces;
+    const JobDev &J = jobs[jobs[upper_index(nj, have ? piece : npieces - 1u,
+                                            [&](uint32_t i) { return (uint32_t)jobs[i].nth_seg; })].nth];
+    const uint32_t r = (have ? piece : npieces - 1u) - (uint32_t)J.seg_base;
+    const uint32_t lt = r / J.nseg, sg = r - lt * J.nseg, tile = J.tile_base + lt;
     const uint32_t *sw = mask + J.sum_base + (size_t)lt * J.sum_words;
+    const uint32_t *mw = mask + J.mask_base + (size_t)lt * J.mask_words;
+    const uint32_t s0 = sg * J.seg_words, s1 = have ? min(s0 + J.seg_words, J.sum_words) : s0;
+    // Steps over the piece's nonzero mask words in order, up to 32 a step, one a
+    // lane (m, at index wi): false when there are none left.
+    uint32_t sb = s0, v = 0, vincl = 0, vtotal = 0, vk = 0, m = 0, wi = 0;
+    auto step = [&]() -> bool {
+        while (vk >= vtotal) {
+            if (sb >= s1) return false;
+            v = sb + lane < s1 ? sw[sb + lane] : 0u;
+            vincl = warp_incl(__popc(v), lane);
+            vtotal = __shfl_sync(FULL, vincl, 31);
+            vk = 0;
+            sb += 32u;
+        }
+        const uint32_t k = vk + lane, L = lane_of(vincl, k), vL = __shfl_sync(FULL, v, L);
+        const uint32_t ex = __shfl_sync(FULL, vincl - __popc(v), L);
+        wi = (sb - 32u + L) * 32u + nth_bit(vL, k - ex + 1u);
+        m = k < vtotal ? mw[wi] : 0u;
+        vk += 32u;
+        return true;
+    };
+    // Entries of the piece.
+    uint32_t n = 0, steps = 0;
+    while (step()) {
+        n += __popc(m);
+        ++steps;
+    }
+    n = __reduce_add_sync(FULL, n);
+    // Their place: one atomic per block.
+    if (lane == 0) place[w] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long sum = 0;
+        for (uint32_t i = 0; i < RF_LIST_WARPS; ++i) sum += place[i];
+        unsigned long long at = sum ? atomicAdd(cursor, sum) : 0ull;
+        for (uint32_t i = 0; i < RF_LIST_WARPS; ++i) {
+            const unsigned long long c = place[i];
+            place[i] = at;
+            at += c;
+        }
+    }
+    __syncthreads();
+    if (!have) return;
+    unsigned long long off = place[w];
+    const bool fits = off + n <= cap;
+    if (lane == 0) {
+        segs[piece] = make_uint2((uint32_t)off, fits ? n : 0u);
+        if (!fits) *ovf = 1u;
+    }
+    if (fits && n) {
+        const bool again = steps > 1u;  // (a single step's words are still here)
+        if (again) {
+            sb = s0;
+            vk = vtotal = 0;
+        }
+        while (!again || step()) {
+            // The words' triangles, 32 at a time, one a lane.
+            const uint32_t incl = warp_incl(__popc(m), lane), total = __shfl_sync(FULL, incl, 31);
+            for (uint32_t q = lane; q - lane < total; q += 32u) {
+                const uint32_t M = lane_of(incl, q), mM = __shfl_sync(FULL, m, M);
+                const uint32_t ex = __shfl_sync(FULL, incl - __popc(m), M), wM = __shfl_sync(FULL, wi, M);
+                if (q < total) {
+                    const uint32_t gt = J.tri_base + wM * 32u + nth_bit(mM, q - ex + 1u);
+                    const uint32_t p = toff[gt], c = tcnt[gt];
+                    list[off + q] = make_uint2(p | (c - 1u) << RF_ENT_SHIFT, c == 1u ? f2u(rprims[p].zmax) : 0x7FFFFFFFu);
+                }
+            }
+            off += total;
+            if (!again) break;
+        }
+    }
+    if (sg != 0u) return;
+    // The tile's work item.
     uint32_t c = 0;
     for (uint32_t i = lane; i < J.sum_words; i += 32) c += __popc(sw[i]);
-    c = __reduce_add_sync(0xFFFFFFFFu, c);
+    c = __reduce_add_sync(FULL, c);
     if (2u * c >= J.mask_words) {
         // Half the mask words or more are nonzero: they say little about
         // the count, so count the bits (a few small busy scenes do this).
-        const uint32_t *mw = mask + J.mask_base + (size_t)lt * J.mask_words;
         c = 0;
         for (uint32_t i = lane; i < J.mask_words; i += 32) c += __popc(mw[i]);
-        c = __reduce_add_sync(0xFFFFFFFFu, c);
+        c = __reduce_add_sync(FULL, c);
     }
     if (lane == 0) {
         const unsigned long long share2 = 2ull * *marks / slots;
@@ -1560,11 +1683,12 @@ k_tile_items(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__res
         // Heavy: more than twice the frame's mean; taken before the rest.
         const bool heavy = crowded || (c > RF_HEAVY_MIN && c > 2ull * *marks / ntiles);
         items[tile] = heavy ? RF_ITEM_SKIP : tile << RF_ITEM_SHIFT;
+        uint32_t *extra = extras + J.group, *first = items + ntiles + (size_t)RF_SPLIT_K * J.group_tile;
         if (crowded) {
-            const uint32_t at = ntiles + atomicAdd(extra, RF_SPLIT_K);
-            for (uint32_t k = 1; k <= RF_SPLIT_K; ++k) items[at + k - 1] = (tile << RF_ITEM_SHIFT) | k;
+            const uint32_t at = atomicAdd(extra, RF_SPLIT_K);
+            for (uint32_t k = 1; k <= RF_SPLIT_K; ++k) first[at + k - 1] = (tile << RF_ITEM_SHIFT) | k;
         } else if (heavy) {
-            items[ntiles + atomicAdd(extra, 1u)] = tile << RF_ITEM_SHIFT;
+            first[atomicAdd(extra, 1u)] = tile << RF_ITEM_SHIFT;
         }
     }
 }
@@ -1640,10 +1764,9 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
                          RasterPrim *rprims, uint32_t *mask, uint32_t *live, unsigned long long *marks,
                          StatsDev *stats, uint32_t *counters, int nsm, cudaStream_t s,
                          const uint32_t *perm, const uint32_t *ptri, int kind) {
-    cudaError_t e = cudaMemsetAsync(rows_total, 0, 8, s);  // the frame's row-record words
+    cudaError_t e = cudaMemsetAsync(rows_total, 0, 16, s);  // the frame's row-record words, the lists' cursor
     if (e != cudaSuccess) return e;
-    if (nt == 0)  // no setup pass to zero the work-list counter
-        return cudaMemsetAsync(counters + RF_CNT_ITEMS, 0, 4, s);
+    if (nt == 0) return cudaSuccess;
     uint32_t blocks = min((nt + RF_SETUP_THREADS - 1) / RF_SETUP_THREADS, (uint32_t)nsm * 32);
     // The live list has room for every output triangle three times over:
     // the triangles for k_bin from the start, those with at most 8 rows from
@@ -1655,7 +1778,7 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
                                                 prims, rows_total, rprims, live,
                                                 counters + RF_CNT_LIVE, live_small,
                                                 counters + RF_CNT_LIVE_SMALL, live_mid,
-                                                counters + RF_CNT_LIVE_MID, counters + RF_CNT_ITEMS,
+                                                counters + RF_CNT_LIVE_MID,
                                                 stats, perm, ptri);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -1684,28 +1807,43 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_items(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles,
-                         const unsigned long long *marks, uint32_t slots, uint32_t *items,
-                         uint32_t *counters, cudaStream_t s) {
+cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles, uint32_t npieces,
+                         const uint32_t *toff, const uint32_t *tcnt, const RasterPrim *rprims,
+                         const unsigned long long *marks, uint32_t slots, uint32_t *items, uint32_t *counters,
+                         uint2 *segs, uint2 *list, unsigned long long *cursor, unsigned long long cap,
+                         cudaStream_t s) {
     if (ntiles == 0) return cudaSuccess;
-    k_tile_items<<<(uint32_t)(((uint64_t)ntiles * 32 + 255) / 256), 256, 0, s>>>(
-        jobs, nj, mask, ntiles, marks, slots ? slots : 1u, items, counters + RF_CNT_ITEMS);
+    k_tile_lists<<<(npieces + RF_LIST_WARPS - 1) / RF_LIST_WARPS, RF_LIST_WARPS * 32, 0, s>>>(
+        jobs, nj, mask, ntiles, npieces, toff, tcnt, rprims, marks, slots ? slots : 1u, items,
+        counters + RF_CNT_ITEMS_G, segs, list, cursor, cap, counters + RF_CNT_LISTOVF);
     return cudaGetLastError();
 }
 
-cudaError_t launch_raster(uint32_t tile_w, int kind, bool fast, const JobDev *jobs, uint32_t nj,
-                          const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims,
-                          const uint32_t *rows, const uint32_t *tcnt, const uint32_t *toff,
-                          const uint32_t *mask, uint32_t ntiles, const uint32_t *items, const uint32_t *nitems,
-                          uint32_t *queue,
-                          StatsDev *stats, uint32_t warps, int nsm, cudaStream_t s) {
-    if (ntiles == 0) return cudaSuccess;
-    switch (tile_w) {
-        case 8: return launch_raster_tw8(kind, fast, jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        case 16: return launch_raster_tw16(kind, fast, jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        case 64: return launch_raster_tw64(kind, fast, jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        default: return launch_raster_tw32(kind, fast, jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
+cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng, const JobDev *jobs, uint32_t nj,
+                          const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, const uint32_t *rows,
+                          const uint32_t *tcnt, const uint32_t *toff, const uint32_t *mask, const uint2 *segs,
+                          const uint2 *list, uint32_t ntiles_all, const uint32_t *items_all, uint32_t *counters,
+                          StatsDev *stats, uint32_t warps, int nsm, const cudaStream_t *st, uint32_t nst) {
+    const uint32_t *listovf = counters + RF_CNT_LISTOVF;
+    for (uint32_t g = 0; g < ng; ++g) {
+        const uint32_t ntiles = groups[g].ntiles, tile0 = groups[g].tile0;
+        if (ntiles == 0) continue;
+        const int kind = groups[g].kind;
+        const bool one = groups[g].fast;
+        const uint32_t *items = items_all + tile0, *first = items_all + ntiles_all + (size_t)RF_SPLIT_K * tile0;
+        const uint32_t *nfirst = counters + RF_CNT_ITEMS_G + g;
+        uint32_t *queue = counters + RF_CNT_QUEUE_G + g;
+        const cudaStream_t s = st[g % nst];
+        cudaError_t e;
+        switch (tile_w) {
+            case 8: e = one ? launch_raster_tw8(kind, RF_RASTER_ARGS) : launch_raster_any_tw8(kind, RF_RASTER_ARGS); break;
+            case 16: e = one ? launch_raster_tw16(kind, RF_RASTER_ARGS) : launch_raster_any_tw16(kind, RF_RASTER_ARGS); break;
+            case 64: e = one ? launch_raster_tw64(kind, RF_RASTER_ARGS) : launch_raster_any_tw64(kind, RF_RASTER_ARGS); break;
+            default: e = one ? launch_raster_tw32(kind, RF_RASTER_ARGS) : launch_raster_any_tw32(kind, RF_RASTER_ARGS); break;
+        }
+        if (e != cudaSuccess) return e;
     }
+    return cudaSuccess;
 }
 
 cudaError_t launch_cull(DrawDev *draws, uint32_t nd, StatsDev *stats, int nsm, cudaStream_t s) {

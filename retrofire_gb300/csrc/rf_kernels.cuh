@@ -36,6 +36,16 @@
 // row arithmetic y0r + j must stay exact in f32.  Such halves count in oob.
 #define RF_MAX_COORD 4194304.0f
 #define RF_RASTER_MAX_THREADS 256
+// The jobs of a frame are laid out by raster group: one shader kind (or
+// RF_K_ANY: jobs that mix kinds) and one context (the default one on a depth
+// target, or any other).  Every group has a raster kernel of its own and its
+// own part of the work list.
+#define RF_MAX_GROUPS (2 * (RF_K_ANY + 1))
+struct RasterGroup {
+    int32_t kind;
+    bool fast;
+    uint32_t tile0, ntiles;
+};
 
 // counters[] slots
 #define RF_CNT_POOL 0     // pool slots used
@@ -43,19 +53,21 @@
 #define RF_CNT_POLYOVF 2  // polygons that exceeded RF_POLY_CAP vertices
 #define RF_CNT_BADIDX 3   // triangles with an out-of-range vertex index
 #define RF_CNT_PRIMS 4    // total output prims (scan total)
-#define RF_CNT_QUEUE 5    // tile queue head
+#define RF_CNT_QUEUE 5    // tile queue head of the line pass
 #define RF_CNT_ROWSOVF 6  // triangles rasterised without row records (buffer full)
 #define RF_CNT_LIVE 7     // output triangles that passed the face-cull test
-#define RF_CNT_ITEMS 8    // rasteriser work items after the first ntiles (slices of crowded tiles)
 #define RF_CNT_CLIPQ 10   // triangles queued for clipping
 #define RF_CNT_LIVE_SMALL 11  // live triangles binned eight lanes each (at most 8 rows)
 #define RF_CNT_LIVE_MID 12    // live triangles binned sixteen lanes each (9 to 16 rows)
-#define RF_CNT_N 16
+#define RF_CNT_QUEUE_G 16     // + g: work-list queue head of raster group g
+#define RF_CNT_ITEMS_G (RF_CNT_QUEUE_G + RF_MAX_GROUPS)  // + g: its heavy tiles and crowded tiles' slices
+#define RF_CNT_LISTOVF (RF_CNT_ITEMS_G + RF_MAX_GROUPS)  // nonzero: the triangle lists did not fit
+#define RF_CNT_N (RF_CNT_LISTOVF + 1)
 #define RF_SCAN_BLOCK_ITEMS 4096u  // values one scan block takes (one launch instead of three)
 
 namespace rfk {
-// counters (optional): POOL, QUEUE, LIVE (all three lists), PRIMS and CLIPQ
-// zeroed for the kernels after it, and *marks (the binning pass's total of
+// counters (optional): POOL, LIVE (all three lists), PRIMS, CLIPQ and the
+// groups' slots zeroed for the kernels after it, and *marks (the binning pass's total of
 // (triangle, tile) bits).
 cudaError_t launch_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv, float4 *cpos,
                           uint8_t *coc, uint32_t *counters, unsigned long long *marks,
@@ -87,7 +99,7 @@ cudaError_t launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t 
 // binning (k_bin_small for triangles of at most 8 and of 9 to 16 rows,
 // then k_bin).  rows holds rows_cap words; rows_total (zeroed here)
 // receives the words the frame asked for, each triangle's records placed
-// by k_setup from it; live (room for three times every output triangle)
+// by k_setup from it (rows_total[1], zeroed too, is the lists' cursor); live (room for three times every output triangle)
 // receives the index of each triangle that passes the face-cull test: the
 // regular ones with at most 8 rows on the target (counters[RF_CNT_LIVE_SMALL]) in its second
 // third, with 9 to 16 rows (counters[RF_CNT_LIVE_MID]) in its last, the
@@ -102,17 +114,32 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
                          unsigned long long *marks, StatsDev *stats, uint32_t *counters, int nsm,
                          cudaStream_t s, const uint32_t *perm = nullptr, const uint32_t *ptri = nullptr,
                          int kind = RF_K_ANY);
-// The rasteriser's work list from the tile masks and the marks total
-// (slots: the warps the rasteriser keeps resident, about).  items (room
-// for (RF_SPLIT_K + 1) * ntiles): items[ntiles .. ntiles + extra) first --
-// heavy tiles (tile << RF_ITEM_SHIFT) and the row slices of crowded tiles
-// (tile << RF_ITEM_SHIFT | k, k = 1 .. RF_SPLIT_K) -- then items[0 .. ntiles):
-// tile t << RF_ITEM_SHIFT in index
-// order, RF_ITEM_SKIP for the tiles already listed; extra is
-// counters[RF_CNT_ITEMS] (zeroed by launch_setup).
-cudaError_t launch_items(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles,
-                         const unsigned long long *marks, uint32_t slots, uint32_t *items,
-                         uint32_t *counters, cudaStream_t s);
+// The tiles' triangle lists and the rasteriser's work list, from the tile
+// masks and the marks total (slots: the warps the rasteriser keeps resident,
+// about).
+// Lists: the set bits of every tile's mask as entries, one per input
+// triangle -- x: its first output triangle | (its outputs - 1) <<
+// RF_ENT_SHIFT, y: the depth bound of a single output (RasterPrim::zmax),
+// NaN for more -- in submission order.  A tile's list comes in J.nseg pieces
+// (segs[J.seg_base + tile * J.nseg + k]: offset, entries), each placed by
+// atomics on *cursor (zeroed by launch_setup); past cap entries the piece is
+// not written and counters[RF_CNT_LISTOVF] is set: the rasteriser then walks
+// the masks itself.
+// Work list: items (room for (RF_SPLIT_K + 1) * ntiles): items[ntiles ..
+// ntiles + extra) first -- heavy tiles (tile << RF_ITEM_SHIFT) and the row
+// slices of crowded tiles (tile << RF_ITEM_SHIFT | k, k = 1 .. RF_SPLIT_K) --
+// then items[0 .. ntiles): tile t << RF_ITEM_SHIFT in index order,
+// RF_ITEM_SKIP for the tiles already listed; extra is
+// counters[RF_CNT_ITEMS_G + g], the list per raster group g: its tiles are
+// tile0 .. tile0 + n and its first part starts at ntiles + RF_SPLIT_K * tile0.
+#define RF_ENT_SHIFT 29u
+#define RF_ENT_MASK ((1u << RF_ENT_SHIFT) - 1u)
+static_assert(RF_MAX_FAN <= 8, "an entry holds a fan's size");
+cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles, uint32_t npieces,
+                         const uint32_t *toff, const uint32_t *tcnt, const RasterPrim *rprims,
+                         const unsigned long long *marks, uint32_t slots, uint32_t *items, uint32_t *counters,
+                         uint2 *segs, uint2 *list, unsigned long long *cursor, unsigned long long cap,
+                         cudaStream_t s);
 #ifndef RF_SPLIT_K
 #define RF_SPLIT_K 4  // row slices of a crowded tile (RF_TILE_H / RF_SPLIT_K rows each)
 #endif
@@ -121,25 +148,29 @@ cudaError_t launch_items(const JobDev *jobs, uint32_t nj, const uint32_t *mask, 
 static_assert(RF_TILE_H % RF_SPLIT_K == 0 && RF_SPLIT_K < 16, "row slices");
 #define RF_ITEM_SKIP 0xFFFFFFFEu  // a work-list entry taken elsewhere in the list
 #define RF_MAX_TILES (1u << (31 - RF_ITEM_SHIFT))  // tiles of one frame or batch
-cudaError_t launch_raster(uint32_t tile_w, int kind, bool fast, const JobDev *jobs, uint32_t nj,
-                          const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims,
-                          const uint32_t *rows, const uint32_t *tcnt, const uint32_t *toff,
-                          const uint32_t *mask, uint32_t ntiles, const uint32_t *items, const uint32_t *nitems,
-                          uint32_t *queue,
-                          StatsDev *stats, uint32_t warps, int nsm, cudaStream_t s);
-#define RF_DECL_RASTER_TW(TW)                                                                  \
-    cudaError_t launch_raster_tw##TW(int kind, bool fast, const JobDev *jobs, uint32_t nj,      \
-                                     const DrawDev *draws, const PrimRec *prims,                \
-                                     const RasterPrim *rprims, const uint32_t *rows,            \
-                                     const uint32_t *tcnt, const uint32_t *toff,                \
-                                     const uint32_t *mask, uint32_t ntiles, const uint32_t *items, \
-                                     const uint32_t *nitems, uint32_t *queue, StatsDev *stats,    \
-                                     uint32_t warps, int nsm, cudaStream_t s);
+// The launchers per tile width (rf_raster.cuh).
+#define RF_RASTER_PARAMS                                                                              \
+    const JobDev *jobs, uint32_t nj, const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, \
+        const uint32_t *rows, const uint32_t *tcnt, const uint32_t *toff, const uint32_t *mask,         \
+        const uint2 *segs, const uint2 *list, const uint32_t *listovf, const uint32_t *items, uint32_t ntiles, const uint32_t *first, const uint32_t *nfirst,          \
+        uint32_t *queue, StatsDev *stats, uint32_t warps, int nsm, cudaStream_t s
+#define RF_RASTER_ARGS \
+    jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, segs, list, listovf, items, ntiles, first, nfirst, queue, stats, warps, nsm, s
+#define RF_DECL_RASTER_TW(TW)                                         \
+    cudaError_t launch_raster_tw##TW(int kind, RF_RASTER_PARAMS);      \
+    cudaError_t launch_raster_any_tw##TW(int kind, RF_RASTER_PARAMS);
 RF_DECL_RASTER_TW(8)
 RF_DECL_RASTER_TW(16)
 RF_DECL_RASTER_TW(32)
 RF_DECL_RASTER_TW(64)
 #undef RF_DECL_RASTER_TW
+// The raster pass: a launch per group, on the streams st[0 .. nst) in turn
+// (the caller orders the side streams after and before its own).
+cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng, const JobDev *jobs, uint32_t nj,
+                          const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, const uint32_t *rows,
+                          const uint32_t *tcnt, const uint32_t *toff, const uint32_t *mask, const uint2 *segs,
+                          const uint2 *list, uint32_t ntiles, const uint32_t *items, uint32_t *counters,
+                          StatsDev *stats, uint32_t warps, int nsm, const cudaStream_t *st, uint32_t nst);
 cudaError_t launch_fill(uint32_t *color, float *depth, size_t n, uint32_t px, float z,
                         uint32_t flags, int nsm, cudaStream_t s);
 // Object culling of the draws with RF_DRAW_CULL_BBOX (sets DrawDev::culled

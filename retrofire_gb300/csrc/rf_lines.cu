@@ -59,10 +59,11 @@ __device__ __forceinline__ uint32_t lzdiv_mask(int32_t shader) {
 
 // Shaded colour of a fragment with varyings v (v[0] = z, v[1..] attributes
 // after to_screen), packed in the target's format.
-__device__ uint32_t lshade(const DrawDev &d, const float *v, int32_t fmt) {
+__device__ uint32_t lshade(const DrawDev &dd, const float *v, int32_t fmt) {
     using namespace rfr;
+    const Paint d(dd);
     uint32_t c;
-    switch (d.shader) {
+    switch (dd.shader) {
         case RF_K_FLAT: c = Kind<RF_K_FLAT>::shade(d, v); break;
         case RF_K_GOURAUD: c = Kind<RF_K_GOURAUD>::shade(d, v); break;
         case RF_K_TEXTURED: c = Kind<RF_K_TEXTURED>::shade(d, v); break;

@@ -59,12 +59,15 @@ constexpr size_t OFF_PRIMS =
     al(OFF_POOL + (size_t)RF_NOALLOC_MAX_TRIS * RF_POLY_STORE * sizeof(PolyVert));
 constexpr size_t OFF_MASK = al(OFF_PRIMS + (size_t)RF_NOALLOC_MAX_TRIS * RF_MAX_FAN * sizeof(PrimRec));
 constexpr size_t OFF_ROWTOT = al(OFF_MASK + (size_t)MAX_TILES * (MASK_WORDS + SUM_WORDS) * 4);
-constexpr size_t OFF_RPRIMS = al(OFF_ROWTOT + 8);
+constexpr size_t OFF_RPRIMS = al(OFF_ROWTOT + 16);
 constexpr size_t OFF_LIVE =
     al(OFF_RPRIMS + (size_t)RF_NOALLOC_MAX_TRIS * RF_MAX_FAN * sizeof(RasterPrim));
 constexpr size_t OFF_MARKS = al(OFF_LIVE + (size_t)RF_NOALLOC_MAX_TRIS * RF_MAX_FAN * 12);
 constexpr size_t OFF_ITEMS = al(OFF_MARKS + 16);
-constexpr size_t OFF_ROWS = al(OFF_ITEMS + (size_t)MAX_TILES * (RF_SPLIT_K + 1) * 4);
+constexpr size_t OFF_SEGS = al(OFF_ITEMS + (size_t)MAX_TILES * (RF_SPLIT_K + 1) * 4);
+constexpr size_t LIST_CAP = 32768;  // entries of the tiles' triangle lists (the masks are walked past it)
+constexpr size_t OFF_LIST = al(OFF_SEGS + (size_t)MAX_TILES * 8);
+constexpr size_t OFF_ROWS = al(OFF_LIST + LIST_CAP * 8);
 // The rest of the area holds row records; triangles whose records do not
 // fit are rasterised from their setup records instead (same results).
 constexpr size_t ROWS_WORDS = (RF_NOALLOC_SCRATCH_BYTES - OFF_ROWS) / 4;
@@ -205,6 +208,8 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
     J.mask_words = (ntri + 31) / 32;
     J.mask_base = 0;
     J.sum_words = (J.mask_words + 31) / 32;
+    J.nseg = 1;
+    J.seg_words = J.sum_words;
     J.sum_base = (uint64_t)J.tiles_x * J.tiles_y * J.mask_words;  // summaries after the masks
     if (clear_rgba) {
         J.clear_flags |= 1u;
@@ -237,6 +242,7 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
     unsigned long long *marks = reinterpret_cast<unsigned long long *>(base + OFF_MARKS);
     uint32_t *items = reinterpret_cast<uint32_t *>(base + OFF_ITEMS);
     uint32_t *rows = reinterpret_cast<uint32_t *>(base + OFF_ROWS);
+    uint2 *segs = reinterpret_cast<uint2 *>(base + OFF_SEGS), *list = reinterpret_cast<uint2 *>(base + OFF_LIST);
 
     // ---- zero what the kernels accumulate into, then the pass itself
     NA_CK(cudaMemsetAsync(sd, 0, sizeof(StatsDev), s));
@@ -256,12 +262,13 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
         NA_CK(rfk::launch_setup(dd, 1, jd, ntri, TILE_W, cpos, tcnt, toff, tpoly, pool, prims,
                                 rowtot, rows, ROWS_WORDS, rprims, mask, live,
                                 marks, sd, cnt, nsm, s, nullptr, nullptr, shader));
-        NA_CK(rfk::launch_items(jd, 1, mask, ntiles, marks, (uint32_t)nsm * 16u, items, cnt, s));
+        NA_CK(rfk::launch_lists(jd, 1, mask, ntiles, ntiles, toff, tcnt, rprims, marks, (uint32_t)nsm * 16u, items,
+                                cnt, segs, list, rowtot + 1, LIST_CAP, s));
         const bool fast = depth && flags->depth_test == RF_DEPTH_LESS && flags->color_write &&
                           flags->depth_write;
-        NA_CK(rfk::launch_raster(TILE_W, shader, fast, jd, 1, dd, prims, rprims, rows, tcnt, toff,
-                                 mask, ntiles, items, cnt + RF_CNT_ITEMS,
-                                 cnt + RF_CNT_QUEUE, sd, WARPS, nsm, s));
+        const RasterGroup group{shader, fast, 0u, ntiles};
+        NA_CK(rfk::launch_raster(TILE_W, &group, 1, jd, 1, dd, prims, rprims, rows, tcnt, toff, mask, segs, list, ntiles, items,
+                                 cnt, sd, WARPS, nsm, &s, 1));
     }
     if (stats) {
         StatsDev hs{};

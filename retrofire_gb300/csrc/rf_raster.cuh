@@ -12,21 +12,34 @@
 
 // ---------------------------------------------------------------------------
 // K4: tile rasteriser.
-// A warp owns one tile of RF_TILE_H rows x TW columns at a time; lane r owns
-// row r of the tile for the whole tile, so per-pixel submission order is the
-// order in which the lane walks the triangle list — no atomics, no sorting.
-// Colour and depth sit in shared memory column-major (word x*32 + r): the
-// bank of every access is the lane id, whatever x each lane is at.
-// Each lane reads its row's record (written by the binning pass from the
-// reference's own running sums: the clipped span, the varyings at its first
-// fragment and at its first tile boundary), enters the tile from one of
-// those -- or, in a third or later tile of a long span, with an exact jump
-// (rfx::jump) of whole tile widths from the boundary values -- then steps
-// pixel by pixel like Iter::next.  Warps take work items (a tile, or a row
-// slice of a crowded one) from the list k_tile_items builds; triangle
-// headers and row records come in through cp.async rings in shared memory,
-// and a tile of whole 32-column blocks goes back to HBM through the copy
-// engine (cp.async.bulk, one 128-byte row per lane).
+// A warp owns one tile of RF_TILE_H rows x TW columns (or a row slice of a
+// crowded one) at a time.  Colour and depth sit in shared memory column-major
+// (word x*32 + row).  The warp takes the tile's triangles from its list
+// (k_tile_lists) in submission order, 32 at a time on a table, and draws their
+// scanlines -- the items -- in one of two ways:
+//   by row   lane r walks row r's triangles, one a round; a round's spans lie
+//            on different rows, so every pixel sees its fragments in order
+//            without a test.  The spans are cut into 8-pixel segments, the
+//            ones the depths hide are dropped, and the rest queue up so that
+//            full warps draw them.  For triangles of many rows.
+//   packed   32 items a pass, a lane each, whatever triangles they belong to;
+//            a span that meets an earlier one of its row waits for it.  For
+//            triangles of few rows, which would leave most rows' lanes idle.
+// An item starts from its row record (the reference's own running sums: the
+// clipped span, the varyings at its first fragment and at its first tile
+// boundary), copied to shared memory one round ahead (cp.async); in a third
+// or later tile of a long span the boundary values are stepped on.  Then it
+// steps pixel by pixel like Iter::next.
+// What bounds it: the chain of dependent instructions of each warp (16 warps
+// per SM, 38 % of issue slots), so what counts is instructions per triangle:
+// one warp pass per triangle -- lane = row, most lanes idle on small
+// triangles -- measured 478 us on the 500 k-triangle grid at 1080p (now 89),
+// 337 us on 10 k instanced cubes (122), 2.40 ms on 64 uneven scenes (0.62)
+// and 236 us on 100 k triangles of 1..10^4 px^2 (169).
+// The loop's code has to stay small: with every helper inlined (8,000
+// instructions) warps waited on instruction fetch as long as they worked.
+// A tile of whole 32-column blocks goes back to HBM through the copy engine
+// (cp.async.bulk, one 128-byte row per lane).
 // ---------------------------------------------------------------------------
 namespace rfr {
 using namespace rfx;
@@ -63,7 +76,17 @@ __device__ __forceinline__ uint32_t to_color4(float r, float g, float b) {
            0xFF000000u;
 }
 
-__device__ __forceinline__ uint32_t sample_tex(const DrawDev &d, float tu, float tv) {
+// What shading reads of a draw, copied to registers once per span (lanes of
+// one pass may be at different draws).
+struct Paint {
+    const uint32_t *tex;
+    uint32_t tw, th, flat_rgba;
+    int32_t sampler;
+    __device__ __forceinline__ explicit Paint(const DrawDev &d)
+        : tex(d.tex), tw(d.tw), th(d.th), flat_rgba(d.flat_rgba), sampler(d.sampler) {}
+};
+
+__device__ __forceinline__ uint32_t sample_tex(const Paint &d, float tu, float tv) {
     const float w = (float)d.tw, h = (float)d.th;
     uint32_t u, v;
     if (d.sampler == RF_K_REPEAT_POT) {  // tex.rs:240-266
@@ -92,7 +115,7 @@ struct Kind {
     // The texel a fragment samples (textured kinds; any varyings give an
     // in-range index), then the colour from it: shade() split in two so
     // several fragments' texel loads can be in flight together.
-    __device__ static __forceinline__ uint32_t texel(const DrawDev &d, const float *v) {
+    __device__ static __forceinline__ uint32_t texel(const Paint &d, const float *v) {
         if constexpr (KIND == RF_K_TEXTURED) return sample_tex(d, fdiv(v[1], v[0]), fdiv(v[2], v[0]));
         else if constexpr (KIND == RF_K_TEX_GOURAUD) return sample_tex(d, fdiv(v[4], v[0]), fdiv(v[5], v[0]));
         else return 0u;
@@ -109,7 +132,7 @@ struct Kind {
     }
     // shade() packed into the target's pixel format (sel: pack_selector,
     // rsel: rgb_selector of it).
-    __device__ static __forceinline__ uint32_t shade_px(const DrawDev &d, const float *v, uint32_t sel,
+    __device__ static __forceinline__ uint32_t shade_px(const Paint &d, const float *v, uint32_t sel,
                                                         uint32_t rsel) {
         if constexpr (KIND == RF_K_GOURAUD) {
             // color.rs:253-263 as in to_color4, the bytes permuted at once
@@ -118,7 +141,7 @@ struct Kind {
             return pack_px(shade(d, v), sel);
         }
     }
-    __device__ static __forceinline__ uint32_t shade(const DrawDev &d, const float *v) {
+    __device__ static __forceinline__ uint32_t shade(const Paint &d, const float *v) {
         if constexpr (KIND == RF_K_FLAT) {
             return d.flat_rgba;
         } else if constexpr (KIND == RF_K_GOURAUD) {
@@ -149,8 +172,8 @@ struct TileCtx {
     uint32_t *scol;
     float *sdep;
     float *smin;
-    uint32_t lane;
-    uint32_t y;       // this lane's row
+    uint32_t row;     // the tile row this lane is at: its own, or its item's
+    uint32_t y;       // the target row of tile row `lane`
     uint32_t tx0;     // first column of the tile
     uint32_t tx1;     // one past the last column of the tile inside the target
     uint32_t tw;      // tile width (a power of two)
@@ -163,184 +186,159 @@ struct TileCtx {
     unsigned long long frags_o;
 };
 
-// Fragments a..b-1 of one scanline into the tile (raster.rs:60-69,
-// target.rs:163-198): v = varyings of fragment a, stepped by dv per pixel.
-template <int KIND, bool FAST>
-__device__ __forceinline__ uint32_t pixels(TileCtx &T, const DrawDev &d, float *v, const float *dv,
-                                           uint32_t a, uint32_t b) {
-    constexpr int NC = Kind<KIND>::NC;
-    uint32_t idx = (a - T.tx0) * RF_TILE_H + T.lane;
-    const uint32_t end = (b - T.tx0) * RF_TILE_H + T.lane;
-    if constexpr (FAST) {
-        // Four pixels per iteration: their depths are loaded together (this
-        // lane alone writes its row, so they cannot change meanwhile); only
-        // the running sums chain from pixel to pixel.
-        uint32_t nout = 0;
-        for (; idx + 3 * RF_TILE_H < end; idx += 4 * RF_TILE_H) {
-            const float c0 = T.sdep[idx], c1 = T.sdep[idx + RF_TILE_H];
-            const float c2 = T.sdep[idx + 2 * RF_TILE_H], c3 = T.sdep[idx + 3 * RF_TILE_H];
-            float v1[NC], v2[NC], v3[NC];
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                v1[c] = fadd(v[c], dv[c]);
-                v2[c] = fadd(v1[c], dv[c]);
-                v3[c] = fadd(v2[c], dv[c]);
-            }
-            // ctx.rs:86-89 with Some(Less)
-            const bool p0 = c0 < v[0], p1 = c1 < v1[0], p2 = c2 < v2[0], p3 = c3 < v3[0];
-            if constexpr (Kind<KIND>::TEXTURED) {
-                // The passing fragments' texels are loaded together, then used.
-                uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0;
-                if (p0) t0 = Kind<KIND>::texel(d, v);
-                if (p1) t1 = Kind<KIND>::texel(d, v1);
-                if (p2) t2 = Kind<KIND>::texel(d, v2);
-                if (p3) t3 = Kind<KIND>::texel(d, v3);
-                if (p0) {
-                    T.scol[idx] = pack_px(Kind<KIND>::from_texel(t0, v), T.fmt);
-                    T.sdep[idx] = v[0];
-                    ++nout;
-                }
-                if (p1) {
-                    T.scol[idx + RF_TILE_H] = pack_px(Kind<KIND>::from_texel(t1, v1), T.fmt);
-                    T.sdep[idx + RF_TILE_H] = v1[0];
-                    ++nout;
-                }
-                if (p2) {
-                    T.scol[idx + 2 * RF_TILE_H] = pack_px(Kind<KIND>::from_texel(t2, v2), T.fmt);
-                    T.sdep[idx + 2 * RF_TILE_H] = v2[0];
-                    ++nout;
-                }
-                if (p3) {
-                    T.scol[idx + 3 * RF_TILE_H] = pack_px(Kind<KIND>::from_texel(t3, v3), T.fmt);
-                    T.sdep[idx + 3 * RF_TILE_H] = v3[0];
-                    ++nout;
-                }
-            } else if constexpr (KIND == RF_K_GOURAUD_SRGB) {
-                // Three powf per pixel: only the passing pixels are shaded.
-                if (p0) {
-                    T.scol[idx] = pack_px(Kind<KIND>::shade(d, v), T.fmt);
-                    T.sdep[idx] = v[0];
-                }
-                if (p1) {
-                    T.scol[idx + RF_TILE_H] = pack_px(Kind<KIND>::shade(d, v1), T.fmt);
-                    T.sdep[idx + RF_TILE_H] = v1[0];
-                }
-                if (p2) {
-                    T.scol[idx + 2 * RF_TILE_H] = pack_px(Kind<KIND>::shade(d, v2), T.fmt);
-                    T.sdep[idx + 2 * RF_TILE_H] = v2[0];
-                }
-                if (p3) {
-                    T.scol[idx + 3 * RF_TILE_H] = pack_px(Kind<KIND>::shade(d, v3), T.fmt);
-                    T.sdep[idx + 3 * RF_TILE_H] = v3[0];
-                }
-                nout += (uint32_t)p0 + (uint32_t)p1 + (uint32_t)p2 + (uint32_t)p3;
-            } else {
-                // Flat and Gouraud shading are a few instructions and read no
-                // memory: every pixel's colour is computed and only the
-                // stores depend on the depth test (no branches around the
-                // arithmetic).
-                const uint32_t k0 = Kind<KIND>::shade_px(d, v, T.fmt, T.rfmt);
-                const uint32_t k1 = Kind<KIND>::shade_px(d, v1, T.fmt, T.rfmt);
-                const uint32_t k2 = Kind<KIND>::shade_px(d, v2, T.fmt, T.rfmt);
-                const uint32_t k3 = Kind<KIND>::shade_px(d, v3, T.fmt, T.rfmt);
-                if (p0) {
-                    T.scol[idx] = k0;
-                    T.sdep[idx] = v[0];
-                }
-                if (p1) {
-                    T.scol[idx + RF_TILE_H] = k1;
-                    T.sdep[idx + RF_TILE_H] = v1[0];
-                }
-                if (p2) {
-                    T.scol[idx + 2 * RF_TILE_H] = k2;
-                    T.sdep[idx + 2 * RF_TILE_H] = v2[0];
-                }
-                if (p3) {
-                    T.scol[idx + 3 * RF_TILE_H] = k3;
-                    T.sdep[idx + 3 * RF_TILE_H] = v3[0];
-                }
-                nout += (uint32_t)p0 + (uint32_t)p1 + (uint32_t)p2 + (uint32_t)p3;
-            }
-#pragma unroll
-            for (int c = 0; c < NC; ++c) v[c] = fadd(v3[c], dv[c]);
-        }
-        for (; idx != end; idx += RF_TILE_H) {
-            const float z = v[0];
-            if (T.sdep[idx] < z) {
-                T.scol[idx] = Kind<KIND>::shade_px(d, v, T.fmt, T.rfmt);
-                T.sdep[idx] = z;
-                ++nout;
-            }
-#pragma unroll
-            for (int c = 0; c < NC; ++c) v[c] = fadd(v[c], dv[c]);
-        }
-        T.frags_o += nout;
-        return nout;
+template <int KIND>
+struct PreNC {
+    static constexpr int NC = KIND == RF_K_ANY ? RF_NC : Kind<KIND == RF_K_ANY ? 0 : KIND>::NC;
+    static constexpr int NP = (NC + 1) / 2;  // pairs of components
+};
+__host__ __device__ constexpr uint32_t row_words(int nc) { return 1u + 2u * (uint32_t)nc; }
+__device__ __forceinline__ uint32_t kind_nc(uint32_t kind) {
+    return kind == RF_K_FLAT ? 1u : kind == RF_K_TEXTURED ? 3u : kind == RF_K_TEX_GOURAUD ? 6u : 4u;
+}
+
+
+template <int KIND>
+__device__ __forceinline__ uint32_t shade_any(uint32_t kind, const Paint &d, const float *v, uint32_t sel,
+                                              uint32_t rsel) {
+    if constexpr (KIND != RF_K_ANY) {
+        return Kind<KIND == RF_K_ANY ? 0 : KIND>::shade_px(d, v, sel, rsel);
     } else {
-        for (; idx != end; idx += RF_TILE_H) {
-            const float z = v[0];
+        switch (kind) {
+            case RF_K_FLAT: return Kind<RF_K_FLAT>::shade_px(d, v, sel, rsel);
+            case RF_K_GOURAUD: return Kind<RF_K_GOURAUD>::shade_px(d, v, sel, rsel);
+            case RF_K_TEXTURED: return Kind<RF_K_TEXTURED>::shade_px(d, v, sel, rsel);
+            case RF_K_TEX_GOURAUD: return Kind<RF_K_TEX_GOURAUD>::shade_px(d, v, sel, rsel);
+            default: return Kind<RF_K_GOURAUD_SRGB>::shade_px(d, v, sel, rsel);
+        }
+    }
+}
+
+// U fragments of one scanline into the tile (raster.rs:60-69, target.rs:
+// 163-198), those before `end` of them: v = the varyings of the fragment at
+// word idx of the tile, as pairs stepped two at a time (each half of
+// add.rn.f32x2 rounds as the single addition).  U > 1: the depths are
+// loaded together (this lane alone writes these pixels meanwhile), and so
+// are the texels; a load past `end` stays inside the warp's area.
+// Advances idx and v; returns how many passed (FAST).
+template <int KIND, bool FAST, int U>
+__device__ __forceinline__ uint32_t px_group(TileCtx &T, const Paint &d, uint32_t kind, float2 *v, const float2 *dv,
+                                             uint32_t &idx, uint32_t end) {
+    constexpr int NP = PreNC<KIND>::NP;
+    constexpr int K1 = KIND == RF_K_ANY ? 0 : KIND;
+    float cur[U];
+    bool p[U];
+    float w[U][2 * NP];
+    float2 x[NP];
+#pragma unroll
+    for (int u = 0; u < U; ++u) cur[u] = FAST || T.has_depth ? T.sdep[idx + u * RF_TILE_H] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < NP; ++c) x[c] = v[c];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+            w[u][2 * c] = x[c].x;
+            w[u][2 * c + 1] = x[c].y;
+            x[c] = __fadd2_rn(x[c], dv[c]);
+        }
+        const bool in = U == 1 || idx + u * RF_TILE_H < end;
+        if constexpr (FAST) {
+            p[u] = in && cur[u] < w[u][0];  // ctx.rs:86-89 with Some(Less)
+        } else {
             bool pass = true;
             if (T.has_depth) {
-                const float cur = T.sdep[idx];
                 switch (T.depth_test) {  // ctx.rs:86-89
                     case RF_K_DEPTH_NONE: pass = true; break;
-                    case RF_K_DEPTH_LESS: pass = cur < z; break;
-                    case RF_K_DEPTH_EQUAL: pass = cur == z; break;
-                    default: pass = cur > z; break;
+                    case RF_K_DEPTH_LESS: pass = cur[u] < w[u][0]; break;
+                    case RF_K_DEPTH_EQUAL: pass = cur[u] == w[u][0]; break;
+                    default: pass = cur[u] > w[u][0]; break;
                 }
             }
-            if (pass) {
-                if (T.color_write) {
-                    T.scol[idx] = Kind<KIND>::shade_px(d, v, T.fmt, T.rfmt);
-                    T.frags_o += 1;
-                }
-                if (T.has_depth && T.depth_write) T.sdep[idx] = z;
-            }
-    #pragma unroll
-            for (int c = 0; c < NC; ++c) v[c] = fadd(v[c], dv[c]);
+            p[u] = in && pass;
         }
-        return 0;
     }
+#pragma unroll
+    for (int c = 0; c < NP; ++c) v[c] = x[c];
+    uint32_t nout = 0;
+    if constexpr (FAST && U > 1 && KIND != RF_K_ANY && Kind<K1>::TEXTURED) {
+        uint32_t t[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) t[u] = p[u] ? Kind<K1>::texel(d, w[u]) : 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (p[u]) {
+                T.scol[idx + u * RF_TILE_H] = pack_px(Kind<K1>::from_texel(t[u], w[u]), T.fmt);
+                T.sdep[idx + u * RF_TILE_H] = w[u][0];
+                ++nout;
+            }
+    } else if constexpr (FAST && U > 1 && (KIND == RF_K_FLAT || KIND == RF_K_GOURAUD)) {
+        // A few instructions that read no memory: every pixel's colour is
+        // computed and only the stores depend on the depth test.
+        uint32_t k[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) k[u] = Kind<K1>::shade_px(d, w[u], T.fmt, T.rfmt);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (p[u]) {
+                T.scol[idx + u * RF_TILE_H] = k[u];
+                T.sdep[idx + u * RF_TILE_H] = w[u][0];
+            }
+            nout += p[u] ? 1u : 0u;
+        }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (p[u]) {
+                if (FAST || T.color_write) {
+                    T.scol[idx + u * RF_TILE_H] = shade_any<KIND>(kind, d, w[u], T.fmt, T.rfmt);
+                    ++nout;
+                }
+                if (FAST || (T.has_depth && T.depth_write)) T.sdep[idx + u * RF_TILE_H] = w[u][0];
+            }
+    }
+    idx += U * RF_TILE_H;
+    return nout;
 }
 
 // FAST path: the minimum current depth of segment s of the lane's row.
 __device__ __forceinline__ void seg_refresh(TileCtx &T, uint32_t s) {
-    const uint32_t base = s * RF_SEG * RF_TILE_H + T.lane;
+    const uint32_t base = s * RF_SEG * RF_TILE_H + T.row;
     float m = T.sdep[base];
 #pragma unroll
     for (uint32_t x = 1; x < RF_SEG; ++x) m = fminf(m, T.sdep[base + x * RF_TILE_H]);
-    T.smin[s * RF_TILE_H + T.lane] = m;
+    T.smin[s * RF_TILE_H + T.row] = m;
 }
 
-// FAST path: true when no fragment a..b-1 can pass Less: an upper bound of
-// the span's running z is <= the current depth of every pixel it covers.
-// z_k = fl(z_{k-1} + dz) never rises when dz <= 0, so its maximum is za; for
-// dz > 0 (all values positive, normal range) k <= 63 rounded additions stay
-// within (1+2^-24)^k of za + k dz, and fl(za + k dz) is within (1-2^-24)^2
-// of it, so fl(e * (1 + 2^-16)) bounds every z_k.  NaN z or depth never
-// skips here (the comparisons are false) and never passes later.
-__device__ __forceinline__ bool span_hidden(const TileCtx &T, float za, float dz, uint32_t a,
-                                            uint32_t b) {
-    float zhi;
-    if (dz <= 0.0f) {
-        zhi = za;
-    } else if (dz > 0.0f && za >= 1e-30f) {
-        const float e = fadd(za, fmul((float)(b - a - 1u), dz));
-        zhi = fmul(e, 1.0000152587890625f);  // 1 + 2^-16
-    } else {
-        return false;
-    }
-    const uint32_t s0 = (a - T.tx0) / RF_SEG, s1 = (b - 1u - T.tx0) / RF_SEG;
-    float lo = T.smin[s0 * RF_TILE_H + T.lane];
-    for (uint32_t s = s0 + 1; s <= s1; ++s) lo = fminf(lo, T.smin[s * RF_TILE_H + T.lane]);
-    return zhi <= lo;
+// FAST path: an upper bound of the running z of n fragments (n <= 64) from
+// z0 on.  z_k = fl(z_{k-1} + dz) never rises when dz <= 0, so its maximum is
+// z0; for dz > 0 (all values positive, normal range) k <= 63 rounded
+// additions stay within (1+2^-24)^k of z0 + k dz, and fl(z0 + k dz) is
+// within (1-2^-24)^2 of it, so fl(e * (1 + 2^-16)) bounds every z_k.
+// Otherwise NaN: no bound (comparisons with it are false, so nothing is
+// skipped; a NaN z never passes Less either).
+__device__ __forceinline__ float depth_bound(float z0, float dz, uint32_t n) {
+    const float e = fmul(fadd(z0, fmul((float)(n - 1u), dz)), 1.0000152587890625f);  // 1 + 2^-16
+    return dz <= 0.0f ? z0 : dz > 0.0f && z0 >= 1e-30f ? e : __int_as_float(0x7FFFFFFF);
 }
+
+// ... and true when no fragment a..b-1 of a span can pass Less: the bound is
+// <= the current depth of every pixel it covers.
+__device__ __forceinline__ bool span_hidden(const TileCtx &T, float za, float dz, uint32_t a, uint32_t b) {
+    const uint32_t s0 = (a - T.tx0) / RF_SEG, s1 = (b - 1u - T.tx0) / RF_SEG;
+    float lo = T.smin[s0 * RF_TILE_H + T.row];
+    for (uint32_t s = s0 + 1; s <= s1; ++s) lo = fminf(lo, T.smin[s * RF_TILE_H + T.row]);
+    return depth_bound(za, dz, b - a) <= lo;
+}
+
+// rfx::jump out of line: the rasteriser's loop has to stay small (its
+// instructions are fetched again on every pass).
+static __device__ __noinline__ float jump_far(float s, float d, uint32_t k) { return jump(s, d, k); }
 
 // The lane's scanline j of half H (raster.rs:84-113), clipped to the tile,
 // then its fragments (raster.rs:60-69) into the tile (target.rs:163-198).
 // FAST: the default context (depth test Less, colour and depth writes on).
 template <int KIND, bool FAST>
-__device__ __forceinline__ void span(TileCtx &T, const DrawDev &d, const HalfRec *__restrict__ H,
+__device__ __forceinline__ void span(TileCtx &T, const Paint &d, const HalfRec *__restrict__ H,
                                      const HalfRuns *__restrict__ U, uint32_t j) {
     constexpr int NC = Kind<KIND>::NC;
     const float lx = row_value(H, U, RF_R_LX, j);
@@ -370,9 +368,18 @@ __device__ __forceinline__ void span(TileCtx &T, const DrawDev &d, const HalfRec
         dv[c] = H->dvdx[c];
         const float c0 = row_value(H, U, RF_R_C + c, j);
         const float adj = fadd(c0, fmul(fsub(fadd(c0, dv[c]), c0), tshift));
-        v[c] = jump(adj, dv[c], k0);
+        v[c] = jump_far(adj, dv[c], k0);
     }
-    pixels<KIND, FAST>(T, d, v, dv, a, b);
+    constexpr int NP = PreNC<KIND>::NP;
+    float2 v2[NP], dv2[NP];
+#pragma unroll
+    for (int c = 0; c < NP; ++c) {
+        v2[c] = make_float2(v[2 * c], 2 * c + 1 < NC ? v[2 * c + 1 < NC ? 2 * c + 1 : 0] : 0.0f);
+        dv2[c] = make_float2(dv[2 * c], 2 * c + 1 < NC ? dv[2 * c + 1 < NC ? 2 * c + 1 : 0] : 0.0f);
+    }
+    uint32_t idx = (a - T.tx0) * RF_TILE_H + T.row;
+    const uint32_t end = (b - T.tx0) * RF_TILE_H + T.row;
+    while (idx < end) T.frags_o += px_group<KIND, FAST, 1>(T, d, (uint32_t)KIND, v2, dv2, idx, end);
 }
 
 // Which scanline of a half lands on row y: row(j) = (y0r + j) as usize =
@@ -398,7 +405,7 @@ __device__ __forceinline__ void rows_for(const HalfRec *__restrict__ H, uint32_t
 }
 
 template <int KIND, bool FAST>
-__device__ __forceinline__ void raster_prim_k(TileCtx &T, const DrawDev &d, const PrimRec *__restrict__ P) {
+__device__ __forceinline__ void raster_prim_k(TileCtx &T, const Paint &d, const PrimRec *__restrict__ P) {
     if (!T.row_ok) return;
     // The two halves cover disjoint rows, so each lane walks only the half
     // holding its row and both halves run in one pass of the warp.  Only
@@ -426,59 +433,19 @@ __device__ __forceinline__ void raster_prim_k(TileCtx &T, const DrawDev &d, cons
     }
 }
 
-// Row records in shared memory: per staged triangle one slot of
-// RF_ROW_WORDS(NC) words per lane, word w of lane L at w * 32 + L (the bank
-// is the lane).  Each lane copies its own row's record (cp.async, 4 bytes a
-// word) two triangles ahead of its use; a lane whose row the triangle does
-// not cover stores word 0 = 0 (an empty span).
+// Row records in shared memory: one slot of row_words(NC) words per lane,
+// word w of lane L at w * 32 + L (the bank is the lane).
+// The row record at src into this lane's part of a slot (cp.async, 4 bytes a
+// word), or an empty span (word 0 = 0) for a lane without one.
 template <int KIND>
-struct PreNC {
-    static constexpr int NC = KIND == RF_K_ANY ? RF_NC : Kind<KIND == RF_K_ANY ? 0 : KIND>::NC;
-};
-__host__ __device__ constexpr uint32_t row_words(int nc) { return 1u + 2u * (uint32_t)nc; }
-
-// Word indices of RasterPrim fields.
-#define RF_RPW_FLAGS 1
-#define RF_RPW_BASE 3
-#define RF_RPW_STRIDE 4
-#define RF_RPW_Y0 5
-#define RF_RPW_C0 6
-#define RF_RPW_Y1 7
-#define RF_RPW_C1 8
-#define RF_RPW_ZMAX (9 + 2 * RF_NC)
-static_assert(offsetof(RasterPrim, zmax) == 4 * RF_RPW_ZMAX, "RasterPrim word layout");
-static_assert(offsetof(RasterPrim, flags) == 4 * RF_RPW_FLAGS && offsetof(RasterPrim, base) == 4 * RF_RPW_BASE &&
-                  offsetof(RasterPrim, stride) == 4 * RF_RPW_STRIDE && offsetof(RasterPrim, y0) == 4 * RF_RPW_Y0 &&
-                  offsetof(RasterPrim, c0) == 4 * RF_RPW_C0 && offsetof(RasterPrim, y1) == 4 * RF_RPW_Y1 &&
-                  offsetof(RasterPrim, c1) == 4 * RF_RPW_C1,
-              "RasterPrim word layout");
-
-// Row records of one triangle whose header H sits in shared memory;
-// present = the triangle exists.  Every lane calls this together.
-template <int KIND>
-__device__ __forceinline__ void stage_rows(const TileCtx &T, uint32_t *slot, bool present,
-                                           const RasterPrim *H, const uint32_t *__restrict__ rows) {
-    const uint32_t flags = H->flags;
-    const uint32_t rbase = H->base;
-    const uint32_t stride = H->stride;  // 1 + 2 NC of its own kind
-    const uint32_t y0 = H->y0, c0 = H->c0, y1 = H->y1, c1 = H->c1;
-    uint32_t *dst = slot + T.lane;
-    if (!present || !T.row_ok || (flags & (RF_RP_LIVE | RF_RP_ROWS)) != (RF_RP_LIVE | RF_RP_ROWS)) {
+__device__ __forceinline__ void stage_row(uint32_t *slot, uint32_t lane, bool present, uint32_t kind,
+                                          const uint32_t *src) {
+    uint32_t *dst = slot + lane;
+    if (!present) {
         dst[0] = 0u;
         return;
     }
-    const uint32_t y = T.y;
-    uint32_t j;
-    if (y - y0 < c0) {
-        j = y - y0;
-    } else if (y - y1 < c1) {
-        j = c0 + (y - y1);
-    } else {
-        dst[0] = 0u;
-        return;
-    }
-    const uint32_t *src = rows + rbase + (size_t)j * stride;
-    const uint32_t nw = KIND == RF_K_ANY ? stride : row_words(PreNC<KIND>::NC);
+    const uint32_t nw = KIND == RF_K_ANY ? row_words((int)kind_nc(kind)) : row_words(PreNC<KIND>::NC);
 #pragma unroll
     for (uint32_t w = 0; w < row_words(PreNC<KIND>::NC); ++w) {
         if (w < nw) {
@@ -488,73 +455,64 @@ __device__ __forceinline__ void stage_rows(const TileCtx &T, uint32_t *slot, boo
     }
 }
 
-template <int KIND, bool FAST>
-__device__ __forceinline__ void raster_rows(TileCtx &T, const DrawDev &d, const RasterPrim *__restrict__ R,
-                                            uint32_t *slot) {
-    constexpr int NC = Kind<KIND>::NC;
-    uint32_t *rs = slot + T.lane;
-    const uint32_t w0 = rs[0];
-    const uint32_t xs = w0 & 0xFFFFu, xe = w0 >> 16;
-    const uint32_t a = xs > T.tx0 ? xs : T.tx0;
-    const uint32_t b = xe < T.tx1 ? xe : T.tx1;
-    if (a >= b) return;
-    const uint32_t hh = T.y - R->y0 < R->c0 ? 0u : 1u;
-    // The span starts in this tile (k = 0 from its first pixel) or enters it
-    // at a tile boundary at or after its first one (k steps from there).
+// One item -- a scanline of a triangle inside the tile: its record sits in
+// this lane's part of a slot (rs), its span [a, b) is clipped to the tile
+// (xs: the span's first pixel).  v, dv: its varyings at pixel a and their
+// steps.  The span starts in this tile, or enters it at its first tile
+// boundary -- both values are in the record -- or at a later one: then the
+// boundary values take the steps between.  Up to RF_STEP_MAX of them one
+// after the other (two components an instruction: 64 instructions for 32
+// pixels of Gouraud, where the exact jump takes about 100 a component);
+// further ones by the jump, in place.
+#define RF_STEP_MAX 128u
+template <int KIND>
+__device__ __forceinline__ void item_load(const TileCtx &T, const float *dvdx, uint32_t *rs, uint32_t nc,
+                                          uint32_t xs, uint32_t a, float2 *v, float2 *dv) {
+    constexpr int NC = PreNC<KIND>::NC, NP = PreNC<KIND>::NP;
     const bool first = a == xs;
-    const uint32_t k = first ? 0u : a - ((xs & ~(T.tw - 1u)) + T.tw);
-    const uint32_t off = first ? 1u : 1u + NC;
-    if (k) {
-        // A third or later tile of the span: step the boundary values in
-        // place (the lane's own slot), one component at a time (a rolled
-        // loop keeps the jump's code out of the per-component unrolling).
+    uint32_t k = first ? 0u : a - ((xs & ~(T.tw - 1u)) + T.tw);
+    const uint32_t off = first ? 1u : 1u + nc;
+    if (k > RF_STEP_MAX) {
 #pragma unroll 1
-        for (int c = 0; c < NC; ++c)
-            rs[(off + c) * RF_TILE_H] = f2u(jump(u2f(rs[(off + c) * RF_TILE_H]), R->dvdx[hh][c], k));
+        for (uint32_t c = 0; c < nc; ++c)
+            rs[(off + c) * RF_TILE_H] = f2u(jump_far(u2f(rs[(off + c) * RF_TILE_H]), dvdx[c], k));
+        k = 0;
     }
-    float v[NC], dv[NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        dv[c] = R->dvdx[hh][c];
-        v[c] = u2f(rs[(off + c) * RF_TILE_H]);
+    for (int c = 0; c < NP; ++c) {
+        dv[c] = reinterpret_cast<const float2 *>(dvdx)[c];
+        v[c].x = u2f(rs[(off + 2 * c) * RF_TILE_H]);
+        // (a pair past the kind's components: a value the record's words do not hold)
+        v[c].y = 2 * c + 1 < NC ? u2f(rs[(off + 2 * c + 1) * RF_TILE_H]) : 0.0f;
     }
-    if constexpr (FAST) {
-        if (span_hidden(T, v[0], dv[0], a, b)) return;
-        if (pixels<KIND, FAST>(T, d, v, dv, a, b)) {
-            const uint32_t s1 = (b - 1u - T.tx0) / RF_SEG;
-            for (uint32_t s = (a - T.tx0) / RF_SEG; s <= s1; ++s) seg_refresh(T, s);
+#pragma unroll 1
+    for (; k; k -= 8u) {  // (whole tile widths)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+#pragma unroll
+            for (int c = 0; c < NP; ++c) v[c] = __fadd2_rn(v[c], dv[c]);
         }
-    } else {
-        pixels<KIND, FAST>(T, d, v, dv, a, b);
     }
 }
 
+// A triangle without row records, from its PrimRec: lane = row (T.row = lane).
 template <int KIND, bool FAST>
-__device__ __forceinline__ void raster_one(TileCtx &T, const DrawDev &d, const RasterPrim *__restrict__ R,
-                                           const PrimRec *__restrict__ P, uint32_t *rs) {
-    if (R->flags & RF_RP_ROWS) raster_rows<KIND, FAST>(T, d, R, rs);
-    else raster_prim_k<KIND, FAST>(T, d, P);
-}
-
-// KIND: the shader kind of every draw of the job, or RF_K_ANY (dispatch per
-// triangle).
-template <int KIND, bool FAST>
-__device__ __forceinline__ void raster_prim(TileCtx &T, const DrawDev *__restrict__ draws,
-                                            const RasterPrim *__restrict__ R,
-                                            const PrimRec *__restrict__ P, uint32_t *rs) {
-    if (!(R->flags & RF_RP_LIVE)) return;
-    const DrawDev &d = draws[R->draw];
+__device__ __noinline__ uint32_t raster_prim_slow(TileCtx T, uint32_t kind, const DrawDev *__restrict__ draw,
+                                                  const PrimRec *__restrict__ P) {
+    T.frags_o = 0;
+    const Paint d(*draw);
     if constexpr (KIND != RF_K_ANY) {
-        raster_one<KIND == RF_K_ANY ? 0 : KIND, FAST>(T, d, R, P, rs);
+        raster_prim_k<KIND == RF_K_ANY ? 0 : KIND, FAST>(T, d, P);
     } else {
-        switch (R->kind) {
-            case RF_K_FLAT: raster_one<RF_K_FLAT, FAST>(T, d, R, P, rs); break;
-            case RF_K_GOURAUD: raster_one<RF_K_GOURAUD, FAST>(T, d, R, P, rs); break;
-            case RF_K_TEXTURED: raster_one<RF_K_TEXTURED, FAST>(T, d, R, P, rs); break;
-            case RF_K_TEX_GOURAUD: raster_one<RF_K_TEX_GOURAUD, FAST>(T, d, R, P, rs); break;
-            default: raster_one<RF_K_GOURAUD_SRGB, FAST>(T, d, R, P, rs); break;
+        switch (kind) {
+            case RF_K_FLAT: raster_prim_k<RF_K_FLAT, FAST>(T, d, P); break;
+            case RF_K_GOURAUD: raster_prim_k<RF_K_GOURAUD, FAST>(T, d, P); break;
+            case RF_K_TEXTURED: raster_prim_k<RF_K_TEXTURED, FAST>(T, d, P); break;
+            case RF_K_TEX_GOURAUD: raster_prim_k<RF_K_TEX_GOURAUD, FAST>(T, d, P); break;
+            default: raster_prim_k<RF_K_GOURAUD_SRGB, FAST>(T, d, P); break;
         }
     }
+    return (uint32_t)T.frags_o;
 }
 
 // FAST path: the least current depth over the tile's rows this warp owns
@@ -563,19 +521,10 @@ template <int TW>
 __device__ __forceinline__ float tile_depth_min(const TileCtx &T) {
     float m = __int_as_float(0x7F800000);
     if (T.row_ok)
-        for (uint32_t sg = 0; sg < (uint32_t)TW / RF_SEG; ++sg) m = fminf(m, T.smin[sg * RF_TILE_H + T.lane]);
+        for (uint32_t sg = 0; sg < (uint32_t)TW / RF_SEG; ++sg) m = fminf(m, T.smin[sg * RF_TILE_H + T.row]);
 #pragma unroll
     for (int sft = 16; sft > 0; sft >>= 1) m = fminf(m, __shfl_xor_sync(0xFFFFFFFFu, m, sft));
     return m;
-}
-
-// FAST path: no fragment of triangle R can pass Less in a tile whose depths
-// are all >= tzmin (R->zmax bounds its fragments' depths from above; a NaN
-// on either side never skips).
-template <bool FAST>
-__device__ __forceinline__ bool hidden(const RasterPrim *R, float tzmin) {
-    if constexpr (FAST) return R->zmax <= tzmin;
-    else return false;
 }
 
 // Warp-wide selection of set bits in order: lane L offers the bits b (lane
@@ -646,15 +595,11 @@ static __device__ __noinline__ WarpTake warp_take(uint32_t b, uint32_t want, uin
 // time; the nonzero mask words they name are then fetched 32 at a time
 // (lane e loads entry e), so an empty stretch of the mask costs nothing.
 // Both gathers pick their next 32 set bits with one warp-wide prefix count
-// (warp_take), not bit by bit.  The next 32 input triangles are gathered at
-// once, lane k holding the k-th one's output range (toff, tcnt loaded in
-// parallel), so one load latency covers 32 triangles.  Warp-uniform state;
-// every lane calls next() together.
+// (warp_take), not bit by bit.  Warp-uniform state; every lane calls
+// gather_tris() together.
 struct PrimIter {
     const uint32_t *tmask;  // the tile's mask words
     const uint32_t *tsum;   // the tile's summary words
-    const uint32_t *toff;
-    const uint32_t *tcnt;
     uint32_t nsum, tri_base, lane;
     // Summary words, 128 at a time: lane L holds words sb + 32 c + L in
     // s[c]; the cursor is chunk sc, lane sl, and srem = the bits of that
@@ -663,22 +608,25 @@ struct PrimIter {
     // Gathered mask words: lane e holds entry e (index widx, value wval),
     // wn of them; the cursor is entry wi with wrem = its bits not taken yet.
     uint32_t widx, wval, wn, wi, wrem;
-    uint32_t p, pend;
-    uint32_t boff, bcnt, bn;      // the gathered batch (lane k: entry k)
-    uint32_t keep;                // entries of the batch still to walk
-    float bz;                     // lane k: entry k's depth bound (RasterPrim::zmax; NaN: none)
-    float zcut;                   // entries whose bound is <= zcut are passed over (NaN: none)
-    const RasterPrim *rprims;
-    uint32_t slo, shi;            // rows of a row-slice item (slo >= shi: the whole tile)
+    uint32_t fidx, fval, fn;  // the word batch after it
     bool started, done;           // a window was loaded; the summary words are all read
 
     __device__ __forceinline__ uint32_t chunk_word() const {
         return sc == 0 ? s0 : (sc == 1 ? s1 : (sc == 2 ? s2 : s3));
     }
-    // The next up to 32 nonzero mask words, in order, into the word batch.
+    // The batch fetched ahead becomes the word batch, and the next up to 32
+    // nonzero mask words, in order, are fetched.
     __device__ __forceinline__ void gather_words() {
+        wn = fn;
+        widx = fidx;
+        wval = fval;
+        wi = 0;
+        wrem = __shfl_sync(0xFFFFFFFFu, wval, 0);
+        fetch_words();
+    }
+    __device__ __forceinline__ void fetch_words() {
         uint32_t n = 0, mine = 0;
-        for (;;) {
+        while (!done) {
             if (!started || sc == 4) {  // next window of summary words
                 if (started) sb += 128;
                 started = true;
@@ -719,11 +667,9 @@ struct PrimIter {
             }
             if (n == 32u) break;
         }
-        wn = n;
-        wi = 0;
-        widx = mine;
-        wval = lane < n ? tmask[mine] : 0u;
-        wrem = __shfl_sync(0xFFFFFFFFu, wval, 0);
+        fn = n;
+        fidx = mine;
+        fval = lane < n ? tmask[mine] : 0u;
     }
     // The next up to 32 input triangles (set bits), in order: lane k holds
     // the k-th one's global index in mine; returns how many.
@@ -732,9 +678,8 @@ struct PrimIter {
         mine = 0;
         while (n < 32u) {
             if (wi >= wn) {
-                if (done) break;  // no summary words left
+                if (fn == 0u) break;  // no mask words left
                 gather_words();
-                if (wn == 0) break;
             }
             const uint32_t b = (lane < wi || lane >= wn) ? 0u : (lane == wi ? wrem : wval);
             WarpTake t = warp_take(b, 32u - n, n, lane);
@@ -750,76 +695,26 @@ struct PrimIter {
         }
         return n;
     }
-    __device__ __forceinline__ void refill() {
-        uint32_t mine;
-        const uint32_t n = gather_tris(mine);
-        bn = n;
-        bool take = lane < n;
-        bz = __int_as_float(0x7FFFFFFF);
-        if (lane < n) {
-            boff = __ldg(toff + mine);
-            bcnt = __ldg(tcnt + mine);
-            if (bcnt == 1u) {
-                // An unclipped triangle: its depth bound, for passing it over
-                // in a tile whose depths have all risen to it (next()) ...
-                const uint32_t *h = reinterpret_cast<const uint32_t *>(rprims + boff);
-                bz = __ldg(reinterpret_cast<const float *>(h) + RF_RPW_ZMAX);
-                if (slo < shi) {
-                    // ... and, in a row slice of a crowded tile, whether its
-                    // rows meet the slice.
-                    const uint32_t fl = __ldg(h + RF_RPW_FLAGS);
-                    const uint32_t y0 = __ldg(h + RF_RPW_Y0), c0 = __ldg(h + RF_RPW_C0);
-                    const uint32_t y1 = __ldg(h + RF_RPW_Y1), c1 = __ldg(h + RF_RPW_C1);
-                    if (fl & RF_RP_ROWS)
-                        take = (c0 && y0 < shi && y0 + c0 > slo) || (c1 && y1 < shi && y1 + c1 > slo);
-                }
-            }
-        }
-        // (entries passed over for their depth bound now are tested again
-        // against the bound of the moment in next())
-        keep = __ballot_sync(0xFFFFFFFFu, take && !(bz <= zcut));
-    }
     __device__ __forceinline__ void init() {
         sb = s0 = s1 = s2 = s3 = sc = sl = srem = 0;
-        widx = wval = wn = wi = wrem = p = pend = 0;
-        boff = bcnt = bn = keep = 0;
-        bz = zcut = __int_as_float(0x7FFFFFFF);
+        widx = wval = wn = wi = wrem = 0;
         started = done = false;
-    }
-    __device__ __forceinline__ uint32_t next() {
-        while (p >= pend) {
-            while (keep == 0u) {
-                refill();
-                if (bn == 0) return 0xFFFFFFFFu;
-            }
-            const uint32_t k = __ffs(keep) - 1;
-            keep &= keep - 1u;
-            // Passed over: triangles no pixel of the tile can take any more
-            // (depth bound <= the tile's least depth, which only rises; a
-            // NaN on either side never passes over).
-            if (__shfl_sync(0xFFFFFFFFu, bz, k) <= zcut) continue;
-            p = __shfl_sync(0xFFFFFFFFu, boff, k);
-            pend = p + __shfl_sync(0xFFFFFFFFu, bcnt, k);
-        }
-        return p++;
+        fn = 0;
+        fetch_words();
     }
 };
 
-// Asynchronous copy of one triangle header into this warp's staging slot
-// (16 bytes per lane, lanes 0..5); committed by commit_stage().
-__device__ __forceinline__ void stage_prim(RasterPrim *slot, const RasterPrim *src, uint32_t lane) {
-    static_assert(sizeof(RasterPrim) % 16 == 0, "RasterPrim must be a whole number of 16-byte chunks");
-    static_assert(sizeof(RasterPrim) <= 64 * 16, "RasterPrim is staged in at most two rounds");
-    constexpr uint32_t CHUNKS = sizeof(RasterPrim) / 16;
-    if (src) {
-#pragma unroll
-        for (uint32_t c = lane; c < CHUNKS; c += 32) {
-            const uint32_t sa = (uint32_t)__cvta_generic_to_shared(reinterpret_cast<char *>(slot) + c * 16);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa),
-                         "l"(reinterpret_cast<const char *>(src) + c * 16)
-                         : "memory");
-        }
-    }
+// The next up to 32 input triangles of a tile whose lists did not fit, from
+// its masks: entries like the lists' (0 with y = 0 for none), n of them.
+// (Out of line, the iterator in local memory: a frame or two until the
+// library has grown the lists.)
+static __device__ __noinline__ uint2 mask_batch(PrimIter *it, const uint32_t *toff, const uint32_t *tcnt,
+                                                uint32_t lane, uint32_t *n) {
+    uint32_t mine;
+    const uint32_t k = it->gather_tris(mine);
+    *n = k;
+    if (lane >= k) return make_uint2(0u, 0u);
+    return make_uint2(__ldg(toff + mine) | (__ldg(tcnt + mine) - 1u) << RF_ENT_SHIFT, 0x7FFFFFFFu);
 }
 
 // One commit group per call on every lane (copies issued since the last).
@@ -835,30 +730,28 @@ __device__ __forceinline__ void wait_staged_but() {
 
 }  // namespace rfr
 
-// Shared-memory words per warp: colour and depth tiles, the ring of staged
-// triangle headers, the ring of staged row records, the depth-segment minima.
-// Pipeline distances of the rasteriser: a triangle's header is copied into
-// shared memory HA triangles before its turn (a ring of HA + 1 slots), its
-// row records RA before (a ring of RA + 1).
-// Narrow tiles hold fewer pixels per triangle, so their iterations are
-// shorter and the row records are copied further ahead.
-#define RF_ROW_AHEAD_NARROW 2  // tile widths 8 and 16
-#define RF_ROW_AHEAD_WIDE 2    // tile widths 32 and 64
-template <int TW>
-struct Pipe {
-    static constexpr int RA = TW <= 16 ? RF_ROW_AHEAD_NARROW : RF_ROW_AHEAD_WIDE;
-    static constexpr int HA = 2 * RA + 1 > 8 ? 2 * RA + 1 : 8;
-    static constexpr uint32_t HS = (uint32_t)HA + 1u;  // header slots
-    static constexpr uint32_t RS = (uint32_t)RA + 1u;  // row-record slots
-};
-// The header and row-record rings double as the row-major staging buffer
-// of the coalesced tile load and store (32 rows of min(TW, 32) + 1 words),
-// so the region is the larger of the two.
+// Shared-memory words per warp: the colour and depth tiles, a work region,
+// the depth-segment minima.  The work region is the row-major staging of the
+// coalesced tile load and store (32 rows of min(TW, 32) + 1 words) while a
+// tile moves, and between the two, in this order: the ring of output
+// triangles not looked at yet, the table of the triangles being drawn (a
+// uint4, the pixel steps, the draw and the depth bound of each), each row's
+// current table entry, the queue of segments, two slots of row records.
+constexpr uint32_t RF_CAND_WORDS = 256u;  // 31 left over and a batch of 32 fans fit
+static_assert(31 + 32 * RF_MAX_FAN <= RF_CAND_WORDS, "ring size");
+constexpr uint32_t RF_TAB_WORDS = (4u + 2u * RF_NC + 2u) * 32u;
+// By row from this many scanlines a triangle in the tile: at 6 the grid's
+// raster takes 158 us and the crates' 77, at 10 and 16 139 and 57; the fill
+// frame's triangles (18) are even at all three.
+constexpr uint32_t RF_ROW_MEAN = 10u;
 template <int TW, int KIND>
-__host__ __device__ constexpr uint32_t raster_ring_words() {
-    return Pipe<TW>::HS * (uint32_t)(sizeof(RasterPrim) / 4) +
-           Pipe<TW>::RS * rfr::row_words(rfr::PreNC<KIND>::NC) * RF_TILE_H;
-}
+struct Region {
+    static constexpr int NC = rfr::PreNC<KIND>::NC, NP = rfr::PreNC<KIND>::NP;
+    static constexpr uint32_t QN = RF_TILE_H * ((uint32_t)TW / RF_SEG);  // segments of a tile
+    static constexpr uint32_t QUEUE = QN * (1u + NC);
+    static constexpr uint32_t SLOT = rfr::row_words(NC) * RF_TILE_H;
+    static constexpr uint32_t WORDS = RF_CAND_WORDS + RF_TAB_WORDS + RF_TILE_H + QUEUE + 2u * SLOT;
+};
 template <int TW>
 __host__ __device__ constexpr uint32_t raster_stage_words() {
     return RF_TILE_H * ((TW < 32 ? (uint32_t)TW : 32u) + 1u);
@@ -866,8 +759,7 @@ __host__ __device__ constexpr uint32_t raster_stage_words() {
 template <int TW, int KIND>
 __host__ __device__ constexpr uint32_t raster_warp_words() {
     return 2u * TW * RF_TILE_H +
-           (raster_ring_words<TW, KIND>() > raster_stage_words<TW>() ? raster_ring_words<TW, KIND>()
-                                                                     : raster_stage_words<TW>()) +
+           (Region<TW, KIND>::WORDS > raster_stage_words<TW>() ? Region<TW, KIND>::WORDS : raster_stage_words<TW>()) +
            ((uint32_t)TW / RF_SEG) * RF_TILE_H;
 }
 
@@ -978,223 +870,526 @@ __device__ __forceinline__ void bulk_store_drain() {
 
 }  // namespace rfr
 
-// KIND: shader kind of every draw of the job (or RF_K_ANY); FAST: the
+struct RasterArgs {
+    const JobDev *jobs;
+    const DrawDev *draws;
+    const PrimRec *prims;
+    const RasterPrim *rprims;
+    const uint32_t *rows, *tcnt, *toff, *mask;
+    const uint2 *segs, *list;  // the tiles' triangle lists
+    const uint32_t *listovf;   // nonzero: they did not fit, walk the masks
+    const uint32_t *items, *first, *nfirst;  // the group's part of the work list
+    uint32_t *queue;
+    StatsDev *stats;
+    uint32_t nj, ntiles;  // ntiles: the group's
+};
+
+namespace rfr {
+
+// One work item (a tile, or the row slice `slice` >= 1 of one) of job J.
+// KIND: the shader kind of every draw of the job, or RF_K_ANY; FAST: the
 // default context (depth test Less, colour and depth writes) on a target
 // with depth.
 template <int TW, int KIND, bool FAST>
-__global__ void __launch_bounds__(RF_RASTER_MAX_THREADS, 2)
-k_raster(const JobDev *__restrict__ jobs, uint32_t nj, const DrawDev *__restrict__ draws,
-         const PrimRec *__restrict__ prims, const RasterPrim *__restrict__ rprims,
-         const uint32_t *__restrict__ rows, const uint32_t *__restrict__ tcnt,
-         const uint32_t *__restrict__ toff, const uint32_t *__restrict__ mask,
-         uint32_t ntiles_total, const uint32_t *__restrict__ items, const uint32_t *__restrict__ nitems_dev,
-         uint32_t *__restrict__ tile_queue, StatsDev *__restrict__ stats) {
+__device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J, uint32_t ji, uint32_t tile,
+                                            uint32_t slice, uint32_t *smem, uint32_t lane) {
+    constexpr uint32_t NONE = 0xFFFFFFFFu, FULL = 0xFFFFFFFFu;
+    using G = Region<TW, KIND>;
+    constexpr int NC = G::NC, NP = G::NP;
+    constexpr uint32_t WORDS = raster_warp_words<TW, KIND>();
+    uint32_t *scol = smem;
+    float *sdep = reinterpret_cast<float *>(scol + TW * RF_TILE_H);
+    uint32_t *stg = scol + 2 * TW * RF_TILE_H;  // the work region
+    uint32_t *cand = stg;
+    uint4 *tab = reinterpret_cast<uint4 *>(stg + RF_CAND_WORDS);
+    float *tab_dv = reinterpret_cast<float *>(tab + 32);  // [entry][half][component]
+    uint32_t *tab_draw = reinterpret_cast<uint32_t *>(tab_dv + 2u * RF_NC * 32u);
+    float *tab_z = reinterpret_cast<float *>(tab_draw + 32);
+    uint32_t *row_entry = tab_draw + 64;  // entry | half << 5 | kind << 8
+    uint32_t *segq = row_entry + RF_TILE_H;
+    uint32_t *rslots = segq + G::QUEUE;
+    const uint32_t lt = tile - J.tile_base;
+    const uint32_t tyi = lt / J.tiles_x, txi = lt - tyi * J.tiles_x;
+    TileCtx T;
+    T.scol = scol;
+    T.sdep = sdep;
+    T.smin = reinterpret_cast<float *>(scol + WORDS - ((uint32_t)TW / RF_SEG) * RF_TILE_H);
+    T.row = lane;
+    T.tx0 = txi * TW;
+    T.tx1 = min(T.tx0 + (uint32_t)TW, J.w);
+    T.tw = TW;
+    const uint32_t ty0 = tyi * RF_TILE_H;
+    T.y = ty0 + lane;
+    constexpr uint32_t SLICE_H = RF_TILE_H / RF_SPLIT_K;
+    T.row_ok = T.y < J.h && (slice == 0 || lane / SLICE_H == slice - 1u);
+    T.has_depth = J.depth != nullptr;
+    T.depth_test = J.depth_test;
+    T.color_write = J.color_write != 0;
+    T.depth_write = J.depth_write != 0;
+    T.fmt = pack_selector(J.pixfmt);
+    T.rfmt = rgb_selector(T.fmt);
+    T.frags_o = 0;
+    const uint32_t ncols = T.tx1 - T.tx0;
+    const size_t row_off = (size_t)T.y * J.w + T.tx0;
+    const uint32_t rows_ok = __ballot_sync(FULL, T.row_ok);
+    // Coalesced 16-byte row transfers (tile_rows_coalesced) when the
+    // tile's rows hold its full width and start 16-byte aligned.
+    const bool vec = ((J.w | T.tx0) & 3u) == 0u && ncols == (uint32_t)TW &&
+                     (((uintptr_t)J.color | (uintptr_t)J.depth) & 15u) == 0u;
+    uint32_t *gcol = J.color + (size_t)ty0 * J.w + T.tx0;
+    uint32_t *gdep = reinterpret_cast<uint32_t *>(J.depth) + (size_t)ty0 * J.w + T.tx0;
+    auto load_tile = [&]() {
+        const bool cc = J.clear_flags & 1u, cd = (J.clear_flags & 2u) != 0u;
+        if (vec) {
+            if (cc) {
+                for (uint32_t x = 0; x < (uint32_t)TW; ++x) scol[x * RF_TILE_H + lane] = J.clear_px;
+            } else {
+                tile_rows_coalesced<TW, true>(scol, stg, gcol, J.w, rows_ok, lane);
+            }
+            if (T.has_depth) {
+                if (cd) {
+                    for (uint32_t x = 0; x < (uint32_t)TW; ++x) sdep[x * RF_TILE_H + lane] = J.clear_z;
+                } else {
+                    tile_rows_coalesced<TW, true>(reinterpret_cast<uint32_t *>(sdep), stg, gdep, J.w, rows_ok, lane);
+                }
+            }
+        } else {
+            for (uint32_t x = 0; x < (uint32_t)TW; ++x) {
+                const uint32_t i = x * RF_TILE_H + lane;
+                const bool in = T.row_ok && x < ncols;
+                scol[i] = cc ? J.clear_px : (in ? J.color[row_off + x] : 0u);
+                if (T.has_depth) sdep[i] = cd ? J.clear_z : (in ? J.depth[row_off + x] : 0.0f);
+            }
+        }
+    };
+    // FAST: the tile's least current depth (a lower bound of every pixel
+    // a span may write), for skipping whole triangles (RasterPrim::zmax).
+    // Columns past the target's edge hold +inf, so they bound nothing
+    // (they are never written back).
+    float tzmin = 0.0f;
+    // The target rows of this item: the tile's, or its slice's.
+    const uint32_t ys = slice ? ty0 + (slice - 1u) * SLICE_H : ty0;
+    const uint32_t ye = min(slice ? ys + SLICE_H : ty0 + RF_TILE_H, J.h);
+    const uint32_t below = (1u << lane) - 1u, upto = below | (1u << lane);
+    constexpr int U_SEG = KIND == RF_K_ANY ? 1 : KIND == RF_K_GOURAUD_SRGB || !FAST ? 2 : 4;
+    constexpr int U_PACK = KIND == RF_K_ANY ? 1 : 2;
+    constexpr bool PAINTED = KIND != RF_K_GOURAUD && KIND != RF_K_GOURAUD_SRGB;  // shading reads the draw
+
+    // The item at row `row` of table entry ki whose record is in this lane's
+    // part rs of a slot: its span [a, b) in the tile, and the varyings it
+    // starts with.  False when it has no pixels here.
+    auto enter = [&](uint32_t ki, uint32_t row, uint32_t *rs, float2 *v, float2 *dv, uint32_t &a, uint32_t &b,
+                     uint32_t &half, uint32_t &kind) -> bool {
+        const uint32_t w0 = rs[0];
+        const uint32_t xs = w0 & 0xFFFFu, xe = w0 >> 16;
+        a = xs > T.tx0 ? xs : T.tx0;
+        b = xe < T.tx1 ? xe : T.tx1;
+        if (a >= b) return false;
+        const uint4 e = tab[ki];
+        if constexpr (KIND == RF_K_ANY) kind = e.z >> 16;
+        half = row < ((e.z >> 8) & 0xFFu) ? 0u : 1u;
+        const float *dvdx = tab_dv + (ki * 2u + half) * RF_NC;
+        const uint32_t nc = KIND == RF_K_ANY ? kind_nc(kind) : (uint32_t)NC;
+        item_load<KIND>(T, dvdx, rs, nc, xs, a, v, dv);
+        return true;
+    };
+    // The record of row r of the entry's in-tile rows into this lane's part of a slot.
+    auto stage = [&](uint32_t *slot, bool have, const uint4 &e, uint32_t r) {
+        const uint32_t kd = e.z >> 16;
+        const uint32_t stride = KIND == RF_K_ANY ? row_words((int)kind_nc(kd)) : row_words(NC);
+        stage_row<KIND>(slot, lane, have, kd, A.rows + e.x + (size_t)r * stride);
+        commit_stage();
+    };
+
+    // The tile's list, a batch of 32 entries at a time (the next one already
+    // loaded: ent, n_ent of them): the entries the tile does not hide go on
+    // to the ring as output triangles.
+    const bool walk = *A.listovf != 0u;
+    PrimIter it;  // (only when the masks are walked)
+    const uint2 *segs = A.segs + J.seg_base + (size_t)lt * J.nseg;
+    uint32_t sb = 0, slive = 0, ent_off = 0, ent_left = 0, n_ent = 0;
+    uint2 seg = make_uint2(0u, 0u), ent = make_uint2(0u, 0u);
+    auto next_entries = [&]() {
+        if (walk) {
+            ent = mask_batch(&it, A.toff, A.tcnt, lane, &n_ent);
+            return;
+        }
+        n_ent = 0;
+        if (ent_left == 0u) {
+            while (slive == 0u) {
+                if (sb >= J.nseg) return;
+                seg = sb + lane < J.nseg ? segs[sb + lane] : make_uint2(0u, 0u);
+                slive = __ballot_sync(FULL, seg.y != 0u);
+                sb += 32u;
+            }
+            const uint32_t k = __ffs(slive) - 1u;
+            slive &= slive - 1u;
+            ent_off = __shfl_sync(FULL, seg.x, k);
+            ent_left = __shfl_sync(FULL, seg.y, k);
+        }
+        n_ent = min(ent_left, 32u);
+        ent = lane < n_ent ? __ldg(A.list + ent_off + lane) : make_uint2(0u, 0u);
+        ent_off += n_ent;
+        ent_left -= n_ent;
+    };
+    if (walk) {
+        it.tmask = A.mask + J.mask_base + (size_t)lt * J.mask_words;
+        it.tsum = A.mask + J.sum_base + (size_t)lt * J.sum_words;
+        it.nsum = J.sum_words;
+        it.tri_base = J.tri_base;
+        it.lane = lane;
+        it.init();
+    }
+    // `todo`: the lanes of the 32 output triangles taken whose triangle has
+    // scanlines in the tile and is not on the table yet, `slows` those
+    // without row records.
+    uint32_t todo = 0, slows = 0;
+    uint32_t p = NONE, nr = 0, a0hs = 0, rb = 0, hdraw = 0;
+    float zmax = 0.0f;
+    uint32_t chead = 0, ncand = 0;  // the ring
+    uint32_t nt = 0;                // triangles on the table
+    bool done = false;
+    next_entries();
+    const bool any = n_ent != 0u;
+    const bool loaded = any || J.clear_flags != 0u;  // (the tile comes in to be drawn into or cleared)
+    if (loaded) {
+        load_tile();
+        if constexpr (FAST) {
+            for (uint32_t x = ncols; x < (uint32_t)TW; ++x) sdep[x * RF_TILE_H + lane] = __int_as_float(0x7F800000);
+            for (uint32_t sg = 0; sg < (uint32_t)TW / RF_SEG; ++sg) seg_refresh(T, sg);
+            tzmin = tile_depth_min<TW>(T);
+        }
+        __syncwarp();
+    }
+    while (any) {
+        if (!todo && !done) {
+            while (ncand < 32u && n_ent) {
+                // FAST: a triangle whose depth bound is at most the tile's
+                // least depth passes no fragment (the tile's depths only
+                // rise; a NaN on either side never skips).
+                const bool keep = lane < n_ent && !(FAST && __uint_as_float(ent.y) <= tzmin);
+                const uint32_t q = ent.x & RF_ENT_MASK, fan = ent.x >> RF_ENT_SHIFT;  // outputs q .. q + fan
+                const uint32_t km = __ballot_sync(FULL, keep);
+                uint32_t at = chead + ncand + __popc(km & below);
+                if (__any_sync(FULL, keep && fan)) {  // fans of clipped triangles among them
+                    uint32_t more = keep ? fan : 0u;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(FULL, more, o);
+                        if (lane >= (uint32_t)o) more += y;
+                    }
+                    ncand += __shfl_sync(FULL, more, 31);
+                    if (keep) {
+                        at += more - fan;
+                        for (uint32_t i = 1; i <= fan; ++i) cand[(at + i) & (RF_CAND_WORDS - 1u)] = q + i;
+                    }
+                }
+                if (keep) cand[at & (RF_CAND_WORDS - 1u)] = q;
+                ncand += __popc(km);
+                next_entries();
+            }
+            __syncwarp();
+            done = ncand == 0u;
+            p = lane < ncand ? cand[(chead + lane) & (RF_CAND_WORDS - 1u)] : NONE;
+            const uint32_t took = min(ncand, 32u);
+            chead += took;
+            ncand -= took;
+            uint4 h0 = make_uint4(0u, 0u, 0u, 0u), h1 = h0, h2 = h0;
+            if (p != NONE) {
+                const uint4 *h = reinterpret_cast<const uint4 *>(A.rprims + p);
+                h0 = __ldg(h);
+                h1 = __ldg(h + 1);
+                h2 = __ldg(h + 2);
+            }
+            nr = 0;
+            bool slow = false;
+            if (p != NONE) {
+                const bool live = (h0.y & RF_RP_LIVE) != 0u, recs = (h0.y & RF_RP_ROWS) != 0u;
+                slow = live && !recs;
+                zmax = __uint_as_float(h2.y);
+                hdraw = h0.x;
+                if (live && recs && !(FAST && zmax <= tzmin)) {
+                    const uint32_t y0 = h1.y, c0 = h1.z, y1 = h1.w, c1 = h2.x;
+                    const uint32_t l0 = max(y0, ys), e0 = min(y0 + c0, ye);
+                    const uint32_t l1 = max(y1, ys), e1 = min(y1 + c1, ye);
+                    const uint32_t n0 = c0 && l0 < e0 ? e0 - l0 : 0u, n1 = c1 && l1 < e1 ? e1 - l1 : 0u;
+                    nr = n0 + n1;  // (the halves meet: y1 = y0 + c0 where both have rows)
+                    const uint32_t a0 = (n0 ? l0 : l1) - ty0;
+                    a0hs = a0 | (a0 + n0) << 8 | h0.z << 16;
+                    rb = h0.w + (n0 ? l0 - y0 : c0 + (l1 - y1)) * h1.x;
+                }
+            }
+            slows = __ballot_sync(FULL, slow);
+            todo = __ballot_sync(FULL, nr != 0u) | slows;
+        }
+        // Onto the table, up to the first triangle without records or until
+        // it is full.
+        {
+            const uint32_t stop = slows & todo ? (uint32_t)__ffs(slows & todo) - 1u : 32u;
+            const uint32_t m = stop < 32u ? todo & ((1u << stop) - 1u) : todo;
+            const uint32_t at = nt + __popc(m & below);
+            const bool put = ((m >> lane) & 1u) && at < 32u;
+            if (put) {
+                tab[at] = make_uint4(rb, nr, a0hs, p);
+                tab_draw[at] = hdraw;
+                tab_z[at] = zmax;
+#pragma unroll
+                for (uint32_t c = 0; c < 2u * RF_NC / 4u; ++c) {
+                    const uint32_t sa = (uint32_t)__cvta_generic_to_shared(tab_dv + at * (2u * RF_NC) + 4u * c);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa),
+                                 "l"(&A.rprims[p].dvdx[0][0] + 4u * c)
+                                 : "memory");
+                }
+            }
+            const uint32_t took = __ballot_sync(FULL, put);
+            nt += __popc(took);
+            todo &= ~took;
+        }
+        const uint32_t slow_now = todo && ((slows >> (__ffs(todo) - 1)) & 1u) ? todo & (0u - todo) : 0u;
+        if (!todo && !done) continue;  // the table has room left
+
+        // The table's triangles, scanline by scanline.  (Their steps arrive
+        // with the first row records.)
+        __syncwarp();
+        if (nt) {
+            const uint4 te = lane < nt ? tab[lane] : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t n = te.y;
+            uint32_t ex = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, ex, o);
+                if (lane >= (uint32_t)o) ex += y;
+            }
+            const uint32_t total = __shfl_sync(FULL, ex, 31);
+            ex -= n;
+            float2 v[NP], dv[NP];
+            uint32_t sl = 0;
+            if (total >= RF_ROW_MEAN * nt) {
+                // By row: lane r takes row r's triangles in order, one a
+                // round, passing over those its row hides.  A round's spans
+                // never meet; cut into segments of RF_SEG pixels, the
+                // visible ones queue up and are drawn on full warps.
+                uint32_t rm = n ? (n < 32u ? (1u << n) - 1u : FULL) << (te.z & 0xFFu) : 0u;  // this triangle's rows
+#pragma unroll
+                for (uint32_t sft = 16, m = 0x0000FFFFu; sft; sft >>= 1, m ^= m << sft) {
+                    const uint32_t o = __shfl_xor_sync(FULL, rm, sft);
+                    rm = lane & sft ? (rm & ~m) | ((o >> sft) & m) : (rm & m) | ((o << sft) & ~m);
+                }  // now the triangles of this lane's row
+                uint32_t kin = 0;
+                bool haven = false;
+                auto stage_next = [&]() {
+                    haven = false;
+                    if (rm) {
+                        float rmin = -__int_as_float(0x7F800000);
+                        if constexpr (FAST) {
+                            rmin = T.smin[lane];
+#pragma unroll
+                            for (uint32_t sg = 1; sg < (uint32_t)TW / RF_SEG; ++sg)
+                                rmin = fminf(rmin, T.smin[sg * RF_TILE_H + lane]);
+                        }
+                        do {  // the next one this row does not hide
+                            kin = __ffs(rm) - 1u;
+                            rm &= rm - 1u;
+                            haven = !(FAST && tab_z[kin] <= rmin);
+                        } while (!haven && rm);
+                    }
+                    const uint4 e = tab[kin];
+                    stage(rslots + sl * G::SLOT, haven, e, lane - (e.z & 0xFFu));
+                };
+                stage_next();
+                T.row = lane;
+                while (__any_sync(FULL, haven)) {
+                    const uint32_t ki = kin;
+                    bool act = haven;
+                    uint32_t *rs = rslots + sl * G::SLOT + lane;
+                    sl ^= 1u;
+                    stage_next();
+                    wait_staged_but<1>();
+                    uint32_t kind = (uint32_t)KIND, half = 0, a = 0, b = 0;
+                    act = act && enter(ki, lane, rs, v, dv, a, b, half, kind);
+                    uint32_t x = a - T.tx0;
+                    const uint32_t xe = b - T.tx0;
+                    if (act) row_entry[lane] = ki | half << 5 | kind << 8;
+                    uint32_t nq = 0;
+                    while (__any_sync(FULL, act)) {
+                        const uint32_t sg = x / RF_SEG, xn = min(xe, (sg + 1u) * RF_SEG), len = xn - x;
+                        bool vis = act;
+                        if constexpr (FAST)
+                            vis = act && !(depth_bound(v[0].x, dv[0].x, len) <= T.smin[sg * RF_TILE_H + lane]);
+                        const uint32_t vm = __ballot_sync(FULL, vis);
+                        if (vis) {
+                            uint32_t *q = segq + nq + __popc(vm & below);
+                            q[0] = (x * RF_TILE_H + lane) | len << 16;
+#pragma unroll
+                            for (int c = 0; c < NC; ++c) q[(1 + c) * G::QN] = f2u(c & 1 ? v[c / 2].y : v[c / 2].x);
+                        }
+                        nq += __popc(vm);
+                        x = xn;
+                        act = act && x < xe;
+                        if (TW > (int)RF_SEG && act) {
+#pragma unroll
+                            for (uint32_t i = 0; i < RF_SEG; ++i)
+                                if (i < len) {
+#pragma unroll
+                                    for (int c = 0; c < NP; ++c) v[c] = __fadd2_rn(v[c], dv[c]);
+                                }
+                        }
+                    }
+                    __syncwarp();
+#pragma unroll 1
+                    for (uint32_t j = lane; j < nq; j += 32u) {
+                        const uint32_t w = segq[j];
+                        uint32_t idx = w & 0xFFFFu;
+                        const uint32_t first = idx, end = idx + (w >> 16) * RF_TILE_H, row = idx & 31u;
+                        const uint32_t re0 = row_entry[row], re = (re0 & 31u) * 2u + ((re0 >> 5) & 1u);
+                        float2 sv[NP], sd[NP];
+#pragma unroll
+                        for (int c = 0; c < NP; ++c) {
+                            sv[c].x = u2f(segq[j + (1 + 2 * c) * G::QN]);
+                            sv[c].y = 2 * c + 1 < NC ? u2f(segq[j + (2 + 2 * c) * G::QN]) : 0.0f;
+                            sd[c] = reinterpret_cast<const float2 *>(tab_dv + re * RF_NC)[c];
+                        }
+                        const Paint paint(A.draws[PAINTED ? tab_draw[re0 & 31u] : 0u]);
+                        uint32_t nout = 0;
+                        do nout += px_group<KIND, FAST, U_SEG>(T, paint, KIND == RF_K_ANY ? re0 >> 8 : (uint32_t)KIND,
+                                                               sv, sd, idx, end);
+                        while (idx < end);
+                        T.frags_o += nout;
+                        if constexpr (FAST) {
+                            T.row = row;
+                            if (nout) seg_refresh(T, first / (RF_SEG * RF_TILE_H));
+                        }
+                    }
+                    __syncwarp();
+                    T.row = lane;
+                }
+            } else {
+                // Packed: 32 scanlines a pass, in submission order, one a
+                // lane.  Spans of one row that meet are drawn in that order:
+                // each waits for the lower lanes it overlaps.
+                if (n) tab[lane].y = ex;
+                __syncwarp();
+                uint32_t kin = 0, rown = 0;
+                auto stage_pass = [&](uint32_t base) {
+                    // the last triangle that starts at or before the item, and its row there
+                    const uint32_t starts = __reduce_or_sync(FULL, n && ex - base < 32u ? 1u << (ex - base) : 0u);
+                    const uint32_t before = __popc(__ballot_sync(FULL, n && ex < base));
+                    const bool have = base + lane < total;
+                    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+                    if (have) {
+                        kin = before + __popc(starts & upto) - 1u;
+                        e = tab[kin];
+                        rown = (e.z & 0xFFu) + (base + lane - e.y);
+                    }
+                    stage(rslots + sl * G::SLOT, have, e, base + lane - e.y);
+                };
+                stage_pass(0u);
+#pragma unroll 1
+                for (uint32_t base = 0; base < total; base += 32u) {
+                    const uint32_t ki = kin, row = rown;
+                    uint32_t *rs = rslots + sl * G::SLOT + lane;
+                    sl ^= 1u;
+                    stage_pass(base + 32u);
+                    wait_staged_but<1>();
+                    uint32_t kind = (uint32_t)KIND, half = 0, a = 0, b = 0;
+                    T.row = row;
+                    bool act = base + lane < total && enter(ki, row, rs, v, dv, a, b, half, kind);
+                    if constexpr (FAST) act = act && !span_hidden(T, v[0].x, dv[0].x, a, b);
+                    uint32_t pend = __ballot_sync(FULL, act);
+                    uint32_t lower = __match_any_sync(FULL, act ? row : 32u + lane) & below;
+                    uint32_t wait = 0;
+                    while (__any_sync(FULL, lower != 0u)) {
+                        const uint32_t src = lower ? (uint32_t)__ffs(lower) - 1u : lane;
+                        const uint32_t oa = __shfl_sync(FULL, a, src), ob = __shfl_sync(FULL, b, src);
+                        if (lower && oa < b && a < ob) wait |= 1u << src;
+                        lower &= lower - 1u;
+                    }
+                    const Paint paint(A.draws[PAINTED && act ? tab_draw[ki] : 0u]);
+                    while (pend) {
+                        const bool go = ((pend >> lane) & 1u) && (wait & pend) == 0u;
+                        if (go) {
+                            uint32_t idx = (a - T.tx0) * RF_TILE_H + row;
+                            const uint32_t end = (b - T.tx0) * RF_TILE_H + row;
+                            uint32_t nout = 0;
+                            do nout += px_group<KIND, FAST, U_PACK>(T, paint, kind, v, dv, idx, end);
+                            while (idx < end);
+                            T.frags_o += nout;
+                            if constexpr (FAST) {
+                                if (nout)
+                                    for (uint32_t sg = (a - T.tx0) / RF_SEG; sg <= (b - 1u - T.tx0) / RF_SEG; ++sg)
+                                        seg_refresh(T, sg);
+                            }
+                        }
+                        pend &= ~__ballot_sync(FULL, go);
+                        __syncwarp();  // (the depths written before the next round reads them)
+                    }
+                }
+                T.row = lane;
+            }
+            __syncwarp();
+            nt = 0;
+            if constexpr (FAST) tzmin = tile_depth_min<TW>(T);
+        }
+        if (slow_now) {
+            const uint32_t l = __ffs(slow_now) - 1u;
+            const uint32_t ps = __shfl_sync(FULL, p, l), ds = __shfl_sync(FULL, hdraw, l);
+            T.frags_o += raster_prim_slow<KIND, FAST>(T, (uint32_t)A.draws[ds].shader, A.draws + ds, A.prims + ps);
+            __syncwarp();
+            todo &= ~slow_now;
+        }
+        if (done) break;
+    }
+    if (loaded) {
+        if (vec) {
+            if constexpr (TW % 32 == 0) {
+                tile_store_bulk<TW>(scol, reinterpret_cast<uint32_t *>(sdep), T.has_depth, stg, gcol, gdep, J.w,
+                                    rows_ok, lane);
+            } else {
+                tile_rows_coalesced<TW, false>(scol, stg, gcol, J.w, rows_ok, lane);
+                if (T.has_depth)
+                    tile_rows_coalesced<TW, false>(reinterpret_cast<uint32_t *>(sdep), stg, gdep, J.w, rows_ok, lane);
+            }
+        } else if (T.row_ok) {
+            for (uint32_t x = 0; x < ncols; ++x) {
+                const uint32_t i = x * RF_TILE_H + lane;
+                J.color[row_off + x] = scol[i];
+                if (T.has_depth) J.depth[row_off + x] = sdep[i];
+            }
+        }
+    }
+    __syncwarp();
+    warp_add_u64(&A.stats[ji].frags_o, T.frags_o, true);
+}
+
+}  // namespace rfr
+
+// Persistent warps over the work list of one raster group.
+template <int TW, int KIND, bool FAST>
+__global__ void __launch_bounds__(RF_RASTER_MAX_THREADS, 2) k_raster(const __grid_constant__ RasterArgs A) {
     using namespace rfr;
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr uint32_t WARP_WORDS = raster_warp_words<TW, KIND>();
     static_assert(WARP_WORDS % 4u == 0u && (2u * TW * RF_TILE_H) % 4u == 0u,
                   "each warp's area and its staging start 16-byte aligned (bulk copies)");
-    constexpr uint32_t RW = row_words(PreNC<KIND>::NC) * RF_TILE_H;  // words per row slot
-    uint32_t *scol = smem + warp * WARP_WORDS;
-    float *sdep = reinterpret_cast<float *>(scol + TW * RF_TILE_H);
-    RasterPrim *stage = reinterpret_cast<RasterPrim *>(scol + 2 * TW * RF_TILE_H);
-    uint32_t *rslots = scol + 2 * TW * RF_TILE_H + Pipe<TW>::HS * (sizeof(RasterPrim) / 4);
-    uint32_t *stg = scol + 2 * TW * RF_TILE_H;  // tile staging (the rings, when idle)
-    float *smin = reinterpret_cast<float *>(scol + WARP_WORDS - ((uint32_t)TW / RF_SEG) * RF_TILE_H);
     // Queue position q: the heavy tiles and crowded-tile slices first
-    // (items[ntiles + q]), then every other tile in index order.
-    const uint32_t nfirst = *nitems_dev;
-    const uint32_t nitems = ntiles_total + nfirst;
+    // (first[q]), then every other tile in index order.
+    const uint32_t nfirst = *A.nfirst;
+    const uint32_t nitems = A.ntiles + nfirst;
     for (;;) {
         uint32_t item = 0;
         if (lane == 0) {
             do {
-                const uint32_t pos = atomicAdd(tile_queue, 1u);
-                item = pos >= nitems ? 0xFFFFFFFFu
-                                     : items[pos < nfirst ? ntiles_total + pos : pos - nfirst];
+                const uint32_t pos = atomicAdd(A.queue, 1u);
+                item = pos >= nitems ? 0xFFFFFFFFu : (pos < nfirst ? A.first[pos] : A.items[pos - nfirst]);
             } while (item == RF_ITEM_SKIP);
         }
         item = __shfl_sync(0xFFFFFFFFu, item, 0);
         if (item == 0xFFFFFFFFu) break;
         const uint32_t tile = item >> RF_ITEM_SHIFT, slice = item & ((1u << RF_ITEM_SHIFT) - 1u);  // 0: the whole tile
-        if (tile >= ntiles_total) break;
         if constexpr (TW % 32 == 0) bulk_store_drain();  // (the last tile's write-back)
-        const uint32_t ji = upper_index(nj, tile, [&](uint32_t i) { return jobs[i].tile_base; });
-        const JobDev &J = jobs[ji];
-        const uint32_t lt = tile - J.tile_base;
-        const uint32_t tyi = lt / J.tiles_x, txi = lt - tyi * J.tiles_x;
-        TileCtx T;
-        T.scol = scol;
-        T.sdep = sdep;
-        T.smin = smin;
-        T.lane = lane;
-        T.tx0 = txi * TW;
-        T.tx1 = min(T.tx0 + (uint32_t)TW, J.w);
-        T.tw = TW;
-        const uint32_t ty0 = tyi * RF_TILE_H;
-        T.y = ty0 + lane;
-        constexpr uint32_t SLICE_H = RF_TILE_H / RF_SPLIT_K;
-        T.row_ok = T.y < J.h && (slice == 0 || lane / SLICE_H == slice - 1u);
-        T.has_depth = J.depth != nullptr;
-        T.depth_test = J.depth_test;
-        T.color_write = J.color_write != 0;
-        T.depth_write = J.depth_write != 0;
-        T.fmt = pack_selector(J.pixfmt);
-        T.rfmt = rgb_selector(T.fmt);
-        T.frags_o = 0;
-        const uint32_t ncols = T.tx1 - T.tx0;
-        const size_t row_off = (size_t)T.y * J.w + T.tx0;
-        const uint32_t rows_ok = __ballot_sync(0xFFFFFFFFu, T.row_ok);
-        // Coalesced 16-byte row transfers (tile_rows_coalesced) when the
-        // tile's rows hold its full width and start 16-byte aligned.
-        const bool vec = ((J.w | T.tx0) & 3u) == 0u && ncols == (uint32_t)TW &&
-                         (((uintptr_t)J.color | (uintptr_t)J.depth) & 15u) == 0u;
-        uint32_t *gcol = J.color + (size_t)ty0 * J.w + T.tx0;
-        uint32_t *gdep = reinterpret_cast<uint32_t *>(J.depth) + (size_t)ty0 * J.w + T.tx0;
-        bool loaded = false;
-        auto load_tile = [&]() {
-            const bool cc = J.clear_flags & 1u, cd = (J.clear_flags & 2u) != 0u;
-            if (vec) {
-                if (cc) {
-                    for (uint32_t x = 0; x < (uint32_t)TW; ++x) scol[x * RF_TILE_H + lane] = J.clear_px;
-                } else {
-                    tile_rows_coalesced<TW, true>(scol, stg, gcol, J.w, rows_ok, lane);
-                }
-                if (T.has_depth) {
-                    if (cd) {
-                        for (uint32_t x = 0; x < (uint32_t)TW; ++x) sdep[x * RF_TILE_H + lane] = J.clear_z;
-                    } else {
-                        tile_rows_coalesced<TW, true>(reinterpret_cast<uint32_t *>(sdep), stg, gdep, J.w,
-                                                      rows_ok, lane);
-                    }
-                }
-            } else {
-                for (uint32_t x = 0; x < (uint32_t)TW; ++x) {
-                    const uint32_t i = x * RF_TILE_H + lane;
-                    const bool in = T.row_ok && x < ncols;
-                    scol[i] = cc ? J.clear_px : (in ? J.color[row_off + x] : 0u);
-                    if (T.has_depth) sdep[i] = cd ? J.clear_z : (in ? J.depth[row_off + x] : 0.0f);
-                }
-            }
-        };
-        // FAST: the tile's least current depth (a lower bound of every pixel
-        // a span may write), for skipping whole triangles (RasterPrim::zmax).
-        // Columns past the target's edge hold +inf, so they bound nothing
-        // (they are never written back).
-        float tzmin = 0.0f;
-        auto load_tile_and_bounds = [&]() {
-            load_tile();
-            if constexpr (FAST) {
-                for (uint32_t x = ncols; x < (uint32_t)TW; ++x) sdep[x * RF_TILE_H + lane] = __int_as_float(0x7F800000);
-                for (uint32_t sg = 0; sg < (uint32_t)TW / RF_SEG; ++sg) seg_refresh(T, sg);
-                tzmin = tile_depth_min<TW>(T);
-            }
-        };
-        PrimIter it;
-        it.tmask = mask + J.mask_base + (size_t)lt * J.mask_words;
-        it.tsum = mask + J.sum_base + (size_t)lt * J.sum_words;
-        it.toff = toff;
-        it.tcnt = tcnt;
-        it.nsum = J.sum_words;
-        it.rprims = rprims;
-        it.slo = slice ? tyi * RF_TILE_H + (slice - 1u) * SLICE_H : 0u;
-        it.shi = slice ? it.slo + SLICE_H : 0u;
-        it.tri_base = J.tri_base;
-        it.lane = lane;
-        it.init();
-        // Software pipeline over the tile's triangles t0, t1, ...: iteration
-        // i rasterises t_i while the headers of t_{i+1} .. t_{i+HA} and the
-        // row records of t_{i+1} .. t_{i+RA} are in flight (cp.async into
-        // the shared-memory rings).  Iteration i issues the header of
-        // t_{i+HA} and the rows of t_{i+RA} as one commit group G_i, then
-        // waits for all but the newest RA groups: the rows of t_i (G_{i-RA})
-        // and every header up to t_{i+HA-RA} are then complete.  The rows of
-        // t_{i+RA} need its header, from G_{i+RA-HA}, complete by the wait of
-        // iteration i-1 since HA >= 2 RA + 1.
-        constexpr uint32_t NONE = 0xFFFFFFFFu;
-        constexpr int HA = Pipe<TW>::HA, RA = Pipe<TW>::RA;
-        constexpr uint32_t HS = Pipe<TW>::HS, RS = Pipe<TW>::RS;
-        static_assert(RA >= 1 && HA >= 2 * RA + 1 && HS == (uint32_t)HA + 1u, "pipeline shape");
-        uint32_t q[HA + 1];  // t_i .. t_{i+HA}
-        q[0] = it.next();
-        if (q[0] != NONE) {
-            load_tile_and_bounds();
-            loaded = true;
-            if constexpr (FAST) it.zcut = tzmin;
-#pragma unroll
-            for (int k = 1; k <= HA; ++k) q[k] = q[k - 1] != NONE ? it.next() : NONE;
-            // Headers of t_0 .. t_{HA-1} (t_{HA} comes with G_0), waited
-            // for at once before the first row records are staged.
-#pragma unroll
-            for (int k = 0; k < HA; ++k)
-                if (q[k] != NONE) stage_prim(stage + k, rprims + q[k], lane);
-            commit_stage();
-            wait_staged_but<0>();
-#pragma unroll
-            for (int k = 0; k < RA; ++k) {
-                stage_rows<KIND>(T, rslots + k * RW, q[k] != NONE && !hidden<FAST>(stage + k, tzmin), stage + k, rows);
-                commit_stage();
-            }
-            uint32_t r = 0;  // row slot of t_i (mod RA+1)
-            uint32_t h = 0;  // header slot of t_i (mod HA+1)
-            uint32_t visits = 0;  // triangles rasterised (FAST: tzmin refreshed every 8)
-            for (;;) {
-                const uint32_t hn = h == 0 ? HS - 1 : h - 1;                // t_{i+HA}: t_{i-1}'s old slot
-                const uint32_t hr = h + RA >= HS ? h + RA - HS : h + RA;    // t_{i+RA}
-                const uint32_t rr = r == 0 ? RS - 1 : r - 1;                // t_{i+RA}: t_{i-1}'s old slot
-                if (q[HA] != NONE) stage_prim(stage + hn, rprims + q[HA], lane);
-                // A triangle whose depth bound is at most the tile's least
-                // depth fails the Less test at every pixel: its rows are not
-                // fetched and its visit is skipped (the tile's depths only rise).
-                stage_rows<KIND>(T, rslots + rr * RW, q[RA] != NONE && !hidden<FAST>(stage + hr, tzmin),
-                                 stage + hr, rows);
-                commit_stage();
-                wait_staged_but<RA>();
-                if (!hidden<FAST>(stage + h, tzmin)) {
-                    raster_prim<KIND, FAST>(T, draws, stage + h, prims + q[0], rslots + r * RW);
-                    if constexpr (FAST) {
-                        if ((++visits & 7u) == 0u) it.zcut = tzmin = tile_depth_min<TW>(T);
-                    }
-                }
-                __syncwarp();
-                if (q[1] == NONE) break;
-                const uint32_t qn = q[HA] != NONE ? it.next() : NONE;
-#pragma unroll
-                for (int k = 0; k < HA; ++k) q[k] = q[k + 1];
-                q[HA] = qn;
-                r = r + 1 == RS ? 0 : r + 1;
-                h = h + 1 == HS ? 0 : h + 1;
-            }
-            asm volatile("cp.async.wait_all;\n" ::: "memory");
-            __syncwarp();
-        }
-        if (!loaded && J.clear_flags) {
-            load_tile();
-            loaded = true;
-        }
-        if (loaded) {
-            if (vec) {
-                if constexpr (TW % 32 == 0) {
-                    tile_store_bulk<TW>(scol, reinterpret_cast<uint32_t *>(sdep), T.has_depth, stg, gcol, gdep,
-                                        J.w, rows_ok, lane);
-                } else {
-                    tile_rows_coalesced<TW, false>(scol, stg, gcol, J.w, rows_ok, lane);
-                    if (T.has_depth)
-                        tile_rows_coalesced<TW, false>(reinterpret_cast<uint32_t *>(sdep), stg, gdep, J.w,
-                                                       rows_ok, lane);
-                }
-            } else if (T.row_ok) {
-                for (uint32_t x = 0; x < ncols; ++x) {
-                    const uint32_t i = x * RF_TILE_H + lane;
-                    J.color[row_off + x] = scol[i];
-                    if (T.has_depth) J.depth[row_off + x] = sdep[i];
-                }
-            }
-        }
-        __syncwarp();
-        const uint32_t j0 = __shfl_sync(0xFFFFFFFFu, ji, 0);
-        warp_add_u64(&stats[j0].frags_o, T.frags_o, true);
+        const uint32_t ji = A.jobs[upper_index(A.nj, tile, [&](uint32_t i) { return A.jobs[i].nth_tile; })].nth;
+        raster_tile<TW, KIND, FAST>(A, A.jobs[ji], ji, tile, slice, smem + warp * WARP_WORDS, lane);
     }
     // (shared memory stays allocated until the last write-back has read it)
     if constexpr (TW % 32 == 0) bulk_store_drain();
@@ -1227,12 +1422,7 @@ static cudaError_t opt_in_smem(K kernel, int bytes) {
 }
 
 template <int TW, int KIND, bool FAST>
-static cudaError_t launch_raster_k(const JobDev *jobs, uint32_t nj, const DrawDev *draws,
-                                   const PrimRec *prims, const RasterPrim *rprims,
-                                   const uint32_t *rows, const uint32_t *tcnt,
-                                   const uint32_t *toff, const uint32_t *mask, uint32_t ntiles,
-                                   const uint32_t *items, const uint32_t *nitems, uint32_t *queue,
-                                   StatsDev *stats, uint32_t warps, int nsm, cudaStream_t s) {
+static cudaError_t launch_raster_k(RF_RASTER_PARAMS) {
     // Shared memory per block: at most the 227 KB opt-in limit, so the
     // block takes as many warps as fit (wide tiles of the generic kind).
     constexpr size_t SMEM_MAX = 227 * 1024;
@@ -1249,37 +1439,23 @@ static cudaError_t launch_raster_k(const JobDev *jobs, uint32_t nj, const DrawDe
     const uint32_t need = (ntiles + warps - 1) / warps;  // (a few crowded-tile slices more are shared out)
     if (blocks > need) blocks = need;
     if (blocks == 0) blocks = 1;
-    k_raster<TW, KIND, FAST><<<blocks, warps * 32, smem, s>>>(jobs, nj, draws, prims, rprims, rows,
-                                                             tcnt, toff, mask, ntiles, items, nitems, queue, stats);
+    const RasterArgs A{jobs, draws, prims, rprims, rows, tcnt, toff, mask, segs, list, listovf,
+                       items, first, nfirst, queue, stats, nj, ntiles};
+    k_raster<TW, KIND, FAST><<<blocks, warps * 32, smem, s>>>(A);
     return cudaGetLastError();
 }
 
-// Launcher for one tile width: picks the kernel specialised for the job's
-// shader kind and context (fast = the default context on a depth target;
-// any other context runs the generic kernel).
-template <int TW>
-static cudaError_t launch_raster_for_width(int kind, bool fast, const JobDev *jobs, uint32_t nj,
-                                           const DrawDev *draws, const PrimRec *prims,
-                                           const RasterPrim *rprims, const uint32_t *rows,
-                                           const uint32_t *tcnt, const uint32_t *toff,
-                                           const uint32_t *mask, uint32_t ntiles, const uint32_t *items, const uint32_t *nitems,
-                          uint32_t *queue,
-                                           StatsDev *stats, uint32_t warps, int nsm, cudaStream_t s) {
-    if (!fast)
-        return launch_raster_k<TW, RF_K_ANY, false>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
+// The launcher of one tile width and context: the kernel of the group's
+// shader kind.
+template <int TW, bool FAST>
+static cudaError_t launch_raster_for_width(int kind, RF_RASTER_PARAMS) {
     switch (kind) {
-        case RF_K_FLAT:
-            return launch_raster_k<TW, RF_K_FLAT, true>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        case RF_K_GOURAUD:
-            return launch_raster_k<TW, RF_K_GOURAUD, true>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        case RF_K_TEXTURED:
-            return launch_raster_k<TW, RF_K_TEXTURED, true>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        case RF_K_TEX_GOURAUD:
-            return launch_raster_k<TW, RF_K_TEX_GOURAUD, true>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        case RF_K_GOURAUD_SRGB:
-            return launch_raster_k<TW, RF_K_GOURAUD_SRGB, true>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
-        default:
-            return launch_raster_k<TW, RF_K_ANY, true>(jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, ntiles, items, nitems, queue, stats, warps, nsm, s);
+        case RF_K_FLAT: return launch_raster_k<TW, RF_K_FLAT, FAST>(RF_RASTER_ARGS);
+        case RF_K_GOURAUD: return launch_raster_k<TW, RF_K_GOURAUD, FAST>(RF_RASTER_ARGS);
+        case RF_K_TEXTURED: return launch_raster_k<TW, RF_K_TEXTURED, FAST>(RF_RASTER_ARGS);
+        case RF_K_TEX_GOURAUD: return launch_raster_k<TW, RF_K_TEX_GOURAUD, FAST>(RF_RASTER_ARGS);
+        case RF_K_GOURAUD_SRGB: return launch_raster_k<TW, RF_K_GOURAUD_SRGB, FAST>(RF_RASTER_ARGS);
+        default: return launch_raster_k<TW, RF_K_ANY, FAST>(RF_RASTER_ARGS);
     }
 }
 

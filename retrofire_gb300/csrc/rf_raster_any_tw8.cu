@@ -1,0 +1,9 @@
+// rf_raster_any_tw8.cu — tile rasteriser kernels for 8-pixel-wide tiles, any
+// context.
+#include "rf_raster.cuh"
+
+namespace rfk {
+cudaError_t launch_raster_any_tw8(int kind, RF_RASTER_PARAMS) {
+    return launch_raster_for_width<8, false>(kind, RF_RASTER_ARGS);
+}
+}  // namespace rfk

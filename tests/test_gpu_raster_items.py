@@ -1,0 +1,123 @@
+"""The rasteriser's ways of giving scanlines to lanes, against the oracle bit
+for bit: triangles of few rows (32 scanlines packed to a pass), of about ten
+(the line between the two ways) and of many (a lane per row), spans from one
+pixel to across many tiles, coincident triangles (ties, and scanlines of one
+row that wait for each other), clipped fans among them; the walk over the tile
+masks when the triangle lists do not fit; jobs of every raster group in one
+batch."""
+import numpy as np
+import pytest
+
+import retrofire_gb300 as rf
+from retrofire_gb300 import mat, scenes
+from rfhelp import DrawSpec, assert_parity, gpu_render, oracle_render
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def built():
+    from retrofire_gb300 import build
+    build.build()
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+
+
+NATTR = {rf.FLAT: 0, rf.GOURAUD: 3, rf.TEXTURED: 2, rf.TEX_GOURAUD: 5, rf.GOURAUD_SRGB: 3}
+
+
+def tris(seed, n, w, h, size, kind=rf.GOURAUD, repeat=1, cross=0.0):
+    """n clip-space triangles inside boxes of size = (xmin, xmax, ymin, ymax)
+    px at random places, each repeated; a share crossing the near plane."""
+    rng = np.random.default_rng(seed)
+    x0, x1, y0, y1 = size
+    c = rng.uniform([0, 0], [w, h], (n, 2))
+    e = np.stack([rng.uniform(x0, x1, n), rng.uniform(y0, y1, n)], 1)
+    px = c[:, None, :] + rng.uniform(-0.5, 0.5, (n, 3, 2)) * e[:, None, :]
+    px = np.repeat(px, repeat, 0)
+    n *= repeat
+    wv = rng.uniform(1.0, 3.0, (n, 3))
+    z = rng.uniform(-0.9, 0.9, (n, 3))
+    z[rng.random(n) < cross, 0] = -1.4
+    clip = np.stack([(px[..., 0] / (w / 2.0) - 1.0) * wv, (px[..., 1] / (h / 2.0) - 1.0) * wv, z * wv, wv], -1)
+    verts = np.concatenate([clip, rng.uniform(0.0, 1.0, (n, 3, NATTR[kind]))], -1)
+    verts = verts.reshape(3 * n, -1).astype(np.float32)
+    tex = scenes.noise_texture(64, seed) if kind in (rf.TEXTURED, rf.TEX_GOURAUD) else None
+    return DrawSpec(verts, np.arange(3 * n, dtype=np.uint32).reshape(n, 3), kind, pos_dim=4,
+                    flat_rgba=0xFF336699, tex=tex)
+
+
+SHAPES = {
+    "dots": dict(n=3000, size=(1, 3, 1, 3)),
+    "slivers": dict(n=1500, size=(8, 40, 1, 3)),
+    "ten_rows": dict(n=1200, size=(4, 30, 9, 24)),
+    "tall": dict(n=200, size=(2, 12, 60, 200)),
+    "wide": dict(n=150, size=(300, 900, 20, 80)),
+    "ties": dict(n=60, size=(3, 40, 2, 40), repeat=40),
+    "fans": dict(n=600, size=(5, 80, 5, 80), cross=0.4),
+}
+
+
+@pytest.mark.parametrize("tw", [8, 16, 32, 64])
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_items_match_oracle(shape, tw):
+    w, h = 700, 203
+    kw = dict(SHAPES[shape])
+    n, size = kw.pop("n"), kw.pop("size")
+    for kind, ctx in ((rf.GOURAUD, rf.Context(face_cull=rf.CULL_NONE)),
+                      (rf.TEX_GOURAUD, rf.Context(face_cull=rf.CULL_NONE)),
+                      (rf.TEXTURED, rf.Context(face_cull=rf.CULL_NONE, depth_test=rf.DEPTH_NONE))):
+        d = [tris(len(shape) + tw, n, w, h, size, kind, **kw)]
+        vp = mat.viewport(0, 0, w, h)
+        assert_parity(gpu_render(d, vp, w, h, ctx=ctx, tile=(tw, 4)), oracle_render(d, vp, w, h, ctx=ctx),
+                      what="%s kind %d width %d" % (shape, kind, tw))
+
+
+def test_lists_that_do_not_fit():
+    """More (triangle, tile) pairs than the lists first hold (2^20): the
+    masks are walked, then the lists have grown; same image both times."""
+    w, h = 1024, 512
+    d = [tris(5, 700, w, h, (1500, 2500, 800, 1500))]
+    vp = mat.viewport(0, 0, w, h)
+    ctx = rf.Context(face_cull=rf.CULL_NONE)
+    ref = oracle_render(d, vp, w, h, ctx=ctx)
+    dev = rf.Device()
+    try:
+        for _ in range(3):
+            assert_parity(gpu_render(d, vp, w, h, ctx=ctx, tile=(8, 4), device=dev), ref)
+    finally:
+        dev.close()
+
+
+def test_every_raster_group_in_one_batch():
+    """Jobs of every shader kind, and of mixed kinds, under the default
+    context and another, in an order that interleaves the groups."""
+    dev = rf.Device()
+    w, h = 150, 90
+    vp = mat.viewport(0, 0, w, h)
+    jobs, keep = [], []
+    try:
+        for i in range(18):
+            kinds = [i % 6] if i % 6 < 5 else [rf.FLAT, rf.TEX_GOURAUD, rf.GOURAUD]
+            ctx = rf.Context(face_cull=rf.CULL_NONE, depth_test=(rf.DEPTH_LESS, rf.DEPTH_GREATER)[i // 6 % 2],
+                             depth_clear=float("inf") if i // 6 % 2 == 0 else 0.1)
+            ds = [tris(100 + i + k, 80, w, h, (2, 60, 2, 60), k) for k in kinds]
+            tg = rf.Framebuf(w, h, device=dev)
+            tg.clear(ctx.color_clear, ctx.depth_clear)
+            items = []
+            for d in ds:
+                m = rf.Mesh(d.verts, d.faces, pos_dim=4, device=dev)
+                t = rf.Texture(d.tex, device=dev) if d.tex is not None else None
+                keep += [m] + ([t] if t else [])
+                items.append((m, rf.Shader(d.shader, d.flat_rgba, t), None))
+            keep.append(tg)
+            jobs.append((rf.Scene(tg, items, vp, ctx), ds, ctx, 1 if rf.GOURAUD_SRGB in kinds else 0))
+        stats = rf.render_batch([j[0] for j in jobs], device=dev)
+        for (sc, ds, ctx, tol), st in zip(jobs, stats):
+            col, dep = sc.target.read()
+            assert_parity((col, dep, st), oracle_render(ds, vp, w, h, ctx=ctx), color_tol=tol)
+    finally:
+        for x in keep:
+            x.close()
+        dev.close()
