@@ -93,7 +93,7 @@ struct UploadBuf {
 
 // An instantiated launch sequence and the frame shape it was captured for.
 struct GraphKey {
-    uint64_t v[13 + RF_MAX_GROUPS];
+    uint64_t v[13 + 3 * RF_MAX_GROUPS];
     bool operator==(const GraphKey &o) const { return memcmp(v, o.v, sizeof v) == 0; }
 };
 struct GraphEntry {
@@ -176,7 +176,6 @@ struct rf_ctx {
     DrawDev *hdraws = nullptr;
     size_t ndraws = 0;
     bool any_cull = false;  // a draw asks for object culling
-    int kind = 0;           // the shader kind of every draw, or RF_K_ANY
     std::vector<JobDev> hjobs;
     std::vector<RasterGroup> groups;
     // Frames of several raster groups: the second launches on a side stream,
@@ -471,13 +470,29 @@ void group_jobs(rf_ctx *ctx) {
     for (uint32_t g = 0; g < RF_MAX_GROUPS; ++g)
         if (seen & (1u << g)) {
             dense[g] = (uint32_t)gr.size();
-            gr.push_back(RasterGroup{(int32_t)(g / 2), g % 2 == 0, 0u, 0u});
+            gr.push_back(RasterGroup{(int32_t)(g / 2), g % 2 == 0, 0u, 0u, 0u, 0u, 0u});
         }
     for (JobDev &J : hj) J.group = dense[J.group];
     uint32_t n = 0;
     for (uint32_t g = 0; g < gr.size(); ++g)
         for (size_t j = 0; j < hj.size(); ++j)
             if (hj[j].group == g) hj[n++].nth = (uint32_t)j;
+}
+
+// Setup blocks of every job and group (from the jobs' triangle ranges).
+void layout_blocks(std::vector<JobDev> &hj, std::vector<RasterGroup> &gr) {
+    uint32_t blocks = 0;
+    for (RasterGroup &g : gr) g.nblocks = g.ntri = 0;
+    for (JobDev &at : hj) {
+        const JobDev &J = hj[at.nth];
+        RasterGroup &g = gr[J.group];
+        if (g.nblocks == 0) g.block0 = blocks;
+        at.nth_block = blocks;
+        const uint32_t n = (J.ntri + RF_SETUP_THREADS - 1) / RF_SETUP_THREADS;
+        g.nblocks += n;
+        g.ntri += J.ntri;
+        blocks += n;
+    }
 }
 
 // Tile and mask fields of every job, and the groups' tile ranges, for tile
@@ -521,7 +536,6 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
     Mesh *mesh = nullptr;
     rf_texture tex_h = 0;
     Texture *tex = nullptr;
-    int frame_kind = RF_K_ANY;
     host.assign(nin, JobHost{});
     uint64_t nv = 0, nt = 0;
     uint64_t tiles = 0;
@@ -602,7 +616,6 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
             continue;
         }
         ctx->any_cull = ctx->any_cull || culls;
-        frame_kind = hj.empty() || frame_kind == kind ? kind : (int)RF_K_ANY;
         const Target &tg = *ji.tg;
         JobDev J{};
         J.color = tg.color;
@@ -632,9 +645,9 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
         hj.push_back(J);
     }
     group_jobs(ctx);
+    layout_blocks(hj, ctx->groups);
     layout_tiles(hj, ctx->groups, TW);
     ctx->ndraws = nd;
-    ctx->kind = frame_kind;
     nv_out = nv;
     nt_out = nt;
     return RF_OK;
@@ -742,7 +755,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     if ((st = ensure(ctx, ctx->scan, rfk::scan_scratch_words((uint32_t)nt) * 4))) return st;
     if ((st = ensure(ctx, ctx->rowtot, 16))) return st;
     if ((st = ensure(ctx, ctx->rprims, (size_t)nt * RF_MAX_FAN * sizeof(RasterPrim)))) return st;
-    if ((st = ensure(ctx, ctx->live, (size_t)nt * RF_MAX_FAN * 12))) return st;  // three lists
+    if ((st = ensure(ctx, ctx->live, (size_t)nt * RF_MAX_FAN * 8))) return st;  // two lists
     if ((st = ensure(ctx, ctx->marks, 8))) return st;
     if ((st = ensure(ctx, ctx->items, (size_t)ntiles * (RF_SPLIT_K + 1) * 4))) return st;
     if (!ctx->rows_need_host) {
@@ -769,7 +782,6 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     if ((st = ensure(ctx, ctx->segs, (size_t)pieces(hj) * 8))) return st;
 
     cudaStream_t s = ctx->stream;
-    const int kind = ctx->kind;
     const bool any_cull = ctx->any_cull;
     const uint32_t ng = (uint32_t)ctx->groups.size();
     if (ng > 1 && !ctx->side) {
@@ -831,12 +843,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     const JobDev *jd = reinterpret_cast<const JobDev *>(P<char>(ctx->draws) + jobs_at(ndraws));
     auto enqueue = [&](bool marks) -> rf_status {
         auto mark = [&](int i) -> cudaError_t { return marks ? cudaEventRecord(ev[i], s) : cudaSuccess; };
-        CK(cudaMemsetAsync(ctx->mask.p, 0, mask_words * 4, s));
-        if (per_job) CK(cudaMemsetAsync(kst, 0, nj * sizeof(StatsDev), s));
         CK(mark(RF_STAGE_VERTEX));
+        CK(rfk::launch_zero(P<uint32_t>(ctx->mask), mask_words, kst, per_job ? nj : 0u,
+                            P<unsigned long long>(ctx->rowtot), P<unsigned long long>(ctx->marks), counters,
+                            ctx->nsm, s));
         if (any_cull) CK(rfk::launch_cull(P<DrawDev>(ctx->draws), ndraws, kst, ctx->nsm, s));
         CK(rfk::launch_vertex(dd, ndraws, (uint32_t)nv, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
-                              counters, P<unsigned long long>(ctx->marks),
                               ctx->nsm, s));
         CK(mark(RF_STAGE_CLIP));
         // (each triangle's output slots placed by the clip kernels: no scan)
@@ -846,12 +858,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
                             P<uint32_t>(ctx->toff), true));
         CK(mark(RF_STAGE_SCAN));
         CK(mark(RF_STAGE_SETUP));
-        CK(rfk::launch_setup(dd, ndraws, jd, (uint32_t)nt, TW, P<float4>(ctx->cpos),
+        CK(rfk::launch_setup(dd, ndraws, jd, nj, ctx->groups.data(), ng, (uint32_t)nt, TW, P<float4>(ctx->cpos),
                              P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->toff), P<uint32_t>(ctx->tpoly),
                              P<PolyVert>(ctx->pool), P<PrimRec>(ctx->prims), P<unsigned long long>(ctx->rowtot),
                              P<uint32_t>(ctx->rows), ctx->rows_cap, P<RasterPrim>(ctx->rprims),
                              P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
-                             kst, counters, ctx->nsm, s, nullptr, nullptr, kind));
+                             kst, counters, ctx->nsm, s));
         CK(rfk::launch_lists(jd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(hj), P<uint32_t>(ctx->toff),
                              P<uint32_t>(ctx->tcnt), P<RasterPrim>(ctx->rprims), P<unsigned long long>(ctx->marks),
                              (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, P<uint2>(ctx->segs),
@@ -874,11 +886,13 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     uint64_t sort_kernels = 0;
     auto enqueue_sorted = [&]() -> rf_status {
         auto mark = [&](int i) -> cudaError_t { return ctx->timing ? cudaEventRecord(ev[i], s) : cudaSuccess; };
-        if (per_job) CK(cudaMemsetAsync(kst, 0, nj * sizeof(StatsDev), s));
         CK(mark(RF_STAGE_VERTEX));
+        // (the masks are zeroed later, once their size is known)
+        CK(rfk::launch_zero(nullptr, 0, kst, per_job ? nj : 0u, P<unsigned long long>(ctx->rowtot),
+                            P<unsigned long long>(ctx->marks), counters, ctx->nsm, s));
         if (any_cull) CK(rfk::launch_cull(P<DrawDev>(ctx->draws), ndraws, kst, ctx->nsm, s));
         CK(rfk::launch_vertex(dd, ndraws, (uint32_t)nv, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
-                              counters, P<unsigned long long>(ctx->marks), ctx->nsm, s));
+                              ctx->nsm, s));
         CK(mark(RF_STAGE_CLIP));
         CK(rfk::launch_clip(dd, ndraws, (uint32_t)nt, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
                             P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->tpoly), P<uint32_t>(ctx->toff),
@@ -923,6 +937,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         }
         for (JobDev &J : vj) J.mask_words = (J.ntri + 31) / 32;
         layout_masks(vj);
+        layout_blocks(vj, ctx->groups);
         const size_t vmask = vj.back().sum_base + (size_t)vj.back().tiles_x * vj.back().tiles_y * vj.back().sum_words;
         const uint32_t n32 = (uint32_t)np;
         if ((st2 = ensure(ctx, ctx->mask, std::max<size_t>(vmask, 1) * 4))) return st2;
@@ -948,12 +963,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
                              P<uint32_t>(ctx->scan), s));
         CK(cudaMemsetAsync(ctx->mask.p, 0, vmask * 4, s));
         CK(rfk::launch_iota(P<uint32_t>(ctx->vtoff), P<uint32_t>(ctx->vtcnt), n32, s));
-        CK(rfk::launch_setup(vdd, ndraws, vjd, n32, TW, P<float4>(ctx->cpos), P<uint32_t>(ctx->tcnt),
-                             P<uint32_t>(ctx->toff), P<uint32_t>(ctx->tpoly), P<PolyVert>(ctx->pool),
-                             P<PrimRec>(ctx->prims), P<unsigned long long>(ctx->rowtot),
+        CK(rfk::launch_setup(vdd, ndraws, vjd, nj, ctx->groups.data(), ng, n32, TW, P<float4>(ctx->cpos),
+                             P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->toff), P<uint32_t>(ctx->tpoly),
+                             P<PolyVert>(ctx->pool), P<PrimRec>(ctx->prims), P<unsigned long long>(ctx->rowtot),
                              P<uint32_t>(ctx->rows), ctx->rows_cap, P<RasterPrim>(ctx->rprims),
                              P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
-                             kst, counters, ctx->nsm, s, P<uint32_t>(ctx->perm), P<uint32_t>(ctx->ptri), kind));
+                             kst, counters, ctx->nsm, s, P<uint32_t>(ctx->perm), P<uint32_t>(ctx->ptri)));
         CK(rfk::launch_lists(vjd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(vj), P<uint32_t>(ctx->vtoff),
                              P<uint32_t>(ctx->vtcnt), P<RasterPrim>(ctx->rprims), P<unsigned long long>(ctx->marks),
                              (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, P<uint2>(ctx->segs),
@@ -976,11 +991,15 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     } else if (ctx->graphs && !ctx->timing) {
         GraphKey key{};
         const uint64_t kv[] = {ctx->gen, ndraws, nj, nv, nt, ntiles, mask_words, TW, ctx->warps,
-                               (uint64_t)(kind + 16) | (any_cull ? 0x100u : 0u), per_job ? 1u : 0u, ctx->rows_cap, ctx->list_cap};
-        static_assert(sizeof kv + RF_MAX_GROUPS * 8 == sizeof key.v, "graph key size");
+                               pieces(hj), (any_cull ? 2u : 0u) | (per_job ? 1u : 0u), ctx->rows_cap, ctx->list_cap};
+        static_assert(sizeof kv + 3 * RF_MAX_GROUPS * 8 == sizeof key.v, "graph key size");
         memcpy(key.v, kv, sizeof kv);
-        for (const RasterGroup &g : ctx->groups)  // (a group's slot is never 0: it has tiles)
-            key.v[13 + g.kind * 2 + (g.fast ? 0 : 1)] = g.ntiles;
+        for (const RasterGroup &g : ctx->groups) {  // (a group present has tiles)
+            uint64_t *k = key.v + 13 + 3 * (g.kind * 2 + (g.fast ? 0 : 1));
+            k[0] = g.ntiles;
+            k[1] = g.ntri;
+            k[2] = g.nblocks;
+        }
         GraphEntry *hit = nullptr;
         for (GraphEntry &g : ctx->gcache)
             if (g.key == key) hit = &g;
@@ -1018,11 +1037,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         CK(cudaEventRecord(tuned->e1, s));
         tuned->pending = true;
     }
-    // vertex, clip (2), setup, bin (3: 8- and 16-lane groups, then warps),
-    // work list, raster (one launch a group; + the stats fold; a depth-sorted frame adds the
-    // scan of the fan counts, 3 launches or 1 for one block, and its sort)
+    // zero, vertex, clip (2), lists, and per group setup, bin (2: 16-lane
+    // groups, then warps) and raster (+ the stats fold; a depth-sorted frame
+    // adds the scan of the fan counts, 3 launches or 1 for one block, and its
+    // sort)
     const uint64_t scan_kernels = sorted ? (nt <= RF_SCAN_BLOCK_ITEMS ? 1 : 3) : 0;
-    ctx->kernels += 8 + ng + scan_kernels + (per_job ? 1 : 0) + (any_cull ? 1 : 0) + sort_kernels;
+    ctx->kernels += 5 + 4 * ng + scan_kernels + (per_job ? 1 : 0) + (any_cull ? 1 : 0) + sort_kernels;
     if (!ctx->rows_evt_pending) {
         CK(cudaMemcpyAsync(ctx->rows_need_host, ctx->rowtot.p, 16, cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(ctx->rows_evt, s));
@@ -1402,7 +1422,7 @@ rf_status rf_render_lines(rf_ctx *ctx, rf_mesh mesh, int32_t shader, const rf_un
         CK(cudaMemsetAsync(counters + RF_CNT_QUEUE, 0, 4, s));
         CK(cudaMemsetAsync(ctx->lmask.p, 0, mwords * 4, s));
         CK(rfk::launch_vertex(P<DrawDev>(ctx->draws), 1, m.nverts, P<float4>(ctx->cpos),
-                              P<uint8_t>(ctx->coc), nullptr, nullptr, ctx->nsm, s));
+                              P<uint8_t>(ctx->coc), ctx->nsm, s));
         CK(rfk::launch_lines(P<DrawDev>(ctx->draws), P<JobDev>(ctx->jobs), m.ntri, P<float4>(ctx->cpos),
                              P<uint8_t>(ctx->coc), P<LineRec>(ctx->lrec), P<uint32_t>(ctx->lmask), ntiles,
                              counters + RF_CNT_QUEUE, P<StatsDev>(ctx->stats), ctx->nsm, s));

@@ -28,6 +28,7 @@
 #define RF_POLY_STORE 9      // stored polygon vertices: a triangle clipped by 6 planes has <= 9
 #define RF_MAX_FAN (RF_POLY_STORE - 2)  // fan triangles per input triangle
 #define RF_TILE_H 32         // tile height = one warp lane per row
+#define RF_SETUP_THREADS 64  // triangles a setup block takes at a time
 
 struct DrawDev {
     const float *verts;
@@ -68,6 +69,7 @@ struct JobDev {
     // Not of this job, but the tile layout's directory: the job whose tiles
     // (and list pieces) come nth when laid out by group, and where they start.
     uint32_t nth, nth_tile;
+    uint32_t nth_block, pad_; // ... and its first setup block (RF_SETUP_THREADS triangles each)
     uint64_t nth_seg;
     uint64_t sum_base;        // word offset of the job's tile-0 summary (after every job's masks)
     uint32_t nseg, seg_words; // a tile's triangle list comes in nseg pieces of seg_words summary words

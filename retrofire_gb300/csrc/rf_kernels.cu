@@ -1,6 +1,7 @@
 // rf_kernels.cu — CUDA kernels of the triangle render path (sm_103a).
 //
 // Stage map (reference call stack: core/src/render.rs:134-207):
+//   k_zero       the frame's masks and counters
 //   k_vertex     vertex shader + ClipVert::new         render.rs:157-165
 //   k_clip       status; the crossing triangles queue  clip.rs:245-267
 //   k_clip_poly  Sutherland-Hodgman on the queue       clip.rs:283-301,350-400
@@ -16,6 +17,8 @@
 //                fragment shading, pixel packing       (rf_raster.cuh)
 //   k_fill       Frame::clear without a later render   front/src/lib.rs:103-120
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "rf_exact.cuh"
 #include "rf_internal.cuh"
@@ -59,25 +62,34 @@ __device__ __forceinline__ uint32_t zdiv_mask_of(int32_t shader) {
 
 }  // namespace
 
+// What a frame's kernels accumulate into, zeroed in one launch: the tile
+// masks (n16 16-byte words; their buffer is padded to that), the jobs' stats
+// slots, the row and list totals, the marks total and the counters that do
+// not run on from frame to frame.
+__global__ void k_zero(uint4 *__restrict__ mask, size_t n16, unsigned long long *__restrict__ js, uint32_t njs,
+                       unsigned long long *__restrict__ totals, unsigned long long *__restrict__ marks,
+                       uint32_t *__restrict__ counters) {
+    const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = i0; i < n16; i += step) mask[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (size_t i = i0; i < njs; i += step) js[i] = 0ull;
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < 2) totals[threadIdx.x] = 0ull;
+        if (threadIdx.x == 0) {
+            *marks = 0ull;
+            counters[RF_CNT_POOL] = 0;
+            counters[RF_CNT_PRIMS] = 0;
+            counters[RF_CNT_CLIPQ] = 0;
+        }
+        if (threadIdx.x < RF_CNT_N - RF_CNT_QUEUE_G) counters[RF_CNT_QUEUE_G + threadIdx.x] = 0;  // the groups' and LISTOVF
+    }
+}
+
 // ---------------------------------------------------------------------------
 // K1: vertex shader (mvp.apply, mat.rs:952-973, or clip-space passthrough)
 // and outcode (clip.rs:240-242, 303-309).
 // ---------------------------------------------------------------------------
 __global__ void k_vertex(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nv_total,
-                         float4 *__restrict__ cpos, uint8_t *__restrict__ coc,
-                         uint32_t *__restrict__ counters, unsigned long long *__restrict__ marks) {
-    if (blockIdx.x == 0) {  // the frame's counters, for the kernels after this one
-        if (counters && threadIdx.x == 0) {
-            counters[RF_CNT_POOL] = 0;
-            counters[RF_CNT_LIVE] = 0;
-            counters[RF_CNT_LIVE_SMALL] = 0;
-            counters[RF_CNT_LIVE_MID] = 0;
-            counters[RF_CNT_PRIMS] = 0;
-            counters[RF_CNT_CLIPQ] = 0;
-            *marks = 0;
-        }
-        if (counters && threadIdx.x <= 2 * RF_MAX_GROUPS) counters[RF_CNT_QUEUE_G + threadIdx.x] = 0;  // .. LISTOVF
-    }
+                         float4 *__restrict__ cpos, uint8_t *__restrict__ coc) {
     // Warp-uniform loop (the draw lookup is shared by the warp's lanes).
     for (uint32_t wbase = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); wbase < nv_total;
          wbase += gridDim.x * blockDim.x) {
@@ -626,8 +638,9 @@ struct SV {  // screen-space vertex: (ScreenPt, V) without the unused y step
 };
 
 // raster.rs:248-302 scan(): fills one HalfRec.
-__device__ void scan_setup(float y0, float y1, const SV &l0, const SV &l1, const SV &r0,
-                           const SV &r1, uint32_t nc, HalfRec &h) {
+template <int NCL>
+__device__ __forceinline__ void scan_setup(float y0, float y1, const SV &l0, const SV &l1, const SV &r0,
+                                           const SV &r1, uint32_t nc, HalfRec &h) {
     const float recip_dy = fdiv(1.0f, fsub(y1, y0));
     const float dlx = fmul(fsub(l1.x, l0.x), recip_dy);
     const float drx = fmul(fsub(r1.x, r0.x), recip_dy);
@@ -643,8 +656,9 @@ __device__ void scan_setup(float y0, float y1, const SV &l0, const SV &l1, const
     h.d[RF_R_RX] = drx;
     st[RF_R_LX] = fadd(l0.x, fmul(fsub(fadd(l0.x, dlx), l0.x), yt));
     st[RF_R_RX] = fadd(r0.x, fmul(drx, yt));
+#pragma unroll
     for (uint32_t c = 0; c < RF_NC; ++c) {
-        if (c < nc) {
+        if (c < NCL && c < nc) {
             const float dl = fmul(fsub(l1.c[c], l0.c[c]), recip_dy);
             const float dr = fmul(fsub(r1.c[c], r0.c[c]), recip_dy);
             const float l0s = fadd(l0.c[c], dl), r0s = fadd(r0.c[c], dr);
@@ -657,6 +671,7 @@ __device__ void scan_setup(float y0, float y1, const SV &l0, const SV &l1, const
             st[RF_R_C + c] = 0.0f;
         }
     }
+#pragma unroll
     for (uint32_t r = 0; r < RF_NR; ++r) h.b0[r] = f2u(st[r]);
 }
 
@@ -686,229 +701,6 @@ __device__ void half_runs(const HalfRec &h, HalfRuns &u, uint32_t r) {
 
 }  // namespace
 
-#define RF_SETUP_THREADS 64
-__global__ void __launch_bounds__(RF_SETUP_THREADS)
-k_setup(const DrawDev *__restrict__ draws, uint32_t nd,
-                        const JobDev *__restrict__ jobs, uint32_t nt_total,
-                        const float4 *__restrict__ cpos, const uint32_t *__restrict__ tcnt,
-                        const uint32_t *__restrict__ toff, const uint32_t *__restrict__ tpoly,
-                        const PolyVert *__restrict__ pool, PrimRec *__restrict__ prims,
-                        unsigned long long *__restrict__ rows_total, RasterPrim *__restrict__ rprims,
-                        uint32_t *__restrict__ live, uint32_t *__restrict__ live_n,
-                        uint32_t *__restrict__ live_small, uint32_t *__restrict__ live_small_n,
-                        uint32_t *__restrict__ live_mid, uint32_t *__restrict__ live_mid_n,
-                        StatsDev *__restrict__ stats,
-                        const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ptri) {
-    // Each thread builds its record in shared memory; the warp then writes
-    // the records out with coalesced 16-byte stores.  Only triangles that
-    // pass the face-cull test get a record, and their indices are appended
-    // to the live list the binning pass walks.
-    // (the record's first RF_PRIM_CORE_BYTES only: the binade runs, needed
-    // by few triangles, go straight to global memory)
-    __shared__ __align__(16) uint4 sbuf[RF_SETUP_THREADS][RF_PRIM_CORE_BYTES / 16];
-    const uint32_t lane = threadIdx.x & 31, wbase = threadIdx.x & ~31u;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    // Depth-sorted frames (perm != nullptr): thread gt is the gt-th clipped
-    // triangle in sorted order, perm[gt] its index in clipped order, ptri
-    // the input triangle it came from; the draws' tri_base / ntri count
-    // clipped triangles then, and src_tri_base locates the input ones.
-    for (uint32_t base = blockIdx.x * blockDim.x; base < nt_total; base += stride) {
-        const uint32_t gt = base + threadIdx.x;
-        const bool active = gt < nt_total;
-        const uint32_t cnt = active ? (perm ? 1u : tcnt[gt]) : 0u;
-        uint32_t job = 0xFFFFFFFFu;
-        unsigned long long prims_o = 0;
-        uint32_t di = 0, t = 0, nc = 0, na = 0, zm = 0, slot = RF_NO_POLY, p0 = 0, fan0 = 0;
-        const uint32_t dwarp = warp_upper_index(nd, active ? gt : nt_total - 1,
-                                                [&](uint32_t i) { return draws[i].tri_base; });
-        if (cnt) {
-            di = dwarp;
-            job = draws[di].job;
-            nc = 1 + nattr_of(draws[di].shader);
-            na = nc - 1;
-            zm = zdiv_mask_of(draws[di].shader);
-            if (perm) {
-                const uint32_t pc = perm[gt], tin = ptri[pc];
-                t = tin - draws[di].src_tri_base;
-                slot = tpoly[tin];
-                fan0 = pc - toff[tin];
-                p0 = gt;
-            } else {
-                t = gt - draws[di].tri_base;
-                slot = tpoly[gt];
-                p0 = toff[gt];
-            }
-        }
-        const uint32_t maxc = __reduce_max_sync(0xFFFFFFFFu, cnt);
-        for (uint32_t c = 0; c < maxc; ++c) {
-            const bool have = c < cnt;
-            bool keep = false;  // passes the face-cull test
-            uint32_t list = 0;  // ... and its binning list: 0 k_bin, 1 / 2 k_bin_small (8 / 16 lanes)
-            if (have) {
-                const DrawDev &d = draws[di];
-                const JobDev &J = jobs[job];
-                // Gather the three clip-space vertices of this (fan) triangle.
-                float pos[3][4], at[3][RF_MAX_ATTR];
-                for (int k = 0; k < 3; ++k) {
-                    if (slot == RF_NO_POLY) {
-                        const uint32_t li = d.idx[3 * (size_t)t + k];
-                        const float4 p = cpos[d.vert_base + li];
-                        pos[k][0] = p.x; pos[k][1] = p.y; pos[k][2] = p.z; pos[k][3] = p.w;
-                        const float *src = d.verts + (size_t)li * d.stride + d.pos_dim;
-                        for (uint32_t a = 0; a < na; ++a) at[k][a] = src[a];
-                    } else {
-                        const PolyVert &v = pool[(size_t)slot * RF_POLY_STORE + (k == 0 ? 0 : fan0 + c + k)];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) pos[k][q] = v.pos[q];
-                        for (uint32_t a = 0; a < na; ++a) at[k][a] = v.a[a];
-                    }
-                }
-                // prim.rs:62-88 to_screen + viewport (mat.rs:945-949).
-                SV sv[3];
-                for (int k = 0; k < 3; ++k) {
-                    const float w = pos[k][3];
-                    const float ndc[4] = {fdiv(pos[k][0], w), fdiv(pos[k][1], w), fdiv(1.0f, w), 1.0f};
-                    sv[k].x = dot4(J.vp + 0, ndc);
-                    sv[k].y = dot4(J.vp + 4, ndc);
-                    sv[k].c[0] = dot4(J.vp + 8, ndc);
-                    for (uint32_t a = 0; a < RF_MAX_ATTR; ++a)
-                        sv[k].c[1 + a] = a < na ? (((zm >> a) & 1u) ? fdiv(at[k][a], w) : at[k][a]) : 0.0f;
-                }
-                // Winding (geom/prim.rs:152-156, 288-294) and face_cull (ctx.rs:95-101).
-                const float ux = fsub(sv[1].x, sv[0].x), uy = fsub(sv[1].y, sv[0].y);
-                const float vx = fsub(sv[2].x, sv[0].x), vy = fsub(sv[2].y, sv[0].y);
-                const float wz = fadd(fadd(0.0f, fmul(-uy, vx)), fmul(ux, vy));
-                const bool backface = wz < 0.0f;
-                const bool culled = (J.face_cull == RF_K_CULL_BACK && backface) ||
-                                    (J.face_cull == RF_K_CULL_FRONT && !backface);
-                keep = !culled;
-                if (culled && cnt > 1) {
-                    // A piece of a clipped triangle: the rasteriser walks
-                    // every piece of a triangle it meets and skips this one.
-                    RasterPrim *R = rprims + p0 + c;
-                    R->draw = di;
-                    R->flags = 0u;
-                    R->kind = d.shader;
-                    R->zmax = __int_as_float(0x7F800000);
-                }
-                if (!culled) {
-                // This thread's slot: the fields before `runs` only.
-                PrimRec &P = *reinterpret_cast<PrimRec *>(sbuf[threadIdx.x]);
-                P.draw = di;
-                P.live = 1u;
-                P.tri = gt;
-                P.kind = d.shader;
-                P.rloc = 0;
-                P.rwords = 0;
-                P.job = job;
-                prims_o += 1;
-                // raster.rs:185-224 tri_fill: stable sort by y (total_cmp).
-                SV v0 = sv[0], v1 = sv[1], v2 = sv[2], tmp;
-                if (total_key(v0.y) > total_key(v1.y)) { tmp = v0; v0 = v1; v1 = tmp; }
-                if (total_key(v1.y) > total_key(v2.y)) { tmp = v1; v1 = v2; v2 = tmp; }
-                if (total_key(v0.y) > total_key(v1.y)) { tmp = v0; v0 = v1; v1 = tmp; }
-                const float tt = fdiv(fsub(v1.y, v0.y), fsub(v2.y, v0.y));
-                SV mid1;
-                mid1.x = lerp(v0.x, v2.x, tt);
-                mid1.y = v1.y;
-                for (uint32_t q = 0; q < RF_NC; ++q) mid1.c[q] = lerp(v0.c[q], v2.c[q], tt);
-                const bool mid0_left = v1.x < mid1.x;
-                const SV &left = mid0_left ? v1 : mid1;
-                const SV &right = mid0_left ? mid1 : v1;
-                scan_setup(v0.y, v1.y, v0, left, v0, right, nc, P.half[0]);
-                scan_setup(v1.y, v2.y, left, v2, right, v2, nc, P.half[1]);
-                // Row records for the scanlines that land on the target's
-                // rows, unless a half starts above the buffer (its rows map
-                // onto row 0 several times: rasterised from this record).
-                uint32_t rows = 0;
-                bool regular = true;
-                for (int hh = 0; hh < 2; ++hh) {
-                    const HalfRec &H = P.half[hh];
-                    if (H.n == 0 || !(fabsf(H.y0r) < RF_MAX_COORD)) continue;
-                    const int32_t Y = (int32_t)fsub(H.y0r, 0.5f);
-                    if (Y < 0) regular = false;
-                    const int64_t in = min((int64_t)H.n, max((int64_t)0, (int64_t)J.h - Y));
-                    rows += (uint32_t)in;
-                }
-                const uint64_t w = regular ? (uint64_t)rows * (1u + 2u * nc) : 0u;
-                if (w < 0x40000000ull) P.rwords = (uint32_t)w;
-                if (P.rwords != 0u) list = rows <= 8u ? 1u : rows <= 16u ? 2u : 0u;
-                if (P.rwords == 0u) {  // rasterised from this record: it needs the runs
-                    PrimRec *G = prims + p0 + c;
-                    for (int hh = 0; hh < 2; ++hh)
-                        for (uint32_t r = 0; r < RF_NR; ++r) half_runs(P.half[hh], G->runs[hh], r);
-                }
-                }
-            }
-            __syncwarp();
-            // Room for this step's row records: one atomic per warp on the
-            // frame's running total, each lane's block after the lower
-            // lanes' (the records' place in the buffer is free; each
-            // triangle's own records stay contiguous).  An offset past 32
-            // bits is clamped, so the binning pass finds no room for it.
-            {
-                PrimRec &P = *reinterpret_cast<PrimRec *>(sbuf[threadIdx.x]);
-                const unsigned long long w = keep ? P.rwords : 0u;
-                unsigned long long incl = w;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                    if (lane >= (uint32_t)o) incl += y;
-                }
-                const unsigned long long total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-                unsigned long long at = 0;
-                if (total && lane == 0) at = atomicAdd(rows_total, total);
-                at = __shfl_sync(0xFFFFFFFFu, at, 0) + (incl - w);
-                if (w) P.rloc = at < 0xFFFFFFFFull ? (uint32_t)at : 0xFFFFFFFFu;
-            }
-            __syncwarp();
-            uint32_t bal = __ballot_sync(0xFFFFFFFFu, keep);
-            const uint32_t dst = p0 + c;
-            // Append this step's live triangles to their lists.
-            for (uint32_t which = 0; which < 3; ++which) {
-                const uint32_t b = __ballot_sync(0xFFFFFFFFu, keep && list == which);
-                if (!b) continue;
-                uint32_t *cnt_w = which == 0 ? live_n : which == 1 ? live_small_n : live_mid_n;
-                uint32_t *list_w = which == 0 ? live : which == 1 ? live_small : live_mid;
-                const uint32_t lead = __ffs(b) - 1;
-                uint32_t at = 0;
-                if (lane == lead) at = atomicAdd(cnt_w, (uint32_t)__popc(b));
-                at = __shfl_sync(0xFFFFFFFFu, at, lead);
-                if ((b >> lane) & 1u) list_w[at + __popc(b & ((1u << lane) - 1u))] = dst;
-            }
-            // Write out the records built in this step, one per pass.
-            while (bal) {
-                const uint32_t l = __ffs(bal) - 1;
-                bal &= bal - 1;
-                const uint32_t dl = __shfl_sync(0xFFFFFFFFu, dst, l);
-                const uint4 *src = sbuf[wbase + l];
-                uint4 *out = reinterpret_cast<uint4 *>(prims + dl);
-                if (lane < RF_PRIM_CORE_BYTES / 16) out[lane] = src[lane];
-            }
-            __syncwarp();
-        }
-        // Stats, aggregated per warp when all lanes share one job.
-        const uint32_t hasjob = __ballot_sync(0xFFFFFFFFu, job != 0xFFFFFFFFu);
-        if (hasjob) {
-            const uint32_t j0 = __shfl_sync(0xFFFFFFFFu, job, __ffs(hasjob) - 1);
-            const bool same = __all_sync(0xFFFFFFFFu, job == j0 || job == 0xFFFFFFFFu);
-            if (same || job != 0xFFFFFFFFu) {
-                StatsDev *S = stats + (same ? j0 : job);
-                warp_add_u64(&S->prims_o, prims_o, same);
-                warp_add_u64(&S->verts_o, 3ull * prims_o, same);
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// K3b: scanline statistics and tile binning, one warp per triangle.
-// For every scanline of both halves (ScanlineIter::next, raster.rs:80-114)
-// the lane owning that row computes the exact edge values (closed-form run or
-// the general loop), then frags.i / oob as rasterize_fb counts them
-// (target.rs:259-264) and the pixel columns it covers; a warp reduction per
-// 32-row band gives the tiles to mark in the job's bitmask.
-// ---------------------------------------------------------------------------
 namespace {
 
 // k steps of Iter::next on the first N components, side by side.
@@ -1038,6 +830,369 @@ __device__ __forceinline__ void row_record(float lx, float rx, const float *cv, 
 
 }  // namespace
 
+// A thread's record in shared memory: an odd number of words, so that the
+// lanes' accesses to one field hit 32 banks.
+#define RF_SETUP_WORDS (RF_PRIM_CORE_BYTES / 4 + 1)
+static_assert(RF_SETUP_WORDS % 2 == 1 && RF_SETUP_WORDS * 4 >= sizeof(RasterPrim), "setup slots");
+// Triangles of at most RF_INLINE_ROWS rows on the target, no wider than
+// RF_INLINE_WIDTH px, are binned by the thread that sets them up.
+#define RF_INLINE_ROWS 8u
+#define RF_INLINE_WIDTH 128.0f
+// NCT: the components (1 + attributes) of every triangle of the launch, or
+// 0 when its draws mix shader kinds.
+template <int NCT>
+__global__ void __launch_bounds__(RF_SETUP_THREADS)
+k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict__ jobs, uint32_t nj,
+        uint32_t block0, uint32_t nblocks, uint32_t tile_w, const float4 *__restrict__ cpos, const uint32_t *__restrict__ tcnt,
+        const uint32_t *__restrict__ toff, const uint32_t *__restrict__ tpoly, const PolyVert *__restrict__ pool,
+        PrimRec *__restrict__ prims, unsigned long long *__restrict__ rows_total, uint32_t *__restrict__ rows,
+        unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint32_t *__restrict__ mask,
+        uint32_t *__restrict__ live, uint32_t *__restrict__ live_n, uint32_t *__restrict__ live_mid,
+        uint32_t *__restrict__ live_mid_n, unsigned long long *__restrict__ marks, StatsDev *__restrict__ stats,
+        const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ptri) {
+    constexpr uint32_t FULL = 0xFFFFFFFFu, NONE = 0xFFFFFFFFu;
+    constexpr int NCL = NCT ? NCT : RF_NC;
+    // Each thread builds its record in shared memory; the warp then writes
+    // the records out with coalesced stores.  Only triangles that pass the
+    // face-cull test get one: the small ones are binned here -- rows walked,
+    // row records and tile bits written -- and leave a RasterPrim, the others
+    // a PrimRec (its first RF_PRIM_CORE_BYTES; the binade runs, needed by few
+    // triangles, go straight to global memory) and an entry on a live list
+    // for the binning pass.
+    __shared__ uint32_t sbuf[RF_SETUP_THREADS][RF_SETUP_WORDS];
+    const uint32_t lane = threadIdx.x & 31, wbase = threadIdx.x & ~31u;
+    const uint32_t tw_log2 = __ffs(tile_w) - 1;
+    uint32_t acc_marks = 0;
+    // Depth-sorted frames (perm != nullptr): thread gt is the gt-th clipped
+    // triangle in sorted order, perm[gt] its index in clipped order, ptri
+    // the input triangle it came from; the draws' tri_base / ntri count
+    // clipped triangles then, and src_tri_base locates the input ones.
+    // A block's triangles belong to one job.
+    for (uint32_t blk = block0 + blockIdx.x; blk < block0 + nblocks; blk += gridDim.x) {
+        const uint32_t nth = upper_index(nj, blk, [&](uint32_t i) { return jobs[i].nth_block; });
+        const uint32_t job = jobs[nth].nth;
+        const JobDev &J = jobs[job];
+        const uint32_t base = J.tri_base + (blk - jobs[nth].nth_block) * RF_SETUP_THREADS;
+        const uint32_t gt = base + threadIdx.x;
+        const bool active = gt < J.tri_base + J.ntri;
+        const uint32_t cnt = active ? (perm ? 1u : tcnt[gt]) : 0u;
+        unsigned long long prims_o = 0, frags_i = 0, oob = 0;
+        uint32_t di = 0, t = 0, nc = NCL, na = NCL - 1, zm = 0, slot = RF_NO_POLY, p0 = 0, fan0 = 0;
+        const uint32_t dwarp = warp_upper_index(nd, active ? gt : J.tri_base + J.ntri - 1u,
+                                                [&](uint32_t i) { return draws[i].tri_base; });
+        if (cnt) {
+            di = dwarp;
+            if constexpr (NCT == 0) {
+                nc = 1 + nattr_of(draws[di].shader);
+                na = nc - 1;
+            }
+            zm = zdiv_mask_of(draws[di].shader);
+            if (perm) {
+                const uint32_t pc = perm[gt], tin = ptri[pc];
+                t = tin - draws[di].src_tri_base;
+                slot = tpoly[tin];
+                fan0 = pc - toff[tin];
+                p0 = gt;
+            } else {
+                t = gt - draws[di].tri_base;
+                slot = tpoly[gt];
+                p0 = toff[gt];
+            }
+        }
+        const uint32_t maxc = __reduce_max_sync(FULL, cnt);
+        for (uint32_t c = 0; c < maxc; ++c) {
+            const bool have = c < cnt;
+            bool keep = false;      // passes the face-cull test
+            bool mid = false;       // for k_bin_small's list
+            bool small = false;     // binned here
+            uint32_t inr[2] = {0u, 0u}, y0[2] = {0u, 0u};  // a small triangle's rows on the target, per half
+            PrimRec &P = *reinterpret_cast<PrimRec *>(sbuf[threadIdx.x]);  // (the fields before `runs` only)
+            if (have) {
+                const DrawDev &d = draws[di];
+                // Gather the three clip-space vertices of this (fan) triangle.
+                float pos[3][4], at[3][RF_MAX_ATTR];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if (slot == RF_NO_POLY) {
+                        const uint32_t li = d.idx[3 * (size_t)t + k];
+                        const float4 p = cpos[d.vert_base + li];
+                        pos[k][0] = p.x; pos[k][1] = p.y; pos[k][2] = p.z; pos[k][3] = p.w;
+                        const float *src = d.verts + (size_t)li * d.stride + d.pos_dim;
+#pragma unroll
+                        for (int a = 0; a < NCL - 1; ++a)
+                            if ((uint32_t)a < na) at[k][a] = src[a];
+                    } else {
+                        const PolyVert &v = pool[(size_t)slot * RF_POLY_STORE + (k == 0 ? 0 : fan0 + c + k)];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) pos[k][q] = v.pos[q];
+#pragma unroll
+                        for (int a = 0; a < NCL - 1; ++a)
+                            if ((uint32_t)a < na) at[k][a] = v.a[a];
+                    }
+                }
+                // prim.rs:62-88 to_screen + viewport (mat.rs:945-949).
+                SV sv[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const float w = pos[k][3];
+                    const float ndc[4] = {fdiv(pos[k][0], w), fdiv(pos[k][1], w), fdiv(1.0f, w), 1.0f};
+                    sv[k].x = dot4(J.vp + 0, ndc);
+                    sv[k].y = dot4(J.vp + 4, ndc);
+                    sv[k].c[0] = dot4(J.vp + 8, ndc);
+#pragma unroll
+                    for (int a = 0; a < RF_MAX_ATTR; ++a)
+                        sv[k].c[1 + a] = a < NCL - 1 && (uint32_t)a < na ? (((zm >> a) & 1u) ? fdiv(at[k][a], w) : at[k][a]) : 0.0f;
+                }
+                // Winding (geom/prim.rs:152-156, 288-294) and face_cull (ctx.rs:95-101).
+                const float ux = fsub(sv[1].x, sv[0].x), uy = fsub(sv[1].y, sv[0].y);
+                const float vx = fsub(sv[2].x, sv[0].x), vy = fsub(sv[2].y, sv[0].y);
+                const float wz = fadd(fadd(0.0f, fmul(-uy, vx)), fmul(ux, vy));
+                const bool backface = wz < 0.0f;
+                const bool culled = (J.face_cull == RF_K_CULL_BACK && backface) ||
+                                    (J.face_cull == RF_K_CULL_FRONT && !backface);
+                keep = !culled;
+                if (culled && cnt > 1) {
+                    // A piece of a clipped triangle: the rasteriser walks
+                    // every piece of a triangle it meets and skips this one.
+                    RasterPrim *R = rprims + p0 + c;
+                    R->draw = di;
+                    R->flags = 0u;
+                    R->kind = d.shader;
+                    R->zmax = __int_as_float(0x7F800000);
+                }
+                if (!culled) {
+                    P.draw = di;
+                    P.live = 1u;
+                    P.tri = gt;
+                    P.kind = d.shader;
+                    P.rloc = 0;
+                    P.rwords = 0;
+                    P.job = job;
+                    prims_o += 1;
+                    // (how wide, before the sort)
+                    const float wide = fsub(fmaxf(fmaxf(sv[0].x, sv[1].x), sv[2].x),
+                                            fminf(fminf(sv[0].x, sv[1].x), sv[2].x));
+                    // raster.rs:185-224 tri_fill: stable sort by y (total_cmp).
+                    SV v0 = sv[0], v1 = sv[1], v2 = sv[2], tmp;
+                    if (total_key(v0.y) > total_key(v1.y)) { tmp = v0; v0 = v1; v1 = tmp; }
+                    if (total_key(v1.y) > total_key(v2.y)) { tmp = v1; v1 = v2; v2 = tmp; }
+                    if (total_key(v0.y) > total_key(v1.y)) { tmp = v0; v0 = v1; v1 = tmp; }
+                    const float tt = fdiv(fsub(v1.y, v0.y), fsub(v2.y, v0.y));
+                    SV mid1;
+                    mid1.x = lerp(v0.x, v2.x, tt);
+                    mid1.y = v1.y;
+#pragma unroll
+                    for (uint32_t q = 0; q < RF_NC; ++q) mid1.c[q] = q < NCL ? lerp(v0.c[q], v2.c[q], tt) : 0.0f;
+                    // (left and right picked component by component: no
+                    // references into the two, which would put them in memory)
+                    const bool mid0_left = v1.x < mid1.x;
+                    SV left, right;
+                    left.x = mid0_left ? v1.x : mid1.x;
+                    right.x = mid0_left ? mid1.x : v1.x;
+                    left.y = right.y = v1.y;
+#pragma unroll
+                    for (uint32_t q = 0; q < RF_NC; ++q) {
+                        left.c[q] = mid0_left ? v1.c[q] : mid1.c[q];
+                        right.c[q] = mid0_left ? mid1.c[q] : v1.c[q];
+                    }
+                    scan_setup<NCL>(v0.y, v1.y, v0, left, v0, right, nc, P.half[0]);
+                    scan_setup<NCL>(v1.y, v2.y, left, v2, right, v2, nc, P.half[1]);
+                    // Row records for the scanlines that land on the target's
+                    // rows, unless a half starts above the buffer (its rows map
+                    // onto row 0 several times: rasterised from this record).
+                    uint32_t nrows = 0;
+                    unsigned long long below = 0;  // rows past the buffer, or a half out of range
+                    bool regular = true;
+#pragma unroll
+                    for (int hh = 0; hh < 2; ++hh) {
+                        const HalfRec &H = P.half[hh];
+                        if (H.n == 0) continue;
+                        if (!(fabsf(H.y0r) < RF_MAX_COORD)) {
+                            below += 1;
+                            continue;
+                        }
+                        const int32_t Y = (int32_t)fsub(H.y0r, 0.5f);
+                        if (Y < 0) regular = false;
+                        const int64_t in = min((int64_t)H.n, max((int64_t)0, (int64_t)J.h - Y));
+                        below += (unsigned long long)((int64_t)H.n - in);
+                        inr[hh] = (uint32_t)in;
+                        y0[hh] = in ? (uint32_t)Y : 0u;
+                        nrows += (uint32_t)in;
+                    }
+                    const uint64_t w = regular ? (uint64_t)nrows * (1u + 2u * nc) : 0u;
+                    if (w < 0x40000000ull) P.rwords = (uint32_t)w;
+                    if (P.rwords != 0u) {
+                        small = nrows <= RF_INLINE_ROWS && wide <= RF_INLINE_WIDTH;
+                        mid = !small && nrows <= 16u;
+                        if (small) oob += below;  // (the binning pass counts the others')
+                    } else {  // rasterised from this record: it needs the runs
+                        PrimRec *G = prims + p0 + c;
+                        for (int hh = 0; hh < 2; ++hh)
+                            for (uint32_t r = 0; r < RF_NR; ++r) half_runs(P.half[hh], G->runs[hh], r);
+                    }
+                }
+            }
+            __syncwarp();
+            // Room for this step's row records: one atomic per warp on the
+            // frame's running total, each lane's block after the lower
+            // lanes' (the records' place in the buffer is free; each
+            // triangle's own records stay contiguous).  An offset past 32
+            // bits is clamped, so the binning pass finds no room for it.
+            {
+                const unsigned long long w = keep ? P.rwords : 0u;
+                unsigned long long incl = w;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned long long y = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= (uint32_t)o) incl += y;
+                }
+                const unsigned long long total = __shfl_sync(FULL, incl, 31);
+                unsigned long long at = 0;
+                if (total && lane == 0) at = atomicAdd(rows_total, total);
+                at = __shfl_sync(FULL, at, 0) + (incl - w);
+                if (w) P.rloc = at < 0xFFFFFFFFull ? (uint32_t)at : 0xFFFFFFFFu;
+                if (small && (unsigned long long)P.rloc + w > rows_cap) {  // no room: k_bin's path
+                    small = false;
+                    for (int hh = 0; hh < 2; ++hh)  // (its rows past the buffer are counted there)
+                        oob -= P.half[hh].n == 0              ? 0ull
+                               : !(fabsf(P.half[hh].y0r) < RF_MAX_COORD) ? 1ull
+                                                               : (unsigned long long)(P.half[hh].n - inr[hh]);
+                }
+            }
+            // The small triangles' rows, walked in order by their thread
+            // (ScanlineIter::next), and the tiles they cover.
+            uint32_t lo[2] = {NONE, NONE}, hi[2] = {0u, 0u}, band0 = 0;  // per 32-row band: covered columns
+            float zhi = -__int_as_float(0x7F800000);
+            if (small) {
+                const uint32_t rstride = 1u + 2u * nc;
+                uint32_t *rec = rows + P.rloc;
+                band0 = (inr[0] ? y0[0] : y0[1]) / RF_TILE_H;
+#pragma unroll 1
+                for (int hh = 0; hh < 2; ++hh) {
+                    const HalfRec &H = P.half[hh];
+                    float v[2 + NCL], st[2 + NCL], dvx[NCL];
+#pragma unroll
+                    for (int r = 0; r < 2 + NCL; ++r) {
+                        v[r] = u2f(H.b0[r]);
+                        st[r] = H.d[r];
+                    }
+#pragma unroll
+                    for (int q = 0; q < NCL; ++q) dvx[q] = H.dvdx[q];
+                    const uint32_t n = inr[hh];
+#pragma unroll 1
+                    for (uint32_t j = 0; j < n; ++j) {
+                        RowOut o{0, 0, NONE, 0};
+                        row_record<NCT>(v[0], v[1], v + 2, 1u, dvx, nc, J.w, tile_w, rec, o, zhi);
+                        rec += rstride;
+                        frags_i += o.frags_i;
+                        oob += o.oob;
+                        if (o.px0 < o.px1) {
+                            const bool second = (y0[hh] + j) / RF_TILE_H != band0;
+                            if (second) {
+                                lo[1] = min(lo[1], o.px0);
+                                hi[1] = max(hi[1], o.px1);
+                            } else {
+                                lo[0] = min(lo[0], o.px0);
+                                hi[0] = max(hi[0], o.px1);
+                            }
+                        }
+#pragma unroll
+                        for (int r = 0; r < 2 + NCL; ++r) v[r] = fadd(v[r], st[r]);
+                    }
+                }
+            }
+            // Their tile bits, a tile a lane at a time; lanes at the same tile
+            // (neighbours of a mesh mostly are) share one atomic: the warp's
+            // triangles are consecutive bits.
+            {
+                const uint32_t n0 = lo[0] < hi[0] ? ((hi[0] - 1u) >> tw_log2) - (lo[0] >> tw_log2) + 1u : 0u;
+                const uint32_t n1 = lo[1] < hi[1] ? ((hi[1] - 1u) >> tw_log2) - (lo[1] >> tw_log2) + 1u : 0u;
+                acc_marks += n0 + n1;
+                for (uint32_t i = 0; __any_sync(FULL, i < n0 + n1); ++i) {
+                    const bool on = i < n0 + n1;
+                    uint32_t lt = NONE;
+                    if (on) {
+                        const uint32_t b = i < n0 ? 0u : 1u;
+                        lt = (band0 + b) * J.tiles_x + (b ? (lo[1] >> tw_log2) + (i - n0) : (lo[0] >> tw_log2) + i);
+                    }
+                    const uint32_t peers = __match_any_sync(FULL, lt);
+                    if (on && (uint32_t)__ffs(peers) - 1u == lane) {
+                        // (the warp's triangles are one mask word: lane L's is bit L)
+                        const uint32_t wd = (base - J.tri_base + wbase) >> 5;
+                        atomicOr(mask + J.mask_base + (size_t)lt * J.mask_words + wd, peers);
+                        atomicOr(mask + J.sum_base + (size_t)lt * J.sum_words + (wd >> 5), 1u << (wd & 31u));
+                    }
+                }
+            }
+            const uint32_t smalls = __ballot_sync(FULL, small);
+            uint32_t bal = __ballot_sync(FULL, keep);
+            const uint32_t dst = p0 + c;
+            if (small) {  // the slot now holds its RasterPrim (dvdx's source lies past it)
+                const uint32_t base_w = P.rloc;
+                const int32_t kind = P.kind;
+                const HalfRec &H0 = P.half[0], &H1 = P.half[1];
+                static_assert(sizeof(RasterPrim) <= offsetof(PrimRec, half) + offsetof(HalfRec, dvdx), "in place");
+                RasterPrim &R = *reinterpret_cast<RasterPrim *>(sbuf[threadIdx.x]);
+                R.draw = di;
+                R.flags = RF_RP_LIVE | RF_RP_ROWS;
+                R.kind = kind;
+                R.base = base_w;
+                R.stride = 1u + 2u * nc;
+                R.y0 = y0[0];
+                R.c0 = inr[0];
+                R.y1 = y0[1];
+                R.c1 = inr[1];
+                R.zmax = zhi;
+#pragma unroll
+                for (int q = 0; q < RF_NC; ++q) {
+                    R.dvdx[0][q] = H0.dvdx[q];
+                    R.dvdx[1][q] = H1.dvdx[q];
+                }
+            }
+            // Append this step's other live triangles to their lists.
+            for (uint32_t which = 0; which < 2; ++which) {
+                const uint32_t b = __ballot_sync(FULL, keep && !small && mid == (which == 1u));
+                if (!b) continue;
+                const uint32_t lead = __ffs(b) - 1;
+                uint32_t at = 0;
+                if (lane == lead) at = atomicAdd(which ? live_mid_n : live_n, (uint32_t)__popc(b));
+                at = __shfl_sync(FULL, at, lead);
+                if ((b >> lane) & 1u) (which ? live_mid : live)[at + __popc(b & ((1u << lane) - 1u))] = dst;
+            }
+            __syncwarp();
+            // Write out the records built in this step, one per pass.
+            while (bal) {
+                const uint32_t l = __ffs(bal) - 1;
+                bal &= bal - 1;
+                const uint32_t dl = __shfl_sync(FULL, dst, l);
+                const uint32_t *src = sbuf[wbase + l];
+                if ((smalls >> l) & 1u) {
+                    if (lane < sizeof(RasterPrim) / 4) reinterpret_cast<uint32_t *>(rprims + dl)[lane] = src[lane];
+                } else {
+                    uint32_t *out = reinterpret_cast<uint32_t *>(prims + dl);
+                    out[lane] = src[lane];
+                    if (lane + 32u < RF_PRIM_CORE_BYTES / 4) out[lane + 32u] = src[lane + 32u];
+                }
+            }
+            __syncwarp();
+        }
+        StatsDev *S = stats + job;
+        warp_add_u64(&S->prims_o, prims_o, true);
+        warp_add_u64(&S->verts_o, 3ull * prims_o, true);
+        warp_add_u64(&S->frags_i, frags_i, true);
+        warp_add_u64(&S->oob, oob, true);
+    }
+    warp_add_u64(marks, acc_marks, true);
+}
+
+// ---------------------------------------------------------------------------
+// K3b: scanline statistics and tile binning, one warp per triangle.
+// For every scanline of both halves (ScanlineIter::next, raster.rs:80-114)
+// the lane owning that row computes the exact edge values (closed-form run or
+// the general loop), then frags.i / oob as rasterize_fb counts them
+// (target.rs:259-264) and the pixel columns it covers; a warp reduction per
+// 32-row band gives the tiles to mark in the job's bitmask.
+// ---------------------------------------------------------------------------
 // NCT: the components (1 + attributes) of every triangle of the launch, or
 // 0 when its draws mix shader kinds (taken per triangle).
 template <int NCT>
@@ -1046,14 +1201,14 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
       PrimRec *__restrict__ prims, const uint32_t *__restrict__ live, uint32_t tile_w,
       uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims,
       uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
-      unsigned long long *__restrict__ marks) {
+      unsigned long long *__restrict__ marks, const uint32_t *__restrict__ live_n) {
     const uint32_t lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & 7;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const uint32_t tw_log2 = __ffs(tile_w) - 1;  // tile widths are powers of two
     // Only the triangles that passed the face-cull test (the live list, in
     // no particular order: every output below depends on the triangle alone).
-    const uint32_t nl = counters[RF_CNT_LIVE];
+    const uint32_t nl = *live_n;
     // Two record slots per warp of the 256-thread block: the next triangle's
     // record is copied (cp.async) while the current one is walked.
     __shared__ __align__(16) uint4 sbuf[8][2][RF_PRIM_CORE_BYTES / 16];  // records' first parts
@@ -1336,7 +1491,8 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             const uint32_t *__restrict__ live_small, uint32_t *__restrict__ live, uint32_t tile_w,
             uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint32_t *__restrict__ mask,
             StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
-            unsigned long long *__restrict__ marks, uint32_t count_slot) {
+            unsigned long long *__restrict__ marks, const uint32_t *__restrict__ small_n,
+            uint32_t *__restrict__ live_n) {
     static_assert(G == 8 || G == 16, "group sizes");
     constexpr uint32_t NG = 32 / G;  // groups per warp
     constexpr uint32_t NONE = 0xFFFFFFFFu;
@@ -1346,7 +1502,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
     const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const uint32_t ng = (gridDim.x * blockDim.x) / G;
     const uint32_t tw_log2 = __ffs(tile_w) - 1;
-    const uint32_t nl = counters[count_slot];
+    const uint32_t nl = *small_n;
     __shared__ __align__(16) uint4 sbuf[8][NG][RF_PRIM_CORE_BYTES / 16];  // records' first parts
     __shared__ __align__(16) RasterPrim srp[8][NG];
     __shared__ float stab[8][NG][RF_NR][G];  // quantity q of row r at [q][r]
@@ -1396,7 +1552,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             J = &jobs[job];
             base = P->rloc;
             if (base + P->rwords > rows_cap) {  // no room for its records: k_bin's path
-                if (gl == 0) live[atomicAdd(&counters[RF_CNT_LIVE], 1u)] = e;
+                if (gl == 0) live[atomicAdd(live_n, 1u)] = e;
                 run = false;
             }
         }
@@ -1708,12 +1864,20 @@ __global__ void k_fill(uint32_t *__restrict__ color, float *__restrict__ depth, 
 // ---------------------------------------------------------------------------
 namespace rfk {
 
+cudaError_t launch_zero(uint32_t *mask, size_t mask_words, StatsDev *js, uint32_t njobs, unsigned long long *totals,
+                        unsigned long long *marks, uint32_t *counters, int nsm, cudaStream_t s) {
+    const size_t n16 = (mask_words + 3) / 4;
+    const uint32_t blocks = (uint32_t)std::min<size_t>((n16 + 255) / 256 + 1, (size_t)nsm * 8);
+    k_zero<<<blocks, 256, 0, s>>>(reinterpret_cast<uint4 *>(mask), n16, reinterpret_cast<unsigned long long *>(js),
+                                  njobs * (uint32_t)(sizeof(StatsDev) / 8), totals, marks, counters);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv, float4 *cpos,
-                          uint8_t *coc, uint32_t *counters, unsigned long long *marks,
-                          int nsm, cudaStream_t s) {
+                          uint8_t *coc, int nsm, cudaStream_t s) {
     if (nv == 0) return cudaSuccess;
     uint32_t blocks = min((nv + 255) / 256, (uint32_t)nsm * 16);
-    k_vertex<<<blocks, 256, 0, s>>>(draws, nd, nv, cpos, coc, counters, marks);
+    k_vertex<<<blocks, 256, 0, s>>>(draws, nd, nv, cpos, coc);
     return cudaGetLastError();
 }
 
@@ -1756,55 +1920,52 @@ cudaError_t launch_mesh_bbox(const float *verts, uint32_t nverts, uint32_t strid
     return cudaGetLastError();
 }
 
-cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, uint32_t nt,
-                         uint32_t tile_w, const float4 *cpos, const uint32_t *tcnt,
-                         const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
+cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, uint32_t nj,
+                         const RasterGroup *groups, uint32_t ng, uint32_t nt, uint32_t tile_w, const float4 *cpos,
+                         const uint32_t *tcnt, const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
                          PrimRec *prims, unsigned long long *rows_total, uint32_t *rows,
-                         unsigned long long rows_cap,
-                         RasterPrim *rprims, uint32_t *mask, uint32_t *live, unsigned long long *marks,
-                         StatsDev *stats, uint32_t *counters, int nsm, cudaStream_t s,
-                         const uint32_t *perm, const uint32_t *ptri, int kind) {
-    cudaError_t e = cudaMemsetAsync(rows_total, 0, 16, s);  // the frame's row-record words, the lists' cursor
-    if (e != cudaSuccess) return e;
-    if (nt == 0) return cudaSuccess;
-    uint32_t blocks = min((nt + RF_SETUP_THREADS - 1) / RF_SETUP_THREADS, (uint32_t)nsm * 32);
-    // The live list has room for every output triangle three times over:
-    // the triangles for k_bin from the start, those with at most 8 rows from
-    // a third of the way, those with 9 to 16 rows from two thirds.  (A
-    // depth-sorted frame's triangles are single clipped pieces.)
-    const size_t live_cap = perm ? (size_t)nt : (size_t)nt * RF_MAX_FAN;
-    uint32_t *live_small = live + live_cap, *live_mid = live + 2 * live_cap;
-    k_setup<<<blocks, RF_SETUP_THREADS, 0, s>>>(draws, nd, jobs, nt, cpos, tcnt, toff, tpoly, pool,
-                                                prims, rows_total, rprims, live,
-                                                counters + RF_CNT_LIVE, live_small,
-                                                counters + RF_CNT_LIVE_SMALL, live_mid,
-                                                counters + RF_CNT_LIVE_MID,
-                                                stats, perm, ptri);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    // The small triangles, eight lanes each, then one warp per other live
-    // output triangle (with the small ones that found no room for their
-    // records); the counts are only known on the device.
-    auto bin = k_bin<0>;
-    auto bin8 = k_bin_small<0, 8>;
-    auto bin16 = k_bin_small<0, 16>;
-    switch (kind) {  // components per triangle: 1 + the kind's attributes
-        case RF_K_FLAT: bin = k_bin<1>; bin8 = k_bin_small<1, 8>; bin16 = k_bin_small<1, 16>; break;
-        case RF_K_TEXTURED: bin = k_bin<3>; bin8 = k_bin_small<3, 8>; bin16 = k_bin_small<3, 16>; break;
-        case RF_K_GOURAUD:
-        case RF_K_GOURAUD_SRGB: bin = k_bin<4>; bin8 = k_bin_small<4, 8>; bin16 = k_bin_small<4, 16>; break;
-        case RF_K_TEX_GOURAUD: bin = k_bin<6>; bin8 = k_bin_small<6, 8>; bin16 = k_bin_small<6, 16>; break;
-        default: break;
+                         unsigned long long rows_cap, RasterPrim *rprims, uint32_t *mask, uint32_t *live,
+                         unsigned long long *marks, StatsDev *stats, uint32_t *counters, int nsm,
+                         cudaStream_t s, const uint32_t *perm, const uint32_t *ptri) {
+    // (A depth-sorted frame's triangles are single clipped pieces.)
+    const size_t fan = perm ? 1 : RF_MAX_FAN;
+    uint32_t *big = live, *mid = live + (size_t)nt * fan;
+    for (uint32_t g = 0; g < ng; ++g) {
+        const uint32_t gt = groups[g].ntri;
+        if (gt == 0) continue;
+        auto setup = k_setup<0>;
+        auto bin = k_bin<0>;
+        auto bin16 = k_bin_small<0, 16>;
+        switch (groups[g].kind) {  // components per triangle: 1 + the kind's attributes
+            case RF_K_FLAT: setup = k_setup<1>; bin = k_bin<1>; bin16 = k_bin_small<1, 16>; break;
+            case RF_K_TEXTURED: setup = k_setup<3>; bin = k_bin<3>; bin16 = k_bin_small<3, 16>; break;
+            case RF_K_GOURAUD:
+            case RF_K_GOURAUD_SRGB: setup = k_setup<4>; bin = k_bin<4>; bin16 = k_bin_small<4, 16>; break;
+            case RF_K_TEX_GOURAUD: setup = k_setup<6>; bin = k_bin<6>; bin16 = k_bin_small<6, 16>; break;
+            default: break;
+        }
+        uint32_t *big_n = counters + RF_CNT_LIVE_G + g, *mid_n = counters + RF_CNT_LIVE_MID_G + g;
+        const uint32_t blocks = min(groups[g].nblocks, (uint32_t)nsm * 32);
+        setup<<<blocks, RF_SETUP_THREADS, 0, s>>>(draws, nd, jobs, nj, groups[g].block0, groups[g].nblocks, tile_w,
+                                                  cpos, tcnt, toff, tpoly, pool, prims, rows_total, rows, rows_cap,
+                                                  rprims, mask, big, big_n, mid, mid_n, marks, stats, perm, ptri);
+        cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        // The triangles left for the binning pass, sixteen lanes each up to
+        // 16 rows, then one warp per other live output triangle (with the
+        // smaller ones that found no room for their records); the counts are
+        // only known on the device.
+        const uint32_t sblocks = min((gt + 31) / 32, (uint32_t)nsm * 4);
+        bin16<<<sblocks, 256, 0, s>>>(jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, mask, stats,
+                                      counters, marks, mid_n, big_n);
+        const uint32_t wblocks = min((gt * 2 + 7) / 8, (uint32_t)nsm * 16);
+        bin<<<wblocks, 256, 0, s>>>(draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, mask, stats,
+                                    counters, marks, big_n);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        big += (size_t)gt * fan;
+        mid += (size_t)gt * fan;
     }
-    const uint32_t sblocks = min((nt + 31) / 32, (uint32_t)nsm * 4);
-    bin8<<<sblocks, 256, 0, s>>>(jobs, prims, live_small, live, tile_w, rows, rows_cap, rprims, mask, stats,
-                                 counters, marks, RF_CNT_LIVE_SMALL);
-    bin16<<<sblocks, 256, 0, s>>>(jobs, prims, live_mid, live, tile_w, rows, rows_cap, rprims, mask, stats,
-                                  counters, marks, RF_CNT_LIVE_MID);
-    const uint32_t wblocks = min((nt * 2 + 7) / 8, (uint32_t)nsm * 16);
-    bin<<<wblocks, 256, 0, s>>>(draws, jobs, prims, live, tile_w, rows, rows_cap, rprims, mask, stats,
-                                counters, marks);
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles, uint32_t npieces,

@@ -38,13 +38,16 @@
 #define RF_RASTER_MAX_THREADS 256
 // The jobs of a frame are laid out by raster group: one shader kind (or
 // RF_K_ANY: jobs that mix kinds) and one context (the default one on a depth
-// target, or any other).  Every group has a raster kernel of its own and its
-// own part of the work list.
+// target, or any other).  Every group has setup, binning and raster launches
+// of its own, specialised for its kind, its own live lists and its own part
+// of the work list.
 #define RF_MAX_GROUPS (2 * (RF_K_ANY + 1))
 struct RasterGroup {
     int32_t kind;
     bool fast;
     uint32_t tile0, ntiles;
+    uint32_t block0, nblocks;  // setup blocks
+    uint32_t ntri;             // triangles
 };
 
 // counters[] slots
@@ -55,23 +58,24 @@ struct RasterGroup {
 #define RF_CNT_PRIMS 4    // total output prims (scan total)
 #define RF_CNT_QUEUE 5    // tile queue head of the line pass
 #define RF_CNT_ROWSOVF 6  // triangles rasterised without row records (buffer full)
-#define RF_CNT_LIVE 7     // output triangles that passed the face-cull test
 #define RF_CNT_CLIPQ 10   // triangles queued for clipping
-#define RF_CNT_LIVE_SMALL 11  // live triangles binned eight lanes each (at most 8 rows)
-#define RF_CNT_LIVE_MID 12    // live triangles binned sixteen lanes each (9 to 16 rows)
 #define RF_CNT_QUEUE_G 16     // + g: work-list queue head of raster group g
 #define RF_CNT_ITEMS_G (RF_CNT_QUEUE_G + RF_MAX_GROUPS)  // + g: its heavy tiles and crowded tiles' slices
-#define RF_CNT_LISTOVF (RF_CNT_ITEMS_G + RF_MAX_GROUPS)  // nonzero: the triangle lists did not fit
+#define RF_CNT_LIVE_G (RF_CNT_ITEMS_G + RF_MAX_GROUPS)   // + g: its live triangles, binned a warp each
+#define RF_CNT_LIVE_MID_G (RF_CNT_LIVE_G + RF_MAX_GROUPS)  // + g: ... sixteen lanes each (at most 16 rows)
+#define RF_CNT_LISTOVF (RF_CNT_LIVE_MID_G + RF_MAX_GROUPS)  // nonzero: the triangle lists did not fit
 #define RF_CNT_N (RF_CNT_LISTOVF + 1)
 #define RF_SCAN_BLOCK_ITEMS 4096u  // values one scan block takes (one launch instead of three)
 
 namespace rfk {
-// counters (optional): POOL, LIVE (all three lists), PRIMS, CLIPQ and the
-// groups' slots zeroed for the kernels after it, and *marks (the binning pass's total of
-// (triangle, tile) bits).
+// Zeroes what a frame accumulates into: the masks (the buffer holds a multiple
+// of 16 bytes), the jobs' stats slots js[0 .. njobs), totals[0..2) (row words,
+// list entries), *marks (the binning pass's total of (triangle, tile) bits)
+// and the frame's counters.
+cudaError_t launch_zero(uint32_t *mask, size_t mask_words, StatsDev *js, uint32_t njobs, unsigned long long *totals,
+                        unsigned long long *marks, uint32_t *counters, int nsm, cudaStream_t s);
 cudaError_t launch_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv, float4 *cpos,
-                          uint8_t *coc, uint32_t *counters, unsigned long long *marks,
-                          int nsm, cudaStream_t s);
+                          uint8_t *coc, int nsm, cudaStream_t s);
 // Clip status, the clipping of the triangles that cross a plane, and each
 // input triangle's fan count tcnt.  queue: room for nt triangle indices.
 // place: each input triangle's first output slot into toff, taken from a
@@ -95,25 +99,24 @@ cudaError_t launch_mesh_bbox(const float *verts, uint32_t nverts, uint32_t strid
 size_t scan_scratch_words(uint32_t n);
 cudaError_t launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *scratch,
                         uint32_t *total, cudaStream_t s);
-// Triangle setup (k_setup), then scanline statistics, row records and tile
-// binning (k_bin_small for triangles of at most 8 and of 9 to 16 rows,
-// then k_bin).  rows holds rows_cap words; rows_total (zeroed here)
-// receives the words the frame asked for, each triangle's records placed
-// by k_setup from it (rows_total[1], zeroed too, is the lists' cursor); live (room for three times every output triangle)
-// receives the index of each triangle that passes the face-cull test: the
-// regular ones with at most 8 rows on the target (counters[RF_CNT_LIVE_SMALL]) in its second
-// third, with 9 to 16 rows (counters[RF_CNT_LIVE_MID]) in its last, the
-// rest (counters[RF_CNT_LIVE]) in its first; *marks receives the
-// (triangle, tile) bits set in all.  kind: the shader kind of every draw,
-// or RF_K_ANY (the binning kernels are specialised for the first).
-cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, uint32_t nt,
-                         uint32_t tile_w, const float4 *cpos, const uint32_t *tcnt,
-                         const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
+// Triangle setup (k_setup: also the row records and tile bits of triangles
+// of a few rows), then scanline statistics, row records and tile binning of
+// the others (k_bin_small for at most 16 rows, then k_bin), per raster group.
+// rows holds rows_cap words; rows_total receives the words the frame asked
+// for, each triangle's records placed by k_setup from it (rows_total[1] is
+// the lists' cursor); live (room for twice every output triangle) receives
+// the index of each triangle left for the binning pass, group after group:
+// those for k_bin (counters[RF_CNT_LIVE_G + g]) in its first half, the regular
+// ones with at most 16 rows on the target (counters[RF_CNT_LIVE_MID_G + g])
+// in its second; *marks receives the (triangle, tile) bits set in all.
+// sorted: perm and ptri give the depth-sorted order (rf_sort.cu).
+cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, uint32_t nj,
+                         const RasterGroup *groups, uint32_t ng, uint32_t nt, uint32_t tile_w, const float4 *cpos,
+                         const uint32_t *tcnt, const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
                          PrimRec *prims, unsigned long long *rows_total, uint32_t *rows,
                          unsigned long long rows_cap, RasterPrim *rprims, uint32_t *mask, uint32_t *live,
                          unsigned long long *marks, StatsDev *stats, uint32_t *counters, int nsm,
-                         cudaStream_t s, const uint32_t *perm = nullptr, const uint32_t *ptri = nullptr,
-                         int kind = RF_K_ANY);
+                         cudaStream_t s, const uint32_t *perm = nullptr, const uint32_t *ptri = nullptr);
 // The tiles' triangle lists and the rasteriser's work list, from the tile
 // masks and the marks total (slots: the warps the rasteriser keeps resident,
 // about).
@@ -122,7 +125,7 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
 // RF_ENT_SHIFT, y: the depth bound of a single output (RasterPrim::zmax),
 // NaN for more -- in submission order.  A tile's list comes in J.nseg pieces
 // (segs[J.seg_base + tile * J.nseg + k]: offset, entries), each placed by
-// atomics on *cursor (zeroed by launch_setup); past cap entries the piece is
+// atomics on *cursor; past cap entries the piece is
 // not written and counters[RF_CNT_LISTOVF] is set: the rasteriser then walks
 // the masks itself.
 // Work list: items (room for (RF_SPLIT_K + 1) * ntiles): items[ntiles ..

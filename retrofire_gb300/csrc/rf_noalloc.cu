@@ -62,7 +62,7 @@ constexpr size_t OFF_ROWTOT = al(OFF_MASK + (size_t)MAX_TILES * (MASK_WORDS + SU
 constexpr size_t OFF_RPRIMS = al(OFF_ROWTOT + 16);
 constexpr size_t OFF_LIVE =
     al(OFF_RPRIMS + (size_t)RF_NOALLOC_MAX_TRIS * RF_MAX_FAN * sizeof(RasterPrim));
-constexpr size_t OFF_MARKS = al(OFF_LIVE + (size_t)RF_NOALLOC_MAX_TRIS * RF_MAX_FAN * 12);
+constexpr size_t OFF_MARKS = al(OFF_LIVE + (size_t)RF_NOALLOC_MAX_TRIS * RF_MAX_FAN * 8);
 constexpr size_t OFF_ITEMS = al(OFF_MARKS + 16);
 constexpr size_t OFF_SEGS = al(OFF_ITEMS + (size_t)MAX_TILES * (RF_SPLIT_K + 1) * 4);
 constexpr size_t LIST_CAP = 32768;  // entries of the tiles' triangle lists (the masks are walked past it)
@@ -254,19 +254,18 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
     } else {
         k_na_put<<<1, 32, 0, s>>>(d, J, dd, jd);
         NA_CK(cudaGetLastError());
-        NA_CK(cudaMemsetAsync(mask, 0, (size_t)ntiles * (J.mask_words + J.sum_words) * 4, s));
-        NA_CK(rfk::launch_vertex(dd, 1, nverts, cpos, coc, cnt, marks, nsm, s));
+        NA_CK(rfk::launch_zero(mask, (size_t)ntiles * (J.mask_words + J.sum_words), sd, 1, rowtot, marks, cnt, nsm, s));
+        NA_CK(rfk::launch_vertex(dd, 1, nverts, cpos, coc, nsm, s));
         NA_CK(rfk::launch_clip(dd, 1, ntri, cpos, coc, tcnt, tpoly, toff, pool, RF_NOALLOC_MAX_TRIS,
                                cnt, nsm, s, toff, false));  // (the scan places the outputs)
         NA_CK(rfk::launch_scan(tcnt, toff, ntri, scan, cnt + RF_CNT_PRIMS, s));
-        NA_CK(rfk::launch_setup(dd, 1, jd, ntri, TILE_W, cpos, tcnt, toff, tpoly, pool, prims,
-                                rowtot, rows, ROWS_WORDS, rprims, mask, live,
-                                marks, sd, cnt, nsm, s, nullptr, nullptr, shader));
-        NA_CK(rfk::launch_lists(jd, 1, mask, ntiles, ntiles, toff, tcnt, rprims, marks, (uint32_t)nsm * 16u, items,
-                                cnt, segs, list, rowtot + 1, LIST_CAP, s));
         const bool fast = depth && flags->depth_test == RF_DEPTH_LESS && flags->color_write &&
                           flags->depth_write;
-        const RasterGroup group{shader, fast, 0u, ntiles};
+        const RasterGroup group{shader, fast, 0u, ntiles, 0u, (ntri + RF_SETUP_THREADS - 1) / RF_SETUP_THREADS, ntri};
+        NA_CK(rfk::launch_setup(dd, 1, jd, 1, &group, 1, ntri, TILE_W, cpos, tcnt, toff, tpoly, pool, prims,
+                                rowtot, rows, ROWS_WORDS, rprims, mask, live, marks, sd, cnt, nsm, s));
+        NA_CK(rfk::launch_lists(jd, 1, mask, ntiles, ntiles, toff, tcnt, rprims, marks, (uint32_t)nsm * 16u, items,
+                                cnt, segs, list, rowtot + 1, LIST_CAP, s));
         NA_CK(rfk::launch_raster(TILE_W, &group, 1, jd, 1, dd, prims, rprims, rows, tcnt, toff, mask, segs, list, ntiles, items,
                                  cnt, sd, WARPS, nsm, &s, 1));
     }

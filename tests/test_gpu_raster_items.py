@@ -51,6 +51,7 @@ def tris(seed, n, w, h, size, kind=rf.GOURAUD, repeat=1, cross=0.0):
 SHAPES = {
     "dots": dict(n=3000, size=(1, 3, 1, 3)),
     "slivers": dict(n=1500, size=(8, 40, 1, 3)),
+    "ribbons": dict(n=400, size=(150, 600, 1, 6)),
     "ten_rows": dict(n=1200, size=(4, 30, 9, 24)),
     "tall": dict(n=200, size=(2, 12, 60, 200)),
     "wide": dict(n=150, size=(300, 900, 20, 80)),
