@@ -139,11 +139,12 @@ struct rf_ctx {
     std::unordered_map<uint64_t, Target> targets;
     // per-frame scratch
     DevBuf draws, jobs, cpos, coc, tcnt, toff, tpoly, pool, prims, mask, scan, counters, stats;
-    DevBuf rowtot, rows, rprims, live, marks, items, jstats, clipq, segs, list;
+    DevBuf rowtot, rows, rprims, live, marks, items, jstats, clipq, segs, list, ent, tacc;
     DevBuf lrec, lmask;  // line pass
+    bool mask_suspect = false;  // a frame was cut short after its masks may have been marked
     // depth-sorted frames: sorted order, source triangles, per-draw counts,
     // sort scratch, the setup pass's draws / jobs, the raster's unit arrays
-    DevBuf perm, ptri, nout, dsort, vdraws, vjobs, vtoff, vtcnt;
+    DevBuf perm, ptri, nout, dsort, vdraws, vjobs;
     uint32_t *nout_host = nullptr;  // pinned, grown with the draw count
     size_t nout_host_cap = 0;
     // CUDA graphs of the launch sequence, keyed by frame shape (graph mode).
@@ -705,6 +706,20 @@ rf_status tune_tile(rf_ctx *ctx, const uint64_t key[5], uint32_t &TW, TuneState 
     return RF_OK;
 }
 
+// Room for the tile masks, which are all zero between frames: a new buffer is
+// zeroed, and so is one that a frame cut short by an error may have left
+// marked.
+rf_status ensure_mask(rf_ctx *ctx, size_t words) {
+    const void *old = ctx->mask.p;
+    rf_status st = ensure(ctx, ctx->mask, words * 4);
+    if (st) return st;
+    if (ctx->mask.p != old || ctx->mask_suspect) {
+        CK(cudaMemsetAsync(ctx->mask.p, 0, ctx->mask.cap, ctx->stream));
+        ctx->mask_suspect = false;
+    }
+    return RF_OK;
+}
+
 // One frame: the jobs of `in` (distinct targets), each with its draws in
 // order, as one pass of the pipeline over all of them.  per_job: kernels
 // count into per-job slots (ctx->jstats), folded into the running total at
@@ -751,7 +766,9 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     const uint32_t pool_cap = (uint32_t)nt;
     if ((st = ensure(ctx, ctx->pool, (size_t)pool_cap * RF_POLY_STORE * sizeof(PolyVert)))) return st;
     if ((st = ensure(ctx, ctx->prims, (size_t)nt * RF_MAX_FAN * sizeof(PrimRec)))) return st;
-    if ((st = ensure(ctx, ctx->mask, mask_words * 4))) return st;
+    if ((st = ensure_mask(ctx, mask_words))) return st;
+    if ((st = ensure(ctx, ctx->tacc, (size_t)ntiles * 8))) return st;
+    if ((st = ensure(ctx, ctx->ent, (size_t)nt * 8))) return st;
     if ((st = ensure(ctx, ctx->scan, rfk::scan_scratch_words((uint32_t)nt) * 4))) return st;
     if ((st = ensure(ctx, ctx->rowtot, 16))) return st;
     if ((st = ensure(ctx, ctx->rprims, (size_t)nt * RF_MAX_FAN * sizeof(RasterPrim)))) return st;
@@ -791,15 +808,14 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     }
     // The raster pass, its groups on two streams so that one group's last
     // tiles overlap the other's first.
-    auto raster = [&](const JobDev *jobs, const DrawDev *draws, const uint32_t *tcnt, const uint32_t *toff,
-                      uint32_t *counters, StatsDev *stats) -> rf_status {
+    auto raster = [&](const JobDev *jobs, const DrawDev *draws, uint32_t *counters, StatsDev *stats) -> rf_status {
         const cudaStream_t st2[2] = {ctx->stream, ctx->side};
         if (ng > 1) {
             CK(cudaEventRecord(ctx->side_fork, ctx->stream));
             CK(cudaStreamWaitEvent(ctx->side, ctx->side_fork, 0));
         }
         CK(rfk::launch_raster(TW, ctx->groups.data(), ng, jobs, nj, draws, P<PrimRec>(ctx->prims),
-                              P<RasterPrim>(ctx->rprims), P<uint32_t>(ctx->rows), tcnt, toff, P<uint32_t>(ctx->mask),
+                              P<RasterPrim>(ctx->rprims), P<uint32_t>(ctx->rows), P<uint2>(ctx->ent), P<uint32_t>(ctx->mask),
                               P<uint2>(ctx->segs), P<uint2>(ctx->list), ntiles, P<uint32_t>(ctx->items), counters, stats, ctx->warps, ctx->nsm, st2,
                               ng > 1 ? 2u : 1u));
         if (ng > 1) {
@@ -844,12 +860,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     auto enqueue = [&](bool marks) -> rf_status {
         auto mark = [&](int i) -> cudaError_t { return marks ? cudaEventRecord(ev[i], s) : cudaSuccess; };
         CK(mark(RF_STAGE_VERTEX));
-        CK(rfk::launch_zero(P<uint32_t>(ctx->mask), mask_words, kst, per_job ? nj : 0u,
-                            P<unsigned long long>(ctx->rowtot), P<unsigned long long>(ctx->marks), counters,
-                            ctx->nsm, s));
+        CK(rfk::launch_zero(P<uint32_t>(ctx->mask), ctx->mask.cap / 4, false, kst, per_job ? nj : 0u,
+                            P<unsigned long long>(ctx->tacc), ntiles, P<unsigned long long>(ctx->rowtot),
+                            P<unsigned long long>(ctx->marks), counters, ctx->nsm, s));
         if (any_cull) CK(rfk::launch_cull(P<DrawDev>(ctx->draws), ndraws, kst, ctx->nsm, s));
         CK(rfk::launch_vertex(dd, ndraws, (uint32_t)nv, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
-                              ctx->nsm, s));
+                              counters, ctx->nsm, s));
         CK(mark(RF_STAGE_CLIP));
         // (each triangle's output slots placed by the clip kernels: no scan)
         CK(rfk::launch_clip(dd, ndraws, (uint32_t)nt, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
@@ -862,14 +878,14 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
                              P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->toff), P<uint32_t>(ctx->tpoly),
                              P<PolyVert>(ctx->pool), P<PrimRec>(ctx->prims), P<unsigned long long>(ctx->rowtot),
                              P<uint32_t>(ctx->rows), ctx->rows_cap, P<RasterPrim>(ctx->rprims),
-                             P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
+                             P<uint2>(ctx->ent), P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
                              kst, counters, ctx->nsm, s));
-        CK(rfk::launch_lists(jd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(hj), P<uint32_t>(ctx->toff),
-                             P<uint32_t>(ctx->tcnt), P<RasterPrim>(ctx->rprims), P<unsigned long long>(ctx->marks),
+        CK(rfk::launch_lists(jd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(hj), P<uint2>(ctx->ent),
+                             P<unsigned long long>(ctx->tacc), P<unsigned long long>(ctx->marks),
                              (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, P<uint2>(ctx->segs),
                              P<uint2>(ctx->list), P<unsigned long long>(ctx->rowtot) + 1, ctx->list_cap, s));
         CK(mark(RF_STAGE_RASTER));
-        rf_status st2 = raster(jd, dd, P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->toff), counters, kst);
+        rf_status st2 = raster(jd, dd, counters, kst);
         if (st2) return st2;
         CK(mark(RF_STAGE_N));
         if (per_job) CK(rfk::launch_stats_fold(kst, nj, P<StatsDev>(ctx->stats), s));
@@ -887,12 +903,12 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     auto enqueue_sorted = [&]() -> rf_status {
         auto mark = [&](int i) -> cudaError_t { return ctx->timing ? cudaEventRecord(ev[i], s) : cudaSuccess; };
         CK(mark(RF_STAGE_VERTEX));
-        // (the masks are zeroed later, once their size is known)
-        CK(rfk::launch_zero(nullptr, 0, kst, per_job ? nj : 0u, P<unsigned long long>(ctx->rowtot),
+        CK(rfk::launch_zero(P<uint32_t>(ctx->mask), ctx->mask.cap / 4, false, kst, per_job ? nj : 0u,
+                            P<unsigned long long>(ctx->tacc), ntiles, P<unsigned long long>(ctx->rowtot),
                             P<unsigned long long>(ctx->marks), counters, ctx->nsm, s));
         if (any_cull) CK(rfk::launch_cull(P<DrawDev>(ctx->draws), ndraws, kst, ctx->nsm, s));
         CK(rfk::launch_vertex(dd, ndraws, (uint32_t)nv, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
-                              ctx->nsm, s));
+                              counters, ctx->nsm, s));
         CK(mark(RF_STAGE_CLIP));
         CK(rfk::launch_clip(dd, ndraws, (uint32_t)nt, P<float4>(ctx->cpos), P<uint8_t>(ctx->coc),
                             P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->tpoly), P<uint32_t>(ctx->toff),
@@ -940,15 +956,16 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         layout_blocks(vj, ctx->groups);
         const size_t vmask = vj.back().sum_base + (size_t)vj.back().tiles_x * vj.back().tiles_y * vj.back().sum_words;
         const uint32_t n32 = (uint32_t)np;
-        if ((st2 = ensure(ctx, ctx->mask, std::max<size_t>(vmask, 1) * 4))) return st2;
+        ctx->mask_suspect = false;  // (nothing marked yet)
+        if ((st2 = ensure_mask(ctx, std::max<size_t>(vmask, 1)))) return st2;
+        ctx->mask_suspect = true;
         if ((st2 = ensure(ctx, ctx->perm, (size_t)std::max<uint32_t>(n32, 1) * 4))) return st2;
         if ((st2 = ensure(ctx, ctx->ptri, (size_t)std::max<uint32_t>(n32, 1) * 4))) return st2;
         if ((st2 = ensure(ctx, ctx->dsort, rfk::dsort_scratch_bytes(n32)))) return st2;
         if ((st2 = ensure(ctx, ctx->scan,
                           rfk::scan_scratch_words(std::max<uint32_t>(rfk::dsort_scan_items(n32), (uint32_t)nt)) * 4)))
             return st2;
-        if ((st2 = ensure(ctx, ctx->vtoff, (size_t)std::max<uint32_t>(n32, 1) * 4))) return st2;
-        if ((st2 = ensure(ctx, ctx->vtcnt, (size_t)std::max<uint32_t>(n32, 1) * 4))) return st2;
+        if ((st2 = ensure(ctx, ctx->ent, (size_t)std::max<uint32_t>(n32, 1) * 8))) return st2;
         if ((st2 = ensure(ctx, ctx->segs, (size_t)pieces(vj) * 8))) return st2;
         if ((st2 = ensure(ctx, ctx->vdraws, vd.size() * sizeof(DrawDev)))) return st2;
         if ((st2 = ensure(ctx, ctx->vjobs, vj.size() * sizeof(JobDev)))) return st2;
@@ -961,31 +978,30 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
                              P<uint32_t>(ctx->toff), P<uint32_t>(ctx->tpoly), P<PolyVert>(ctx->pool),
                              counters, P<uint32_t>(ctx->perm), P<uint32_t>(ctx->ptri), ctx->dsort.p,
                              P<uint32_t>(ctx->scan), s));
-        CK(cudaMemsetAsync(ctx->mask.p, 0, vmask * 4, s));
-        CK(rfk::launch_iota(P<uint32_t>(ctx->vtoff), P<uint32_t>(ctx->vtcnt), n32, s));
         CK(rfk::launch_setup(vdd, ndraws, vjd, nj, ctx->groups.data(), ng, n32, TW, P<float4>(ctx->cpos),
                              P<uint32_t>(ctx->tcnt), P<uint32_t>(ctx->toff), P<uint32_t>(ctx->tpoly),
                              P<PolyVert>(ctx->pool), P<PrimRec>(ctx->prims), P<unsigned long long>(ctx->rowtot),
                              P<uint32_t>(ctx->rows), ctx->rows_cap, P<RasterPrim>(ctx->rprims),
-                             P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
+                             P<uint2>(ctx->ent), P<uint32_t>(ctx->mask), P<uint32_t>(ctx->live), P<unsigned long long>(ctx->marks),
                              kst, counters, ctx->nsm, s, P<uint32_t>(ctx->perm), P<uint32_t>(ctx->ptri)));
-        CK(rfk::launch_lists(vjd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(vj), P<uint32_t>(ctx->vtoff),
-                             P<uint32_t>(ctx->vtcnt), P<RasterPrim>(ctx->rprims), P<unsigned long long>(ctx->marks),
+        CK(rfk::launch_lists(vjd, nj, P<uint32_t>(ctx->mask), ntiles, pieces(vj), P<uint2>(ctx->ent),
+                             P<unsigned long long>(ctx->tacc), P<unsigned long long>(ctx->marks),
                              (uint32_t)ctx->nsm * 16u, P<uint32_t>(ctx->items), counters, P<uint2>(ctx->segs),
                              P<uint2>(ctx->list), P<unsigned long long>(ctx->rowtot) + 1, ctx->list_cap, s));
         CK(mark(RF_STAGE_RASTER));
-        if ((st2 = raster(vjd, vdd, P<uint32_t>(ctx->vtcnt), P<uint32_t>(ctx->vtoff), counters, kst))) return st2;
+        if ((st2 = raster(vjd, vdd, counters, kst))) return st2;
         CK(mark(RF_STAGE_N));
         if (per_job) CK(rfk::launch_stats_fold(kst, nj, P<StatsDev>(ctx->stats), s));
         // draw counts, sort keys, per digit pass a histogram, a scan of 1 or 3
-        // launches and a scatter, the unit arrays
+        // launches and a scatter
         const uint32_t dpasses = 4 + (ndraws > 1 ? (ndraws > 256 ? (ndraws > 65536 ? 3 : 2) : 1) : 0);
         const uint32_t sitems = rfk::dsort_scan_items(n32);
-        sort_kernels = 2 + (n32 ? 1 + dpasses * (2 + (sitems <= RF_SCAN_BLOCK_ITEMS ? 1 : 3)) + 1 : 0);
+        sort_kernels = 2 + (n32 ? 1 + dpasses * (2 + (sitems <= RF_SCAN_BLOCK_ITEMS ? 1 : 3)) : 0);
         return RF_OK;
     };
 
     if (tuned) CK(cudaEventRecord(tuned->e0, s));
+    ctx->mask_suspect = true;  // (until every launch is queued)
     if (sorted) {
         if ((st = enqueue_sorted())) return st;
     } else if (ctx->graphs && !ctx->timing) {
@@ -1033,6 +1049,7 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     } else {
         if ((st = enqueue(ctx->timing))) return st;
     }
+    ctx->mask_suspect = false;
     if (tuned) {
         CK(cudaEventRecord(tuned->e1, s));
         tuned->pending = true;
@@ -1242,9 +1259,8 @@ rf_status rf_ctx_destroy(rf_ctx *ctx) {
     DevBuf *bufs[] = {&ctx->draws, &ctx->jobs, &ctx->cpos, &ctx->coc, &ctx->tcnt, &ctx->toff,
                       &ctx->tpoly, &ctx->pool, &ctx->prims, &ctx->mask, &ctx->scan,
                       &ctx->counters, &ctx->stats,
-                      &ctx->rowtot, &ctx->clipq, &ctx->rows, &ctx->rprims, &ctx->live, &ctx->marks, &ctx->items, &ctx->segs, &ctx->list, &ctx->jstats, &ctx->lrec, &ctx->lmask,
-                      &ctx->perm, &ctx->ptri, &ctx->nout, &ctx->dsort, &ctx->vdraws, &ctx->vjobs,
-                      &ctx->vtoff, &ctx->vtcnt};
+                      &ctx->rowtot, &ctx->clipq, &ctx->rows, &ctx->rprims, &ctx->live, &ctx->marks, &ctx->items, &ctx->segs, &ctx->list, &ctx->ent, &ctx->tacc, &ctx->jstats, &ctx->lrec, &ctx->lmask,
+                      &ctx->perm, &ctx->ptri, &ctx->nout, &ctx->dsort, &ctx->vdraws, &ctx->vjobs};
     for (UploadBuf &u : ctx->uploads) {
         if (u.p) cudaFreeHost(u.p);
         if (u.copied) cudaEventDestroy(u.copied);
@@ -1422,7 +1438,7 @@ rf_status rf_render_lines(rf_ctx *ctx, rf_mesh mesh, int32_t shader, const rf_un
         CK(cudaMemsetAsync(counters + RF_CNT_QUEUE, 0, 4, s));
         CK(cudaMemsetAsync(ctx->lmask.p, 0, mwords * 4, s));
         CK(rfk::launch_vertex(P<DrawDev>(ctx->draws), 1, m.nverts, P<float4>(ctx->cpos),
-                              P<uint8_t>(ctx->coc), ctx->nsm, s));
+                              P<uint8_t>(ctx->coc), nullptr, ctx->nsm, s));
         CK(rfk::launch_lines(P<DrawDev>(ctx->draws), P<JobDev>(ctx->jobs), m.ntri, P<float4>(ctx->cpos),
                              P<uint8_t>(ctx->coc), P<LineRec>(ctx->lrec), P<uint32_t>(ctx->lmask), ntiles,
                              counters + RF_CNT_QUEUE, P<StatsDev>(ctx->stats), ctx->nsm, s));

@@ -14,8 +14,10 @@
 //   prim[p]  PrimRec  triangle setup: two ScanlineIter starts (raster.rs:248-302)
 //   mask     u32      per tile, one bit per input triangle of the job that
 //                     touches the tile; bit order = submission order
-//   list     uint2    the tiles' set bits as triangle entries (RF_ENT_*), in
-//                     submission order, a piece per (tile, segment)
+//   ent[t]   uint2    t's entry in the tiles' lists (RF_ENT_*): its outputs
+//                     and their depth bound; written for every t with a bit
+//   list     uint2    the tiles' set bits as those entries, in submission
+//                     order, a piece per (tile, segment)
 #ifndef RF_INTERNAL_CUH
 #define RF_INTERNAL_CUH
 
@@ -127,7 +129,7 @@ struct PrimRec {
     uint32_t rloc;    // word offset of its row records in the frame's row buffer
     uint32_t rwords;  // words of row records; 0 = rasterised from this record instead
     uint32_t job;     // scene (job) of its draw
-    uint32_t pad_;
+    uint32_t fan;     // 1: one of several pieces of a clipped triangle
     HalfRec half[2];  // what the binning pass reads (RF_PRIM_CORE_BYTES)
     HalfRuns runs[2]; // written only for a triangle without row records
 };

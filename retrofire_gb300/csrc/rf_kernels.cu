@@ -62,16 +62,21 @@ __device__ __forceinline__ uint32_t zdiv_mask_of(int32_t shader) {
 
 }  // namespace
 
-// What a frame's kernels accumulate into, zeroed in one launch: the tile
-// masks (n16 16-byte words; their buffer is padded to that), the jobs' stats
-// slots, the row and list totals, the marks total and the counters that do
-// not run on from frame to frame.
-__global__ void k_zero(uint4 *__restrict__ mask, size_t n16, unsigned long long *__restrict__ js, uint32_t njs,
-                       unsigned long long *__restrict__ totals, unsigned long long *__restrict__ marks,
-                       uint32_t *__restrict__ counters) {
+// What a frame's kernels accumulate into, zeroed in one launch: the jobs'
+// stats slots, the tiles' entry counts, the row and list totals, the marks
+// total and the counters that do not run on from frame to frame.  The tile
+// masks (n16 16-byte words) are zero already -- k_tile_lists leaves them so --
+// unless the dirty counter says otherwise: zeroing them every frame took 39 us
+// of the 500 k-triangle grid's frame (255 MB at tile width 16).
+__global__ void k_zero(uint4 *__restrict__ mask, size_t n16, const uint32_t *__restrict__ dirty,
+                       unsigned long long *__restrict__ js, uint32_t njs, unsigned long long *__restrict__ tacc,
+                       uint32_t ntiles, unsigned long long *__restrict__ totals,
+                       unsigned long long *__restrict__ marks, uint32_t *__restrict__ counters) {
     const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = i0; i < n16; i += step) mask[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (!dirty || *dirty)
+        for (size_t i = i0; i < n16; i += step) mask[i] = make_uint4(0u, 0u, 0u, 0u);
     for (size_t i = i0; i < njs; i += step) js[i] = 0ull;
+    for (size_t i = i0; i < ntiles; i += step) tacc[i] = 0ull;
     if (blockIdx.x == 0) {
         if (threadIdx.x < 2) totals[threadIdx.x] = 0ull;
         if (threadIdx.x == 0) {
@@ -80,7 +85,7 @@ __global__ void k_zero(uint4 *__restrict__ mask, size_t n16, unsigned long long 
             counters[RF_CNT_PRIMS] = 0;
             counters[RF_CNT_CLIPQ] = 0;
         }
-        if (threadIdx.x < RF_CNT_N - RF_CNT_QUEUE_G) counters[RF_CNT_QUEUE_G + threadIdx.x] = 0;  // the groups' and LISTOVF
+        if (threadIdx.x < RF_CNT_N - RF_CNT_QUEUE_G) counters[RF_CNT_QUEUE_G + threadIdx.x] = 0;  // the groups'
     }
 }
 
@@ -89,7 +94,8 @@ __global__ void k_zero(uint4 *__restrict__ mask, size_t n16, unsigned long long 
 // and outcode (clip.rs:240-242, 303-309).
 // ---------------------------------------------------------------------------
 __global__ void k_vertex(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nv_total,
-                         float4 *__restrict__ cpos, uint8_t *__restrict__ coc) {
+                         float4 *__restrict__ cpos, uint8_t *__restrict__ coc, uint32_t *__restrict__ counters) {
+    if (counters && blockIdx.x == 0 && threadIdx.x == 0) counters[RF_CNT_MASKDIRTY] = 0;  // (k_zero is done)
     // Warp-uniform loop (the draw lookup is shared by the warp's lanes).
     for (uint32_t wbase = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); wbase < nv_total;
          wbase += gridDim.x * blockDim.x) {
@@ -846,8 +852,8 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
         uint32_t block0, uint32_t nblocks, uint32_t tile_w, const float4 *__restrict__ cpos, const uint32_t *__restrict__ tcnt,
         const uint32_t *__restrict__ toff, const uint32_t *__restrict__ tpoly, const PolyVert *__restrict__ pool,
         PrimRec *__restrict__ prims, unsigned long long *__restrict__ rows_total, uint32_t *__restrict__ rows,
-        unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint32_t *__restrict__ mask,
-        uint32_t *__restrict__ live, uint32_t *__restrict__ live_n, uint32_t *__restrict__ live_mid,
+        unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint2 *__restrict__ ent,
+        uint32_t *__restrict__ mask, uint32_t *__restrict__ live, uint32_t *__restrict__ live_n, uint32_t *__restrict__ live_mid,
         uint32_t *__restrict__ live_mid_n, unsigned long long *__restrict__ marks, StatsDev *__restrict__ stats,
         const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ptri) {
     constexpr uint32_t FULL = 0xFFFFFFFFu, NONE = 0xFFFFFFFFu;
@@ -900,6 +906,9 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
             }
         }
         const uint32_t maxc = __reduce_max_sync(FULL, cnt);
+        // The entry of a triangle of several pieces; a single one's comes with
+        // its depth bound.
+        if (cnt > 1u) ent[gt] = make_uint2(p0 | (cnt - 1u) << RF_ENT_SHIFT, 0x7FFFFFFFu);
         for (uint32_t c = 0; c < maxc; ++c) {
             const bool have = c < cnt;
             bool keep = false;      // passes the face-cull test
@@ -968,6 +977,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                     P.rloc = 0;
                     P.rwords = 0;
                     P.job = job;
+                    P.fan = cnt > 1u ? 1u : 0u;
                     prims_o += 1;
                     // (how wide, before the sort)
                     const float wide = fsub(fmaxf(fmaxf(sv[0].x, sv[1].x), sv[2].x),
@@ -1127,6 +1137,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
             const uint32_t smalls = __ballot_sync(FULL, small);
             uint32_t bal = __ballot_sync(FULL, keep);
             const uint32_t dst = p0 + c;
+            if (small && cnt == 1u) ent[gt] = make_uint2(dst, f2u(zhi));
             if (small) {  // the slot now holds its RasterPrim (dvdx's source lies past it)
                 const uint32_t base_w = P.rloc;
                 const int32_t kind = P.kind;
@@ -1200,7 +1211,7 @@ __global__ void __launch_bounds__(256, 4)
 k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
       PrimRec *__restrict__ prims, const uint32_t *__restrict__ live, uint32_t tile_w,
       uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims,
-      uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
+      uint2 *__restrict__ ent, uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
       unsigned long long *__restrict__ marks, const uint32_t *__restrict__ live_n) {
     const uint32_t lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & 7;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1460,6 +1471,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
             }
         }
         __syncwarp();
+        if (lane == 0 && !P->fan) ent[P->tri] = make_uint2(p, f2u(R->zmax));
         {
             const uint4 *src = reinterpret_cast<const uint4 *>(R);
             uint4 *dst = reinterpret_cast<uint4 *>(rprims + p);
@@ -1489,8 +1501,8 @@ template <int NCT, uint32_t G>
 __global__ void __launch_bounds__(256, 4)
 k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             const uint32_t *__restrict__ live_small, uint32_t *__restrict__ live, uint32_t tile_w,
-            uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint32_t *__restrict__ mask,
-            StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
+            uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint2 *__restrict__ ent,
+            uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
             unsigned long long *__restrict__ marks, const uint32_t *__restrict__ small_n,
             uint32_t *__restrict__ live_n) {
     static_assert(G == 8 || G == 16, "group sizes");
@@ -1647,6 +1659,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             // The triangle's depth bound: the largest of its rows'.
             for (int o2 = G / 2; o2 > 0; o2 >>= 1) zhi = fmaxf(zhi, __shfl_xor_sync(gmask, zhi, o2));
             if (gl == 0) R->zmax = zhi;
+            if (gl == 0 && !P->fan) ent[P->tri] = make_uint2(e, f2u(zhi));
             __syncwarp(gmask);
             const uint4 *rs = reinterpret_cast<const uint4 *>(R);
             uint4 *dst = reinterpret_cast<uint4 *>(rprims + e);
@@ -1685,11 +1698,8 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
 // triangles in order: a row belongs to one slice).  The list is the heavy
 // tiles and the slices of the crowded ones, in no particular order, then
 // every tile in index order, RF_ITEM_SKIP where the tile went to the first
-// part.  A tile's nonzero mask words (the set bits of its summary words)
-// stand for its triangle count: at most the count, about it where the tile's
-// triangles are scattered through the submission order; where most words are
-// nonzero the bits are counted instead.  A crowded tile is one whose count
-// exceeds twice the frame's marks per resident warp: its walk alone would
+// part.  A crowded tile is one whose triangles
+// exceed twice the frame's marks per resident warp: its walk alone would
 // outlast two warps' fair shares of the pass, so splitting it shortens the
 // pass.
 #define RF_SPLIT_MIN 64u  // a tile with fewer binned triangles is never split
@@ -1733,12 +1743,11 @@ __device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t k) {
 }  // namespace
 
 __global__ void __launch_bounds__(RF_LIST_WARPS * 32)
-k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__restrict__ mask,
-             uint32_t ntiles, uint32_t npieces, const uint32_t *__restrict__ toff,
-             const uint32_t *__restrict__ tcnt, const RasterPrim *__restrict__ rprims,
-             const unsigned long long *__restrict__ marks, uint32_t slots, uint32_t *__restrict__ items,
+k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict__ mask,
+             uint32_t ntiles, uint32_t npieces, const uint2 *__restrict__ ent,
+             unsigned long long *__restrict__ tacc, const unsigned long long *__restrict__ marks, uint32_t slots, uint32_t *__restrict__ items,
              uint32_t *__restrict__ extras, uint2 *__restrict__ segs, uint2 *__restrict__ list,
-             unsigned long long *__restrict__ cursor, unsigned long long cap, uint32_t *__restrict__ ovf) {
+             unsigned long long *__restrict__ cursor, unsigned long long cap, uint32_t *__restrict__ dirty) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t piece = blockIdx.x * RF_LIST_WARPS + w;
@@ -1748,8 +1757,8 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__res
                                             [&](uint32_t i) { return (uint32_t)jobs[i].nth_seg; })].nth];
     const uint32_t r = (have ? piece : npieces - 1u) - (uint32_t)J.seg_base;
     const uint32_t lt = r / J.nseg, sg = r - lt * J.nseg, tile = J.tile_base + lt;
-    const uint32_t *sw = mask + J.sum_base + (size_t)lt * J.sum_words;
-    const uint32_t *mw = mask + J.mask_base + (size_t)lt * J.mask_words;
+    uint32_t *sw = mask + J.sum_base + (size_t)lt * J.sum_words;
+    uint32_t *mw = mask + J.mask_base + (size_t)lt * J.mask_words;
     const uint32_t s0 = sg * J.seg_words, s1 = have ? min(s0 + J.seg_words, J.sum_words) : s0;
     // Steps over the piece's nonzero mask words in order, up to 32 a step, one a
     // lane (m, at index wi): false when there are none left.
@@ -1795,8 +1804,8 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__res
     unsigned long long off = place[w];
     const bool fits = off + n <= cap;
     if (lane == 0) {
-        segs[piece] = make_uint2((uint32_t)off, fits ? n : 0u);
-        if (!fits) *ovf = 1u;
+        segs[piece] = make_uint2((uint32_t)off, fits ? n : RF_SEG_WALK);
+        if (!fits) *dirty = 1u;
     }
     if (fits && n) {
         const bool again = steps > 1u;  // (a single step's words are still here)
@@ -1805,34 +1814,29 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, const uint32_t *__res
             vk = vtotal = 0;
         }
         while (!again || step()) {
+            if (m) mw[wi] = 0u;  // (read for the last time)
             // The words' triangles, 32 at a time, one a lane.
             const uint32_t incl = warp_incl(__popc(m), lane), total = __shfl_sync(FULL, incl, 31);
             for (uint32_t q = lane; q - lane < total; q += 32u) {
                 const uint32_t M = lane_of(incl, q), mM = __shfl_sync(FULL, m, M);
                 const uint32_t ex = __shfl_sync(FULL, incl - __popc(m), M), wM = __shfl_sync(FULL, wi, M);
-                if (q < total) {
-                    const uint32_t gt = J.tri_base + wM * 32u + nth_bit(mM, q - ex + 1u);
-                    const uint32_t p = toff[gt], c = tcnt[gt];
-                    list[off + q] = make_uint2(p | (c - 1u) << RF_ENT_SHIFT, c == 1u ? f2u(rprims[p].zmax) : 0x7FFFFFFFu);
-                }
+                if (q < total) list[off + q] = __ldg(ent + J.tri_base + wM * 32u + nth_bit(mM, q - ex + 1u));
             }
             off += total;
             if (!again) break;
         }
     }
-    if (sg != 0u) return;
-    // The tile's work item.
-    uint32_t c = 0;
-    for (uint32_t i = lane; i < J.sum_words; i += 32) c += __popc(sw[i]);
-    c = __reduce_add_sync(FULL, c);
-    if (2u * c >= J.mask_words) {
-        // Half the mask words or more are nonzero: they say little about
-        // the count, so count the bits (a few small busy scenes do this).
-        c = 0;
-        for (uint32_t i = lane; i < J.mask_words; i += 32) c += __popc(mw[i]);
-        c = __reduce_add_sync(FULL, c);
-    }
+    if (fits)
+        for (uint32_t i = s0 + lane; i < s1; i += 32u)
+            if (sw[i]) sw[i] = 0u;
+    // The tile's work item, by the last of its pieces to come here.
     if (lane == 0) {
+        uint32_t c = n;
+        if (J.nseg > 1u) {
+            const unsigned long long before = atomicAdd(tacc + tile, (1ull << 32) + n);
+            if ((uint32_t)(before >> 32) + 1u != J.nseg) return;
+            c += (uint32_t)before;
+        }
         const unsigned long long share2 = 2ull * *marks / slots;
         const uint32_t thr = (uint32_t)min(max((unsigned long long)RF_SPLIT_MIN, share2), 0xFFFFFFFFull);
         const bool crowded = c > thr;
@@ -1864,20 +1868,24 @@ __global__ void k_fill(uint32_t *__restrict__ color, float *__restrict__ depth, 
 // ---------------------------------------------------------------------------
 namespace rfk {
 
-cudaError_t launch_zero(uint32_t *mask, size_t mask_words, StatsDev *js, uint32_t njobs, unsigned long long *totals,
+cudaError_t launch_zero(uint32_t *mask, size_t mask_words, bool masks, StatsDev *js, uint32_t njobs,
+                        unsigned long long *tacc, uint32_t ntiles, unsigned long long *totals,
                         unsigned long long *marks, uint32_t *counters, int nsm, cudaStream_t s) {
-    const size_t n16 = (mask_words + 3) / 4;
-    const uint32_t blocks = (uint32_t)std::min<size_t>((n16 + 255) / 256 + 1, (size_t)nsm * 8);
-    k_zero<<<blocks, 256, 0, s>>>(reinterpret_cast<uint4 *>(mask), n16, reinterpret_cast<unsigned long long *>(js),
-                                  njobs * (uint32_t)(sizeof(StatsDev) / 8), totals, marks, counters);
+    const size_t n16 = mask_words / 4;
+    // (a grid for the masks only when they are certain to be cleared)
+    const size_t work = std::max<size_t>(masks ? n16 : 0, ntiles);
+    const uint32_t blocks = (uint32_t)std::min<size_t>((work + 255) / 256 + 1, (size_t)nsm * 8);
+    k_zero<<<blocks, 256, 0, s>>>(reinterpret_cast<uint4 *>(mask), n16, masks ? nullptr : counters + RF_CNT_MASKDIRTY,
+                                  reinterpret_cast<unsigned long long *>(js),
+                                  njobs * (uint32_t)(sizeof(StatsDev) / 8), tacc, ntiles, totals, marks, counters);
     return cudaGetLastError();
 }
 
 cudaError_t launch_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv, float4 *cpos,
-                          uint8_t *coc, int nsm, cudaStream_t s) {
+                          uint8_t *coc, uint32_t *counters, int nsm, cudaStream_t s) {
     if (nv == 0) return cudaSuccess;
     uint32_t blocks = min((nv + 255) / 256, (uint32_t)nsm * 16);
-    k_vertex<<<blocks, 256, 0, s>>>(draws, nd, nv, cpos, coc);
+    k_vertex<<<blocks, 256, 0, s>>>(draws, nd, nv, cpos, coc, counters);
     return cudaGetLastError();
 }
 
@@ -1924,7 +1932,7 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
                          const RasterGroup *groups, uint32_t ng, uint32_t nt, uint32_t tile_w, const float4 *cpos,
                          const uint32_t *tcnt, const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
                          PrimRec *prims, unsigned long long *rows_total, uint32_t *rows,
-                         unsigned long long rows_cap, RasterPrim *rprims, uint32_t *mask, uint32_t *live,
+                         unsigned long long rows_cap, RasterPrim *rprims, uint2 *ent, uint32_t *mask, uint32_t *live,
                          unsigned long long *marks, StatsDev *stats, uint32_t *counters, int nsm,
                          cudaStream_t s, const uint32_t *perm, const uint32_t *ptri) {
     // (A depth-sorted frame's triangles are single clipped pieces.)
@@ -1948,7 +1956,7 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
         const uint32_t blocks = min(groups[g].nblocks, (uint32_t)nsm * 32);
         setup<<<blocks, RF_SETUP_THREADS, 0, s>>>(draws, nd, jobs, nj, groups[g].block0, groups[g].nblocks, tile_w,
                                                   cpos, tcnt, toff, tpoly, pool, prims, rows_total, rows, rows_cap,
-                                                  rprims, mask, big, big_n, mid, mid_n, marks, stats, perm, ptri);
+                                                  rprims, ent, mask, big, big_n, mid, mid_n, marks, stats, perm, ptri);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         // The triangles left for the binning pass, sixteen lanes each up to
@@ -1956,10 +1964,10 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
         // smaller ones that found no room for their records); the counts are
         // only known on the device.
         const uint32_t sblocks = min((gt + 31) / 32, (uint32_t)nsm * 4);
-        bin16<<<sblocks, 256, 0, s>>>(jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, mask, stats,
+        bin16<<<sblocks, 256, 0, s>>>(jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                       counters, marks, mid_n, big_n);
         const uint32_t wblocks = min((gt * 2 + 7) / 8, (uint32_t)nsm * 16);
-        bin<<<wblocks, 256, 0, s>>>(draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, mask, stats,
+        bin<<<wblocks, 256, 0, s>>>(draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                     counters, marks, big_n);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         big += (size_t)gt * fan;
@@ -1968,24 +1976,23 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
     return cudaSuccess;
 }
 
-cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles, uint32_t npieces,
-                         const uint32_t *toff, const uint32_t *tcnt, const RasterPrim *rprims,
-                         const unsigned long long *marks, uint32_t slots, uint32_t *items, uint32_t *counters,
+cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, uint32_t *mask, uint32_t ntiles, uint32_t npieces,
+                         const uint2 *ent, unsigned long long *tacc, const unsigned long long *marks,
+                         uint32_t slots, uint32_t *items, uint32_t *counters,
                          uint2 *segs, uint2 *list, unsigned long long *cursor, unsigned long long cap,
                          cudaStream_t s) {
     if (ntiles == 0) return cudaSuccess;
     k_tile_lists<<<(npieces + RF_LIST_WARPS - 1) / RF_LIST_WARPS, RF_LIST_WARPS * 32, 0, s>>>(
-        jobs, nj, mask, ntiles, npieces, toff, tcnt, rprims, marks, slots ? slots : 1u, items,
-        counters + RF_CNT_ITEMS_G, segs, list, cursor, cap, counters + RF_CNT_LISTOVF);
+        jobs, nj, mask, ntiles, npieces, ent, tacc, marks, slots ? slots : 1u, items,
+        counters + RF_CNT_ITEMS_G, segs, list, cursor, cap, counters + RF_CNT_MASKDIRTY);
     return cudaGetLastError();
 }
 
 cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng, const JobDev *jobs, uint32_t nj,
                           const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, const uint32_t *rows,
-                          const uint32_t *tcnt, const uint32_t *toff, const uint32_t *mask, const uint2 *segs,
+                          const uint2 *ent, const uint32_t *mask, const uint2 *segs,
                           const uint2 *list, uint32_t ntiles_all, const uint32_t *items_all, uint32_t *counters,
                           StatsDev *stats, uint32_t warps, int nsm, const cudaStream_t *st, uint32_t nst) {
-    const uint32_t *listovf = counters + RF_CNT_LISTOVF;
     for (uint32_t g = 0; g < ng; ++g) {
         const uint32_t ntiles = groups[g].ntiles, tile0 = groups[g].tile0;
         if (ntiles == 0) continue;

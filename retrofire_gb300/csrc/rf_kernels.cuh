@@ -58,24 +58,27 @@ struct RasterGroup {
 #define RF_CNT_PRIMS 4    // total output prims (scan total)
 #define RF_CNT_QUEUE 5    // tile queue head of the line pass
 #define RF_CNT_ROWSOVF 6  // triangles rasterised without row records (buffer full)
+#define RF_CNT_MASKDIRTY 9 // nonzero: the tile masks were not left zero
 #define RF_CNT_CLIPQ 10   // triangles queued for clipping
 #define RF_CNT_QUEUE_G 16     // + g: work-list queue head of raster group g
 #define RF_CNT_ITEMS_G (RF_CNT_QUEUE_G + RF_MAX_GROUPS)  // + g: its heavy tiles and crowded tiles' slices
 #define RF_CNT_LIVE_G (RF_CNT_ITEMS_G + RF_MAX_GROUPS)   // + g: its live triangles, binned a warp each
 #define RF_CNT_LIVE_MID_G (RF_CNT_LIVE_G + RF_MAX_GROUPS)  // + g: ... sixteen lanes each (at most 16 rows)
-#define RF_CNT_LISTOVF (RF_CNT_LIVE_MID_G + RF_MAX_GROUPS)  // nonzero: the triangle lists did not fit
-#define RF_CNT_N (RF_CNT_LISTOVF + 1)
+#define RF_CNT_N (RF_CNT_LIVE_MID_G + RF_MAX_GROUPS)
 #define RF_SCAN_BLOCK_ITEMS 4096u  // values one scan block takes (one launch instead of three)
 
 namespace rfk {
-// Zeroes what a frame accumulates into: the masks (the buffer holds a multiple
-// of 16 bytes), the jobs' stats slots js[0 .. njobs), totals[0..2) (row words,
-// list entries), *marks (the binning pass's total of (triangle, tile) bits)
-// and the frame's counters.
-cudaError_t launch_zero(uint32_t *mask, size_t mask_words, StatsDev *js, uint32_t njobs, unsigned long long *totals,
+// Zeroes what a frame accumulates into: the jobs' stats slots js[0 .. njobs),
+// the tiles' entry counts, totals[0..2) (row words, list entries), *marks
+// (the binning pass's total of (triangle, tile) bits), the frame's counters
+// and -- when the last frame left them dirty, or with `masks` -- the whole mask
+// buffer (mask_words, a multiple of 4).  launch_vertex clears the dirty mark
+// (counters: nullptr for none).
+cudaError_t launch_zero(uint32_t *mask, size_t mask_words, bool masks, StatsDev *js, uint32_t njobs,
+                        unsigned long long *tacc, uint32_t ntiles, unsigned long long *totals,
                         unsigned long long *marks, uint32_t *counters, int nsm, cudaStream_t s);
 cudaError_t launch_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv, float4 *cpos,
-                          uint8_t *coc, int nsm, cudaStream_t s);
+                          uint8_t *coc, uint32_t *counters, int nsm, cudaStream_t s);
 // Clip status, the clipping of the triangles that cross a plane, and each
 // input triangle's fan count tcnt.  queue: room for nt triangle indices.
 // place: each input triangle's first output slot into toff, taken from a
@@ -114,20 +117,23 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
                          const RasterGroup *groups, uint32_t ng, uint32_t nt, uint32_t tile_w, const float4 *cpos,
                          const uint32_t *tcnt, const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
                          PrimRec *prims, unsigned long long *rows_total, uint32_t *rows,
-                         unsigned long long rows_cap, RasterPrim *rprims, uint32_t *mask, uint32_t *live,
+                         unsigned long long rows_cap, RasterPrim *rprims, uint2 *ent, uint32_t *mask, uint32_t *live,
                          unsigned long long *marks, StatsDev *stats, uint32_t *counters, int nsm,
                          cudaStream_t s, const uint32_t *perm = nullptr, const uint32_t *ptri = nullptr);
 // The tiles' triangle lists and the rasteriser's work list, from the tile
 // masks and the marks total (slots: the warps the rasteriser keeps resident,
 // about).
 // Lists: the set bits of every tile's mask as entries, one per input
-// triangle -- x: its first output triangle | (its outputs - 1) <<
+// triangle, in submission order: ent[t], written by the setup and binning
+// passes -- x: its first output triangle | (its outputs - 1) <<
 // RF_ENT_SHIFT, y: the depth bound of a single output (RasterPrim::zmax),
-// NaN for more -- in submission order.  A tile's list comes in J.nseg pieces
-// (segs[J.seg_base + tile * J.nseg + k]: offset, entries), each placed by
-// atomics on *cursor; past cap entries the piece is
-// not written and counters[RF_CNT_LISTOVF] is set: the rasteriser then walks
-// the masks itself.
+// NaN for more.  A tile's list comes in J.nseg pieces (segs[J.seg_base + tile
+// * J.nseg + k]: offset, entries), each placed by atomics on *cursor; a piece
+// that would end past cap entries is marked RF_SEG_WALK instead and the
+// rasteriser walks its masks.  The masks are left zero for the next frame,
+// but for the pieces marked: then counters[RF_CNT_MASKDIRTY] is set and
+// the next launch_zero clears them all.  tacc (a word pair per tile, zeroed
+// by launch_zero) gathers a tile's entries over its pieces.
 // Work list: items (room for (RF_SPLIT_K + 1) * ntiles): items[ntiles ..
 // ntiles + extra) first -- heavy tiles (tile << RF_ITEM_SHIFT) and the row
 // slices of crowded tiles (tile << RF_ITEM_SHIFT | k, k = 1 .. RF_SPLIT_K) --
@@ -138,9 +144,9 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
 #define RF_ENT_SHIFT 29u
 #define RF_ENT_MASK ((1u << RF_ENT_SHIFT) - 1u)
 static_assert(RF_MAX_FAN <= 8, "an entry holds a fan's size");
-cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, const uint32_t *mask, uint32_t ntiles, uint32_t npieces,
-                         const uint32_t *toff, const uint32_t *tcnt, const RasterPrim *rprims,
-                         const unsigned long long *marks, uint32_t slots, uint32_t *items, uint32_t *counters,
+#define RF_SEG_WALK 0xFFFFFFFFu
+cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, uint32_t *mask, uint32_t ntiles, uint32_t npieces,
+                         const uint2 *ent, unsigned long long *tacc, const unsigned long long *marks, uint32_t slots, uint32_t *items, uint32_t *counters,
                          uint2 *segs, uint2 *list, unsigned long long *cursor, unsigned long long cap,
                          cudaStream_t s);
 #ifndef RF_SPLIT_K
@@ -154,11 +160,11 @@ static_assert(RF_TILE_H % RF_SPLIT_K == 0 && RF_SPLIT_K < 16, "row slices");
 // The launchers per tile width (rf_raster.cuh).
 #define RF_RASTER_PARAMS                                                                              \
     const JobDev *jobs, uint32_t nj, const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, \
-        const uint32_t *rows, const uint32_t *tcnt, const uint32_t *toff, const uint32_t *mask,         \
-        const uint2 *segs, const uint2 *list, const uint32_t *listovf, const uint32_t *items, uint32_t ntiles, const uint32_t *first, const uint32_t *nfirst,          \
+        const uint32_t *rows, const uint2 *ent, const uint32_t *mask, const uint2 *segs,                 \
+        const uint2 *list, const uint32_t *items, uint32_t ntiles, const uint32_t *first, const uint32_t *nfirst,          \
         uint32_t *queue, StatsDev *stats, uint32_t warps, int nsm, cudaStream_t s
 #define RF_RASTER_ARGS \
-    jobs, nj, draws, prims, rprims, rows, tcnt, toff, mask, segs, list, listovf, items, ntiles, first, nfirst, queue, stats, warps, nsm, s
+    jobs, nj, draws, prims, rprims, rows, ent, mask, segs, list, items, ntiles, first, nfirst, queue, stats, warps, nsm, s
 #define RF_DECL_RASTER_TW(TW)                                         \
     cudaError_t launch_raster_tw##TW(int kind, RF_RASTER_PARAMS);      \
     cudaError_t launch_raster_any_tw##TW(int kind, RF_RASTER_PARAMS);
@@ -171,7 +177,7 @@ RF_DECL_RASTER_TW(64)
 // (the caller orders the side streams after and before its own).
 cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng, const JobDev *jobs, uint32_t nj,
                           const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, const uint32_t *rows,
-                          const uint32_t *tcnt, const uint32_t *toff, const uint32_t *mask, const uint2 *segs,
+                          const uint2 *ent, const uint32_t *mask, const uint2 *segs,
                           const uint2 *list, uint32_t ntiles, const uint32_t *items, uint32_t *counters,
                           StatsDev *stats, uint32_t warps, int nsm, const cudaStream_t *st, uint32_t nst);
 cudaError_t launch_fill(uint32_t *color, float *depth, size_t n, uint32_t px, float z,
@@ -202,9 +208,6 @@ cudaError_t launch_dsort(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
 // Per-draw clipped-triangle counts only (nout[d]), before np is known.
 cudaError_t launch_draw_counts(const DrawDev *draws, uint32_t nd, uint32_t nt, const uint32_t *toff,
                                const uint32_t *counters, uint32_t *nout, cudaStream_t s);
-// toff[i] = i, tcnt[i] = 1 for i < n: the raster's view of a sorted frame,
-// where every clipped triangle is one unit of the tile masks.
-cudaError_t launch_iota(uint32_t *toff, uint32_t *tcnt, uint32_t n, cudaStream_t s);
 // Writes the GPU's global timer (ns) into *dst when the stream reaches it
 // (dst: device memory or page-locked host memory).
 cudaError_t launch_stamp(unsigned long long *dst, cudaStream_t s);

@@ -67,7 +67,10 @@ constexpr size_t OFF_ITEMS = al(OFF_MARKS + 16);
 constexpr size_t OFF_SEGS = al(OFF_ITEMS + (size_t)MAX_TILES * (RF_SPLIT_K + 1) * 4);
 constexpr size_t LIST_CAP = 32768;  // entries of the tiles' triangle lists (the masks are walked past it)
 constexpr size_t OFF_LIST = al(OFF_SEGS + (size_t)MAX_TILES * 8);
-constexpr size_t OFF_ROWS = al(OFF_LIST + LIST_CAP * 8);
+constexpr size_t OFF_ENT = al(OFF_LIST + LIST_CAP * 8);
+constexpr size_t OFF_TACC = al(OFF_ENT + (size_t)RF_NOALLOC_MAX_TRIS * 8);
+constexpr size_t OFF_ROWS = al(OFF_TACC + (size_t)MAX_TILES * 8);
+static_assert(((size_t)MAX_TILES * (MASK_WORDS + SUM_WORDS)) % 4 == 0, "masks are zeroed 16 bytes at a time");
 // The rest of the area holds row records; triangles whose records do not
 // fit are rasterised from their setup records instead (same results).
 constexpr size_t ROWS_WORDS = (RF_NOALLOC_SCRATCH_BYTES - OFF_ROWS) / 4;
@@ -243,6 +246,8 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
     uint32_t *items = reinterpret_cast<uint32_t *>(base + OFF_ITEMS);
     uint32_t *rows = reinterpret_cast<uint32_t *>(base + OFF_ROWS);
     uint2 *segs = reinterpret_cast<uint2 *>(base + OFF_SEGS), *list = reinterpret_cast<uint2 *>(base + OFF_LIST);
+    uint2 *ent = reinterpret_cast<uint2 *>(base + OFF_ENT);
+    unsigned long long *tacc = reinterpret_cast<unsigned long long *>(base + OFF_TACC);
 
     // ---- zero what the kernels accumulate into, then the pass itself
     NA_CK(cudaMemsetAsync(sd, 0, sizeof(StatsDev), s));
@@ -254,8 +259,9 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
     } else {
         k_na_put<<<1, 32, 0, s>>>(d, J, dd, jd);
         NA_CK(cudaGetLastError());
-        NA_CK(rfk::launch_zero(mask, (size_t)ntiles * (J.mask_words + J.sum_words), sd, 1, rowtot, marks, cnt, nsm, s));
-        NA_CK(rfk::launch_vertex(dd, 1, nverts, cpos, coc, nsm, s));
+        NA_CK(rfk::launch_zero(mask, (size_t)MAX_TILES * (MASK_WORDS + SUM_WORDS), true, sd, 1, tacc, ntiles, rowtot,
+                               marks, cnt, nsm, s));
+        NA_CK(rfk::launch_vertex(dd, 1, nverts, cpos, coc, cnt, nsm, s));
         NA_CK(rfk::launch_clip(dd, 1, ntri, cpos, coc, tcnt, tpoly, toff, pool, RF_NOALLOC_MAX_TRIS,
                                cnt, nsm, s, toff, false));  // (the scan places the outputs)
         NA_CK(rfk::launch_scan(tcnt, toff, ntri, scan, cnt + RF_CNT_PRIMS, s));
@@ -263,10 +269,10 @@ extern "C" rf_status rf_render_noalloc(const float *verts, uint32_t nverts, uint
                           flags->depth_write;
         const RasterGroup group{shader, fast, 0u, ntiles, 0u, (ntri + RF_SETUP_THREADS - 1) / RF_SETUP_THREADS, ntri};
         NA_CK(rfk::launch_setup(dd, 1, jd, 1, &group, 1, ntri, TILE_W, cpos, tcnt, toff, tpoly, pool, prims,
-                                rowtot, rows, ROWS_WORDS, rprims, mask, live, marks, sd, cnt, nsm, s));
-        NA_CK(rfk::launch_lists(jd, 1, mask, ntiles, ntiles, toff, tcnt, rprims, marks, (uint32_t)nsm * 16u, items,
+                                rowtot, rows, ROWS_WORDS, rprims, ent, mask, live, marks, sd, cnt, nsm, s));
+        NA_CK(rfk::launch_lists(jd, 1, mask, ntiles, ntiles, ent, tacc, marks, (uint32_t)nsm * 16u, items,
                                 cnt, segs, list, rowtot + 1, LIST_CAP, s));
-        NA_CK(rfk::launch_raster(TILE_W, &group, 1, jd, 1, dd, prims, rprims, rows, tcnt, toff, mask, segs, list, ntiles, items,
+        NA_CK(rfk::launch_raster(TILE_W, &group, 1, jd, 1, dd, prims, rprims, rows, ent, mask, segs, list, ntiles, items,
                                  cnt, sd, WARPS, nsm, &s, 1));
     }
     if (stats) {

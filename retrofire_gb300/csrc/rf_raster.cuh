@@ -695,8 +695,10 @@ struct PrimIter {
         }
         return n;
     }
-    __device__ __forceinline__ void init() {
-        sb = s0 = s1 = s2 = s3 = sc = sl = srem = 0;
+    // From summary word `first` on (to nsum).
+    __device__ __forceinline__ void init(uint32_t first) {
+        sb = first;
+        s0 = s1 = s2 = s3 = sc = sl = srem = 0;
         widx = wval = wn = wi = wrem = 0;
         started = done = false;
         fn = 0;
@@ -704,17 +706,23 @@ struct PrimIter {
     }
 };
 
-// The next up to 32 input triangles of a tile whose lists did not fit, from
-// its masks: entries like the lists' (0 with y = 0 for none), n of them.
-// (Out of line, the iterator in local memory: a frame or two until the
-// library has grown the lists.)
-static __device__ __noinline__ uint2 mask_batch(PrimIter *it, const uint32_t *toff, const uint32_t *tcnt,
-                                                uint32_t lane, uint32_t *n) {
+// The next up to 32 entries of a list piece that did not fit, from the tile's
+// masks (0 with y = 0 for none), n of them.  (Out of line, the iterator in
+// local memory: a frame or two until the library has grown the lists.)
+static __device__ __noinline__ uint2 mask_batch(PrimIter *it, const uint2 *ent, uint32_t lane, uint32_t *n) {
     uint32_t mine;
     const uint32_t k = it->gather_tris(mine);
     *n = k;
-    if (lane >= k) return make_uint2(0u, 0u);
-    return make_uint2(__ldg(toff + mine) | (__ldg(tcnt + mine) - 1u) << RF_ENT_SHIFT, 0x7FFFFFFFu);
+    return lane < k ? __ldg(ent + mine) : make_uint2(0u, 0u);
+}
+static __device__ __noinline__ void mask_begin(PrimIter *it, const uint32_t *mask, const JobDev *J, uint32_t lt,
+                                               uint32_t piece, uint32_t lane) {
+    it->tmask = mask + J->mask_base + (size_t)lt * J->mask_words;
+    it->tsum = mask + J->sum_base + (size_t)lt * J->sum_words;
+    it->nsum = min((piece + 1u) * J->seg_words, J->sum_words);
+    it->tri_base = J->tri_base;
+    it->lane = lane;
+    it->init(piece * J->seg_words);
 }
 
 // One commit group per call on every lane (copies issued since the last).
@@ -875,9 +883,10 @@ struct RasterArgs {
     const DrawDev *draws;
     const PrimRec *prims;
     const RasterPrim *rprims;
-    const uint32_t *rows, *tcnt, *toff, *mask;
+    const uint32_t *rows;
+    const uint2 *ent;  // the triangles' list entries
+    const uint32_t *mask;
     const uint2 *segs, *list;  // the tiles' triangle lists
-    const uint32_t *listovf;   // nonzero: they did not fit, walk the masks
     const uint32_t *items, *first, *nfirst;  // the group's part of the work list
     uint32_t *queue;
     StatsDev *stats;
@@ -1004,18 +1013,19 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
     // The tile's list, a batch of 32 entries at a time (the next one already
     // loaded: ent, n_ent of them): the entries the tile does not hide go on
     // to the ring as output triangles.
-    const bool walk = *A.listovf != 0u;
-    PrimIter it;  // (only when the masks are walked)
+    bool walk = false;  // the piece's masks are walked (the list did not hold it)
+    PrimIter it;
     const uint2 *segs = A.segs + J.seg_base + (size_t)lt * J.nseg;
     uint32_t sb = 0, slive = 0, ent_off = 0, ent_left = 0, n_ent = 0;
     uint2 seg = make_uint2(0u, 0u), ent = make_uint2(0u, 0u);
     auto next_entries = [&]() {
-        if (walk) {
-            ent = mask_batch(&it, A.toff, A.tcnt, lane, &n_ent);
-            return;
-        }
         n_ent = 0;
-        if (ent_left == 0u) {
+        while (ent_left == 0u) {
+            if (walk) {
+                ent = mask_batch(&it, A.ent, lane, &n_ent);
+                if (n_ent) return;
+                walk = false;
+            }
             while (slive == 0u) {
                 if (sb >= J.nseg) return;
                 seg = sb + lane < J.nseg ? segs[sb + lane] : make_uint2(0u, 0u);
@@ -1026,20 +1036,17 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
             slive &= slive - 1u;
             ent_off = __shfl_sync(FULL, seg.x, k);
             ent_left = __shfl_sync(FULL, seg.y, k);
+            if (ent_left == RF_SEG_WALK) {
+                mask_begin(&it, A.mask, &J, lt, sb - 32u + k, lane);
+                ent_left = 0u;
+                walk = true;
+            }
         }
         n_ent = min(ent_left, 32u);
         ent = lane < n_ent ? __ldg(A.list + ent_off + lane) : make_uint2(0u, 0u);
         ent_off += n_ent;
         ent_left -= n_ent;
     };
-    if (walk) {
-        it.tmask = A.mask + J.mask_base + (size_t)lt * J.mask_words;
-        it.tsum = A.mask + J.sum_base + (size_t)lt * J.sum_words;
-        it.nsum = J.sum_words;
-        it.tri_base = J.tri_base;
-        it.lane = lane;
-        it.init();
-    }
     // `todo`: the lanes of the 32 output triangles taken whose triangle has
     // scanlines in the tile and is not on the table yet, `slows` those
     // without row records.
@@ -1439,8 +1446,7 @@ static cudaError_t launch_raster_k(RF_RASTER_PARAMS) {
     const uint32_t need = (ntiles + warps - 1) / warps;  // (a few crowded-tile slices more are shared out)
     if (blocks > need) blocks = need;
     if (blocks == 0) blocks = 1;
-    const RasterArgs A{jobs, draws, prims, rprims, rows, tcnt, toff, mask, segs, list, listovf,
-                       items, first, nfirst, queue, stats, nj, ntiles};
+    const RasterArgs A{jobs, draws, prims, rprims, rows, ent, mask, segs, list, items, first, nfirst, queue, stats, nj, ntiles};
     k_raster<TW, KIND, FAST><<<blocks, warps * 32, smem, s>>>(A);
     return cudaGetLastError();
 }

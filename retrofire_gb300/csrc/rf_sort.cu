@@ -132,13 +132,6 @@ __global__ void k_draw_counts(const DrawDev *__restrict__ draws, uint32_t nd, ui
     }
 }
 
-__global__ void k_iota(uint32_t *__restrict__ toff, uint32_t *__restrict__ tcnt, uint32_t n) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        toff[i] = i;
-        tcnt[i] = 1u;
-    }
-}
-
 struct SortScratch {
     unsigned long long *k0, *k1;
     uint32_t *v1, *hist, *total;  // hist: counts, then their exclusive scan
@@ -215,12 +208,6 @@ cudaError_t launch_dsort(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
     }
     if (vin != perm) return cudaMemcpyAsync(perm, vin, (size_t)np * 4, cudaMemcpyDeviceToDevice, s);
     return cudaSuccess;
-}
-
-cudaError_t launch_iota(uint32_t *toff, uint32_t *tcnt, uint32_t n, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    k_iota<<<min((n + 255) / 256, 4096u), 256, 0, s>>>(toff, tcnt, n);
-    return cudaGetLastError();
 }
 
 }  // namespace rfk

@@ -85,8 +85,13 @@ def test_lists_that_do_not_fit():
     ref = oracle_render(d, vp, w, h, ctx=ctx)
     dev = rf.Device()
     try:
-        for _ in range(3):
+        # (and the masks that frame left marked do not reach the next one)
+        small = [tris(6, 300, 333, 77, (2, 40, 2, 40))]
+        vs = mat.viewport(0, 0, 333, 77)
+        for _ in range(2):
             assert_parity(gpu_render(d, vp, w, h, ctx=ctx, tile=(8, 4), device=dev), ref)
+            assert_parity(gpu_render(small, vs, 333, 77, tile=(32, 4), device=dev),
+                          oracle_render(small, vs, 333, 77))
     finally:
         dev.close()
 
