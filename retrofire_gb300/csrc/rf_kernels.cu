@@ -709,20 +709,6 @@ __device__ void half_runs(const HalfRec &h, HalfRuns &u, uint32_t r) {
 
 namespace {
 
-// k steps of Iter::next on the first N components, side by side.
-template <int N>
-__device__ __forceinline__ void step_k(float *v, const float *d, uint32_t k) {
-    uint32_t i = 0;
-    for (; i + 4u <= k; i += 4u) {  // four additions per trip, the same sequence
-#pragma unroll
-        for (int c = 0; c < N; ++c) v[c] = fadd(fadd(fadd(fadd(v[c], d[c]), d[c]), d[c]), d[c]);
-    }
-    for (; i < k; ++i) {
-#pragma unroll
-        for (int c = 0; c < N; ++c) v[c] = fadd(v[c], d[c]);
-    }
-}
-
 struct RowOut {
     unsigned long long frags_i;
     uint32_t oob;
@@ -770,68 +756,52 @@ __device__ __forceinline__ float span_depth_bound(float z0, float dz, uint32_t n
 
 // One scanline of a regular triangle (raster.rs:84-113): its span from the
 // row's edge values lx, rx (target.rs:259-264 for frags.i / oob), its row
-// record at rec -- w0 = first | end << 16 of the covered columns, the
-// varyings at the first fragment, then at the span's first tile boundary
-// -- and the bound of its depths into zhi.  cv[c * cs] is component c of
-// the row's interpolated values; dvh the half's per-pixel steps.
+// record at rec -- w0 = first | end << 16 of the covered columns, then the
+// varyings at the first fragment -- and the bound of its depths into zhi.
+// cv[c * cs] is component c of the row's interpolated values; dvh the half's
+// per-pixel steps.
 template <int NCT>
 __device__ __forceinline__ void row_record(float lx, float rx, const float *cv, uint32_t cs,
-                                           const float *dvh, uint32_t nc, uint32_t w, uint32_t tile_w,
-                                           uint32_t *rec, RowOut &o, float &zhi) {
+                                           const float *dvh, uint32_t nc, uint32_t w, uint32_t *rec, RowOut &o, float &zhi) {
     const float x0r = round_up_to_half(lx), x1r = round_up_to_half(rx);
-    const uint64_t xs = as_usize(x0r);
-    uint64_t xe = as_usize(x1r);
-    if (xe < xs) xe = xs;
-    o.frags_i = xe - xs;
-    if (xe > w) o.oob = 1;
-    uint64_t nfr = xe - xs;
-    const uint32_t cnt = as_u32(fsub(x1r, x0r));
-    if (cnt < nfr) nfr = cnt;
     uint32_t w0 = 0;
-    if (nfr && xs < w) {
-        o.px0 = (uint32_t)xs;
-        o.px1 = (uint32_t)(xs + nfr < w ? xs + nfr : w);
-        w0 = o.px0 | (o.px1 << 16);
+    if (fmaxf(x0r, x1r) < 4294967296.0f) {  // both below 2^32 (or NaN): 32-bit casts are exact
+        const uint32_t xs = as_u32(x0r), xe = max(as_u32(x1r), xs);
+        o.frags_i = xe - xs;
+        if (xe > w) o.oob = 1;
+        const uint32_t nfr = min(xe - xs, as_u32(fsub(x1r, x0r)));
+        if (nfr && xs < w) {
+            o.px0 = xs;
+            o.px1 = min(xs + nfr, w);
+            w0 = o.px0 | (o.px1 << 16);
+        }
+    } else {
+        const uint64_t xs = as_usize(x0r);
+        uint64_t xe = as_usize(x1r);
+        if (xe < xs) xe = xs;
+        o.frags_i = xe - xs;
+        if (xe > w) o.oob = 1;
+        uint64_t nfr = xe - xs;
+        const uint32_t cnt = as_u32(fsub(x1r, x0r));
+        if (cnt < nfr) nfr = cnt;
+        if (nfr && xs < w) {
+            o.px0 = (uint32_t)xs;
+            o.px1 = (uint32_t)(xs + nfr < w ? xs + nfr : w);
+            w0 = o.px0 | (o.px1 << 16);
+        }
     }
     rec[0] = w0;
-    // v0.lerp(v0.step(dv_dx), x0 - v0.x)  (raster.rs:102), and the
-    // varyings at the span's first tile boundary.
+    // v0.lerp(v0.step(dv_dx), x0 - v0.x)  (raster.rs:102)
     const float tshift = fsub(x0r, lx);
-    const uint32_t kb = w0 ? tile_w - (o.px0 & (tile_w - 1u)) : 0u;
-    const bool crosses = w0 && o.px0 + kb < o.px1;
-    const uint32_t ksteps = crosses ? kb : 0u;  // <= tile width
-    // The components step side by side (independent chains), each exactly
-    // like Iter::next.
     constexpr uint32_t NCL = NCT ? (uint32_t)NCT : RF_NC;
-    float vb[NCL], dvc[NCL];
-#pragma unroll
-    for (uint32_t c = 0; c < NCL; ++c) {
-        if (c < nc) {
-            const float v = cv[c * cs];
-            dvc[c] = dvh[c];
-            vb[c] = fadd(v, fmul(fsub(fadd(v, dvc[c]), v), tshift));
-            rec[1 + c] = f2u(vb[c]);
-        } else {
-            dvc[c] = 0.0f;
-            vb[c] = 0.0f;
-        }
-    }
-    if (w0) zhi = fmaxf(zhi, span_depth_bound(vb[0], dvc[0], o.px1 - o.px0));
-    if constexpr (NCT != 0) {
-        step_k<NCT>(vb, dvc, ksteps);
-    } else {
-        switch (nc) {  // only the kind's components step
-            case 1: step_k<1>(vb, dvc, ksteps); break;
-            case 2: step_k<2>(vb, dvc, ksteps); break;
-            case 3: step_k<3>(vb, dvc, ksteps); break;
-            case 4: step_k<4>(vb, dvc, ksteps); break;
-            case 5: step_k<5>(vb, dvc, ksteps); break;
-            default: step_k<6>(vb, dvc, ksteps); break;
-        }
-    }
 #pragma unroll
     for (uint32_t c = 0; c < NCL; ++c)
-        if (c < nc) rec[1 + nc + c] = f2u(vb[c]);
+        if (c < nc) {
+            const float v = cv[c * cs], dv = dvh[c];
+            const float vb = fadd(v, fmul(fsub(fadd(v, dv), v), tshift));
+            rec[1 + c] = f2u(vb);
+            if (c == 0 && w0) zhi = fmaxf(zhi, span_depth_bound(vb, dv, o.px1 - o.px0));
+        }
 }
 
 }  // namespace
@@ -1029,7 +999,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                         y0[hh] = in ? (uint32_t)Y : 0u;
                         nrows += (uint32_t)in;
                     }
-                    const uint64_t w = regular ? (uint64_t)nrows * (1u + 2u * nc) : 0u;
+                    const uint64_t w = regular ? (uint64_t)nrows * (1u + nc) : 0u;
                     if (w < 0x40000000ull) P.rwords = (uint32_t)w;
                     if (P.rwords != 0u) {
                         small = nrows <= RF_INLINE_ROWS && wide <= RF_INLINE_WIDTH;
@@ -1074,7 +1044,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
             uint32_t lo[2] = {NONE, NONE}, hi[2] = {0u, 0u}, band0 = 0;  // per 32-row band: covered columns
             float zhi = -__int_as_float(0x7F800000);
             if (small) {
-                const uint32_t rstride = 1u + 2u * nc;
+                const uint32_t rstride = 1u + nc;
                 uint32_t *rec = rows + P.rloc;
                 band0 = (inr[0] ? y0[0] : y0[1]) / RF_TILE_H;
 #pragma unroll 1
@@ -1092,7 +1062,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
 #pragma unroll 1
                     for (uint32_t j = 0; j < n; ++j) {
                         RowOut o{0, 0, NONE, 0};
-                        row_record<NCT>(v[0], v[1], v + 2, 1u, dvx, nc, J.w, tile_w, rec, o, zhi);
+                        row_record<NCT>(v[0], v[1], v + 2, 1u, dvx, nc, J.w, rec, o, zhi);
                         rec += rstride;
                         frags_i += o.frags_i;
                         oob += o.oob;
@@ -1148,7 +1118,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                 R.flags = RF_RP_LIVE | RF_RP_ROWS;
                 R.kind = kind;
                 R.base = base_w;
-                R.stride = 1u + 2u * nc;
+                R.stride = 1u + nc;
                 R.y0 = y0[0];
                 R.c0 = inr[0];
                 R.y1 = y0[1];
@@ -1227,6 +1197,11 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
     // Scanline values of one band: quantity q of the band's row i at
     // [q][i] (rows 16-byte aligned: the walk stores four rows at once).
     __shared__ __align__(16) float stab[8][RF_NR][RF_TILE_H + 4];
+    // A chunk's row records, on their way out: written here a row a lane (the
+    // record's odd length: no bank conflicts), stored as one run of words.  A
+    // lane storing its own record a word at a time made every store 32 partial
+    // sectors.
+    __shared__ uint32_t srec[8][RF_TILE_H * (1 + (NCT ? NCT : RF_NC))];
     auto fetch = [&](uint4 *dst, uint32_t p, bool ok) {
         if (ok) {
             const char *src = reinterpret_cast<const char *>(prims + p);
@@ -1257,22 +1232,24 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
         }
         acc_fi = acc_oob = 0;
     };
-    // One band of the target: reduce the lanes' covered columns and mark the
-    // band's tiles with this triangle's bit.
-    auto mark_band = [&](int64_t band, RowOut &o, const JobDev &J, uint32_t word, uint32_t bit) {
-        const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, o.px0 < o.px1 ? o.px0 : 0xFFFFFFFFu);
-        const uint32_t hi = __reduce_max_sync(0xFFFFFFFFu, o.px0 < o.px1 ? o.px1 : 0u);
-        if (lo < hi) {
-            const uint32_t t0 = lo >> tw_log2, t1 = (hi - 1) >> tw_log2;
-            uint32_t *row = mask + J.mask_base + (size_t)band * J.tiles_x * J.mask_words + word;
+    // Marks the tiles of up to two bands of the target that the lanes' covered
+    // columns meet with this triangle's bit; band: of each lane's row (b0, or
+    // the one below it).
+    auto mark_bands = [&](int64_t b0, int64_t band, RowOut &o, const JobDev &J, uint32_t word, uint32_t bit) {
+        const bool on = o.px0 < o.px1, up = band == b0;
+        const uint32_t lo0 = __reduce_min_sync(0xFFFFFFFFu, on && up ? o.px0 : 0xFFFFFFFFu);
+        const uint32_t hi0 = __reduce_max_sync(0xFFFFFFFFu, on && up ? o.px1 : 0u);
+        const uint32_t lo1 = __reduce_min_sync(0xFFFFFFFFu, on && !up ? o.px0 : 0xFFFFFFFFu);
+        const uint32_t hi1 = __reduce_max_sync(0xFFFFFFFFu, on && !up ? o.px1 : 0u);
+        const uint32_t n0 = lo0 < hi0 ? ((hi0 - 1u) >> tw_log2) - (lo0 >> tw_log2) + 1u : 0u;
+        const uint32_t n1 = lo1 < hi1 ? ((hi1 - 1u) >> tw_log2) - (lo1 >> tw_log2) + 1u : 0u;
+        for (uint32_t k = lane; k < n0 + n1; k += 32u) {
+            const size_t t = k < n0 ? (size_t)b0 * J.tiles_x + (lo0 >> tw_log2) + k
+                                    : (size_t)(b0 + 1) * J.tiles_x + (lo1 >> tw_log2) + (k - n0);
+            atomicOr(mask + J.mask_base + t * J.mask_words + word, bit);
             // ... and the summary bit of that mask word
-            uint32_t *srow = mask + J.sum_base + (size_t)band * J.tiles_x * J.sum_words + (word >> 5);
-            const uint32_t sbit = 1u << (word & 31u);
-            for (uint32_t t = t0 + lane; t <= t1; t += 32) {
-                atomicOr(row + (size_t)t * J.mask_words, bit);
-                atomicOr(srow + (size_t)t * J.sum_words, sbit);
-                ++acc_marks;
-            }
+            atomicOr(mask + J.sum_base + t * J.sum_words + (word >> 5), 1u << (word & 31u));
+            ++acc_marks;
         }
     };
     for (uint32_t i = wid; i < nl; i += nw) {
@@ -1308,7 +1285,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
             const uint32_t word = tl >> 5, bit = 1u << (tl & 31);
             const uint32_t nc = NCT ? (uint32_t)NCT : 1 + nattr_of(P->kind);
             const uint32_t nr = RF_R_C + nc;
-            const uint32_t stride = 1 + 2 * nc;
+            const uint32_t stride = 1 + nc;
             bool regular = P->rwords != 0;
             unsigned long long base = 0;
             if (regular) {
@@ -1396,27 +1373,28 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                         wv = fadd(wv, wd);
                     }
                 };
-                for (int32_t band = (inh[0] | inh[1]) ? ylo / RF_TILE_H : 1; band * RF_TILE_H <= yhi; ++band) {
-                    const int32_t ys = max(ylo, band * RF_TILE_H);
-                    const int32_t ye = min(yhi, band * RF_TILE_H + RF_TILE_H - 1);
-                    const int32_t bs = band * RF_TILE_H;
-                    if (wlane) walk(wv, wd, max(ys, wlo), min(ye, whi), bs);
+                // 32 rows at a time from the triangle's first one (not from the
+                // target's bands: a triangle of 20 rows is one chunk, not two).
+                const int32_t last = (inh[0] | inh[1]) ? yhi : ylo - 1;
+                for (int32_t cs = ylo; cs <= last; cs += RF_TILE_H) {
+                    const int32_t ce = min(last, cs + RF_TILE_H - 1);
+                    if (wlane) walk(wv, wd, max(cs, wlo), min(ce, whi), cs);
                     __syncwarp();
-                    const int32_t y = band * RF_TILE_H + (int32_t)lane;
+                    const int32_t y = cs + (int32_t)lane;
                     const bool in0 = inh[0] && y >= lo0 && y <= hi0;
                     const bool in1 = inh[1] && y >= lo1 && y <= hi1;
                     RowOut o{0, 0, 0xFFFFFFFFu, 0};
-                    if (in0 || in1) {
-                        const uint32_t hh = in0 ? 0u : 1u;
-                        const uint32_t i = (uint32_t)(y - bs);
-                        const uint32_t ridx = in0 ? (uint32_t)(y - lo0) : inh[0] + (uint32_t)(y - lo1);
-                        row_record<NCT>(T[RF_R_LX][i], T[RF_R_RX][i], &T[RF_R_C][i], RF_TILE_H + 4,
-                                        P->half[hh].dvdx, nc, J.w, tile_w, rows + base + (size_t)ridx * stride,
-                                        o, zhi_tri);
-                    }
+                    if (in0 || in1)
+                        row_record<NCT>(T[RF_R_LX][lane], T[RF_R_RX][lane], &T[RF_R_C][lane], RF_TILE_H + 4,
+                                        P->half[in0 ? 0 : 1].dvdx, nc, J.w, srec[wib] + lane * stride, o,
+                                        zhi_tri);
                     acc_fi += o.frags_i;
                     acc_oob += o.oob;
-                    mark_band(band, o, J, word, bit);
+                    mark_bands(cs / RF_TILE_H, y / RF_TILE_H, o, J, word, bit);
+                    __syncwarp();
+                    uint32_t *out = rows + base + (size_t)(uint32_t)(cs - ylo) * stride;
+                    const uint32_t n = (uint32_t)(ce - cs + 1) * stride;
+                    for (uint32_t k = lane; k < n; k += 32u) out[k] = srec[wib][k];
                     __syncwarp();
                 }
                 // The triangle's depth bound: the largest of its rows'.
@@ -1455,7 +1433,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                     }
                     acc_fi += o.frags_i;
                     acc_oob += o.oob;
-                    mark_band(band, o, J, word, bit);
+                    mark_bands(band, band, o, J, word, bit);
                 }
                 // Band 0 not visited (no row y > 0): flush the row-0 walk of
                 // lane 0.  The test is made warp-uniform before the shuffles.
@@ -1466,7 +1444,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                     acc_oob += o0.oob;
                     RowOut z{0, 0, __shfl_sync(0xFFFFFFFFu, o0.px0, 0), __shfl_sync(0xFFFFFFFFu, o0.px1, 0)};
                     if (lane != 0) z = RowOut{0, 0, 0xFFFFFFFFu, 0};
-                    mark_band(0, z, J, word, bit);
+                    mark_bands(0, 0, z, J, word, bit);
                 }
             }
         }
@@ -1518,6 +1496,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
     __shared__ __align__(16) uint4 sbuf[8][NG][RF_PRIM_CORE_BYTES / 16];  // records' first parts
     __shared__ __align__(16) RasterPrim srp[8][NG];
     __shared__ float stab[8][NG][RF_NR][G];  // quantity q of row r at [q][r]
+    __shared__ uint32_t srec[8][NG][G * (1 + (NCT ? NCT : RF_NC))];  // the rows' records, on their way out
     const PrimRec *P = reinterpret_cast<const PrimRec *>(sbuf[wib][g]);
     RasterPrim *R = &srp[wib][g];
     float (*T)[G] = stab[wib][g];
@@ -1574,7 +1553,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             bit = 1u << (tl & 31);
             nc = NCT ? (uint32_t)NCT : 1 + nattr_of(P->kind);
             nr = RF_R_C + nc;
-            stride = 1 + 2 * nc;
+            stride = 1 + nc;
             // Both halves' rows on the target (as in k_bin).
             for (int hh = 0; hh < 2; ++hh) {
                 const HalfRec *H = &P->half[hh];
@@ -1631,9 +1610,11 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             const int64_t y = hh ? Yh[1] + (gl - inh[0]) : Yh[0] + gl;
             yb = (uint32_t)(y / RF_TILE_H);
             row_record<NCT>(T[RF_R_LX][gl], T[RF_R_RX][gl], &T[RF_R_C][gl], G,
-                            P->half[hh].dvdx, nc, J->w, tile_w, rows + base + (size_t)gl * stride, o, zhi);
+                            P->half[hh].dvdx, nc, J->w, srec[wib][g] + gl * stride, o, zhi);
         }
         __syncwarp();
+        if (run)
+            for (uint32_t k = gl; k < nrows * stride; k += G) rows[base + k] = srec[wib][g][k];
         acc_fi += o.frags_i;
         acc_oob += o.oob;
         if (run) {

@@ -26,10 +26,9 @@
 //            a span that meets an earlier one of its row waits for it.  For
 //            triangles of few rows, which would leave most rows' lanes idle.
 // An item starts from its row record (the reference's own running sums: the
-// clipped span, the varyings at its first fragment and at its first tile
-// boundary), copied to shared memory one round ahead (cp.async); in a third
-// or later tile of a long span the boundary values are stepped on.  Then it
-// steps pixel by pixel like Iter::next.
+// clipped span and the varyings at its first fragment), copied to shared
+// memory one round ahead (cp.async); a span that starts left of the tile is
+// stepped to it.  Then it steps pixel by pixel like Iter::next.
 // What bounds it: the chain of dependent instructions of each warp (16 warps
 // per SM, 38 % of issue slots), so what counts is instructions per triangle:
 // one warp pass per triangle -- lane = row, most lanes idle on small
@@ -176,7 +175,6 @@ struct TileCtx {
     uint32_t y;       // the target row of tile row `lane`
     uint32_t tx0;     // first column of the tile
     uint32_t tx1;     // one past the last column of the tile inside the target
-    uint32_t tw;      // tile width (a power of two)
     bool row_ok;
     bool has_depth;
     int32_t depth_test;
@@ -191,7 +189,7 @@ struct PreNC {
     static constexpr int NC = KIND == RF_K_ANY ? RF_NC : Kind<KIND == RF_K_ANY ? 0 : KIND>::NC;
     static constexpr int NP = (NC + 1) / 2;  // pairs of components
 };
-__host__ __device__ constexpr uint32_t row_words(int nc) { return 1u + 2u * (uint32_t)nc; }
+__host__ __device__ constexpr uint32_t row_words(int nc) { return 1u + (uint32_t)nc; }
 __device__ __forceinline__ uint32_t kind_nc(uint32_t kind) {
     return kind == RF_K_FLAT ? 1u : kind == RF_K_TEXTURED ? 3u : kind == RF_K_TEX_GOURAUD ? 6u : 4u;
 }
@@ -458,41 +456,43 @@ __device__ __forceinline__ void stage_row(uint32_t *slot, uint32_t lane, bool pr
 // One item -- a scanline of a triangle inside the tile: its record sits in
 // this lane's part of a slot (rs), its span [a, b) is clipped to the tile
 // (xs: the span's first pixel).  v, dv: its varyings at pixel a and their
-// steps.  The span starts in this tile, or enters it at its first tile
-// boundary -- both values are in the record -- or at a later one: then the
-// boundary values take the steps between.  Up to RF_STEP_MAX of them one
-// after the other (two components an instruction: 64 instructions for 32
-// pixels of Gouraud, where the exact jump takes about 100 a component);
-// further ones by the jump, in place.
+// steps.  A span that starts left of the tile takes the steps between: up to
+// RF_STEP_MAX of them one after the other (two components an instruction: 64
+// instructions for 32 pixels of Gouraud, where the exact jump takes about 100
+// a component), more by the jump, in place.  (Records that also held the
+// varyings at the first tile boundary saved up to a tile's steps here, but
+// were nearly twice as long.)
 #define RF_STEP_MAX 128u
 template <int KIND>
-__device__ __forceinline__ void item_load(const TileCtx &T, const float *dvdx, uint32_t *rs, uint32_t nc,
-                                          uint32_t xs, uint32_t a, float2 *v, float2 *dv) {
+__device__ __forceinline__ void item_load(const float *dvdx, uint32_t *rs, uint32_t nc, uint32_t k, float2 *v,
+                                          float2 *dv) {
     constexpr int NC = PreNC<KIND>::NC, NP = PreNC<KIND>::NP;
-    const bool first = a == xs;
-    uint32_t k = first ? 0u : a - ((xs & ~(T.tw - 1u)) + T.tw);
-    const uint32_t off = first ? 1u : 1u + nc;
     if (k > RF_STEP_MAX) {
 #pragma unroll 1
         for (uint32_t c = 0; c < nc; ++c)
-            rs[(off + c) * RF_TILE_H] = f2u(jump_far(u2f(rs[(off + c) * RF_TILE_H]), dvdx[c], k));
+            rs[(1u + c) * RF_TILE_H] = f2u(jump_far(u2f(rs[(1u + c) * RF_TILE_H]), dvdx[c], k));
         k = 0;
     }
 #pragma unroll
     for (int c = 0; c < NP; ++c) {
         dv[c] = reinterpret_cast<const float2 *>(dvdx)[c];
-        v[c].x = u2f(rs[(off + 2 * c) * RF_TILE_H]);
-        // (a pair past the kind's components: a value the record's words do not hold)
-        v[c].y = 2 * c + 1 < NC ? u2f(rs[(off + 2 * c + 1) * RF_TILE_H]) : 0.0f;
+        v[c].x = u2f(rs[(1 + 2 * c) * RF_TILE_H]);
+        v[c].y = 2 * c + 1 < NC ? u2f(rs[(2 + 2 * c) * RF_TILE_H]) : 0.0f;
     }
 #pragma unroll 1
-    for (; k; k -= 8u) {  // (whole tile widths)
+    for (; k >= 4u; k -= 4u) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
 #pragma unroll
             for (int c = 0; c < NP; ++c) v[c] = __fadd2_rn(v[c], dv[c]);
         }
     }
+#pragma unroll
+    for (uint32_t i = 0; i < 3; ++i)
+        if (i < k) {
+#pragma unroll
+            for (int c = 0; c < NP; ++c) v[c] = __fadd2_rn(v[c], dv[c]);
+        }
 }
 
 // A triangle without row records, from its PrimRec: lane = row (T.row = lane).
@@ -926,7 +926,6 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
     T.row = lane;
     T.tx0 = txi * TW;
     T.tx1 = min(T.tx0 + (uint32_t)TW, J.w);
-    T.tw = TW;
     const uint32_t ty0 = tyi * RF_TILE_H;
     T.y = ty0 + lane;
     constexpr uint32_t SLICE_H = RF_TILE_H / RF_SPLIT_K;
@@ -999,7 +998,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
         half = row < ((e.z >> 8) & 0xFFu) ? 0u : 1u;
         const float *dvdx = tab_dv + (ki * 2u + half) * RF_NC;
         const uint32_t nc = KIND == RF_K_ANY ? kind_nc(kind) : (uint32_t)NC;
-        item_load<KIND>(T, dvdx, rs, nc, xs, a, v, dv);
+        item_load<KIND>(dvdx, rs, nc, a - xs, v, dv);
         return true;
     };
     // The record of row r of the entry's in-tile rows into this lane's part of a slot.
