@@ -11,6 +11,13 @@
 namespace rfd {
 using namespace rfx;
 
+// First in every kernel of a frame: wait for the kernel before it on the
+// stream (launch_next; no wait otherwise), then let the one after it come up.
+__device__ __forceinline__ void grid_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Largest i with key(i) <= x over a sorted array of n records.
 template <class F>
 __device__ __forceinline__ uint32_t upper_index(uint32_t n, uint32_t x, F key) {

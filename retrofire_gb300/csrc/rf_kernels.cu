@@ -72,6 +72,7 @@ __global__ void k_zero(uint4 *__restrict__ mask, size_t n16, const uint32_t *__r
                        unsigned long long *__restrict__ js, uint32_t njs, unsigned long long *__restrict__ tacc,
                        uint32_t ntiles, unsigned long long *__restrict__ totals,
                        unsigned long long *__restrict__ marks, uint32_t *__restrict__ counters) {
+    grid_begin();
     const size_t i0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
     if (!dirty || *dirty)
         for (size_t i = i0; i < n16; i += step) mask[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -95,6 +96,7 @@ __global__ void k_zero(uint4 *__restrict__ mask, size_t n16, const uint32_t *__r
 // ---------------------------------------------------------------------------
 __global__ void k_vertex(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nv_total,
                          float4 *__restrict__ cpos, uint8_t *__restrict__ coc, uint32_t *__restrict__ counters) {
+    grid_begin();
     if (counters && blockIdx.x == 0 && threadIdx.x == 0) counters[RF_CNT_MASKDIRTY] = 0;  // (k_zero is done)
     // Warp-uniform loop (the draw lookup is shared by the warp's lanes).
     for (uint32_t wbase = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); wbase < nv_total;
@@ -175,6 +177,7 @@ __global__ void k_bbox_fold(const float *__restrict__ part, uint32_t nb, float *
 // (view_frustum::status == Hidden, clip.rs:245-267) culls the draw.
 // ---------------------------------------------------------------------------
 __global__ void k_cull(DrawDev *__restrict__ draws, uint32_t nd, StatsDev *__restrict__ stats) {
+    grid_begin();
     for (uint32_t di = blockIdx.x * blockDim.x + threadIdx.x; di < nd; di += gridDim.x * blockDim.x) {
         DrawDev &d = draws[di];
         d.culled = 0;
@@ -250,6 +253,7 @@ __global__ void k_clip(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t 
                        uint32_t *__restrict__ tpoly, uint32_t *__restrict__ queue,
                        uint32_t *__restrict__ counters, uint32_t *__restrict__ toff,
                        uint32_t *__restrict__ prim_total) {
+    grid_begin();
     // Block-uniform loop (the draw lookup is shared by a warp's lanes, the
     // output slots are taken once per block).
     __shared__ uint32_t wslot[2][RF_CLIP_THREADS / 32];
@@ -533,6 +537,7 @@ k_clip_poly(const DrawDev *__restrict__ draws, const float4 *__restrict__ cpos,
             const uint8_t *__restrict__ coc, uint32_t *__restrict__ tcnt,
             uint32_t *__restrict__ tpoly, const uint32_t *__restrict__ queue,
             PolyVert *__restrict__ pool, uint32_t pool_cap, uint32_t *__restrict__ counters) {
+    grid_begin();
     const uint32_t nq = counters[RF_CNT_CLIPQ];
     if (nq <= RF_CLIP_GROUP_MAX) clip_groups(draws, cpos, coc, tcnt, tpoly, queue, pool, pool_cap, counters, nq);
     else clip_threads(draws, cpos, coc, tcnt, tpoly, queue, pool, pool_cap, counters, nq);
@@ -550,6 +555,7 @@ static_assert(SCAN_THREADS * SCAN_ITEMS == RF_SCAN_BLOCK_ITEMS, "scan block size
 __global__ void k_scan_blocks(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
                               uint32_t n, uint32_t *__restrict__ block_sums,
                               uint32_t *__restrict__ total) {
+    grid_begin();
     __shared__ uint32_t warp_sums[32];
     const uint32_t base = blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + threadIdx.x * SCAN_ITEMS;
     uint32_t v[SCAN_ITEMS], s = 0;
@@ -591,6 +597,7 @@ __global__ void k_scan_blocks(const uint32_t *__restrict__ in, uint32_t *__restr
 
 // Single block: exclusive scan of the block sums in place; total -> *total.
 __global__ void k_scan_sums(uint32_t *__restrict__ sums, uint32_t nb, uint32_t *__restrict__ total) {
+    grid_begin();
     __shared__ uint32_t warp_sums[32];
     __shared__ uint32_t carry;
     if (threadIdx.x == 0) carry = 0;
@@ -627,6 +634,7 @@ __global__ void k_scan_sums(uint32_t *__restrict__ sums, uint32_t nb, uint32_t *
 }
 
 __global__ void k_scan_add(uint32_t *__restrict__ out, uint32_t n, const uint32_t *__restrict__ sums) {
+    grid_begin();
     const uint32_t base = blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + threadIdx.x * SCAN_ITEMS;
     const uint32_t add = sums[blockIdx.x];
 #pragma unroll
@@ -826,6 +834,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
         uint32_t *__restrict__ mask, uint32_t *__restrict__ live, uint32_t *__restrict__ live_n, uint32_t *__restrict__ live_mid,
         uint32_t *__restrict__ live_mid_n, unsigned long long *__restrict__ marks, StatsDev *__restrict__ stats,
         const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ptri) {
+    grid_begin();
     constexpr uint32_t FULL = 0xFFFFFFFFu, NONE = 0xFFFFFFFFu;
     constexpr int NCL = NCT ? NCT : RF_NC;
     // Each thread builds its record in shared memory; the warp then writes
@@ -1183,6 +1192,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
       uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims,
       uint2 *__restrict__ ent, uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
       unsigned long long *__restrict__ marks, const uint32_t *__restrict__ live_n) {
+    grid_begin();
     const uint32_t lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & 7;
     const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
@@ -1483,6 +1493,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
             unsigned long long *__restrict__ marks, const uint32_t *__restrict__ small_n,
             uint32_t *__restrict__ live_n) {
+    grid_begin();
     static_assert(G == 8 || G == 16, "group sizes");
     constexpr uint32_t NG = 32 / G;  // groups per warp
     constexpr uint32_t NONE = 0xFFFFFFFFu;
@@ -1729,6 +1740,7 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict_
              unsigned long long *__restrict__ tacc, const unsigned long long *__restrict__ marks, uint32_t slots, uint32_t *__restrict__ items,
              uint32_t *__restrict__ extras, uint2 *__restrict__ segs, uint2 *__restrict__ list,
              unsigned long long *__restrict__ cursor, unsigned long long cap, uint32_t *__restrict__ dirty) {
+    grid_begin();
     constexpr uint32_t FULL = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t piece = blockIdx.x * RF_LIST_WARPS + w;
@@ -1837,6 +1849,7 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict_
 // Frame::clear applied directly (when no render follows before a read).
 __global__ void k_fill(uint32_t *__restrict__ color, float *__restrict__ depth, size_t n,
                        uint32_t px, float z, uint32_t flags) {
+    grid_begin();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
          i += (size_t)gridDim.x * blockDim.x) {
         if (flags & 1u) color[i] = px;
@@ -1866,7 +1879,7 @@ cudaError_t launch_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv, float4
                           uint8_t *coc, uint32_t *counters, int nsm, cudaStream_t s) {
     if (nv == 0) return cudaSuccess;
     uint32_t blocks = min((nv + 255) / 256, (uint32_t)nsm * 16);
-    k_vertex<<<blocks, 256, 0, s>>>(draws, nd, nv, cpos, coc, counters);
+    RF_NEXT(k_vertex, blocks, 256, 0, s, draws, nd, nv, cpos, coc, counters);
     return cudaGetLastError();
 }
 
@@ -1877,11 +1890,11 @@ cudaError_t launch_clip(const DrawDev *draws, uint32_t nd, uint32_t nt, const fl
     if (nt == 0) return cudaSuccess;
     uint32_t *prim_total = place ? counters + RF_CNT_PRIMS : nullptr;
     const uint32_t blocks = min((nt + RF_CLIP_THREADS - 1) / RF_CLIP_THREADS, (uint32_t)nsm * 16);
-    k_clip<<<blocks, RF_CLIP_THREADS, 0, s>>>(draws, nd, nt, coc, tcnt, tpoly, queue, counters, toff, prim_total);
+    RF_NEXT(k_clip, blocks, RF_CLIP_THREADS, 0, s, draws, nd, nt, coc, tcnt, tpoly, queue, counters, toff, prim_total);
     // The queue's length is known on the device only: a grid for all of it
     // at the worst case, each thread striding over what is there.
     const uint32_t pblocks = min((nt + 15) / 16, (uint32_t)nsm * 8);  // 16 triangles per block
-    k_clip_poly<<<pblocks, 256, 0, s>>>(draws, cpos, coc, tcnt, tpoly, queue, pool, pool_cap, counters);
+    RF_NEXT(k_clip_poly, pblocks, 256, 0, s, draws, cpos, coc, tcnt, tpoly, queue, pool, pool_cap, counters);
     return cudaGetLastError();
 }
 
@@ -1893,10 +1906,10 @@ cudaError_t launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t 
                         uint32_t *total, cudaStream_t s) {
     if (n == 0) return cudaMemsetAsync(total, 0, 4, s);
     const uint32_t nb = (n + SCAN_THREADS * SCAN_ITEMS - 1) / (SCAN_THREADS * SCAN_ITEMS);
-    k_scan_blocks<<<nb, SCAN_THREADS, 0, s>>>(in, out, n, scratch, total);
+    RF_NEXT(k_scan_blocks, nb, SCAN_THREADS, 0, s, in, out, n, scratch, total);
     if (nb > 1) {  // one block: its scan is the whole scan
-        k_scan_sums<<<1, 1024, 0, s>>>(scratch, nb, total);
-        k_scan_add<<<nb, SCAN_THREADS, 0, s>>>(out, n, scratch);
+        RF_NEXT(k_scan_sums, 1, 1024, 0, s, scratch, nb, total);
+        RF_NEXT(k_scan_add, nb, SCAN_THREADS, 0, s, out, n, scratch);
     }
     return cudaGetLastError();
 }
@@ -1935,7 +1948,7 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
         }
         uint32_t *big_n = counters + RF_CNT_LIVE_G + g, *mid_n = counters + RF_CNT_LIVE_MID_G + g;
         const uint32_t blocks = min(groups[g].nblocks, (uint32_t)nsm * 32);
-        setup<<<blocks, RF_SETUP_THREADS, 0, s>>>(draws, nd, jobs, nj, groups[g].block0, groups[g].nblocks, tile_w,
+        RF_NEXT(setup, blocks, RF_SETUP_THREADS, 0, s, draws, nd, jobs, nj, groups[g].block0, groups[g].nblocks, tile_w,
                                                   cpos, tcnt, toff, tpoly, pool, prims, rows_total, rows, rows_cap,
                                                   rprims, ent, mask, big, big_n, mid, mid_n, marks, stats, perm, ptri);
         cudaError_t e = cudaGetLastError();
@@ -1945,10 +1958,10 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
         // smaller ones that found no room for their records); the counts are
         // only known on the device.
         const uint32_t sblocks = min((gt + 31) / 32, (uint32_t)nsm * 4);
-        bin16<<<sblocks, 256, 0, s>>>(jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
+        RF_NEXT(bin16, sblocks, 256, 0, s, jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                       counters, marks, mid_n, big_n);
         const uint32_t wblocks = min((gt * 2 + 7) / 8, (uint32_t)nsm * 16);
-        bin<<<wblocks, 256, 0, s>>>(draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
+        RF_NEXT(bin, wblocks, 256, 0, s, draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                     counters, marks, big_n);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         big += (size_t)gt * fan;
@@ -1963,8 +1976,8 @@ cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, uint32_t *mask, uint32
                          uint2 *segs, uint2 *list, unsigned long long *cursor, unsigned long long cap,
                          cudaStream_t s) {
     if (ntiles == 0) return cudaSuccess;
-    k_tile_lists<<<(npieces + RF_LIST_WARPS - 1) / RF_LIST_WARPS, RF_LIST_WARPS * 32, 0, s>>>(
-        jobs, nj, mask, ntiles, npieces, ent, tacc, marks, slots ? slots : 1u, items,
+    RF_NEXT(k_tile_lists, (npieces + RF_LIST_WARPS - 1) / RF_LIST_WARPS, RF_LIST_WARPS * 32, 0, s,
+            jobs, nj, mask, ntiles, npieces, ent, tacc, marks, slots ? slots : 1u, items,
         counters + RF_CNT_ITEMS_G, segs, list, cursor, cap, counters + RF_CNT_MASKDIRTY);
     return cudaGetLastError();
 }
@@ -1998,7 +2011,7 @@ cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t n
 cudaError_t launch_cull(DrawDev *draws, uint32_t nd, StatsDev *stats, int nsm, cudaStream_t s) {
     if (nd == 0) return cudaSuccess;
     const uint32_t blocks = min((nd + 127) / 128, (uint32_t)nsm * 8);
-    k_cull<<<blocks, 128, 0, s>>>(draws, nd, stats);
+    RF_NEXT(k_cull, blocks, 128, 0, s, draws, nd, stats);
     return cudaGetLastError();
 }
 
@@ -2006,6 +2019,7 @@ cudaError_t launch_cull(DrawDev *draws, uint32_t nd, StatsDev *stats, int nsm, c
 // block; stream order makes the plain read-modify-write of *total safe.
 __global__ void __launch_bounds__(256) k_stats_fold(const StatsDev *__restrict__ js, uint32_t n,
                                                     StatsDev *__restrict__ total) {
+    grid_begin();
     constexpr int NF = (int)(sizeof(StatsDev) / sizeof(unsigned long long));
     static_assert(sizeof(StatsDev) == NF * sizeof(unsigned long long), "StatsDev is all counters");
     __shared__ unsigned long long part[NF][8];
@@ -2049,7 +2063,7 @@ cudaError_t launch_stamp(unsigned long long *dst, cudaStream_t s) {
 
 cudaError_t launch_stats_fold(const StatsDev *js, uint32_t n, StatsDev *total, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_stats_fold<<<1, 256, 0, s>>>(js, n, total);
+    RF_NEXT(k_stats_fold, 1, 256, 0, s, js, n, total);
     return cudaGetLastError();
 }
 

@@ -68,6 +68,32 @@ struct RasterGroup {
 #define RF_SCAN_BLOCK_ITEMS 4096u  // values one scan block takes (one launch instead of three)
 
 namespace rfk {
+#if defined(__CUDACC__)
+// A launch that may start while the kernel before it on the stream drains
+// (programmatic dependent launch): its blocks come up and wait in
+// grid_begin() (rf_device.cuh) until that kernel has finished, so the launch
+// latency and the wait for the last block do not add up.  Every kernel
+// launched here calls grid_begin() first.
+template <class... P, class... A>
+cudaError_t launch_next(void (*k)(P...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t s, A... a) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(blocks);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, static_cast<P>(a)...);
+}
+#define RF_NEXT(...)                                          \
+    do {                                                      \
+        const cudaError_t next_ = rfk::launch_next(__VA_ARGS__); \
+        if (next_ != cudaSuccess) return next_;               \
+    } while (0)
+#endif
 // Zeroes what a frame accumulates into: the jobs' stats slots js[0 .. njobs),
 // the tiles' entry counts, totals[0..2) (row words, list entries), *marks
 // (the binning pass's total of (triangle, tile) bits), the frame's counters

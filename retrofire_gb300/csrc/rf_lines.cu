@@ -79,6 +79,7 @@ __global__ void k_line_setup(const DrawDev *__restrict__ draws, const JobDev *__
                              uint32_t nl, const float4 *__restrict__ cpos,
                              const uint8_t *__restrict__ coc, LineRec *__restrict__ recs,
                              uint32_t *__restrict__ mask, StatsDev *__restrict__ stats) {
+    rfd::grid_begin();
     const DrawDev &d = draws[0];
     const JobDev &J = jobs[0];
     const uint32_t na = d.nattr, zm = lzdiv_mask(d.shader);
@@ -198,6 +199,7 @@ __global__ void k_line_setup(const DrawDev *__restrict__ draws, const JobDev *__
 __global__ void k_line_raster(const JobDev *__restrict__ jobs, const LineRec *__restrict__ recs,
                               const uint32_t *__restrict__ mask, uint32_t ntiles,
                               uint32_t *__restrict__ queue, StatsDev *__restrict__ stats) {
+    rfd::grid_begin();
     const JobDev &J = jobs[0];
     const uint32_t lane = threadIdx.x & 31;
     unsigned long long fo = 0;
@@ -271,11 +273,11 @@ cudaError_t launch_lines(const DrawDev *draws, const JobDev *jobs, uint32_t nl, 
                          uint32_t *queue, StatsDev *stats, int nsm, cudaStream_t s) {
     if (nl == 0) return cudaSuccess;
     const uint32_t blocks = min((nl + 127) / 128, (uint32_t)nsm * 8);
-    k_line_setup<<<blocks, 128, 0, s>>>(draws, jobs, nl, cpos, coc, recs, mask, stats);
+    RF_NEXT(k_line_setup, blocks, 128, 0, s, draws, jobs, nl, cpos, coc, recs, mask, stats);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const uint32_t rblocks = min((ntiles + 3) / 4, (uint32_t)nsm * 8);
-    k_line_raster<<<rblocks, 128, 0, s>>>(jobs, recs, mask, ntiles, queue, stats);
+    RF_NEXT(k_line_raster, rblocks, 128, 0, s, jobs, recs, mask, ntiles, queue, stats);
     return cudaGetLastError();
 }
 

@@ -1373,6 +1373,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
 template <int TW, int KIND, bool FAST>
 __global__ void __launch_bounds__(RF_RASTER_MAX_THREADS, 2) k_raster(const __grid_constant__ RasterArgs A) {
     using namespace rfr;
+    grid_begin();
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr uint32_t WARP_WORDS = raster_warp_words<TW, KIND>();
@@ -1446,7 +1447,7 @@ static cudaError_t launch_raster_k(RF_RASTER_PARAMS) {
     if (blocks > need) blocks = need;
     if (blocks == 0) blocks = 1;
     const RasterArgs A{jobs, draws, prims, rprims, rows, ent, mask, segs, list, items, first, nfirst, queue, stats, nj, ntiles};
-    k_raster<TW, KIND, FAST><<<blocks, warps * 32, smem, s>>>(A);
+    RF_NEXT(k_raster<TW, KIND, FAST>, blocks, warps * 32, smem, s, A);
     return cudaGetLastError();
 }
 

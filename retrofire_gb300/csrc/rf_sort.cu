@@ -29,6 +29,7 @@ __global__ void k_dsort_keys(const DrawDev *__restrict__ draws, uint32_t nd, con
                              const uint32_t *__restrict__ toff, const uint32_t *__restrict__ tpoly,
                              const PolyVert *__restrict__ pool, unsigned long long *__restrict__ keys,
                              uint32_t *__restrict__ vals, uint32_t *__restrict__ ptri) {
+    rfd::grid_begin();
     for (uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x; gt < nt; gt += gridDim.x * blockDim.x) {
         const uint32_t cnt = tcnt[gt];
         if (!cnt) continue;
@@ -63,6 +64,7 @@ __device__ __forceinline__ uint32_t digit_of(unsigned long long k, uint32_t shif
 // Per block, how many of its items have each digit: hist[digit * nb + block].
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned long long *__restrict__ keys, uint32_t n,
                                                         uint32_t shift, uint32_t *__restrict__ hist) {
+    rfd::grid_begin();
     __shared__ uint32_t h[RS_DIGITS];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned long l
                                                            uint32_t shift, const uint32_t *__restrict__ offs,
                                                            unsigned long long *__restrict__ kout,
                                                            uint32_t *__restrict__ vout) {
+    rfd::grid_begin();
     constexpr uint32_t NW = RS_THREADS / 32;
     __shared__ uint32_t run[RS_DIGITS];       // next place of each digit
     __shared__ uint32_t wcnt[NW][RS_DIGITS];  // per warp: its items of each digit in this chunk
@@ -120,6 +123,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned long l
 __global__ void k_draw_counts(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nt,
                               const uint32_t *__restrict__ toff, const uint32_t *__restrict__ counters,
                               uint32_t *__restrict__ nout) {
+    rfd::grid_begin();
     const uint32_t total = counters[RF_CNT_PRIMS];
     for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < nd; d += gridDim.x * blockDim.x) {
         const uint32_t t0 = draws[d].tri_base, t1 = t0 + draws[d].ntri;
@@ -169,7 +173,7 @@ size_t dsort_scratch_bytes(uint32_t np) {
 cudaError_t launch_draw_counts(const DrawDev *draws, uint32_t nd, uint32_t nt, const uint32_t *toff,
                                const uint32_t *counters, uint32_t *nout, cudaStream_t s) {
     if (nd == 0) return cudaSuccess;
-    k_draw_counts<<<(nd + 255) / 256, 256, 0, s>>>(draws, nd, nt, toff, counters, nout);
+    RF_NEXT(k_draw_counts, (nd + 255) / 256, 256, 0, s, draws, nd, nt, toff, counters, nout);
     return cudaGetLastError();
 }
 
@@ -182,7 +186,7 @@ cudaError_t launch_dsort(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
     if (np == 0) return cudaSuccess;
     SortScratch S = carve(scratch, np);
     const uint32_t kb = min((nt + 255) / 256, 4096u);
-    k_dsort_keys<<<kb, 256, 0, s>>>(draws, nd, jobs, nt, cpos, tcnt, toff, tpoly, pool, S.k0, perm, ptri);
+    RF_NEXT(k_dsort_keys, kb, 256, 0, s, draws, nd, jobs, nt, cpos, tcnt, toff, tpoly, pool, S.k0, perm, ptri);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // Digits to sort: the 32 key bits, then the draw index's bits.
     uint32_t dbits = 0;
@@ -194,10 +198,10 @@ cudaError_t launch_dsort(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
     uint32_t *offs = S.hist + (size_t)nb * RS_DIGITS;
     for (uint32_t p = 0; p < passes; ++p) {
         const uint32_t shift = 8 * p;
-        k_rs_hist<<<nb, RS_THREADS, 0, s>>>(kin, np, shift, S.hist);
+        RF_NEXT(k_rs_hist, nb, RS_THREADS, 0, s, kin, np, shift, S.hist);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = launch_scan(S.hist, offs, nb * RS_DIGITS, scan_scratch, S.total, s)) != cudaSuccess) return e;
-        k_rs_scatter<<<nb, RS_THREADS, 0, s>>>(kin, vin, np, shift, offs, kout, vout);
+        RF_NEXT(k_rs_scatter, nb, RS_THREADS, 0, s, kin, vin, np, shift, offs, kout, vout);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         unsigned long long *tk = kin;
         kin = kout;
