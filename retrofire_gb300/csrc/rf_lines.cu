@@ -7,11 +7,11 @@
 // k_line_setup: one thread per line; clips it, walks its pixels with the
 // reference's running sum (stats, and the tiles it touches: a per-tile
 // bitmask over the lines, bit order = submission order).
-// k_line_raster: a warp per 32x32 tile takes the tile's lines in order; a
-// line that steps along x gives each column (lane) at most one pixel, one
-// that steps along y each row (lane): the lane's pixel comes from the exact
-// k-step running sum (rfx::jump), so lanes of one line never collide and
-// pixels see the lines in submission order.
+// k_line_raster: a warp per quarter of a 32x32 tile (8 rows, its pixels in
+// shared memory) takes the tile's lines in order, 32 at a time, and their steps
+// inside its columns (a line that steps along x) or rows, 32 of any lines a
+// pass: a lane's pixel comes from the k-step running sum, and lanes that meet
+// in a pixel go in submission order.
 #include "rf_raster.cuh"
 
 using namespace rfx;
@@ -196,71 +196,203 @@ __global__ void k_line_setup(const DrawDev *__restrict__ draws, const JobDev *__
     warp_add_u64(&stats->oob, oob, true);
 }
 
-__global__ void k_line_raster(const JobDev *__restrict__ jobs, const LineRec *__restrict__ recs,
-                              const uint32_t *__restrict__ mask, uint32_t ntiles,
-                              uint32_t *__restrict__ queue, StatsDev *__restrict__ stats) {
+// The k-step running sum from s: one add after the other up to RF_LINE_STEP
+// steps (4 cycles each; a wireframe's lines are mostly shorter), else the exact
+// jump.
+#define RF_LINE_STEP 64u
+__device__ __forceinline__ float line_step(float s, float d, uint32_t k) {
+    if (k > RF_LINE_STEP) return jump(s, d, k);
+#pragma unroll 1
+    for (; k >= 4u; k -= 4u) s = fadd(fadd(fadd(fadd(s, d), d), d), d);
+#pragma unroll
+    for (uint32_t i = 0; i < 3; ++i)
+        if (i < k) s = fadd(s, d);
+    return s;
+}
+
+#define RF_LINE_WARPS 4
+#define RF_LINE_ROWS 8u    // tile rows a warp draws
+#define RF_LINE_PITCH 33u  // words per tile row in shared memory (odd: steep lines hit different banks)
+// Bound by the latencies of the fullest tiles (up to 200 lines of a wireframe of
+// 12,416 at 1280x720): one line a pass, a lane per column or row, each line's
+// record and pixels waited for in turn, took 117 us there.  With a batch's
+// records loaded together, the pixels in shared memory and short lines sharing
+// a pass 65, with short lines stepped instead of jumped 60, and with four warps
+// a tile, RF_LINE_ROWS rows each, 31 (each reads all of the tile's mask, which
+// is in L2, but steps only the lines that can reach its rows).
+__global__ void __launch_bounds__(RF_LINE_WARPS * 32)
+k_line_raster(const JobDev *__restrict__ jobs, const LineRec *__restrict__ recs,
+              const uint32_t *__restrict__ mask, uint32_t ntiles, uint32_t *__restrict__ queue,
+              StatsDev *__restrict__ stats) {
     rfd::grid_begin();
+    constexpr uint32_t FULL = 0xFFFFFFFFu;
+    __shared__ uint32_t s_col[RF_LINE_WARPS][RF_LINE_ROWS * RF_LINE_PITCH];
+    __shared__ float s_dep[RF_LINE_WARPS][RF_LINE_ROWS * RF_LINE_PITCH];
+    __shared__ LineRec s_rec[RF_LINE_WARPS][32];
+    __shared__ uint32_t s_pend[RF_LINE_WARPS][64];  // the tile's lines found, not drawn yet
+    __shared__ uint2 s_item[RF_LINE_WARPS][32];  // per line of the batch with steps here: first step, first item
     const JobDev &J = jobs[0];
-    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t below = (1u << lane) - 1u, upto = below | (1u << lane);
+    uint32_t *col = s_col[wib];
+    float *dep = s_dep[wib];
+    const bool has_depth = J.depth != nullptr, color_write = J.color_write != 0;
+    const bool depth_write = has_depth && J.depth_write != 0;
+    const int32_t test = has_depth ? J.depth_test : RF_K_DEPTH_NONE;
     unsigned long long fo = 0;
     for (;;) {
-        uint32_t tile = 0;
-        if (lane == 0) tile = atomicAdd(queue, 1u);
-        tile = __shfl_sync(0xFFFFFFFFu, tile, 0);
+        uint32_t part = 0;
+        if (lane == 0) part = atomicAdd(queue, 1u);
+        part = __shfl_sync(FULL, part, 0);
+        const uint32_t tile = part / (RF_TILE_H / RF_LINE_ROWS);
         if (tile >= ntiles) break;
         const uint32_t ty = tile / J.tiles_x, tx = tile - ty * J.tiles_x;
-        const uint64_t tx0 = (uint64_t)tx * RF_TILE_H, ty0 = (uint64_t)ty * RF_TILE_H;
-        const uint64_t tx1 = min(tx0 + RF_TILE_H, (uint64_t)J.w);
+        const uint32_t tx0 = tx * RF_TILE_H, tx1 = min(tx0 + RF_TILE_H, J.w);
+        const uint32_t ty0 = ty * RF_TILE_H + part % (RF_TILE_H / RF_LINE_ROWS) * RF_LINE_ROWS;
+        if (ty0 >= J.h) continue;
+        const uint32_t ty1 = min(ty0 + RF_LINE_ROWS, J.h);
         const uint32_t *tm = mask + (size_t)tile * J.mask_words;
-        for (uint32_t wb = 0; wb < J.mask_words; wb += 32) {
-            const uint32_t word = wb + lane < J.mask_words ? tm[wb + lane] : 0u;
-            uint32_t bal = __ballot_sync(0xFFFFFFFFu, word != 0u);
-            while (bal) {
-                const uint32_t src = __ffs(bal) - 1;
-                bal &= bal - 1;
-                uint32_t w = __shfl_sync(0xFFFFFFFFu, word, src);
-                while (w) {
-                    const uint32_t l = (wb + src) * 32 + (__ffs(w) - 1);
-                    w &= w - 1;
-                    const LineRec R = recs[l];
-                    uint64_t x = 0, y = 0;
-                    bool mine = false;
-                    if (R.wide) {  // lane = column
-                        x = tx0 + lane;
-                        if (x < tx1 && x >= R.begin && x - R.begin < R.n) {
-                            y = as_usize(jump(R.s0, R.d, (uint32_t)(x - R.begin)));
-                            mine = y >= ty0 && y < ty0 + RF_TILE_H && y < J.h;
+        bool loaded = false;
+        // The tile's lines in order: 32 mask words at a time (the next four
+        // rounds' already loaded), their set bits on to the pending list, which is
+        // drawn 32 lines at a time.
+        const auto words = [&](uint32_t w) { return w + lane < J.mask_words ? tm[w + lane] : 0u; };
+        uint32_t next[4] = {words(0), words(32), words(64), words(96)};
+        uint32_t word = 0, incl = 0, nlines = 0, lb = 0, wb = 0, pend = 0;
+        for (bool last = false; !last;) {
+            if (lb >= nlines) {
+                last = wb >= J.mask_words;
+                word = last ? 0u : next[0];
+                incl = __popc(word);
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, incl, o);
+                    if (lane >= (uint32_t)o) incl += y;
+                }
+                nlines = __shfl_sync(FULL, incl, 31);
+                lb = 0;
+                wb += 32u;
+                next[0] = next[1];
+                next[1] = next[2];
+                next[2] = next[3];
+                next[3] = words(wb + 96u);
+            }
+            if (lb < nlines) {
+                const uint32_t k = lb + lane;
+                uint32_t L = 0;
+#pragma unroll
+                for (uint32_t step = 16; step >= 1; step >>= 1) {
+                    const uint32_t v = __shfl_sync(FULL, incl, L + step - 1u);
+                    if (v <= k) L += step;
+                }
+                L &= 31u;
+                const uint32_t wl = __shfl_sync(FULL, word, L);
+                const uint32_t ex = __shfl_sync(FULL, incl - __popc(word), L);
+                if (k < nlines)
+                    s_pend[wib][pend + lane] = (wb - 32u + L) * 32u + rfr::nth_set_bit(wl, k - ex + 1u);
+                pend += min(nlines - lb, 32u);
+                lb += 32u;
+            }
+            __syncwarp();
+            if (pend == 0u || (pend < 32u && !last)) continue;
+            {
+                if (!loaded) {
+                    loaded = true;
+#pragma unroll 8
+                    for (uint32_t r = 0; r < RF_LINE_ROWS; ++r)
+                        if (ty0 + r < ty1 && tx0 + lane < tx1) {
+                            const size_t i = (size_t)(ty0 + r) * J.w + tx0 + lane;
+                            col[r * RF_LINE_PITCH + lane] = J.color[i];
+                            if (has_depth) dep[r * RF_LINE_PITCH + lane] = J.depth[i];
                         }
-                    } else {  // lane = row
-                        y = ty0 + lane;
-                        if (y < J.h && y >= R.begin && y - R.begin < R.n) {
-                            x = as_usize(jump(R.s0, R.d, (uint32_t)(y - R.begin)));
-                            mine = x >= tx0 && x < tx1;
+                }
+                const uint32_t here = min(pend, 32u);
+                const uint32_t line = lane < here ? s_pend[wib][lane] : 0u;
+                const uint32_t left = s_pend[wib][32u + lane];  // (past pend: not used)
+                __syncwarp();
+                s_pend[wib][lane] = left;
+                pend -= here;
+                uint32_t n = 0, first = 0;  // this line's steps in the tile's columns (rows)
+                if (lane < here) {
+                    const LineRec R = recs[line];
+                    s_rec[wib][lane] = R;
+                    const uint64_t t0 = R.wide ? tx0 : ty0, t1 = R.wide ? tx1 : ty1;
+                    const uint64_t a = max(R.begin, t0), b = min(R.begin + R.n, t1);
+                    // (a short line along x, a row or more above or below: skipped.
+                    // Its |d| <= 1, so RF_LINE_STEP additions near these rows are
+                    // off by far less than a row; below 0 it draws in row 0.)
+                    const float y0 = R.s0, y1 = fadd(R.s0, fmul(R.d, (float)R.n));
+                    const bool off = R.wide && R.n <= RF_LINE_STEP &&
+                                     (fmaxf(fmaxf(y0, y1), 0.0f) + 1.0f < (float)ty0 ||
+                                      fminf(y0, y1) - 1.0f > (float)ty1);
+                    if (a < b && !off) {
+                        n = (uint32_t)(b - a);
+                        first = (uint32_t)(a - R.begin);
+                    }
+                }
+                uint32_t items = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, items, o);
+                    if (lane >= (uint32_t)o) items += y;
+                }
+                const uint32_t total = __shfl_sync(FULL, items, 31), at = items - n;
+                const uint32_t nz = __ballot_sync(FULL, n != 0u);
+                // (packed: the table's entries are the lines with steps here)
+                if (n) s_item[wib][__popc(nz & below)] = make_uint2(first << 5 | lane, at);
+                __syncwarp();
+#pragma unroll 1
+                for (uint32_t base = 0; base < total; base += 32u) {
+                    const uint32_t starts = __reduce_or_sync(FULL, n && at - base < 32u ? 1u << (at - base) : 0u);
+                    const uint32_t before = __popc(__ballot_sync(FULL, n && at < base));
+                    uint32_t idx = 0xFFFFFFFFu, color = 0;
+                    float z = 0.0f;
+                    if (base + lane < total) {
+                        const uint2 it = s_item[wib][before + __popc(starts & upto) - 1u];
+                        const LineRec &R = s_rec[wib][it.x & 31u];
+                        const uint32_t step = (it.x >> 5) + (base + lane - it.y);
+                        const uint64_t along = R.begin + step, across = as_usize(line_step(R.s0, R.d, step));
+                        const uint64_t x = R.wide ? along : across, y = R.wide ? across : along;
+                        if (x >= tx0 && x < tx1 && y >= ty0 && y < ty1) {
+                            idx = ((uint32_t)y - ty0) * RF_LINE_PITCH + ((uint32_t)x - tx0);
+                            color = R.color;
+                            z = R.z;
                         }
                     }
-                    if (mine) {
-                        const size_t i = (size_t)y * J.w + x;
-                        bool pass = true;
-                        if (J.depth) {
-                            const float cur = J.depth[i];
-                            switch (J.depth_test) {  // ctx.rs:86-89
+                    const uint32_t rank = __popc(__match_any_sync(FULL, idx == 0xFFFFFFFFu ? ~lane : idx) & below);
+                    const uint32_t rounds = __reduce_max_sync(FULL, rank);
+                    for (uint32_t r = 0; r <= rounds; ++r) {
+                        if (idx != 0xFFFFFFFFu && rank == r) {
+                            bool pass = true;
+                            const float cur = has_depth ? dep[idx] : 0.0f;
+                            switch (test) {  // ctx.rs:86-89
                                 case RF_K_DEPTH_NONE: pass = true; break;
-                                case RF_K_DEPTH_LESS: pass = cur < R.z; break;
-                                case RF_K_DEPTH_EQUAL: pass = cur == R.z; break;
-                                default: pass = cur > R.z; break;
+                                case RF_K_DEPTH_LESS: pass = cur < z; break;
+                                case RF_K_DEPTH_EQUAL: pass = cur == z; break;
+                                default: pass = cur > z; break;
+                            }
+                            if (pass) {
+                                if (color_write) {
+                                    col[idx] = color;
+                                    fo += 1;
+                                }
+                                if (depth_write) dep[idx] = z;
                             }
                         }
-                        if (pass) {
-                            if (J.color_write) {
-                                J.color[i] = R.color;
-                                fo += 1;
-                            }
-                            if (J.depth && J.depth_write) J.depth[i] = R.z;
-                        }
+                        __syncwarp();  // (these pixels before the next round's tests)
                     }
-                    __syncwarp();  // this line's pixels before the next line's tests
                 }
             }
+        }
+        if (loaded) {
+#pragma unroll 8
+            for (uint32_t r = 0; r < RF_LINE_ROWS; ++r)
+                if (ty0 + r < ty1 && tx0 + lane < tx1) {
+                    const size_t i = (size_t)(ty0 + r) * J.w + tx0 + lane;
+                    if (color_write) J.color[i] = col[r * RF_LINE_PITCH + lane];
+                    if (depth_write) J.depth[i] = dep[r * RF_LINE_PITCH + lane];
+                }
+            __syncwarp();
         }
     }
     warp_add_u64(&stats->frags_o, fo, true);
@@ -276,8 +408,8 @@ cudaError_t launch_lines(const DrawDev *draws, const JobDev *jobs, uint32_t nl, 
     RF_NEXT(k_line_setup, blocks, 128, 0, s, draws, jobs, nl, cpos, coc, recs, mask, stats);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const uint32_t rblocks = min((ntiles + 3) / 4, (uint32_t)nsm * 8);
-    RF_NEXT(k_line_raster, rblocks, 128, 0, s, jobs, recs, mask, ntiles, queue, stats);
+    const uint32_t rblocks = min((ntiles * (RF_TILE_H / RF_LINE_ROWS) + RF_LINE_WARPS - 1) / RF_LINE_WARPS, (uint32_t)nsm * 8);
+    RF_NEXT(k_line_raster, rblocks, RF_LINE_WARPS * 32, 0, s, jobs, recs, mask, ntiles, queue, stats);
     return cudaGetLastError();
 }
 

@@ -155,3 +155,40 @@ def test_pending_clear_and_counts():
         tg.close()
     finally:
         dev.close()
+
+
+@pytest.mark.parametrize("size", [(33, 9), (64, 40), (257, 31)])
+@pytest.mark.parametrize("shape", ["coincident", "fans", "rows"])
+def test_tile_parts(size, shape):
+    """Many lines through the same pixels, lines longer than a batch's steps
+    and lines along the borders of the rows a warp draws, the target's edges
+    cutting tiles and parts of tiles."""
+    w, h = size
+    rng = np.random.default_rng(w * 7 + h)
+    n = 1100  # (mask words past the first batch of 32)
+    p = np.zeros((2 * n, 4), np.float32)
+    p[:, 3] = 1.0
+    if shape == "coincident":  # a few segments over and over, depths out of order
+        ends = rng.uniform(-1.1, 1.1, size=(12, 2, 2)).astype(np.float32)
+        p[:, :2] = ends[rng.integers(0, 12, n)].reshape(2 * n, 2)
+    elif shape == "fans":  # from one point to everywhere: short and long, steep and flat
+        p[0::2, :2] = np.float32(0.1)
+        r = rng.choice(np.array([0.02, 0.2, 2.0], np.float32), n)
+        a = rng.uniform(0, 2 * np.pi, n).astype(np.float32)
+        p[1::2, 0], p[1::2, 1] = 0.1 + r * np.cos(a), 0.1 + r * np.sin(a)
+    else:  # nearly flat, on and next to row borders, past the top and bottom too
+        y = (rng.integers(-1, h // 8 + 2, n) * 8 + rng.choice([-0.6, -0.5, 0.0, 0.4, 0.5], n)) * 2 / h - 1
+        p[0::2, 1], p[1::2, 1] = y, y + rng.choice([-3.0, 0.0, 0.4, 2.0], n) * 2 / h
+        p[0::2, 0] = rng.uniform(-1.2, 1.0, n)
+        p[1::2, 0] = p[0::2, 0] + rng.choice(np.array([3.0, 30.0, 300.0]), n) * 2 / w
+    z = rng.choice(np.array([0.5, 0.75, 1.0, 1.5], np.float32), n).repeat(2)
+    p *= z[:, None]
+    col = rng.uniform(0, 1, size=(2 * n, 3)).astype(np.float32)
+    v, li = np.concatenate([p, col], 1), np.arange(2 * n, dtype=np.uint32).reshape(n, 2)
+    for ctx in (rf.Context(), rf.Context(depth_test=rf.DEPTH_NONE)):
+        g, o = both(v, li, rf.GOURAUD, mat.viewport(0, 0, w, h), w, h, pos_dim=4, ctx=ctx)
+        assert o[2].frags_o > 100
+        check(g, o, "%s %dx%d" % (shape, w, h))
+    # (the viewport above the target: rows below 0 draw in row 0)
+    g, o = both(v, li, rf.GOURAUD, mat.viewport(0, -20, w, h - 20), w, h, pos_dim=4)
+    check(g, o, "%s %dx%d above" % (shape, w, h))
