@@ -992,11 +992,14 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         if ((st2 = raster(vjd, vdd, counters, kst))) return st2;
         CK(mark(RF_STAGE_N));
         if (per_job) CK(rfk::launch_stats_fold(kst, nj, P<StatsDev>(ctx->stats), s));
-        // draw counts, sort keys, per digit pass a histogram, a scan of 1 or 3
-        // launches and a scatter
+        // draw counts, sort keys, per digit pass a scatter, or a histogram, a
+        // scan of 1 or 3 launches and a scatter
         const uint32_t dpasses = 4 + (ndraws > 1 ? (ndraws > 256 ? (ndraws > 65536 ? 3 : 2) : 1) : 0);
         const uint32_t sitems = rfk::dsort_scan_items(n32);
-        sort_kernels = 2 + (n32 ? 1 + dpasses * (2 + (sitems <= RF_SCAN_BLOCK_ITEMS ? 1 : 3)) : 0);
+        sort_kernels = 2 + (n32 ? 1 + dpasses * (sitems == 0                     ? 1
+                                                       : sitems <= RF_SCAN_BLOCK_ITEMS ? 3
+                                                                                       : 5)
+                                : 0);
         return RF_OK;
     };
 

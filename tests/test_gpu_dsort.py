@@ -94,3 +94,36 @@ def test_batch_mixes_sorted_and_unsorted_jobs():
         for o in objs:
             o.close()
         dev.close()
+
+
+@pytest.mark.parametrize("n", [1, 256, 257, 32768, 32769, 65537, 262144, 262145, 525000])
+def test_sort_sizes(n):
+    """One call of n small triangles none of which is clipped: the sizes at
+    which a pass's blocks take more items and the digits are counted by a scan
+    instead; depths repeat, so that the order of equal keys shows."""
+    rng = np.random.default_rng(n)
+    w, h = 300, 200
+    c = rng.uniform(-0.95, 0.95, (n, 1, 2))
+    xy = c + rng.uniform(-0.03, 0.03, (n, 3, 2))
+    z = np.repeat(rng.choice(np.linspace(-0.9, 0.9, 1 + n // 2), n)[:, None, None], 3, 1)
+    v = np.concatenate([xy, z, np.ones((n, 3, 1)), rng.uniform(0, 1, (n, 3, 3))], -1)
+    d = DrawSpec(v.reshape(3 * n, 7).astype(np.float32), np.arange(3 * n, dtype=np.uint32).reshape(n, 3),
+                 rf.GOURAUD, pos_dim=4)
+    s = scenes.fill_stress(ntri=1, w=w, h=h, seed=1)
+    ctx = rf.Context(depth_sort=rf.SORT_BACK_TO_FRONT, depth_test=rf.DEPTH_NONE, face_cull=rf.CULL_NONE)
+    g, o = both([d], s["vp"], w, h, ctx)
+    assert g[2].prims_o == n
+    for depth in (g[1], o[1]):  # (a sliver's 0 / 0: which NaN it is depends on the processor)
+        depth[np.isnan(depth)] = np.nan
+    assert_parity(g, o, what="%d triangles" % n)
+
+
+def test_sort_many_calls():
+    """300 calls in one frame: the draw's digits (two passes more), odd and
+    even numbers of passes."""
+    for ninst in (40, 300):
+        s = scenes.instanced_cubes(ninst=ninst, w=320, h=200, seed=26, tex_size=32)
+        draws = [DrawSpec(s["verts"], s["faces"], rf.TEX_GOURAUD, m, tex=s["tex"]) for m in s["mvps"]]
+        ctx = rf.Context(depth_sort=rf.SORT_FRONT_TO_BACK, depth_test=rf.DEPTH_NONE)
+        g, o = both(draws, s["vp"], 320, 200, ctx)
+        assert_parity(g, o, what="%d calls" % ninst)
