@@ -30,25 +30,54 @@ __device__ __forceinline__ uint32_t upper_index(uint32_t n, uint32_t x, F key) {
     return lo;
 }
 
+// upper_index by a whole warp for one x (all lanes call): 32 records are
+// looked at a step, so 110,000 take four dependent loads instead of 17
+// (vertex stage of 64 scenes with as many draws: 86 us with a binary search by
+// one lane and a walk by each, 67 with these two; triangle lists 123 -> 118,
+// both rasters 685 -> 664).
+template <class F>
+__device__ __forceinline__ uint32_t warp_find(uint32_t n, uint32_t x, F key) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 1u) {
+        const uint32_t step = (hi - lo + 31u) / 32u, at = lo + lane * step;
+        const uint32_t b = __ballot_sync(0xFFFFFFFFu, lane == 0u || (at < hi && key(at) <= x));
+        lo += (31u - __clz(b)) * step;  // (keys do not decrease: the lanes that hold are the first ones)
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
 // upper_index for the 32 lanes of a warp whose x do not decrease with the
-// lane (all lanes call): one binary search for lane 0's x, then each lane
-// steps forward over the few records between (same result per lane).
+// lane (all lanes call): the search for lane 0's x, then each lane looks
+// through the next records, 32 loaded at a time.
 template <class F>
 __device__ __forceinline__ uint32_t warp_upper_index(uint32_t n, uint32_t x, F key) {
-    const uint32_t x0 = __shfl_sync(0xFFFFFFFFu, x, 0);
-    uint32_t d = 0;
-    if ((threadIdx.x & 31) == 0) d = upper_index(n, x0, key);
-    d = __shfl_sync(0xFFFFFFFFu, d, 0);
-    while (d + 1 < n && key(d + 1) <= x) ++d;
-    return d;
+    if (n <= 1u) return 0u;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = warp_find(n, __shfl_sync(0xFFFFFFFFu, x, 0), key), d = lo;
+    for (;;) {
+        const uint32_t k = lo + lane < n ? key(lo + lane) : 0xFFFFFFFFu;  // (no x is that large)
+        uint32_t i = 0;  // the last of these records not above x
+#pragma unroll
+        for (uint32_t step = 16; step >= 1u; step >>= 1)
+            if (__shfl_sync(0xFFFFFFFFu, k, i + step) <= x) i += step;
+        if (__shfl_sync(0xFFFFFFFFu, k, 0) <= x) d = lo + i;
+        if (!__any_sync(0xFFFFFFFFu, i == 31u)) return d;
+        lo += 31u;
+    }
 }
 
 // Warp-aggregated 64-bit counter add (all 32 lanes must call).
 __device__ __forceinline__ void warp_add_u64(unsigned long long *dst, unsigned long long v,
                                              bool same_dst) {
     if (same_dst) {
+        if (!__any_sync(0xFFFFFFFFu, (v >> 27) != 0ull)) {  // the sum fits 32 bits: one instruction
+            v = __reduce_add_sync(0xFFFFFFFFu, (uint32_t)v);
+        } else {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+        }
         if ((threadIdx.x & 31) == 0 && v) atomicAdd(dst, v);
     } else if (v) {
         atomicAdd(dst, v);

@@ -822,6 +822,13 @@ static_assert(RF_SETUP_WORDS % 2 == 1 && RF_SETUP_WORDS * 4 >= sizeof(RasterPrim
 // RF_INLINE_WIDTH px, are binned by the thread that sets them up.
 #define RF_INLINE_ROWS 8u
 #define RF_INLINE_WIDTH 128.0f
+// Bound by the instructions and their latencies of a warp's 32 triangles, not
+// by the registers' occupancy (12 or 14 blocks a multiprocessor, at 80 or 72
+// registers, were 3 and 9 % slower on the 500 k-triangle grid than the
+// compiler's 8).  There 109 us: with triangles that meet no row dropped (most of
+// it: the binade runs that one such lane made its warp work out) and both
+// halves' rows in one loop, 96.  (Records written five a pass, 16 bytes a lane,
+// instead of one: 103.)
 // NCT: the components (1 + attributes) of every triangle of the launch, or
 // 0 when its draws mix shader kinds.
 template <int NCT>
@@ -854,7 +861,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
     // clipped triangles then, and src_tri_base locates the input ones.
     // A block's triangles belong to one job.
     for (uint32_t blk = block0 + blockIdx.x; blk < block0 + nblocks; blk += gridDim.x) {
-        const uint32_t nth = upper_index(nj, blk, [&](uint32_t i) { return jobs[i].nth_block; });
+        const uint32_t nth = warp_find(nj, blk, [&](uint32_t i) { return jobs[i].nth_block; });
         const uint32_t job = jobs[nth].nth;
         const JobDev &J = jobs[job];
         const uint32_t base = J.tri_base + (blk - jobs[nth].nth_block) * RF_SETUP_THREADS;
@@ -939,15 +946,6 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                 const bool culled = (J.face_cull == RF_K_CULL_BACK && backface) ||
                                     (J.face_cull == RF_K_CULL_FRONT && !backface);
                 keep = !culled;
-                if (culled && cnt > 1) {
-                    // A piece of a clipped triangle: the rasteriser walks
-                    // every piece of a triangle it meets and skips this one.
-                    RasterPrim *R = rprims + p0 + c;
-                    R->draw = di;
-                    R->flags = 0u;
-                    R->kind = d.shader;
-                    R->zmax = __int_as_float(0x7F800000);
-                }
                 if (!culled) {
                     P.draw = di;
                     P.live = 1u;
@@ -1010,7 +1008,10 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                     }
                     const uint64_t w = regular ? (uint64_t)nrows * (1u + nc) : 0u;
                     if (w < 0x40000000ull) P.rwords = (uint32_t)w;
-                    if (P.rwords != 0u) {
+                    if (nrows == 0u) {  // between two rows, or past the buffer: draws nothing
+                        keep = false;
+                        oob += below;
+                    } else if (P.rwords != 0u) {
                         small = nrows <= RF_INLINE_ROWS && wide <= RF_INLINE_WIDTH;
                         mid = !small && nrows <= 16u;
                         if (small) oob += below;  // (the binning pass counts the others')
@@ -1020,6 +1021,15 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                             for (uint32_t r = 0; r < RF_NR; ++r) half_runs(P.half[hh], G->runs[hh], r);
                     }
                 }
+                if (!keep && cnt > 1) {
+                    // A piece of a clipped triangle: the rasteriser walks
+                    // every piece of a triangle it meets and skips this one.
+                    RasterPrim *R = rprims + p0 + c;
+                    R->draw = di;
+                    R->flags = 0u;
+                    R->kind = d.shader;
+                    R->zmax = __int_as_float(0x7F800000);
+                }
             }
             __syncwarp();
             // Room for this step's row records: one atomic per warp on the
@@ -1028,12 +1038,22 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
             // triangle's own records stay contiguous).  An offset past 32
             // bits is clamped, so the binning pass finds no room for it.
             {
-                const unsigned long long w = keep ? P.rwords : 0u;
+                const uint32_t w = keep ? P.rwords : 0u;
                 unsigned long long incl = w;
+                if (!__any_sync(FULL, (w >> 27) != 0u)) {  // (the sum fits 32 bits)
+                    uint32_t lo32 = w;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned long long y = __shfl_up_sync(FULL, incl, o);
-                    if (lane >= (uint32_t)o) incl += y;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(FULL, lo32, o);
+                        if (lane >= (uint32_t)o) lo32 += y;
+                    }
+                    incl = lo32;
+                } else {
+#pragma unroll 1
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned long long y = __shfl_up_sync(FULL, incl, o);
+                        if (lane >= (uint32_t)o) incl += y;
+                    }
                 }
                 const unsigned long long total = __shfl_sync(FULL, incl, 31);
                 unsigned long long at = 0;
@@ -1056,38 +1076,39 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                 const uint32_t rstride = 1u + nc;
                 uint32_t *rec = rows + P.rloc;
                 band0 = (inr[0] ? y0[0] : y0[1]) / RF_TILE_H;
+                // (one loop over both halves: a warp goes on to its longest
+                // triangle's rows, not to the longest upper and lower halves')
+                const uint32_t n0 = inr[0], n = n0 + inr[1];
+                float v[2 + NCL], st[2 + NCL], dvx[NCL];
 #pragma unroll 1
-                for (int hh = 0; hh < 2; ++hh) {
-                    const HalfRec &H = P.half[hh];
-                    float v[2 + NCL], st[2 + NCL], dvx[NCL];
+                for (uint32_t j = 0; j < n; ++j) {
+                    if (j == 0u || j == n0) {
+                        const HalfRec &H = P.half[j < n0 ? 0 : 1];
 #pragma unroll
-                    for (int r = 0; r < 2 + NCL; ++r) {
-                        v[r] = u2f(H.b0[r]);
-                        st[r] = H.d[r];
-                    }
-#pragma unroll
-                    for (int q = 0; q < NCL; ++q) dvx[q] = H.dvdx[q];
-                    const uint32_t n = inr[hh];
-#pragma unroll 1
-                    for (uint32_t j = 0; j < n; ++j) {
-                        RowOut o{0, 0, NONE, 0};
-                        row_record<NCT>(v[0], v[1], v + 2, 1u, dvx, nc, J.w, rec, o, zhi);
-                        rec += rstride;
-                        frags_i += o.frags_i;
-                        oob += o.oob;
-                        if (o.px0 < o.px1) {
-                            const bool second = (y0[hh] + j) / RF_TILE_H != band0;
-                            if (second) {
-                                lo[1] = min(lo[1], o.px0);
-                                hi[1] = max(hi[1], o.px1);
-                            } else {
-                                lo[0] = min(lo[0], o.px0);
-                                hi[0] = max(hi[0], o.px1);
-                            }
+                        for (int r = 0; r < 2 + NCL; ++r) {
+                            v[r] = u2f(H.b0[r]);
+                            st[r] = H.d[r];
                         }
 #pragma unroll
-                        for (int r = 0; r < 2 + NCL; ++r) v[r] = fadd(v[r], st[r]);
+                        for (int q = 0; q < NCL; ++q) dvx[q] = H.dvdx[q];
                     }
+                    RowOut o{0, 0, NONE, 0};
+                    row_record<NCT>(v[0], v[1], v + 2, 1u, dvx, nc, J.w, rec, o, zhi);
+                    rec += rstride;
+                    frags_i += o.frags_i;
+                    oob += o.oob;
+                    if (o.px0 < o.px1) {
+                        const bool second = (j < n0 ? y0[0] + j : y0[1] + (j - n0)) / RF_TILE_H != band0;
+                        if (second) {
+                            lo[1] = min(lo[1], o.px0);
+                            hi[1] = max(hi[1], o.px1);
+                        } else {
+                            lo[0] = min(lo[0], o.px0);
+                            hi[0] = max(hi[0], o.px1);
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < 2 + NCL; ++r) v[r] = fadd(v[r], st[r]);
                 }
             }
             // Their tile bits, a tile a lane at a time; lanes at the same tile
@@ -1114,7 +1135,8 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
                 }
             }
             const uint32_t smalls = __ballot_sync(FULL, small);
-            uint32_t bal = __ballot_sync(FULL, keep);
+            // (a single triangle without a tile bit is on no list: no record)
+            uint32_t bal = __ballot_sync(FULL, keep && !(small && cnt == 1u && lo[0] >= hi[0] && lo[1] >= hi[1]));
             const uint32_t dst = p0 + c;
             if (small && cnt == 1u) ent[gt] = make_uint2(dst, f2u(zhi));
             if (small) {  // the slot now holds its RasterPrim (dvdx's source lies past it)
@@ -1746,8 +1768,8 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict_
     const uint32_t piece = blockIdx.x * RF_LIST_WARPS + w;
     __shared__ unsigned long long place[RF_LIST_WARPS];
     const bool have = piece < npieces;
-    const JobDev &J = jobs[jobs[upper_index(nj, have ? piece : npieces - 1u,
-                                            [&](uint32_t i) { return (uint32_t)jobs[i].nth_seg; })].nth];
+    const JobDev &J = jobs[jobs[warp_find(nj, have ? piece : npieces - 1u,
+                                          [&](uint32_t i) { return (uint32_t)jobs[i].nth_seg; })].nth];
     const uint32_t r = (have ? piece : npieces - 1u) - (uint32_t)J.seg_base;
     const uint32_t lt = r / J.nseg, sg = r - lt * J.nseg, tile = J.tile_base + lt;
     uint32_t *sw = mask + J.sum_base + (size_t)lt * J.sum_words;

@@ -1395,7 +1395,7 @@ __global__ void __launch_bounds__(RF_RASTER_MAX_THREADS, 2) k_raster(const __gri
         if (item == 0xFFFFFFFFu) break;
         const uint32_t tile = item >> RF_ITEM_SHIFT, slice = item & ((1u << RF_ITEM_SHIFT) - 1u);  // 0: the whole tile
         if constexpr (TW % 32 == 0) bulk_store_drain();  // (the last tile's write-back)
-        const uint32_t ji = A.jobs[upper_index(A.nj, tile, [&](uint32_t i) { return A.jobs[i].nth_tile; })].nth;
+        const uint32_t ji = A.jobs[warp_find(A.nj, tile, [&](uint32_t i) { return A.jobs[i].nth_tile; })].nth;
         raster_tile<TW, KIND, FAST>(A, A.jobs[ji], ji, tile, slice, smem + warp * WARP_WORDS, lane);
     }
     // (shared memory stays allocated until the last write-back has read it)

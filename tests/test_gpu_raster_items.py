@@ -127,3 +127,34 @@ def test_every_raster_group_in_one_batch():
         for x in keep:
             x.close()
         dev.close()
+
+
+@pytest.mark.parametrize("ndraws", [31, 33, 1025, 1100])
+def test_many_small_draws(ndraws):
+    """Draws of one triangle (a warp's triangles belong to 32 draws), of none
+    and of many among them: the lookups of a triangle's and a vertex's draw."""
+    rng = np.random.default_rng(ndraws)
+    w, h = 256, 160
+    draws = []
+    for i in range(ndraws):
+        n = int(rng.choice([0, 1, 1, 1, 1, 2, 40], p=[.1, .2, .2, .2, .1, .1, .1]))
+        d = tris(1000 * ndraws + i, max(n, 1), w, h, (2, 30, 1, 20))
+        draws.append(DrawSpec(d.verts, d.faces[:n], rf.GOURAUD, pos_dim=4))
+    vp = mat.viewport(0, 0, w, h)
+    assert_parity(gpu_render(draws, vp, w, h), oracle_render(draws, vp, w, h), what="%d draws" % ndraws)
+
+
+@pytest.mark.parametrize("size", [(1, 200, 0.02, 0.6), (0.02, 0.6, 1, 40)])
+def test_triangles_between_rows_or_columns(size):
+    """Triangles that meet no row (or no column), some of them pieces of
+    clipped ones, some past the target's last row."""
+    w, h = 300, 120
+    d = tris(77, 4000, w, h + 40, size, cross=0.2)
+    d.verts[:, 1] *= (h + 40) / h
+    vp = mat.viewport(0, 0, w, h)
+    for cull in (rf.CULL_BACK, rf.CULL_NONE):
+        ctx = rf.Context(face_cull=cull)
+        g, o = gpu_render([d], vp, w, h, ctx=ctx), oracle_render([d], vp, w, h, ctx=ctx)
+        for depth in (g[1], o[1]):  # (a sliver's 0 / 0: which NaN it is depends on the processor)
+            depth[np.isnan(depth)] = np.nan
+        assert_parity(g, o, what="cull %d" % cull)
