@@ -121,9 +121,10 @@ struct Kind {
     }
     __device__ static __forceinline__ uint32_t from_texel(uint32_t t, const float *v) {
         if constexpr (KIND == RF_K_TEX_GOURAUD) {
-            const float tr = fdiv((float)(t & 0xFFu), 256.0f);
-            const float tg = fdiv((float)((t >> 8) & 0xFFu), 256.0f);
-            const float tb = fdiv((float)((t >> 16) & 0xFFu), 256.0f);
+            // (a power of two: the product is the quotient, exactly)
+            const float tr = fmul((float)(t & 0xFFu), 1.0f / 256.0f);
+            const float tg = fmul((float)((t >> 8) & 0xFFu), 1.0f / 256.0f);
+            const float tb = fmul((float)((t >> 16) & 0xFFu), 1.0f / 256.0f);
             return to_color4(fmul(tr, v[1]), fmul(tg, v[2]), fmul(tb, v[3]));
         } else {
             return t;
@@ -149,11 +150,7 @@ struct Kind {
             // Scanline::fragments: var.z_div(pos.z) (raster.rs:60-69)
             return sample_tex(d, fdiv(v[1], v[0]), fdiv(v[2], v[0]));
         } else if constexpr (KIND == RF_K_TEX_GOURAUD) {
-            const uint32_t t = sample_tex(d, fdiv(v[4], v[0]), fdiv(v[5], v[0]));
-            const float tr = fdiv((float)(t & 0xFFu), 256.0f);
-            const float tg = fdiv((float)((t >> 8) & 0xFFu), 256.0f);
-            const float tb = fdiv((float)((t >> 16) & 0xFFu), 256.0f);
-            return to_color4(fmul(tr, v[1]), fmul(tg, v[2]), fmul(tb, v[3]));
+            return from_texel(texel(d, v), v);
         } else {  // GOURAUD_SRGB: Color3f<LinRgb>::to_srgb (color.rs:383-392)
             const float ig = fdiv(1.0f, 2.2f);
             return to_color4(powf(v[1], ig), powf(v[2], ig), powf(v[3], ig));
@@ -461,8 +458,12 @@ __device__ __forceinline__ void stage_row(uint32_t *slot, uint32_t lane, bool pr
 // instructions for 32 pixels of Gouraud, where the exact jump takes about 100
 // a component), more by the jump, in place.  (Records that also held the
 // varyings at the first tile boundary saved up to a tile's steps here, but
-// were nearly twice as long.)
-#define RF_STEP_MAX 128u
+// were nearly twice as long.)  The line at 128 steps, where lanes that jump no
+// longer wait for each other's branches, was too low by the slowest tile: a
+// round of jumps takes 5,000 cycles, 512 steps 2,000 (raster of a cube 300 px
+// wide 26 -> 19 us, of 10,000 objects 116 -> 101; 256, 1,024 and 4,096 measure
+// the same).
+#define RF_STEP_MAX 512u
 template <int KIND>
 __device__ __forceinline__ void item_load(const float *dvdx, uint32_t *rs, uint32_t nc, uint32_t k, float2 *v,
                                           float2 *dv) {
@@ -979,13 +980,23 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
     const uint32_t ys = slice ? ty0 + (slice - 1u) * SLICE_H : ty0;
     const uint32_t ye = min(slice ? ys + SLICE_H : ty0 + RF_TILE_H, J.h);
     const uint32_t below = (1u << lane) - 1u, upto = below | (1u << lane);
-    constexpr int U_SEG = KIND == RF_K_ANY ? 1 : KIND == RF_K_GOURAUD_SRGB || !FAST ? 2 : 4;
-    constexpr int U_PACK = KIND == RF_K_ANY ? 1 : 2;
+    // Pixels a lane has in flight: as many as the registers and the instruction
+    // cache bear.  Texture with colour: 2 where 4 took 113 us instead of 99 on
+    // 10,000 objects; a texture alone, packed: 8 where 2 took 53 instead of 51 on
+    // 1,600 crates.
+    constexpr int U_SEG = KIND == RF_K_ANY ? 1
+                          : KIND == RF_K_GOURAUD_SRGB || KIND == RF_K_TEX_GOURAUD || !FAST ? 2 : 4;
+    constexpr int U_PACK = KIND == RF_K_ANY ? 1 : KIND == RF_K_TEXTURED && FAST ? 8 : 2;
     // Two lanes a segment where a round leaves room: pays where a pixel costs a
     // texel or the general tests (rasters of 10,000 textured objects 113.7 ->
     // 108.8 us, of 20,000 sorted triangles without depth 117.2 -> 109.8), not
     // for Gouraud's (100,000 triangles 173.1 -> 178.2).
     constexpr bool PAIRS = !FAST || KIND == RF_K_TEXTURED || KIND == RF_K_TEX_GOURAUD;
+    // Four lanes a span where a packed round has few (most of the 32 are hidden
+    // ones): the crates' raster 55 -> 53 us.  Not for texture with colour (the
+    // 10,000 objects 81 -> 76, but the 500 k-triangle grid, whose rounds are
+    // full, 91 -> 94) nor Gouraud (64 scenes 512 -> 521).
+    constexpr bool SPLIT = KIND == RF_K_TEXTURED || KIND == RF_K_GOURAUD_SRGB;
     constexpr bool PAINTED = KIND != RF_K_GOURAUD && KIND != RF_K_GOURAUD_SRGB;  // shading reads the draw
 
     // The item at row `row` of table entry ki whose record is in this lane's
@@ -1310,7 +1321,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
                 stage_pass(0u);
 #pragma unroll 1
                 for (uint32_t base = 0; base < total; base += 32u) {
-                    const uint32_t ki = kin, row = rown;
+                    uint32_t ki = kin, row = rown;
                     uint32_t *rs = rslots + sl * G::SLOT + lane;
                     sl ^= 1u;
                     stage_pass(base + 32u);
@@ -1328,23 +1339,52 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
                         if (lower && oa < b && a < ob) wait |= 1u << src;
                         lower &= lower - 1u;
                     }
-                    const Paint paint(A.draws[PAINTED && act ? tab_draw[ki] : 0u]);
                     while (pend) {
-                        const bool go = ((pend >> lane) & 1u) && (wait & pend) == 0u;
+                        bool go = ((pend >> lane) & 1u) && (wait & pend) == 0u;
+                        const uint32_t gm = __ballot_sync(FULL, go), cnt = __popc(gm);
+                        pend &= ~gm;
+                        if (SPLIT && pend == 0u && cnt <= 8u) {
+                            // The last ones, and few: four lanes a span.
+                            const uint32_t src = nth_set_bit(gm, min(lane >> 2, cnt - 1u) + 1u);
+                            go = lane >> 2 < cnt;
+                            row = __shfl_sync(FULL, row, src);
+                            ki = __shfl_sync(FULL, ki, src);
+                            a = __shfl_sync(FULL, a, src);
+                            b = __shfl_sync(FULL, b, src);
+                            if (KIND == RF_K_ANY) kind = __shfl_sync(FULL, kind, src);
+#pragma unroll
+                            for (int c = 0; c < NP; ++c) {
+                                v[c].x = __shfl_sync(FULL, v[c].x, src);
+                                v[c].y = __shfl_sync(FULL, v[c].y, src);
+                                dv[c].x = __shfl_sync(FULL, dv[c].x, src);
+                                dv[c].y = __shfl_sync(FULL, dv[c].y, src);
+                            }
+                            const uint32_t part = (b - a + 3u) >> 2, skip = part * (lane & 3u);
+#pragma unroll 1
+                            for (uint32_t i = 0; i < skip; ++i) {
+#pragma unroll
+                                for (int c = 0; c < NP; ++c) v[c] = __fadd2_rn(v[c], dv[c]);
+                            }
+                            a += skip;
+                            b = min(b, a + part);
+                            go = go && a < b;
+                            T.row = row;
+                        }
+                        uint32_t nout = 0;
                         if (go) {
+                            const Paint paint(A.draws[PAINTED ? tab_draw[ki] : 0u]);
                             uint32_t idx = (a - T.tx0) * RF_TILE_H + row;
                             const uint32_t end = (b - T.tx0) * RF_TILE_H + row;
-                            uint32_t nout = 0;
                             do nout += px_group<KIND, FAST, U_PACK>(T, paint, kind, v, dv, idx, end);
                             while (idx < end);
                             T.frags_o += nout;
-                            if constexpr (FAST) {
-                                if (nout)
-                                    for (uint32_t sg = (a - T.tx0) / RF_SEG; sg <= (b - 1u - T.tx0) / RF_SEG; ++sg)
-                                        seg_refresh(T, sg);
-                            }
                         }
-                        pend &= ~__ballot_sync(FULL, go);
+                        if constexpr (FAST) {
+                            if (SPLIT) __syncwarp();  // (all of a span's lanes' depths before the least)
+                            if (nout)
+                                for (uint32_t sg = (a - T.tx0) / RF_SEG; sg <= (b - 1u - T.tx0) / RF_SEG; ++sg)
+                                    seg_refresh(T, sg);
+                        }
                         __syncwarp();  // (the depths written before the next round reads them)
                     }
                 }
