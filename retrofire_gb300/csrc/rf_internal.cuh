@@ -149,6 +149,8 @@ static_assert(offsetof(PrimRec, runs) == RF_PRIM_CORE_BYTES && RF_PRIM_CORE_BYTE
 // RasterPrim: the rasteriser's view of one output triangle.
 #define RF_RP_LIVE 1u
 #define RF_RP_ROWS 2u  // row records present (else rasterise from the PrimRec)
+#define RF_RP_EDGES 4u // ... and more than RF_EDGE_ROWS of them: the rasteriser looks which rows meet a tile
+#define RF_EDGE_ROWS 32u
 struct RasterPrim {
     uint32_t draw;
     uint32_t flags;

@@ -1334,7 +1334,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                 }
             }
             if (lane == 0 && regular) {
-                R->flags |= RF_RP_ROWS;
+                R->flags |= RF_RP_ROWS | (P->half[0].n + P->half[1].n > RF_EDGE_ROWS ? RF_RP_EDGES : 0u);
                 R->base = (uint32_t)base;
                 R->stride = stride;
             }

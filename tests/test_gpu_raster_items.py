@@ -158,3 +158,31 @@ def test_triangles_between_rows_or_columns(size):
         for depth in (g[1], o[1]):  # (a sliver's 0 / 0: which NaN it is depends on the processor)
             depth[np.isnan(depth)] = np.nan
         assert_parity(g, o, what="cull %d" % cull)
+
+
+@pytest.mark.parametrize("tile", [(8, 4), (16, 4), (32, 4), (64, 2)])
+@pytest.mark.parametrize("kind", [rf.FLAT, rf.GOURAUD, rf.GOURAUD_SRGB])
+def test_slanted_tall_triangles(tile, kind):
+    """Triangles of 32, 33 and more rows, thin and slanted either way (most of
+    their rows miss a tile they are binned into), vertical, and wider than the
+    target; on a target smaller than the viewport too."""
+    rng = np.random.default_rng(31)
+    w, h, n = 400, 300, 500
+    dy = rng.choice([31.5, 32.0, 33.0, 34.0, 90.0, 280.0], n)
+    dx = rng.choice([0.0, 3.0, -3.0, 40.0, -40.0, 300.0, -300.0, 2000.0, -2000.0], n)
+    x, y = rng.uniform(-50, w, n), rng.uniform(-20, h - 20, n)
+    px = np.stack([np.stack([x, y], 1), np.stack([x + dx, y + dy], 1),
+                   np.stack([x + dx * rng.uniform(0, 1, n) + rng.choice([0.4, 3.0, 30.0], n),
+                             y + dy * rng.uniform(0, 1, n)], 1)], 1)
+    wv = rng.uniform(1.0, 3.0, (n, 3))
+    clip = np.stack([(px[..., 0] / (w / 2.0) - 1.0) * wv, (px[..., 1] / (h / 2.0) - 1.0) * wv,
+                     rng.uniform(-0.9, 0.9, (n, 3)) * wv, wv], -1)
+    v = np.concatenate([clip, rng.uniform(0, 1, (n, 3, NATTR[kind]))], -1).reshape(3 * n, -1).astype(np.float32)
+    d = DrawSpec(v, np.arange(3 * n, dtype=np.uint32).reshape(n, 3), kind, pos_dim=4, flat_rgba=0xFF336699)
+    for ctx, tw, th in ((rf.Context(face_cull=rf.CULL_NONE), w, h),
+                        (rf.Context(face_cull=rf.CULL_NONE, depth_test=rf.DEPTH_NONE), w - 90, h - 70)):
+        vp = mat.viewport(0, 0, w, h)
+        g, o = gpu_render([d], vp, tw, th, ctx=ctx, tile=tile), oracle_render([d], vp, tw, th, ctx=ctx)
+        for depth in (g[1], o[1]):
+            depth[np.isnan(depth)] = np.nan
+        assert_parity(g, o, color_tol=1 if kind == rf.GOURAUD_SRGB else 0, what="tile %r" % (tile,))
