@@ -1216,12 +1216,26 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
       unsigned long long *__restrict__ marks, const uint32_t *__restrict__ live_n) {
     grid_begin();
     const uint32_t lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & 7;
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const uint32_t tw_log2 = __ffs(tile_w) - 1;  // tile widths are powers of two
     // Only the triangles that passed the face-cull test (the live list, in
     // no particular order: every output below depends on the triangle alone).
     const uint32_t nl = *live_n;
+    // Few triangles: `parts` warps of a block share one, each taking every
+    // parts-th 32 rows of it (stepping over the others' rows), so that a tall
+    // triangle is not one warp's chain of rows.  Then a warp has at most one.
+    // Setup stage of a cube 300 px high 32.1 -> 27.8 us, of 1,600 crates 38.6 ->
+    // 36.1; with half as many warps to spare (twice the triangles) 10,000
+    // objects took 83 instead of 80.
+    // Many, two or more a warp: half of the blocks take them all (a block's start
+    // costs: 75,000 triangles 126 us with 16 blocks a multiprocessor, 115 with 8;
+    // 12,000, one a warp, are 2 us better off with 16).
+    const uint32_t nb = nl >= gridDim.x * 16u ? (gridDim.x + 1u) / 2u : gridDim.x;
+    if (blockIdx.x >= nb) return;
+    uint32_t nw = nb * 8u, parts = 1;
+    while (parts < 8u && nl * parts * 4u <= nw) parts *= 2u;
+    const uint32_t part = wib & (parts - 1u);
+    const uint32_t wid = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) / parts;
+    nw /= parts;
     // Two record slots per warp of the 256-thread block: the next triangle's
     // record is copied (cp.async) while the current one is walked.
     __shared__ __align__(16) uint4 sbuf[8][2][RF_PRIM_CORE_BYTES / 16];  // records' first parts
@@ -1284,6 +1298,13 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
             ++acc_marks;
         }
     };
+    auto finish = [&](const PrimRec *P, uint32_t p) {
+        if (lane == 0 && !P->fan) ent[P->tri] = make_uint2(p, f2u(R->zmax));
+        const uint4 *src = reinterpret_cast<const uint4 *>(R);
+        uint4 *dst = reinterpret_cast<uint4 *>(rprims + p);
+        if (lane < sizeof(RasterPrim) / 16) dst[lane] = src[lane];
+    };
+    uint32_t mine = 0xFFFFFFFFu;
     for (uint32_t i = wid; i < nl; i += nw) {
         const uint32_t pnn = i + 2 * nw < nl ? __ldg(live + i + 2 * nw) : 0u;
         __syncwarp();  // the other slot's previous triangle is done
@@ -1324,9 +1345,9 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                 base = P->rloc;
                 if (base + P->rwords > rows_cap) {  // no room: rasterise from the PrimRec
                     regular = false;
-                    if (lane == 0) atomicAdd(&counters[RF_CNT_ROWSOVF], 1u);
+                    if (lane == 0 && part == 0u) atomicAdd(&counters[RF_CNT_ROWSOVF], 1u);
                     // ... which then needs its binade runs (lane r: quantity r).
-                    if (lane < RF_NR) {
+                    if (lane < RF_NR && part == 0u) {
                         half_runs(sP->half[0], prims[p].runs[0], lane);
                         half_runs(sP->half[1], prims[p].runs[1], lane);
                     }
@@ -1349,14 +1370,14 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                 if (n == 0) continue;
                 const float y0r = H->y0r;
                 if (!(fabsf(y0r) < RF_MAX_COORD)) {  // outside the supported range
-                    if (lane == 0) acc_oob += 1;
+                    if (lane == 0 && part == 0u) acc_oob += 1;
                     continue;
                 }
                 // row(j) = max(0, Y + j); |y0r| < 2^22, so the 32-bit convert
                 const int64_t Y = (int32_t)fsub(y0r, 0.5f);
                 // Scanlines at or below the buffer's last row count only in oob.
                 const int64_t in_rows = min((int64_t)n, max((int64_t)0, (int64_t)J.h - Y));
-                if (lane == 0) acc_oob += (unsigned long long)((int64_t)n - in_rows);
+                if (lane == 0 && part == 0u) acc_oob += (unsigned long long)((int64_t)n - in_rows);
                 if (in_rows <= 0) continue;
                 Yh[hh] = Y;
                 inh[hh] = (uint32_t)in_rows;
@@ -1408,8 +1429,14 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                 // 32 rows at a time from the triangle's first one (not from the
                 // target's bands: a triangle of 20 rows is one chunk, not two).
                 const int32_t last = (inh[0] | inh[1]) ? yhi : ylo - 1;
-                for (int32_t cs = ylo; cs <= last; cs += RF_TILE_H) {
+                uint32_t turn = parts - part;  // (a chunk of this warp's when a multiple of parts)
+                for (int32_t cs = ylo; cs <= last; cs += RF_TILE_H, ++turn) {
                     const int32_t ce = min(last, cs + RF_TILE_H - 1);
+                    if (turn & (parts - 1u)) {  // another warp's: stepped over
+                        if (wlane)
+                            for (int32_t k = min(ce, whi) - max(cs, wlo); k >= 0; --k) wv = fadd(wv, wd);
+                        continue;
+                    }
                     if (wlane) walk(wv, wd, max(cs, wlo), min(ce, whi), cs);
                     __syncwarp();
                     const int32_t y = cs + (int32_t)lane;
@@ -1436,7 +1463,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
                 if (lane == 0) R->zmax = zhi_tri;
                 zhi_tri = -__int_as_float(0x7F800000);
             }
-            for (int hh = 0; hh < 2 && !regular; ++hh) {
+            for (int hh = 0; hh < 2 && !regular && part == 0u; ++hh) {
                 const HalfRec *H = &P->half[hh];
                 if (inh[hh] == 0) continue;
                 const int64_t Y = Yh[hh];
@@ -1481,11 +1508,21 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
             }
         }
         __syncwarp();
-        if (lane == 0 && !P->fan) ent[P->tri] = make_uint2(p, f2u(R->zmax));
-        {
-            const uint4 *src = reinterpret_cast<const uint4 *>(R);
-            uint4 *dst = reinterpret_cast<uint4 *>(rprims + p);
-            if (lane < sizeof(RasterPrim) / 16) dst[lane] = src[lane];
+        if (parts > 1u) {  // (its only one: written below)
+            mine = p;
+            break;
+        }
+        finish(P, p);
+    }
+    if (parts > 1u) {  // the largest of the warps' depth bounds
+        __syncthreads();
+        if (mine != 0xFFFFFFFFu && part == 0u) {
+            float z = R->zmax;
+            for (uint32_t k = 1; k < parts; ++k) z = fmaxf(z, srp[wib + k].zmax);
+            __syncwarp();
+            if (lane == 0) R->zmax = z;
+            __syncwarp();
+            finish(reinterpret_cast<const PrimRec *>(sbuf[wib][0]), mine);
         }
     }
     flush();
@@ -1982,7 +2019,7 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
         const uint32_t sblocks = min((gt + 31) / 32, (uint32_t)nsm * 4);
         RF_NEXT(bin16, sblocks, 256, 0, s, jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                       counters, marks, mid_n, big_n);
-        const uint32_t wblocks = min((gt * 2 + 7) / 8, (uint32_t)nsm * 16);
+        const uint32_t wblocks = min(gt, (uint32_t)nsm * 16);
         RF_NEXT(bin, wblocks, 256, 0, s, draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                     counters, marks, big_n);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -186,3 +186,15 @@ def test_slanted_tall_triangles(tile, kind):
         for depth in (g[1], o[1]):
             depth[np.isnan(depth)] = np.nan
         assert_parity(g, o, color_tol=1 if kind == rf.GOURAUD_SRGB else 0, what="tile %r" % (tile,))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 9, 40, 300])
+def test_few_tall_triangles(n):
+    """Few triangles of up to a target's height, several warps to each one's
+    rows: chunks of 32 rows, the last one short; clipped pieces among them."""
+    w, h = 200, 700
+    d = tris(500 + n, n, w, h, (20, 150, 30, 1500), cross=0.2)
+    vp = mat.viewport(0, 0, w, h)
+    for tile in ((8, 4), (32, 4)):
+        g, o = gpu_render([d], vp, w, h, tile=tile), oracle_render([d], vp, w, h)
+        assert_parity(g, o, what="%d triangles, tile %r" % (n, tile))
