@@ -1755,7 +1755,12 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
 // pass.
 #define RF_SPLIT_MIN 64u  // a tile with fewer binned triangles is never split
 #define RF_HEAVY_MIN 16u  // ... nor taken early
-#define RF_LIST_WARPS 8u
+// Warps a block, which takes its lists' place with one atomic: its warps wait
+// for the longest of them, and all wait for memory, so small blocks and as many
+// as 42 registers allow.  Setup stage of the 500 k-triangle grid 148 us with 8
+// warps and 48 registers, 142 so; loading 64 summary words ahead took 62
+// registers and 5 us more.
+#define RF_LIST_WARPS 4u
 namespace {
 // Position of the r-th set bit of v (r >= 1, at most popc(v)): halving
 // search on popcounts.
@@ -1793,7 +1798,7 @@ __device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t k) {
 }
 }  // namespace
 
-__global__ void __launch_bounds__(RF_LIST_WARPS * 32)
+__global__ void __launch_bounds__(RF_LIST_WARPS * 32, 12)
 k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict__ mask,
              uint32_t ntiles, uint32_t npieces, const uint2 *__restrict__ ent,
              unsigned long long *__restrict__ tacc, const unsigned long long *__restrict__ marks, uint32_t slots, uint32_t *__restrict__ items,
@@ -1814,11 +1819,12 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict_
     const uint32_t s0 = sg * J.seg_words, s1 = have ? min(s0 + J.seg_words, J.sum_words) : s0;
     // Steps over the piece's nonzero mask words in order, up to 32 a step, one a
     // lane (m, at index wi): false when there are none left.
+    auto sword = [&](uint32_t b) { return b + lane < s1 ? sw[b + lane] : 0u; };
     uint32_t sb = s0, v = 0, vincl = 0, vtotal = 0, vk = 0, m = 0, wi = 0;
     auto step = [&]() -> bool {
         while (vk >= vtotal) {
             if (sb >= s1) return false;
-            v = sb + lane < s1 ? sw[sb + lane] : 0u;
+            v = sword(sb);
             vincl = warp_incl(__popc(v), lane);
             vtotal = __shfl_sync(FULL, vincl, 31);
             vk = 0;
@@ -1879,8 +1885,13 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict_
         }
     }
     if (fits)
-        for (uint32_t i = s0 + lane; i < s1; i += 32u)
-            if (sw[i]) sw[i] = 0u;
+        for (uint32_t b = s0; b < s1; b += 128u) {  // (four loads in flight)
+            const uint32_t a0 = sword(b), a1 = sword(b + 32u), a2 = sword(b + 64u), a3 = sword(b + 96u);
+            if (a0) sw[b + lane] = 0u;
+            if (a1) sw[b + 32u + lane] = 0u;
+            if (a2) sw[b + 64u + lane] = 0u;
+            if (a3) sw[b + 96u + lane] = 0u;
+        }
     // The tile's work item, by the last of its pieces to come here.
     if (lane == 0) {
         uint32_t c = n;
