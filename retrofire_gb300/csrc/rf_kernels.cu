@@ -1,16 +1,17 @@
 // rf_kernels.cu — CUDA kernels of the triangle render path (sm_103a).
 //
 // Stage map (reference call stack: core/src/render.rs:134-207):
-//   k_zero       the frame's masks and counters
+//   k_zero       the frame's counters and totals
 //   k_vertex     vertex shader + ClipVert::new         render.rs:157-165
 //   k_clip       status; the crossing triangles queue  clip.rs:245-267
 //   k_clip_poly  Sutherland-Hodgman on the queue       clip.rs:283-301,350-400
 //   k_scan_*     order-preserving compaction offsets   (submission order)
 //   k_setup      to_screen, face cull, tri_fill/scan   prim.rs:62-88, raster.rs:185-302
-//                setup, the live list
-//   k_bin        scanline walk: stats (frags.i, oob),  raster.rs:80-114, target.rs:259-264
-//                row records, tile binning, one warp
-//                per live triangle
+//                setup; small triangles binned; the
+//                others onto the live lists
+//   k_bin_small, scanline walk: stats (frags.i, oob),  raster.rs:80-114, target.rs:259-264
+//   k_bin        row records, tile binning, sixteen
+//                lanes or a warp per live triangle
 //   k_tile_lists the tiles' triangle lists and the     (scheduling only)
 //                rasteriser's work list
 //   k_raster     per-tile span fill, depth test,       raster.rs:60-69, target.rs:163-198
@@ -819,7 +820,10 @@ __device__ __forceinline__ void row_record(float lx, float rx, const float *cv, 
 #define RF_SETUP_WORDS (RF_PRIM_CORE_BYTES / 4 + 1)
 static_assert(RF_SETUP_WORDS % 2 == 1 && RF_SETUP_WORDS * 4 >= sizeof(RasterPrim), "setup slots");
 // Triangles of at most RF_INLINE_ROWS rows on the target, no wider than
-// RF_INLINE_WIDTH px, are binned by the thread that sets them up.
+// RF_INLINE_WIDTH px, are binned by the thread that sets them up (500 k-triangle
+// grid: setup stage 200 us, 245 with eight lanes a triangle in a launch of their
+// own; 100,000 triangles 224 and 235).  Larger ones leave a warp waiting for the
+// longest.
 #define RF_INLINE_ROWS 8u
 #define RF_INLINE_WIDTH 128.0f
 // Bound by the instructions and their latencies of a warp's 32 triangles, not
@@ -1200,10 +1204,11 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
 // ---------------------------------------------------------------------------
 // K3b: scanline statistics and tile binning, one warp per triangle.
 // For every scanline of both halves (ScanlineIter::next, raster.rs:80-114)
-// the lane owning that row computes the exact edge values (closed-form run or
-// the general loop), then frags.i / oob as rasterize_fb counts them
-// (target.rs:259-264) and the pixel columns it covers; a warp reduction per
-// 32-row band gives the tiles to mark in the job's bitmask.
+// the lane owning that row takes the exact edge values (from a sequential walk;
+// without row records, a closed-form run or the general loop), then frags.i /
+// oob as rasterize_fb counts them (target.rs:259-264) and the pixel columns it
+// covers; a warp reduction per 32-row chunk gives the tiles to mark in the job's
+// bitmask.
 // ---------------------------------------------------------------------------
 // NCT: the components (1 + attributes) of every triangle of the launch, or
 // 0 when its draws mix shader kinds (taken per triangle).
@@ -1227,8 +1232,8 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
     // 36.1; with half as many warps to spare (twice the triangles) 10,000
     // objects took 83 instead of 80.
     // Many, two or more a warp: half of the blocks take them all (a block's start
-    // costs: 75,000 triangles 126 us with 16 blocks a multiprocessor, 115 with 8;
-    // 12,000, one a warp, are 2 us better off with 16).
+    // costs: setup stage of 75,000 triangles at tile width 8 256 us with 16 blocks
+    // a multiprocessor, 236 with 8; 12,000, one a warp, are 2 us better off with 16).
     const uint32_t nb = nl >= gridDim.x * 16u ? (gridDim.x + 1u) / 2u : gridDim.x;
     if (blockIdx.x >= nb) return;
     uint32_t nw = nb * 8u, parts = 1;
@@ -1530,7 +1535,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
 }
 
 // ---------------------------------------------------------------------------
-// K3c: the same work for small triangles, G = 8 or 16 lanes per triangle.
+// K3c: the same work for small triangles, G = 16 lanes per triangle.
 // A regular triangle with at most G rows on the target (k_setup puts it on
 // that group size's list) would leave most of a warp idle in k_bin, so
 // here a group of G lanes takes it -- 32 / G triangles per warp (its
@@ -1542,8 +1547,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
 // live list instead (k_bin runs after this kernel and takes it with the
 // rest).
 // ---------------------------------------------------------------------------
-static_assert(sizeof(RasterPrim) / 16 <= 8, "a group of eight lanes stores a RasterPrim in one pass");
-// G: lanes per triangle (8 or 16: the list of triangles with at most G rows).
+// G: lanes per triangle (those of at most G rows).
 template <int NCT, uint32_t G>
 __global__ void __launch_bounds__(256, 4)
 k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
@@ -1553,12 +1557,12 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
             unsigned long long *__restrict__ marks, const uint32_t *__restrict__ small_n,
             uint32_t *__restrict__ live_n) {
     grid_begin();
-    static_assert(G == 8 || G == 16, "group sizes");
+    static_assert(G == 16 && sizeof(RasterPrim) / 16 <= G, "a group stores a RasterPrim in one pass");
     constexpr uint32_t NG = 32 / G;  // groups per warp
     constexpr uint32_t NONE = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & 7;
     const uint32_t g = lane / G, gl = lane & (G - 1);  // group of the warp, lane in the group
-    const uint32_t gmask = (G == 16 ? 0xFFFFu : 0xFFu) << (G * g);
+    const uint32_t gmask = 0xFFFFu << (G * g);
     const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / G;
     const uint32_t ng = (gridDim.x * blockDim.x) / G;
     const uint32_t tw_log2 = __ffs(tile_w) - 1;
@@ -1585,7 +1589,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
         }
         acc_fi = acc_oob = 0;
     };
-    // Warp-uniform trips: the four groups of a warp take four consecutive
+    // Warp-uniform trips: the two groups of a warp take two consecutive
     // list entries each trip, and the warp reconverges between the phases
     // (groups left to drift apart would issue their instructions apart).
     for (uint32_t w4 = gid - g; w4 < nl; w4 += ng) {

@@ -32,9 +32,9 @@
 // What bounds it: the chain of dependent instructions of each warp (16 warps
 // per SM, 38 % of issue slots), so what counts is instructions per triangle:
 // one warp pass per triangle -- lane = row, most lanes idle on small
-// triangles -- measured 478 us on the 500 k-triangle grid at 1080p (now 89),
-// 337 us on 10 k instanced cubes (122), 2.40 ms on 64 uneven scenes (0.62)
-// and 236 us on 100 k triangles of 1..10^4 px^2 (169).
+// triangles -- measured 478 us on the 500 k-triangle grid at 1080p (now 90),
+// 337 us on 10 k instanced cubes (81), 2.40 ms on 64 uneven scenes (0.51)
+// and 236 us on 100 k triangles of 1..10^4 px^2 (163).
 // The loop's code has to stay small: with every helper inlined (8,000
 // instructions) warps waited on instruction fetch as long as they worked.
 // A tile of whole 32-column blocks goes back to HBM through the copy engine
