@@ -141,7 +141,7 @@ struct rf_ctx {
     DevBuf draws, jobs, cpos, coc, tcnt, toff, tpoly, pool, prims, mask, scan, counters, stats;
     DevBuf rowtot, rows, rprims, live, marks, items, jstats, clipq, segs, list, ent, tacc;
     DevBuf lrec, lmask;  // line pass
-    bool mask_suspect = false;  // a frame was cut short after its masks may have been marked
+    bool mask_suspect = false;  // the masks may not be zero: a new buffer, or a frame cut short
     // depth-sorted frames: sorted order, source triangles, per-draw counts,
     // sort scratch, the setup pass's draws / jobs, the raster's unit arrays
     DevBuf perm, ptri, nout, dsort, vdraws, vjobs;
@@ -708,12 +708,14 @@ rf_status tune_tile(rf_ctx *ctx, const uint64_t key[5], uint32_t &TW, TuneState 
 
 // Room for the tile masks, which are all zero between frames: a new buffer is
 // zeroed, and so is one that a frame cut short by an error may have left
-// marked.
+// marked.  New is told by its size (an allocation always raises it), not by
+// its address: the larger buffer may get the one just freed.
 rf_status ensure_mask(rf_ctx *ctx, size_t words) {
-    const void *old = ctx->mask.p;
+    const size_t cap = ctx->mask.cap;
     rf_status st = ensure(ctx, ctx->mask, words * 4);
+    if (ctx->mask.cap != cap) ctx->mask_suspect = true;  // (until it is zeroed)
     if (st) return st;
-    if (ctx->mask.p != old || ctx->mask_suspect) {
+    if (ctx->mask_suspect) {
         CK(cudaMemsetAsync(ctx->mask.p, 0, ctx->mask.cap, ctx->stream));
         ctx->mask_suspect = false;
     }

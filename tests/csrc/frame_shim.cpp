@@ -1,0 +1,210 @@
+// Host build of the frame code (rf_api.cu) against a CUDA runtime that is all
+// host memory, for CPU tests of what a frame's buffers hold between frames.
+// Copies, fills and launches happen at once.  An allocation takes the address
+// freed last, whatever its size was, and holds 0xA5 bytes; the kernels' stand-ins
+// do what the frame's contract says of the tile masks: zero when the setup
+// pass marks them, zero again once the list pass has read them.
+#include <sys/mman.h>
+
+#include "../../retrofire_gb300/csrc/rf_api.cu"
+
+namespace {
+constexpr size_t SLOT = 256u << 20;
+constexpr int NSLOTS = 256;
+char *g_base = nullptr;
+int g_next = 0;
+std::vector<int> g_free;
+int g_fail_lists = 0;        // the list pass reports an error this many times
+int g_fail_fill = 0;         // ... a fill of more than a few counters
+uint32_t g_clipped = 1;      // a sorted frame's clipped triangles per input one
+uint64_t g_dirty_words = 0;  // mask words found set when a setup pass began
+uint64_t g_setups = 0, g_same_address = 0;
+size_t g_size[NSLOTS];       // bytes allocated in each slot
+const void *g_last_mask = nullptr;
+size_t g_last_size = 0;
+
+// Words of the masks and summaries the jobs lay out.
+size_t job_words(const JobDev *jobs, uint32_t nj) {
+    size_t n = 0;
+    for (uint32_t j = 0; j < nj; ++j)
+        n = std::max<size_t>(n, jobs[j].sum_base + (size_t)jobs[j].tiles_x * jobs[j].tiles_y * jobs[j].sum_words);
+    return n;
+}
+}  // namespace
+
+extern "C" {
+cudaError_t cudaMalloc(void **p, size_t n) {
+    if (!g_base) {
+        void *m = mmap(nullptr, SLOT * NSLOTS, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+        if (m == MAP_FAILED) return cudaErrorMemoryAllocation;
+        g_base = static_cast<char *>(m);
+    }
+    int slot = g_next;
+    if (!g_free.empty()) {
+        slot = g_free.back();
+        g_free.pop_back();
+    } else if (g_next++ == NSLOTS) {
+        return cudaErrorMemoryAllocation;
+    }
+    if (n > SLOT) return cudaErrorMemoryAllocation;
+    *p = g_base + SLOT * (size_t)slot;
+    g_size[slot] = n;
+    memset(*p, 0xA5, n);
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+    if (p) g_free.push_back((int)((static_cast<char *>(p) - g_base) / (ptrdiff_t)SLOT));
+    return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return (*p = malloc(n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaMallocHost(void **p, size_t n) { return cudaHostAlloc(p, n, 0); }
+cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
+cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t) {
+    if (n > 1024 && g_fail_fill) {
+        --g_fail_fill;
+        return cudaErrorUnknown;
+    }
+    memset(d, v, n);
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr, int) { *v = 4; return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+const char *cudaGetErrorString(cudaError_t) { return "error"; }
+cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = reinterpret_cast<cudaEvent_t>(1); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorNotSupported; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = reinterpret_cast<cudaStream_t>(1); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+}
+
+namespace rfk {
+cudaError_t launch_zero(uint32_t *mask, size_t words, bool masks, StatsDev *js, uint32_t njobs, unsigned long long *tacc,
+                        uint32_t ntiles, unsigned long long *totals, unsigned long long *marks, uint32_t *, int,
+                        cudaStream_t) {
+    if (masks) memset(mask, 0, words * 4);
+    memset(js, 0, njobs * sizeof(StatsDev));
+    memset(tacc, 0, (size_t)ntiles * 8);
+    totals[0] = totals[1] = *marks = 0;
+    return cudaSuccess;
+}
+cudaError_t launch_setup(const DrawDev *, uint32_t, const JobDev *jobs, uint32_t nj, const RasterGroup *, uint32_t,
+                         uint32_t, uint32_t, const float4 *, const uint32_t *, const uint32_t *, const uint32_t *,
+                         const PolyVert *, PrimRec *, unsigned long long *, uint32_t *, unsigned long long, RasterPrim *,
+                         uint2 *, uint32_t *mask, uint32_t *, unsigned long long *, StatsDev *, uint32_t *, int,
+                         cudaStream_t, const uint32_t *, const uint32_t *) {
+    const size_t n = job_words(jobs, nj);
+    for (size_t i = 0; i < n; ++i) g_dirty_words += mask[i] != 0u;
+    ++g_setups;
+    const size_t size = g_size[(reinterpret_cast<char *>(mask) - g_base) / (ptrdiff_t)SLOT];
+    g_same_address += mask == g_last_mask && size > g_last_size;
+    g_last_mask = mask;
+    g_last_size = size;
+    memset(mask, 0xFF, n * 4);  // (all marked)
+    return cudaSuccess;
+}
+cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, uint32_t *mask, uint32_t, uint32_t, const uint2 *,
+                         unsigned long long *, const unsigned long long *, uint32_t, uint32_t *, uint32_t *, uint2 *,
+                         uint2 *, unsigned long long *, unsigned long long, cudaStream_t) {
+    if (g_fail_lists) {
+        --g_fail_lists;
+        return cudaErrorUnknown;
+    }
+    memset(mask, 0, job_words(jobs, nj) * 4);
+    return cudaSuccess;
+}
+cudaError_t launch_draw_counts(const DrawDev *d, uint32_t nd, uint32_t, const uint32_t *, const uint32_t *, uint32_t *nout,
+                               cudaStream_t) {
+    for (uint32_t i = 0; i < nd; ++i) nout[i] = d[i].ntri * g_clipped;
+    return cudaSuccess;
+}
+cudaError_t launch_vertex(const DrawDev *, uint32_t, uint32_t, float4 *, uint8_t *, uint32_t *, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_cull(DrawDev *, uint32_t, StatsDev *, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_clip(const DrawDev *, uint32_t, uint32_t, const float4 *, const uint8_t *, uint32_t *, uint32_t *,
+                        uint32_t *, PolyVert *, uint32_t, uint32_t *, int, cudaStream_t, uint32_t *, bool) { return cudaSuccess; }
+cudaError_t launch_fill(uint32_t *, float *, size_t, uint32_t, float, uint32_t, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_scan(const uint32_t *, uint32_t *, uint32_t, uint32_t *, uint32_t *, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_dsort(const DrawDev *, uint32_t, const JobDev *, uint32_t, uint32_t, const float4 *, const uint32_t *,
+                         const uint32_t *, const uint32_t *, const PolyVert *, const uint32_t *, uint32_t *, uint32_t *,
+                         void *, uint32_t *, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_lines(const DrawDev *, const JobDev *, uint32_t, const float4 *, const uint8_t *, LineRec *, uint32_t *,
+                         uint32_t, uint32_t *, StatsDev *, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_stamp(unsigned long long *, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_raster(uint32_t, const RasterGroup *, uint32_t, const JobDev *, uint32_t, const DrawDev *,
+                          const PrimRec *, const RasterPrim *, const uint32_t *, const uint2 *, const uint32_t *,
+                          const uint2 *, const uint2 *, uint32_t, const uint32_t *, uint32_t *, StatsDev *, uint32_t, int,
+                          const cudaStream_t *, uint32_t) { return cudaSuccess; }
+cudaError_t launch_mesh_bbox(const float *, uint32_t, uint32_t, float *, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_stats_fold(const StatsDev *, uint32_t, StatsDev *, cudaStream_t) { return cudaSuccess; }
+uint32_t dsort_scan_items(uint32_t) { return 0; }
+size_t scan_scratch_words(uint32_t n) { return n / 4096u + 2u; }
+size_t dsort_scratch_bytes(uint32_t n) { return (size_t)n * 32u + 4096u; }
+}  // namespace rfk
+
+namespace {
+// One frame of one mesh of ntri flat triangles on a w x h target.
+rf_status frame(rf_ctx *ctx, uint32_t ntri, uint32_t w, uint32_t h, int32_t sort) {
+    std::vector<float> v(9, 0.5f);
+    std::vector<uint32_t> idx(3 * (size_t)ntri);
+    for (size_t i = 0; i < idx.size(); ++i) idx[i] = (uint32_t)(i % 3);
+    rf_mesh m = 0;
+    rf_target t = 0;
+    rf_status st = rf_mesh_upload(ctx, v.data(), 3, 3, 0, idx.data(), ntri, &m);
+    if (!st) st = rf_target_create(ctx, w, h, RF_ARGB8888, 1, &t);
+    if (!st) {
+        rf_draw d{};
+        d.mesh = m;
+        d.shader = RF_SHADER_FLAT;
+        const float vp[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
+        const rf_context_flags fl{RF_DEPTH_LESS, 1, 1, RF_CULL_BACK, sort};
+        st = rf_render_draws(ctx, &d, 1, vp, t, &fl, nullptr);
+    }
+    if (t) rf_target_destroy(ctx, t);
+    if (m) rf_mesh_destroy(ctx, m);
+    return st;
+}
+}  // namespace
+
+extern "C" {
+// Frames of the given sizes (ntri, w, h, depth_sort, clipped pieces per
+// triangle, 1 when the list pass is to fail, 2 when the zeroing of its masks
+// is), one after the other on one context.  out: mask words found set at the setup passes, setup passes,
+// those whose masks had grown in place; returns the frames that ended in
+// another status than expected.
+uint32_t shim_frames(const uint32_t *f, uint32_t n, uint64_t out[3]) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return 0xFFFFFFFFu;
+    rf_ctx_set_tiling(ctx, 32, 4);
+    g_dirty_words = g_setups = g_same_address = 0;
+    g_last_mask = nullptr;
+    g_last_size = 0;
+    uint32_t bad = 0;
+    for (uint32_t i = 0; i < n; ++i, f += 6) {
+        g_clipped = f[4];
+        g_fail_lists = f[5] == 1u;
+        g_fail_fill = f[5] == 2u;
+        bad += (frame(ctx, f[0], f[1], f[2], (int32_t)f[3]) == RF_OK) != (f[5] == 0u);
+    }
+    rf_ctx_destroy(ctx);
+    out[0] = g_dirty_words;
+    out[1] = g_setups;
+    out[2] = g_same_address;
+    return bad;
+}
+}

@@ -1,0 +1,70 @@
+"""CPU tests of the frame code (retrofire_gb300/csrc/rf_api.cu) against a CUDA
+runtime of host memory (tests/csrc/frame_shim.cpp): what its buffers hold from
+frame to frame."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    inc = os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include")
+    if not os.path.exists(os.path.join(inc, "cuda_runtime.h")):
+        pytest.skip("no CUDA headers")
+    out = str(tmp_path_factory.mktemp("shim") / "libframe.so")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic",
+                           "-I" + inc, os.path.join(HERE, "csrc", "frame_shim.cpp"), "-o", out])
+    L = C.CDLL(out)
+    L.shim_frames.argtypes = [C.c_void_p, C.c_uint32, C.POINTER(C.c_uint64)]
+    L.shim_frames.restype = C.c_uint32
+    return L
+
+
+def frames(L, rows):
+    """(mask words found set, setup passes, masks grown in place) of a run of
+    (ntri, w, h, depth_sort, clipped, fails) frames."""
+    a = np.ascontiguousarray(rows, np.uint32)
+    out = (C.c_uint64 * 3)()
+    assert L.shim_frames(a.ctypes.data, len(a), out) == 0
+    return tuple(out)
+
+
+@pytest.mark.parametrize("sort", [0, 1])
+def test_grown_masks_start_zero(shim, sort):
+    """Masks that grow, step by step, onto the address they had: every frame
+    finds them zero, those after the largest too."""
+    rows = [(n, w, h, sort, 1, 0) for n, w, h in
+            ((40, 64, 64), (700, 320, 240), (40, 64, 64), (9000, 640, 480), (70000, 640, 480), (40, 64, 64))]
+    dirty, setups, grown = frames(shim, rows)
+    assert setups == len(rows)
+    assert grown >= 2  # (the case this is about)
+    assert dirty == 0
+
+
+def test_masks_grown_by_clipped_pieces(shim):
+    """A depth-sorted frame's masks grow a second time, by its clipped
+    triangles, in the middle of the frame."""
+    dirty, setups, grown = frames(shim, [(3000, 320, 240, 1, 1, 0), (3000, 320, 240, 1, 7, 0), (3000, 320, 240, 0, 1, 0)])
+    assert (dirty, setups) == (0, 3) and grown >= 1
+
+
+@pytest.mark.parametrize("sort", [0, 1])
+def test_frame_cut_short(shim, sort):
+    """A frame that fails between marking and reading the masks: the next
+    one finds them zero, larger or smaller."""
+    for after in (40, 700, 9000):
+        dirty, setups, _ = frames(shim, [(700, 320, 240, sort, 1, 0), (700, 320, 240, sort, 1, 1), (after, 320, 240, 0, 1, 0)])
+        assert (dirty, setups) == (0, 3)
+
+
+def test_new_masks_not_zeroed(shim):
+    """A frame that fails between allocating larger masks and zeroing them:
+    the next one zeroes them, though they are large enough by then."""
+    dirty, setups, _ = frames(shim, [(40, 64, 64, 0, 1, 0), (9000, 640, 480, 0, 1, 2), (9000, 640, 480, 0, 1, 0)])
+    assert (dirty, setups) == (0, 2)
