@@ -1334,6 +1334,10 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
                     __syncwarp();
                     T.row = lane;
                 }
+                // Where every row hides every triangle no round has waited for
+                // the table's own copies; the next table, or the tile's
+                // write-back, takes their place.
+                wait_staged_but<0>();
             } else {
                 // Packed: 32 scanlines a pass, in submission order, one a
                 // lane.  Spans of one row that meet are drawn in that order:

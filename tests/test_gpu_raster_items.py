@@ -198,3 +198,41 @@ def test_few_tall_triangles(n):
     for tile in ((8, 4), (32, 4)):
         g, o = gpu_render([d], vp, w, h, tile=tile), oracle_render([d], vp, w, h)
         assert_parity(g, o, what="%d triangles, tile %r" % (n, tile))
+
+
+@pytest.mark.parametrize("tw", [8, 16, 32, 64])
+@pytest.mark.parametrize("kind", [rf.GOURAUD, rf.TEX_GOURAUD, rf.FLAT])
+def test_tables_that_no_row_takes(tw, kind):
+    """Whole tables of 32 triangles (and a last, shorter one) that lie in rows
+    already covered by nearer ones, in tiles with other rows still clear: no
+    round is drawn for them, between tables that are drawn and at the end of a
+    tile."""
+    w, h, rng = 256, 96, np.random.default_rng(tw)
+
+    def rects(n, y0, y1, wv):  # n triangles across the target, rows y0 .. y1 of every 32 covered
+        out = []
+        for i in range(n):
+            b = 32 * (i % 3)
+            out.append([[-300, b + y0], [900, b + y0], [-300, b + 2 * y1 - y0]] if i % 2 else
+                       [[900, b + y1], [-300, b + y1], [900, b + 2 * y0 - y1]])
+        return np.array(out, np.float64), np.full((n, 3), wv)
+
+    parts = [rects(96, 2, 20, 1.0), rects(32, 21, 31, 1.5)]
+    for m in (31, 32, 33, 64, 77):  # farther away, inside the covered rows
+        n = 3 * m
+        c = np.stack([rng.uniform(0, w, n), 32 * (np.arange(n) % 3) + 11.0], 1)
+        px = c[:, None, :] + np.stack([rng.uniform(-90, 90, (n, 3)), np.tile([-6.5, 6.0, 1.0], (n, 1))], -1)
+        parts.append((px, rng.uniform(2.0, 3.0, (n, 3))))
+        parts.append(rects(3, 24, 30, 1.4 - 0.01 * m / 31))
+    parts.append(parts[4])
+    px, wv = (np.concatenate(x) for x in zip(*parts))
+    n = len(px)
+    clip = np.stack([(px[..., 0] / (w / 2.0) - 1.0) * wv, (px[..., 1] / (h / 2.0) - 1.0) * wv, 0.0 * wv, wv], -1)
+    v = np.concatenate([clip, rng.uniform(0, 1, (n, 3, NATTR[kind]))], -1).reshape(3 * n, -1).astype(np.float32)
+    tex = scenes.noise_texture(64, 3) if kind == rf.TEX_GOURAUD else None
+    d = DrawSpec(v, np.arange(3 * n, dtype=np.uint32).reshape(n, 3), kind, pos_dim=4, flat_rgba=0xFF336699, tex=tex)
+    vp, ctx = mat.viewport(0, 0, w, h), rf.Context(face_cull=rf.CULL_NONE)
+    o = oracle_render([d], vp, w, h, ctx=ctx)
+    assert o[2]["frags_o"] > 0
+    for _ in range(3):
+        assert_parity(gpu_render([d], vp, w, h, ctx=ctx, tile=(tw, 4)), o, what="width %d" % tw)
