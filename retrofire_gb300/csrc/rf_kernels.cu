@@ -95,7 +95,7 @@ __global__ void k_zero(uint4 *__restrict__ mask, size_t n16, const uint32_t *__r
 // K1: vertex shader (mvp.apply, mat.rs:952-973, or clip-space passthrough)
 // and outcode (clip.rs:240-242, 303-309).
 // ---------------------------------------------------------------------------
-__global__ void k_vertex(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nv_total,
+__global__ void k_vertex(const DrawDev *draws, uint32_t nd, uint32_t nv_total,
                          float4 *__restrict__ cpos, uint8_t *__restrict__ coc, uint32_t *__restrict__ counters) {
     grid_begin();
     if (counters && blockIdx.x == 0 && threadIdx.x == 0) counters[RF_CNT_MASKDIRTY] = 0;  // (k_zero is done)
@@ -250,7 +250,7 @@ __device__ int clip_plane(int plane, const CV *in, int nin, CV *out, uint32_t na
 // few that cross a plane go to a queue for k_clip_poly, so the clipping
 // loop runs on full warps.
 __global__ void k_clip(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nt_total,
-                       const uint8_t *__restrict__ coc, uint32_t *__restrict__ tcnt,
+                       const uint8_t *coc, uint32_t *__restrict__ tcnt,
                        uint32_t *__restrict__ tpoly, uint32_t *__restrict__ queue,
                        uint32_t *__restrict__ counters, uint32_t *__restrict__ toff,
                        uint32_t *__restrict__ prim_total) {
@@ -341,7 +341,7 @@ __global__ void k_clip(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t 
 // per edge in order, the kept start vertex, then the intersection.
 __device__ __forceinline__ void clip_groups(const DrawDev *__restrict__ draws, const float4 *__restrict__ cpos,
                                             const uint8_t *__restrict__ coc, uint32_t *__restrict__ tcnt,
-                                            uint32_t *__restrict__ tpoly, const uint32_t *__restrict__ queue,
+                                            uint32_t *__restrict__ tpoly, const uint32_t *queue,
                                             PolyVert *__restrict__ pool, uint32_t pool_cap,
                                             uint32_t *__restrict__ counters, uint32_t nq) {
     constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -472,7 +472,7 @@ __device__ __forceinline__ void clip_groups(const DrawDev *__restrict__ draws, c
 // cost more issue slots than it saves latency.
 __device__ __forceinline__ void clip_threads(const DrawDev *__restrict__ draws, const float4 *__restrict__ cpos,
                                              const uint8_t *__restrict__ coc, uint32_t *__restrict__ tcnt,
-                                             uint32_t *__restrict__ tpoly, const uint32_t *__restrict__ queue,
+                                             uint32_t *__restrict__ tpoly, const uint32_t *queue,
                                              PolyVert *__restrict__ pool, uint32_t pool_cap,
                                              uint32_t *__restrict__ counters, uint32_t nq) {
     for (uint32_t qi = blockIdx.x * blockDim.x + threadIdx.x; qi < nq; qi += gridDim.x * blockDim.x) {
@@ -536,7 +536,7 @@ __device__ __forceinline__ void clip_threads(const DrawDev *__restrict__ draws, 
 __global__ void __launch_bounds__(256)
 k_clip_poly(const DrawDev *__restrict__ draws, const float4 *__restrict__ cpos,
             const uint8_t *__restrict__ coc, uint32_t *__restrict__ tcnt,
-            uint32_t *__restrict__ tpoly, const uint32_t *__restrict__ queue,
+            uint32_t *__restrict__ tpoly, const uint32_t *queue,
             PolyVert *__restrict__ pool, uint32_t pool_cap, uint32_t *__restrict__ counters) {
     grid_begin();
     const uint32_t nq = counters[RF_CNT_CLIPQ];
@@ -553,7 +553,7 @@ k_clip_poly(const DrawDev *__restrict__ draws, const float4 *__restrict__ cpos,
 static_assert(SCAN_THREADS * SCAN_ITEMS == RF_SCAN_BLOCK_ITEMS, "scan block size");
 // Exclusive scan of each block's SCAN_THREADS * SCAN_ITEMS values; the block
 // totals go to block_sums, and with a single block the total to *total.
-__global__ void k_scan_blocks(const uint32_t *__restrict__ in, uint32_t *__restrict__ out,
+__global__ void k_scan_blocks(const uint32_t *in, uint32_t *__restrict__ out,
                               uint32_t n, uint32_t *__restrict__ block_sums,
                               uint32_t *__restrict__ total) {
     grid_begin();
@@ -634,7 +634,7 @@ __global__ void k_scan_sums(uint32_t *__restrict__ sums, uint32_t nb, uint32_t *
     if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void k_scan_add(uint32_t *__restrict__ out, uint32_t n, const uint32_t *__restrict__ sums) {
+__global__ void k_scan_add(uint32_t *__restrict__ out, uint32_t n, const uint32_t *sums) {
     grid_begin();
     const uint32_t base = blockIdx.x * (SCAN_THREADS * SCAN_ITEMS) + threadIdx.x * SCAN_ITEMS;
     const uint32_t add = sums[blockIdx.x];
@@ -838,13 +838,13 @@ static_assert(RF_SETUP_WORDS % 2 == 1 && RF_SETUP_WORDS * 4 >= sizeof(RasterPrim
 template <int NCT>
 __global__ void __launch_bounds__(RF_SETUP_THREADS)
 k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict__ jobs, uint32_t nj,
-        uint32_t block0, uint32_t nblocks, uint32_t tile_w, const float4 *__restrict__ cpos, const uint32_t *__restrict__ tcnt,
-        const uint32_t *__restrict__ toff, const uint32_t *__restrict__ tpoly, const PolyVert *__restrict__ pool,
+        uint32_t block0, uint32_t nblocks, uint32_t tile_w, const float4 *__restrict__ cpos, const uint32_t *tcnt,
+        const uint32_t *toff, const uint32_t *tpoly, const PolyVert *pool,
         PrimRec *__restrict__ prims, unsigned long long *__restrict__ rows_total, uint32_t *__restrict__ rows,
         unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint2 *__restrict__ ent,
         uint32_t *__restrict__ mask, uint32_t *__restrict__ live, uint32_t *__restrict__ live_n, uint32_t *__restrict__ live_mid,
         uint32_t *__restrict__ live_mid_n, unsigned long long *__restrict__ marks, StatsDev *__restrict__ stats,
-        const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ptri) {
+        const uint32_t *perm, const uint32_t *ptri) {
     grid_begin();
     constexpr uint32_t FULL = 0xFFFFFFFFu, NONE = 0xFFFFFFFFu;
     constexpr int NCL = NCT ? NCT : RF_NC;
@@ -1215,10 +1215,10 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
 template <int NCT>
 __global__ void __launch_bounds__(256, 4)
 k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
-      PrimRec *__restrict__ prims, const uint32_t *__restrict__ live, uint32_t tile_w,
+      PrimRec *prims, const uint32_t *live, uint32_t tile_w,
       uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims,
       uint2 *__restrict__ ent, uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
-      unsigned long long *__restrict__ marks, const uint32_t *__restrict__ live_n) {
+      unsigned long long *__restrict__ marks, const uint32_t *live_n) {
     grid_begin();
     const uint32_t lane = threadIdx.x & 31, wib = (threadIdx.x >> 5) & 7;
     const uint32_t tw_log2 = __ffs(tile_w) - 1;  // tile widths are powers of two
@@ -1267,8 +1267,8 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
     uint32_t cur = 0;
     // Live-list entries: this warp's current and next triangle (the one
     // after that is loaded one iteration ahead).
-    uint32_t pc = wid < nl ? __ldg(live + wid) : 0u;
-    uint32_t pn = wid + nw < nl ? __ldg(live + wid + nw) : 0u;
+    uint32_t pc = wid < nl ? live[wid] : 0u;
+    uint32_t pn = wid + nw < nl ? live[wid + nw] : 0u;
     fetch(sbuf[wib][0], pc, wid < nl);
     RasterPrim *R = &srp[wib];
     float (*T)[RF_TILE_H + 4] = stab[wib];
@@ -1311,7 +1311,7 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
     };
     uint32_t mine = 0xFFFFFFFFu;
     for (uint32_t i = wid; i < nl; i += nw) {
-        const uint32_t pnn = i + 2 * nw < nl ? __ldg(live + i + 2 * nw) : 0u;
+        const uint32_t pnn = i + 2 * nw < nl ? live[i + 2 * nw] : 0u;
         __syncwarp();  // the other slot's previous triangle is done
         fetch(sbuf[wib][cur ^ 1u], pn, i + nw < nl);
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
@@ -1550,11 +1550,11 @@ k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
 // G: lanes per triangle (those of at most G rows).
 template <int NCT, uint32_t G>
 __global__ void __launch_bounds__(256, 4)
-k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
-            const uint32_t *__restrict__ live_small, uint32_t *__restrict__ live, uint32_t tile_w,
+k_bin_small(const JobDev *__restrict__ jobs, PrimRec *prims,
+            const uint32_t *live_small, uint32_t *__restrict__ live, uint32_t tile_w,
             uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint2 *__restrict__ ent,
             uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
-            unsigned long long *__restrict__ marks, const uint32_t *__restrict__ small_n,
+            unsigned long long *__restrict__ marks, const uint32_t *small_n,
             uint32_t *__restrict__ live_n) {
     grid_begin();
     static_assert(G == 16 && sizeof(RasterPrim) / 16 <= G, "a group stores a RasterPrim in one pass");
@@ -1597,7 +1597,7 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *__restrict__ prims,
         const bool act = i < nl;
         uint32_t e = 0;  // the output triangle
         if (act) {
-            e = __ldg(live_small + i);
+            e = live_small[i];
             const uint4 *src = reinterpret_cast<const uint4 *>(prims + e);
             for (uint32_t q = gl; q < RF_PRIM_CORE_BYTES / 16; q += G) sbuf[wib][g][q] = src[q];
         }
@@ -1804,8 +1804,8 @@ __device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t k) {
 
 __global__ void __launch_bounds__(RF_LIST_WARPS * 32, 12)
 k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict__ mask,
-             uint32_t ntiles, uint32_t npieces, const uint2 *__restrict__ ent,
-             unsigned long long *__restrict__ tacc, const unsigned long long *__restrict__ marks, uint32_t slots, uint32_t *__restrict__ items,
+             uint32_t ntiles, uint32_t npieces, const uint2 *ent,
+             unsigned long long *__restrict__ tacc, const unsigned long long *marks, uint32_t slots, uint32_t *__restrict__ items,
              uint32_t *__restrict__ extras, uint2 *__restrict__ segs, uint2 *__restrict__ list,
              unsigned long long *__restrict__ cursor, unsigned long long cap, uint32_t *__restrict__ dirty) {
     grid_begin();
@@ -1882,7 +1882,7 @@ k_tile_lists(const JobDev *__restrict__ jobs, uint32_t nj, uint32_t *__restrict_
             for (uint32_t q = lane; q - lane < total; q += 32u) {
                 const uint32_t M = lane_of(incl, q), mM = __shfl_sync(FULL, m, M);
                 const uint32_t ex = __shfl_sync(FULL, incl - __popc(m), M), wM = __shfl_sync(FULL, wi, M);
-                if (q < total) list[off + q] = __ldg(ent + J.tri_base + wM * 32u + nth_bit(mM, q - ex + 1u));
+                if (q < total) list[off + q] = ent[J.tri_base + wM * 32u + nth_bit(mM, q - ex + 1u)];
             }
             off += total;
             if (!again) break;
@@ -2091,7 +2091,7 @@ cudaError_t launch_cull(DrawDev *draws, uint32_t nd, StatsDev *stats, int nsm, c
 
 // Per-job stats of a batch folded into the context's running total.  One
 // block; stream order makes the plain read-modify-write of *total safe.
-__global__ void __launch_bounds__(256) k_stats_fold(const StatsDev *__restrict__ js, uint32_t n,
+__global__ void __launch_bounds__(256) k_stats_fold(const StatsDev *js, uint32_t n,
                                                     StatsDev *__restrict__ total) {
     grid_begin();
     constexpr int NF = (int)(sizeof(StatsDev) / sizeof(unsigned long long));

@@ -73,7 +73,12 @@ namespace rfk {
 // (programmatic dependent launch): its blocks come up and wait in
 // grid_begin() (rf_device.cuh) until that kernel has finished, so the launch
 // latency and the wait for the last block do not add up.  Every kernel
-// launched here calls grid_begin() first.
+// launched here calls grid_begin() first.  It is resident while the kernel
+// before it still writes, so it reads what that one writes by plain loads: not
+// through __ldg, nor from a parameter that is const and __restrict__ (or only
+// read, and __restrict__), whose memory must not change while the kernel lives.
+// What earlier kernels wrote is complete by then: each lets its successor come
+// up only after its own wait.
 template <class... P, class... A>
 cudaError_t launch_next(void (*k)(P...), uint32_t blocks, uint32_t threads, size_t smem, cudaStream_t s, A... a) {
     cudaLaunchAttribute at{};

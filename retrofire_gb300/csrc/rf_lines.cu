@@ -76,8 +76,8 @@ __device__ uint32_t lshade(const DrawDev &dd, const float *v, int32_t fmt) {
 }  // namespace
 
 __global__ void k_line_setup(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
-                             uint32_t nl, const float4 *__restrict__ cpos,
-                             const uint8_t *__restrict__ coc, LineRec *__restrict__ recs,
+                             uint32_t nl, const float4 *cpos,
+                             const uint8_t *coc, LineRec *__restrict__ recs,
                              uint32_t *__restrict__ mask, StatsDev *__restrict__ stats) {
     rfd::grid_begin();
     const DrawDev &d = draws[0];
@@ -221,8 +221,8 @@ __device__ __forceinline__ float line_step(float s, float d, uint32_t k) {
 // a tile, RF_LINE_ROWS rows each, 31 (each reads all of the tile's mask, which
 // is in L2, but steps only the lines that can reach its rows).
 __global__ void __launch_bounds__(RF_LINE_WARPS * 32)
-k_line_raster(const JobDev *__restrict__ jobs, const LineRec *__restrict__ recs,
-              const uint32_t *__restrict__ mask, uint32_t ntiles, uint32_t *__restrict__ queue,
+k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
+              const uint32_t *mask, uint32_t ntiles, uint32_t *__restrict__ queue,
               StatsDev *__restrict__ stats) {
     rfd::grid_begin();
     constexpr uint32_t FULL = 0xFFFFFFFFu;

@@ -707,7 +707,7 @@ static __device__ __noinline__ uint2 mask_batch(PrimIter *it, const uint2 *ent, 
     uint32_t mine;
     const uint32_t k = it->gather_tris(mine);
     *n = k;
-    return lane < k ? __ldg(ent + mine) : make_uint2(0u, 0u);
+    return lane < k ? ent[mine] : make_uint2(0u, 0u);
 }
 static __device__ __noinline__ void mask_begin(PrimIter *it, const uint32_t *mask, const JobDev *J, uint32_t lt,
                                                uint32_t piece, uint32_t lane) {
@@ -1081,7 +1081,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
             }
         }
         n_ent = min(ent_left, 32u);
-        ent = lane < n_ent ? __ldg(A.list + ent_off + lane) : make_uint2(0u, 0u);
+        ent = lane < n_ent ? A.list[ent_off + lane] : make_uint2(0u, 0u);
         ent_off += n_ent;
         ent_left -= n_ent;
     };

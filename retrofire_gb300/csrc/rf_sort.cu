@@ -91,7 +91,7 @@ __device__ __forceinline__ uint32_t digit_of(unsigned long long k, uint32_t shif
 }
 
 // Per block, how many of its items have each digit: hist[digit * nb + block].
-__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned long long *__restrict__ keys, uint32_t n,
+__global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned long long *keys, uint32_t n,
                                                         uint32_t shift, uint32_t *__restrict__ hist) {
     rfd::grid_begin();
     __shared__ uint32_t h[RS_DIGITS];
@@ -112,9 +112,9 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const unsigned long long
 // Short: latencies of one block.  20,000 triangles, all passes: 99 us with a
 // count, a scan and eight chunks a block each, 42 us with direct passes.
 template <bool DIRECT>
-__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned long long *__restrict__ kin,
-                                                           const uint32_t *__restrict__ vin, uint32_t n,
-                                                           uint32_t shift, const uint32_t *__restrict__ cnt,
+__global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned long long *kin,
+                                                           const uint32_t *vin, uint32_t n,
+                                                           uint32_t shift, const uint32_t *cnt,
                                                            uint32_t *__restrict__ next_cnt, uint32_t chunk_log2,
                                                            unsigned long long *__restrict__ kout,
                                                            uint32_t *__restrict__ vout) {
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_scatter(const unsigned long l
 }
 
 __global__ void k_draw_counts(const DrawDev *__restrict__ draws, uint32_t nd, uint32_t nt,
-                              const uint32_t *__restrict__ toff, const uint32_t *__restrict__ counters,
+                              const uint32_t *toff, const uint32_t *counters,
                               uint32_t *__restrict__ nout) {
     rfd::grid_begin();
     const uint32_t total = counters[RF_CNT_PRIMS];
