@@ -1940,9 +1940,7 @@ cudaError_t launch_zero(uint32_t *mask, size_t mask_words, bool masks, StatsDev 
                         unsigned long long *tacc, uint32_t ntiles, unsigned long long *totals,
                         unsigned long long *marks, uint32_t *counters, int nsm, cudaStream_t s) {
     const size_t n16 = mask_words / 4;
-    // (a grid for the masks only when they are certain to be cleared)
-    const size_t work = std::max<size_t>(masks ? n16 : 0, ntiles);
-    const uint32_t blocks = (uint32_t)std::min<size_t>((work + 255) / 256 + 1, (size_t)nsm * 8);
+    const uint32_t blocks = zero_blocks(n16, masks, ntiles, nsm);
     k_zero<<<blocks, 256, 0, s>>>(reinterpret_cast<uint4 *>(mask), n16, masks ? nullptr : counters + RF_CNT_MASKDIRTY,
                                   reinterpret_cast<unsigned long long *>(js),
                                   njobs * (uint32_t)(sizeof(StatsDev) / 8), tacc, ntiles, totals, marks, counters);

@@ -105,6 +105,18 @@ cudaError_t launch_next(void (*k)(P...), uint32_t blocks, uint32_t threads, size
 // and -- when the last frame left them dirty, or with `masks` -- the whole mask
 // buffer (mask_words, a multiple of 4).  launch_vertex clears the dirty mark
 // (counters: nullptr for none).
+// Blocks of 256: for the tiles' counts, and for the masks' n16 16-byte words, up to
+// eight blocks a multiprocessor where they are certain to be cleared and two
+// where only the device knows (a block with nothing to clear ends after one
+// load).
+inline uint32_t zero_blocks(size_t n16, bool masks, uint32_t ntiles, int nsm) {
+    auto upto = [&](size_t work, int per_sm) {
+        const size_t b = (work + 255) / 256 + 1, most = (size_t)nsm * per_sm;
+        return b < most ? b : most;
+    };
+    const size_t a = upto(ntiles, 8), b = upto(n16, masks ? 8 : 2);
+    return (uint32_t)(a > b ? a : b);
+}
 cudaError_t launch_zero(uint32_t *mask, size_t mask_words, bool masks, StatsDev *js, uint32_t njobs,
                         unsigned long long *tacc, uint32_t ntiles, unsigned long long *totals,
                         unsigned long long *marks, uint32_t *counters, int nsm, cudaStream_t s);

@@ -207,4 +207,7 @@ uint32_t shim_frames(const uint32_t *f, uint32_t n, uint64_t out[3]) {
     out[2] = g_same_address;
     return bad;
 }
+uint32_t shim_zero_blocks(uint64_t n16, int masks, uint32_t ntiles, int nsm) {
+    return rfk::zero_blocks(n16, masks != 0, ntiles, nsm);
+}
 }

@@ -23,6 +23,8 @@ def shim(tmp_path_factory):
     L = C.CDLL(out)
     L.shim_frames.argtypes = [C.c_void_p, C.c_uint32, C.POINTER(C.c_uint64)]
     L.shim_frames.restype = C.c_uint32
+    L.shim_zero_blocks.argtypes = [C.c_uint64, C.c_int, C.c_uint32, C.c_int]
+    L.shim_zero_blocks.restype = C.c_uint32
     return L
 
 
@@ -68,3 +70,15 @@ def test_new_masks_not_zeroed(shim):
     the next one zeroes them, though they are large enough by then."""
     dirty, setups, _ = frames(shim, [(40, 64, 64, 0, 1, 0), (9000, 640, 480, 0, 1, 2), (9000, 640, 480, 0, 1, 0)])
     assert (dirty, setups) == (0, 2)
+
+
+@pytest.mark.parametrize("mask_mb", [0, 1, 16, 300, 4000])
+@pytest.mark.parametrize("ntiles", [1, 60, 4080, 1 << 20])
+def test_zeroing_grid_covers_masks_left_marked(shim, mask_mb, ntiles):
+    """A frame's zeroing launch after one that left the masks marked: the whole
+    chip clears large masks, whatever target the frame is for; small masks and
+    few tiles take few blocks."""
+    nsm, n16 = 152, mask_mb << 16
+    b = shim.shim_zero_blocks(n16, 0, ntiles, nsm)
+    assert b >= min(n16 // 256, nsm) and b * 256 >= min(ntiles, nsm * 8 * 256)
+    assert b <= max(2 * nsm, min(ntiles // 256 + 2, 8 * nsm)) and b <= (n16 + ntiles) // 256 + 2
