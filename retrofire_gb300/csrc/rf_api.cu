@@ -81,7 +81,10 @@ struct DevBuf {
 // (the runtime copies them out before the call returns); from RF_UPLOAD_PIN
 // bytes on through a ring of page-locked buffers, each free again when the
 // copy that reads it is done -- from ordinary memory such a copy would hold
-// the host until the stream reaches it.
+// the host until the stream reaches it, which is what happens where no more
+// memory can be page-locked.  The ring grows with the draws looked at, not with
+// the count a call claims, and is the context's until it is destroyed: three
+// times the largest frame's descriptors and a quarter.
 constexpr size_t RF_UPLOAD_PIN = 16384;
 constexpr uint32_t RF_UPLOAD_RING = 3;
 struct UploadBuf {
@@ -172,9 +175,10 @@ struct rf_ctx {
     // upload buffer), the jobs in hjobs, which follow the draws there.
     UploadBuf uploads[RF_UPLOAD_RING];
     uint32_t upload_at = 0;
-    std::vector<char> small_upload;
-    UploadBuf *upload = nullptr;  // the ring's buffer in use (nullptr: small_upload)
+    std::vector<char> plain_upload;
+    UploadBuf *upload = nullptr;  // the ring's buffer in use (nullptr: plain_upload)
     DrawDev *hdraws = nullptr;
+    size_t hroom = 0;  // draws it has room for
     size_t ndraws = 0;
     bool any_cull = false;  // a draw asks for object culling
     std::vector<JobDev> hjobs;
@@ -288,28 +292,55 @@ rf_status sync_all(rf_ctx *ctx) {
 // Byte offset of the jobs behind n draws.
 size_t jobs_at(size_t n) { return (n * sizeof(DrawDev) + 255) & ~(size_t)255; }
 
-// Room for the descriptors of up to ndraws draws and njobs jobs.
+// The buffer for the descriptors of up to ndraws draws and njobs jobs: one of
+// the ring as it is (upload_more makes room in it), or ordinary memory for a few.
 rf_status upload_begin(rf_ctx *ctx, size_t ndraws, size_t njobs) {
     const size_t bytes = jobs_at(ndraws) + njobs * sizeof(JobDev);
     if (bytes < RF_UPLOAD_PIN) {
-        if (ctx->small_upload.size() < RF_UPLOAD_PIN) ctx->small_upload.resize(RF_UPLOAD_PIN);
+        if (ctx->plain_upload.size() < RF_UPLOAD_PIN) ctx->plain_upload.resize(RF_UPLOAD_PIN);
         ctx->upload = nullptr;
-        ctx->hdraws = reinterpret_cast<DrawDev *>(ctx->small_upload.data());
+        ctx->hdraws = reinterpret_cast<DrawDev *>(ctx->plain_upload.data());
+        ctx->hroom = ndraws;
         return RF_OK;
     }
     UploadBuf &u = ctx->uploads[ctx->upload_at++ % RF_UPLOAD_RING];
     if (u.pending) CK(cudaEventSynchronize(u.copied));
     u.pending = false;
-    if (u.cap < bytes) {
-        if (u.p) CK(cudaFreeHost(u.p));
-        u.p = nullptr;
-        u.cap = 0;
-        CK(cudaMallocHost(&u.p, bytes + bytes / 4));
-        u.cap = bytes + bytes / 4;
-        if (!u.copied) CK(cudaEventCreateWithFlags(&u.copied, cudaEventDisableTiming));
-    }
+    if (!u.copied) CK(cudaEventCreateWithFlags(&u.copied, cudaEventDisableTiming));
     ctx->upload = &u;
     ctx->hdraws = reinterpret_cast<DrawDev *>(u.p);
+    const size_t rest = njobs * sizeof(JobDev) + 255;
+    ctx->hroom = u.cap > rest ? (u.cap - rest) / sizeof(DrawDev) : 0;
+    return RF_OK;
+}
+
+// Room for more than the n draws built so far, of ndraws the call claims to
+// have: sixteen times as many at once (a first frame of 100,000 draws
+// allocates three times), since any of the rest may still be refused.
+rf_status upload_more(rf_ctx *ctx, size_t n, size_t ndraws, size_t njobs) {
+    const size_t want = std::min(ndraws, std::max<size_t>(256, n * 16));
+    const size_t bytes = jobs_at(want) + njobs * sizeof(JobDev), cap = bytes + bytes / 4;
+    char *p = nullptr;
+    if (ctx->upload && cudaMallocHost(&p, cap) == cudaSuccess) {
+        UploadBuf &u = *ctx->upload;
+        if (n) memcpy(p, u.p, n * sizeof(DrawDev));
+        if (u.p) cudaFreeHost(u.p);
+        u.p = p;
+        u.cap = cap;
+    } else {
+        cudaGetLastError();  // (no more page-locked memory: ordinary memory from here on)
+        try {
+            std::vector<char> v(cap);
+            if (n) memcpy(v.data(), ctx->hdraws, n * sizeof(DrawDev));
+            ctx->plain_upload.swap(v);
+        } catch (const std::bad_alloc &) {
+            return RF_ERR_OOM;
+        }
+        p = ctx->plain_upload.data();
+        ctx->upload = nullptr;
+    }
+    ctx->hdraws = reinterpret_cast<DrawDev *>(p);
+    ctx->hroom = want;
     return RF_OK;
 }
 
@@ -528,7 +559,6 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
     for (uint32_t k = 0; k < nin; ++k) most += in[k].draws ? in[k].ndraws : 0u;
     rf_status us = upload_begin(ctx, most, nin);
     if (us) return us;
-    DrawDev *hd = ctx->hdraws;
     size_t nd = 0;
     ctx->any_cull = false;
     // The objects of the draw before (instances share their mesh and
@@ -563,7 +593,8 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
                 ctx->async_meshes.push_back(&m);
             if (dr.shader < RF_SHADER_FLAT || dr.shader > RF_SHADER_GOURAUD_SRGB) return RF_ERR_BAD_ARG;
             if (m.nattr != nattr_for(dr.shader)) return RF_ERR_BAD_ARG;
-            DrawDev &d = hd[nd];
+            if (nd == ctx->hroom && (us = upload_more(ctx, nd, most, nin))) return us;
+            DrawDev &d = ctx->hdraws[nd];
             d.verts = m.verts;
             d.idx = m.idx;
             d.nverts = m.nverts;

@@ -20,6 +20,9 @@ uint32_t g_clipped = 1;      // a sorted frame's clipped triangles per input one
 uint64_t g_dirty_words = 0;  // mask words found set when a setup pass began
 uint64_t g_setups = 0, g_same_address = 0;
 size_t g_size[NSLOTS];       // bytes allocated in each slot
+size_t g_host_limit = ~(size_t)0, g_host_bytes = 0;  // largest page-locked allocation allowed; bytes asked for
+uint64_t g_bad_draws = 0, g_seen_draws = 0;  // descriptors that reached the device, and wrong ones
+uint32_t g_tris = 1;                         // triangles of every draw
 const void *g_last_mask = nullptr;
 size_t g_last_size = 0;
 
@@ -56,7 +59,10 @@ cudaError_t cudaFree(void *p) {
     if (p) g_free.push_back((int)((static_cast<char *>(p) - g_base) / (ptrdiff_t)SLOT));
     return cudaSuccess;
 }
-cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return (*p = malloc(n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) {
+    g_host_bytes += n;
+    return n <= g_host_limit && (*p = malloc(n)) ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaMallocHost(void **p, size_t n) { return cudaHostAlloc(p, n, 0); }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
@@ -134,7 +140,12 @@ cudaError_t launch_draw_counts(const DrawDev *d, uint32_t nd, uint32_t, const ui
     for (uint32_t i = 0; i < nd; ++i) nout[i] = d[i].ntri * g_clipped;
     return cudaSuccess;
 }
-cudaError_t launch_vertex(const DrawDev *, uint32_t, uint32_t, float4 *, uint8_t *, uint32_t *, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t launch_vertex(const DrawDev *d, uint32_t nd, uint32_t, float4 *, uint8_t *, uint32_t *, int, cudaStream_t) {
+    for (uint32_t i = 0; i < nd; ++i)
+        g_bad_draws += d[i].tri_base != i * g_tris || d[i].mvp[0] != (float)i || d[i].verts == nullptr;
+    g_seen_draws += nd;
+    return cudaSuccess;
+}
 cudaError_t launch_cull(DrawDev *, uint32_t, StatsDev *, int, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_clip(const DrawDev *, uint32_t, uint32_t, const float4 *, const uint8_t *, uint32_t *, uint32_t *,
                         uint32_t *, PolyVert *, uint32_t, uint32_t *, int, cudaStream_t, uint32_t *, bool) { return cudaSuccess; }
@@ -158,22 +169,29 @@ size_t dsort_scratch_bytes(uint32_t n) { return (size_t)n * 32u + 4096u; }
 }  // namespace rfk
 
 namespace {
-// One frame of one mesh of ntri flat triangles on a w x h target.
-rf_status frame(rf_ctx *ctx, uint32_t ntri, uint32_t w, uint32_t h, int32_t sort) {
+// One frame of ndraws draws of one mesh of ntri flat triangles on a w x h
+// target; claims: the number of draws the call says it has (the one after the
+// last is a bad handle then).
+rf_status frame(rf_ctx *ctx, uint32_t ntri, uint32_t w, uint32_t h, int32_t sort, uint32_t ndraws = 1,
+                uint32_t claims = 0) {
     std::vector<float> v(9, 0.5f);
     std::vector<uint32_t> idx(3 * (size_t)ntri);
     for (size_t i = 0; i < idx.size(); ++i) idx[i] = (uint32_t)(i % 3);
+    g_tris = ntri;
     rf_mesh m = 0;
     rf_target t = 0;
     rf_status st = rf_mesh_upload(ctx, v.data(), 3, 3, 0, idx.data(), ntri, &m);
     if (!st) st = rf_target_create(ctx, w, h, RF_ARGB8888, 1, &t);
     if (!st) {
-        rf_draw d{};
-        d.mesh = m;
-        d.shader = RF_SHADER_FLAT;
+        std::vector<rf_draw> d(ndraws + 1);
+        for (uint32_t i = 0; i < ndraws; ++i) {
+            d[i].mesh = m;
+            d[i].shader = RF_SHADER_FLAT;
+            d[i].uniforms.mvp[0] = (float)i;
+        }
         const float vp[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1};
         const rf_context_flags fl{RF_DEPTH_LESS, 1, 1, RF_CULL_BACK, sort};
-        st = rf_render_draws(ctx, &d, 1, vp, t, &fl, nullptr);
+        st = rf_render_draws(ctx, d.data(), claims ? claims : ndraws, vp, t, &fl, nullptr);
     }
     if (t) rf_target_destroy(ctx, t);
     if (m) rf_mesh_destroy(ctx, m);
@@ -209,5 +227,33 @@ uint32_t shim_frames(const uint32_t *f, uint32_t n, uint64_t out[3]) {
 }
 uint32_t shim_zero_blocks(uint64_t n16, int masks, uint32_t ntiles, int nsm) {
     return rfk::zero_blocks(n16, masks != 0, ntiles, nsm);
+}
+// Frames of counts[i] draws each on one context, page-locked allocations above
+// `limit` bytes refused.  out: wrong descriptors, descriptors, page-locked
+// bytes asked for.  Returns the first status that is not RF_OK.
+int32_t shim_draws(const uint32_t *counts, uint32_t n, uint64_t limit, uint64_t out[3]) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return -1;
+    g_host_limit = limit;
+    g_host_bytes = g_bad_draws = g_seen_draws = 0;
+    rf_status st = RF_OK;
+    for (uint32_t i = 0; i < n && !st; ++i) st = frame(ctx, 1, 64, 64, 0, counts[i]);
+    rf_ctx_destroy(ctx);
+    g_host_limit = ~(size_t)0;
+    out[0] = g_bad_draws;
+    out[1] = g_seen_draws;
+    out[2] = g_host_bytes;
+    return st;
+}
+// A call of `good` draws, then a bad handle, that claims to have `claims` draws: its
+// status, and the page-locked bytes it asked for.
+int32_t shim_refused(uint32_t good, uint32_t claims, uint64_t *bytes) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return -1;
+    g_host_bytes = 0;
+    const rf_status st = frame(ctx, 2, 64, 64, 0, good, claims);
+    *bytes = g_host_bytes;
+    rf_ctx_destroy(ctx);
+    return st;
 }
 }

@@ -25,6 +25,8 @@ def shim(tmp_path_factory):
     L.shim_frames.restype = C.c_uint32
     L.shim_zero_blocks.argtypes = [C.c_uint64, C.c_int, C.c_uint32, C.c_int]
     L.shim_zero_blocks.restype = C.c_uint32
+    L.shim_draws.argtypes = [C.c_void_p, C.c_uint32, C.c_uint64, C.POINTER(C.c_uint64)]
+    L.shim_refused.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]
     return L
 
 
@@ -82,3 +84,24 @@ def test_zeroing_grid_covers_masks_left_marked(shim, mask_mb, ntiles):
     b = shim.shim_zero_blocks(n16, 0, ntiles, nsm)
     assert b >= min(n16 // 256, nsm) and b * 256 >= min(ntiles, nsm * 8 * 256)
     assert b <= max(2 * nsm, min(ntiles // 256 + 2, 8 * nsm)) and b <= (n16 + ntiles) // 256 + 2
+
+
+COUNTS = [1, 40, 101, 300, 5000, 7, 20000, 5000, 20, 300]
+
+
+@pytest.mark.parametrize("limit", [1 << 40, 4096, 1 << 20])
+def test_descriptors_arrive(shim, limit):
+    """Every draw's descriptor reaches the device as it was built, whatever the
+    frames before needed, and whether or not memory can be page-locked."""
+    a, out = np.array(COUNTS, np.uint32), (C.c_uint64 * 3)()
+    assert shim.shim_draws(a.ctypes.data, len(a), limit, out) == 0
+    assert (out[0], out[1]) == (0, sum(COUNTS))
+
+
+@pytest.mark.parametrize("good", [0, 1, 255, 256, 257, 3000])
+def test_refused_calls_lock_no_memory_for_what_they_claim(shim, good):
+    """A call whose count is wrong ends at its first bad draw with that draw's
+    status, and page-locks memory for the draws before it at most."""
+    n = C.c_uint64()
+    assert shim.shim_refused(good, 0xFFFFFFFF, C.byref(n)) == 1  # RF_ERR_BAD_HANDLE
+    assert n.value <= 65536 + 2 * 16 * 1.25 * 200 * good
