@@ -559,7 +559,8 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
     for (uint32_t k = 0; k < nin; ++k) most += in[k].draws ? in[k].ndraws : 0u;
     rf_status us = upload_begin(ctx, most, nin);
     if (us) return us;
-    size_t nd = 0;
+    DrawDev *hd = ctx->hdraws;
+    size_t nd = 0, room = ctx->hroom;
     ctx->any_cull = false;
     // The objects of the draw before (instances share their mesh and
     // texture, and a frame may have 10^5 of them).
@@ -593,8 +594,12 @@ rf_status build_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, std::vector<Job
                 ctx->async_meshes.push_back(&m);
             if (dr.shader < RF_SHADER_FLAT || dr.shader > RF_SHADER_GOURAUD_SRGB) return RF_ERR_BAD_ARG;
             if (m.nattr != nattr_for(dr.shader)) return RF_ERR_BAD_ARG;
-            if (nd == ctx->hroom && (us = upload_more(ctx, nd, most, nin))) return us;
-            DrawDev &d = ctx->hdraws[nd];
+            if (nd == room) {
+                if ((us = upload_more(ctx, nd, most, nin))) return us;
+                hd = ctx->hdraws;
+                room = ctx->hroom;
+            }
+            DrawDev &d = hd[nd];
             d.verts = m.verts;
             d.idx = m.idx;
             d.nverts = m.nverts;
