@@ -168,6 +168,7 @@ struct rf_ctx {
     bool rows_evt_pending = false;
     // stats: host-side counts + device-accumulated counts, and what was
     // already handed out by rf_ctx_take_stats / rf_render
+    bool stats_ready = false;  // stats and counters allocated and zeroed
     rf_stats host_acc{};
     rf_stats taken{};
     char last_error[1024] = {0};  // the failing call (as written) and the CUDA message
@@ -402,8 +403,8 @@ rf_status read_totals(rf_ctx *ctx, rf_stats &tot) {
     StatsDev sd{};
     uint32_t cnt[RF_CNT_N] = {0};
     CK(cudaStreamSynchronize(ctx->stream));
-    if (ctx->stats.p) CK(cudaMemcpy(&sd, ctx->stats.p, sizeof sd, cudaMemcpyDeviceToHost));
-    if (ctx->counters.p) CK(cudaMemcpy(cnt, ctx->counters.p, sizeof cnt, cudaMemcpyDeviceToHost));
+    if (ctx->stats_ready) CK(cudaMemcpy(&sd, ctx->stats.p, sizeof sd, cudaMemcpyDeviceToHost));
+    if (ctx->stats_ready) CK(cudaMemcpy(cnt, ctx->counters.p, sizeof cnt, cudaMemcpyDeviceToHost));
     tot = ctx->host_acc;
     tot.prims_o += sd.prims_o;
     tot.verts_o += sd.verts_o;
@@ -420,13 +421,14 @@ rf_status read_totals(rf_ctx *ctx, rf_stats &tot) {
 }
 
 rf_status init_stats(rf_ctx *ctx) {
-    if (ctx->stats.p) return RF_OK;
+    if (ctx->stats_ready) return RF_OK;
     rf_status s = ensure(ctx, ctx->stats, sizeof(StatsDev));
     if (s) return s;
     s = ensure(ctx, ctx->counters, RF_CNT_N * 4);
     if (s) return s;
     CK(cudaMemsetAsync(ctx->stats.p, 0, sizeof(StatsDev), ctx->stream));
     CK(cudaMemsetAsync(ctx->counters.p, 0, RF_CNT_N * 4, ctx->stream));
+    ctx->stats_ready = true;
     return RF_OK;
 }
 

@@ -13,6 +13,8 @@ constexpr size_t SLOT = 256u << 20;
 constexpr int NSLOTS = 256;
 char *g_base = nullptr;
 int g_next = 0;
+int g_fail_alloc = -1;       // the allocation that fails, counted down to (-1: none)
+uint64_t g_null_counters = 0, g_bad_counters = 0;  // zeroing launches without counters; counters of a new context not zero
 std::vector<int> g_free;
 int g_fail_lists = 0;        // the list pass reports an error this many times
 int g_fail_fill = 0;         // ... a fill of more than a few counters
@@ -37,6 +39,7 @@ size_t job_words(const JobDev *jobs, uint32_t nj) {
 
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t n) {
+    if (g_fail_alloc >= 0 && g_fail_alloc-- == 0) return cudaErrorMemoryAllocation;
     if (!g_base) {
         void *m = mmap(nullptr, SLOT * NSLOTS, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
         if (m == MAP_FAILED) return cudaErrorMemoryAllocation;
@@ -102,8 +105,13 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cu
 
 namespace rfk {
 cudaError_t launch_zero(uint32_t *mask, size_t words, bool masks, StatsDev *js, uint32_t njobs, unsigned long long *tacc,
-                        uint32_t ntiles, unsigned long long *totals, unsigned long long *marks, uint32_t *, int,
+                        uint32_t ntiles, unsigned long long *totals, unsigned long long *marks, uint32_t *counters, int,
                         cudaStream_t) {
+    if (!counters) {
+        ++g_null_counters;
+        return cudaSuccess;
+    }
+    for (int i = 0; i < RF_CNT_N; ++i) g_bad_counters += counters[i] != 0u;
     if (masks) memset(mask, 0, words * 4);
     memset(js, 0, njobs * sizeof(StatsDev));
     memset(tacc, 0, (size_t)ntiles * 8);
@@ -253,6 +261,22 @@ int32_t shim_refused(uint32_t good, uint32_t claims, uint64_t *bytes) {
     g_host_bytes = 0;
     const rf_status st = frame(ctx, 2, 64, 64, 0, good, claims);
     *bytes = g_host_bytes;
+    rf_ctx_destroy(ctx);
+    return st;
+}
+// On a new context, a frame whose k-th allocation fails (its mesh and target
+// included), then one that has all it asks for: the first one's status; out: the
+// second's, zeroing launches without counters, counters found set.
+int32_t shim_alloc_fails(uint32_t k, uint64_t out[3]) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return -1;
+    g_null_counters = g_bad_counters = 0;
+    g_fail_alloc = (int)k;
+    const rf_status st = frame(ctx, 5, 64, 64, 0);
+    g_fail_alloc = -1;
+    out[0] = frame(ctx, 5, 64, 64, 0);
+    out[1] = g_null_counters;
+    out[2] = g_bad_counters;
     rf_ctx_destroy(ctx);
     return st;
 }

@@ -26,6 +26,7 @@ def shim(tmp_path_factory):
     L.shim_zero_blocks.argtypes = [C.c_uint64, C.c_int, C.c_uint32, C.c_int]
     L.shim_zero_blocks.restype = C.c_uint32
     L.shim_draws.argtypes = [C.c_void_p, C.c_uint32, C.c_uint64, C.POINTER(C.c_uint64)]
+    L.shim_alloc_fails.argtypes = [C.c_uint32, C.POINTER(C.c_uint64)]
     L.shim_refused.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]
     return L
 
@@ -105,3 +106,13 @@ def test_refused_calls_lock_no_memory_for_what_they_claim(shim, good):
     n = C.c_uint64()
     assert shim.shim_refused(good, 0xFFFFFFFF, C.byref(n)) == 1  # RF_ERR_BAD_HANDLE
     assert n.value <= 65536 + 2 * 16 * 1.25 * 200 * good
+
+
+@pytest.mark.parametrize("k", range(40))
+def test_frame_after_one_out_of_memory(shim, k):
+    """A first frame whose k-th allocation fails, then one that gets its memory:
+    it has counters, and they are zero."""
+    out = (C.c_uint64 * 3)()
+    st = shim.shim_alloc_fails(k, out)
+    assert st in (0, 4)  # RF_ERR_OOM; 0: the frame makes fewer
+    assert tuple(out) == (0, 0, 0)
