@@ -815,10 +815,9 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     if ((st = ensure(ctx, ctx->live, (size_t)nt * RF_MAX_FAN * 8))) return st;  // two lists
     if ((st = ensure(ctx, ctx->marks, 8))) return st;
     if ((st = ensure(ctx, ctx->items, (size_t)ntiles * (RF_SPLIT_K + 1) * 4))) return st;
-    if (!ctx->rows_need_host) {
-        CK(cudaMallocHost(&ctx->rows_need_host, 2 * sizeof(unsigned long long)));
-        CK(cudaEventCreateWithFlags(&ctx->rows_evt, cudaEventDisableTiming));
-    }
+    // (each made once, and looked at one by one: a frame may have failed between them)
+    if (!ctx->rows_need_host) CK(cudaMallocHost(&ctx->rows_need_host, 2 * sizeof(unsigned long long)));
+    if (!ctx->rows_evt) CK(cudaEventCreateWithFlags(&ctx->rows_evt, cudaEventDisableTiming));
     if (ctx->rows_evt_pending && cudaEventQuery(ctx->rows_evt) == cudaSuccess) {
         const uint64_t need = *ctx->rows_need_host;
         if (need > ctx->rows_cap) ctx->rows_cap = need + need / 4;
@@ -841,10 +840,10 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     cudaStream_t s = ctx->stream;
     const bool any_cull = ctx->any_cull;
     const uint32_t ng = (uint32_t)ctx->groups.size();
-    if (ng > 1 && !ctx->side) {
-        CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&ctx->side_join, cudaEventDisableTiming));
+    if (ng > 1) {
+        if (!ctx->side) CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        if (!ctx->side_fork) CK(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
+        if (!ctx->side_join) CK(cudaEventCreateWithFlags(&ctx->side_join, cudaEventDisableTiming));
     }
     // The raster pass, its groups on two streams so that one group's last
     // tiles overlap the other's first.

@@ -13,6 +13,7 @@ constexpr size_t SLOT = 256u << 20;
 constexpr int NSLOTS = 256;
 char *g_base = nullptr;
 int g_next = 0;
+int g_fail_event = -1;       // the event that is not made, counted down to (-1: none)
 int g_fail_alloc = -1;       // the allocation that fails, counted down to (-1: none)
 uint64_t g_null_counters = 0, g_bad_counters = 0;  // zeroing launches without counters; counters of a new context not zero
 std::vector<int> g_free;
@@ -84,13 +85,18 @@ cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "error"; }
-cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = reinterpret_cast<cudaEvent_t>(1); return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t *e) {
+    if (g_fail_event >= 0 && g_fail_event-- == 0) return cudaErrorMemoryAllocation;
+    *e = reinterpret_cast<cudaEvent_t>(1);
+    return cudaSuccess;
+}
+cudaError_t event_ok(cudaEvent_t e) { return e ? cudaSuccess : cudaErrorInvalidResourceHandle; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
-cudaError_t cudaEventQuery(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t e) { return event_ok(e); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return event_ok(e); }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { return event_ok(e); }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
@@ -100,7 +106,7 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaError
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = reinterpret_cast<cudaStream_t>(1); return cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t e, unsigned) { return event_ok(e); }
 }
 
 namespace rfk {
@@ -277,6 +283,38 @@ int32_t shim_alloc_fails(uint32_t k, uint64_t out[3]) {
     out[0] = frame(ctx, 5, 64, 64, 0);
     out[1] = g_null_counters;
     out[2] = g_bad_counters;
+    rf_ctx_destroy(ctx);
+    return st;
+}
+// On a new context, a batch of two raster groups during which the k-th event
+// cannot be made, then the same again with nothing failing: the first one's status;
+// out: the second's.
+int32_t shim_event_fails(uint32_t k, int32_t *out) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return -1;
+    rf_ctx_set_tiling(ctx, 32, 4);
+    const float v[9] = {};
+    const uint32_t idx[3] = {0, 1, 2};
+    rf_mesh m = 0;
+    rf_target t[2] = {0, 0};
+    rf_status st = rf_mesh_upload(ctx, v, 3, 3, 0, idx, 1, &m);
+    for (int i = 0; i < 2 && !st; ++i) st = rf_target_create(ctx, 64, 64, RF_ARGB8888, 1, &t[i]);
+    if (st) return -1;
+    g_tris = 1;
+    rf_draw d{};
+    d.mesh = m;
+    d.shader = RF_SHADER_FLAT;
+    rf_job j[2]{};
+    for (int i = 0; i < 2; ++i) {
+        j[i].target = t[i];
+        j[i].ndraws = 1;
+        j[i].draws = &d;
+        j[i].flags = {i ? RF_DEPTH_GREATER : RF_DEPTH_LESS, 1, 1, RF_CULL_BACK, 0};
+    }
+    g_fail_event = (int)k;
+    st = rf_render_batch(ctx, j, 2, nullptr);
+    g_fail_event = -1;
+    *out = rf_render_batch(ctx, j, 2, nullptr);
     rf_ctx_destroy(ctx);
     return st;
 }

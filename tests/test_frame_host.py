@@ -27,6 +27,7 @@ def shim(tmp_path_factory):
     L.shim_zero_blocks.restype = C.c_uint32
     L.shim_draws.argtypes = [C.c_void_p, C.c_uint32, C.c_uint64, C.POINTER(C.c_uint64)]
     L.shim_alloc_fails.argtypes = [C.c_uint32, C.POINTER(C.c_uint64)]
+    L.shim_event_fails.argtypes = [C.c_uint32, C.POINTER(C.c_int32)]
     L.shim_refused.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]
     return L
 
@@ -116,3 +117,12 @@ def test_frame_after_one_out_of_memory(shim, k):
     st = shim.shim_alloc_fails(k, out)
     assert st in (0, 4)  # RF_ERR_OOM; 0: the frame makes fewer
     assert tuple(out) == (0, 0, 0)
+
+
+@pytest.mark.parametrize("k", range(6))
+def test_frame_after_one_short_of_events(shim, k):
+    """A first batch of two raster groups whose k-th event cannot be made, then
+    one that gets its events: it is rendered."""
+    out = C.c_int32()
+    st = shim.shim_event_fails(k, C.byref(out))
+    assert (st, out.value) in ((4, 0), (0, 0))  # RF_ERR_OOM; 0: the batch makes fewer
