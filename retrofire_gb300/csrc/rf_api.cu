@@ -94,6 +94,9 @@ struct UploadBuf {
     bool pending = false;
 };
 
+// Streams of the raster pass beside the context's own: one a group.
+constexpr uint32_t RF_SIDE_STREAMS = RF_MAX_GROUPS - 1;
+
 // An instantiated launch sequence and the frame shape it was captured for.
 struct GraphKey {
     uint64_t v[13 + 3 * RF_MAX_GROUPS];
@@ -184,10 +187,10 @@ struct rf_ctx {
     bool any_cull = false;  // a draw asks for object culling
     std::vector<JobDev> hjobs;
     std::vector<RasterGroup> groups;
-    // Frames of several raster groups: the second launches on a side stream,
-    // forked and joined by events (lazily made).
-    cudaStream_t side = nullptr;
-    cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    // Frames of several raster groups: all but the first launch on side
+    // streams, forked and joined by events (lazily made).
+    cudaStream_t side[RF_SIDE_STREAMS] = {};
+    cudaEvent_t side_fork = nullptr, side_join[RF_SIDE_STREAMS] = {};
     // stage timing
     bool timing = false;
     std::vector<cudaEvent_t> ev_free;
@@ -494,13 +497,29 @@ uint64_t layout_masks(std::vector<JobDev> &hj) {
 
 // The raster groups present (J.group: kind and context, then the group's
 // index among them), and the order the jobs' tiles are laid out in: by group.
+// Groups of fewer than RF_GROUP_MIN triangles join their context's group of
+// mixed kinds, whose kernels take up to twice as long a triangle but come once:
+// a batch of five kinds, 300 triangles each on 1280 x 720, takes 153 us in five
+// groups and 87 in one, of 10,000 each 199 and 120; two kinds of 30,000 each
+// 213 and 225 (triangles of 40 px), of 80,000 800 and 900, which is where the
+// line lies.
+constexpr uint32_t RF_GROUP_MIN = 32768u;
 void group_jobs(rf_ctx *ctx) {
     auto &hj = ctx->hjobs;
     auto &gr = ctx->groups;
     gr.clear();
-    uint32_t seen = 0;
-    for (const JobDev &J : hj) seen |= 1u << J.group;
-    uint32_t dense[RF_MAX_GROUPS];
+    uint64_t tris[RF_MAX_GROUPS] = {};
+    for (const JobDev &J : hj) tris[J.group] += J.ntri;
+    uint32_t to[RF_MAX_GROUPS], dense[RF_MAX_GROUPS], seen = 0;
+    for (uint32_t g = 0; g < RF_MAX_GROUPS; ++g) to[g] = g;
+    for (uint32_t c = 0; c < 2; ++c) {  // (the default context, then the others)
+        const uint32_t any = RF_K_ANY * 2 + c;
+        uint32_t few = tris[any] ? 1u : 0u;
+        for (uint32_t g = c; g < any; g += 2) few += tris[g] && tris[g] < RF_GROUP_MIN;
+        for (uint32_t g = c; few > 1u && g < any; g += 2)
+            if (tris[g] < RF_GROUP_MIN) to[g] = any;
+    }
+    for (JobDev &J : hj) seen |= 1u << (J.group = to[J.group]);
     for (uint32_t g = 0; g < RF_MAX_GROUPS; ++g)
         if (seen & (1u << g)) {
             dense[g] = (uint32_t)gr.size();
@@ -840,26 +859,29 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
     cudaStream_t s = ctx->stream;
     const bool any_cull = ctx->any_cull;
     const uint32_t ng = (uint32_t)ctx->groups.size();
-    if (ng > 1) {
-        if (!ctx->side) CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
-        if (!ctx->side_fork) CK(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
-        if (!ctx->side_join) CK(cudaEventCreateWithFlags(&ctx->side_join, cudaEventDisableTiming));
+    const uint32_t nside = std::min<uint32_t>(ng - 1u, RF_SIDE_STREAMS);
+    if (nside && !ctx->side_fork) CK(cudaEventCreateWithFlags(&ctx->side_fork, cudaEventDisableTiming));
+    for (uint32_t i = 0; i < nside; ++i) {
+        if (!ctx->side[i]) CK(cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking));
+        if (!ctx->side_join[i]) CK(cudaEventCreateWithFlags(&ctx->side_join[i], cudaEventDisableTiming));
     }
-    // The raster pass, its groups on two streams so that one group's last
-    // tiles overlap the other's first.
+    // The raster pass, a stream a group: one group's last tiles overlap
+    // another's first, and groups of few tiles share the chip (ten groups of
+    // 80,000 triangles on 320 x 240 each: 6.8 ms on two streams, 3.9 on ten).
     auto raster = [&](const JobDev *jobs, const DrawDev *draws, uint32_t *counters, StatsDev *stats) -> rf_status {
-        const cudaStream_t st2[2] = {ctx->stream, ctx->side};
-        if (ng > 1) {
-            CK(cudaEventRecord(ctx->side_fork, ctx->stream));
-            CK(cudaStreamWaitEvent(ctx->side, ctx->side_fork, 0));
+        cudaStream_t st[1 + RF_SIDE_STREAMS] = {ctx->stream};
+        if (nside) CK(cudaEventRecord(ctx->side_fork, ctx->stream));
+        for (uint32_t i = 0; i < nside; ++i) {
+            st[1 + i] = ctx->side[i];
+            CK(cudaStreamWaitEvent(ctx->side[i], ctx->side_fork, 0));
         }
         CK(rfk::launch_raster(TW, ctx->groups.data(), ng, jobs, nj, draws, P<PrimRec>(ctx->prims),
                               P<RasterPrim>(ctx->rprims), P<uint32_t>(ctx->rows), P<uint2>(ctx->ent), P<uint32_t>(ctx->mask),
-                              P<uint2>(ctx->segs), P<uint2>(ctx->list), ntiles, P<uint32_t>(ctx->items), counters, stats, ctx->warps, ctx->nsm, st2,
-                              ng > 1 ? 2u : 1u));
-        if (ng > 1) {
-            CK(cudaEventRecord(ctx->side_join, ctx->side));
-            CK(cudaStreamWaitEvent(ctx->stream, ctx->side_join, 0));
+                              P<uint2>(ctx->segs), P<uint2>(ctx->list), ntiles, P<uint32_t>(ctx->items), counters, stats,
+                              ctx->warps, ctx->nsm, st, 1u + nside));
+        for (uint32_t i = 0; i < nside; ++i) {
+            CK(cudaEventRecord(ctx->side_join[i], ctx->side[i]));
+            CK(cudaStreamWaitEvent(ctx->stream, ctx->side_join[i], 0));
         }
         return RF_OK;
     };
@@ -1096,12 +1118,14 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         CK(cudaEventRecord(tuned->e1, s));
         tuned->pending = true;
     }
-    // zero, vertex, clip (2), lists, and per group setup, bin (2: 16-lane
-    // groups, then warps) and raster (+ the stats fold; a depth-sorted frame
+    // zero, vertex, clip (2), lists, per kind setup and bin (2: 16-lane groups,
+    // then warps) and per group raster (+ the stats fold; a depth-sorted frame
     // adds the scan of the fan counts, 3 launches or 1 for one block, and its
     // sort)
+    uint32_t nkinds = 0;
+    for (uint32_t g = 0; g < ng; ++g) nkinds += g == 0 || ctx->groups[g].kind != ctx->groups[g - 1].kind;
     const uint64_t scan_kernels = sorted ? (nt <= RF_SCAN_BLOCK_ITEMS ? 1 : 3) : 0;
-    ctx->kernels += 5 + 4 * ng + scan_kernels + (per_job ? 1 : 0) + (any_cull ? 1 : 0) + sort_kernels;
+    ctx->kernels += 5 + 3 * nkinds + ng + scan_kernels + (per_job ? 1 : 0) + (any_cull ? 1 : 0) + sort_kernels;
     if (!ctx->rows_evt_pending) {
         CK(cudaMemcpyAsync(ctx->rows_need_host, ctx->rowtot.p, 16, cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(ctx->rows_evt, s));
@@ -1290,9 +1314,11 @@ rf_status rf_ctx_destroy(rf_ctx *ctx) {
     for (auto &kv : ctx->targets) { cudaFree(kv.second.color); cudaFree(kv.second.depth); drop_async(kv.second); }
     if (ctx->up) cudaStreamDestroy(ctx->up);
     if (ctx->down) cudaStreamDestroy(ctx->down);
-    if (ctx->side) cudaStreamDestroy(ctx->side);
+    for (cudaStream_t q : ctx->side)
+        if (q) cudaStreamDestroy(q);
     if (ctx->side_fork) cudaEventDestroy(ctx->side_fork);
-    if (ctx->side_join) cudaEventDestroy(ctx->side_join);
+    for (cudaEvent_t e : ctx->side_join)
+        if (e) cudaEventDestroy(e);
     graphs_drop(ctx);
     for (TuneState &t : ctx->tunes) {
         if (t.e0) cudaEventDestroy(t.e0);

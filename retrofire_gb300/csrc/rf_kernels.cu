@@ -2004,9 +2004,15 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
     // (A depth-sorted frame's triangles are single clipped pieces.)
     const size_t fan = perm ? 1 : RF_MAX_FAN;
     uint32_t *big = live, *mid = live + (size_t)nt * fan;
-    for (uint32_t g = 0; g < ng; ++g) {
-        const uint32_t gt = groups[g].ntri;
+    for (uint32_t g = 0, g1; g < ng; g = g1) {
+        // The groups of one kind, whatever their context: neighbours.
+        uint32_t gt = 0, nblocks = 0;
+        for (g1 = g; g1 < ng && groups[g1].kind == groups[g].kind; ++g1) {
+            gt += groups[g1].ntri;
+            nblocks += groups[g1].nblocks;
+        }
         if (gt == 0) continue;
+        const uint32_t block0 = groups[g].nblocks ? groups[g].block0 : groups[g1 - 1].block0;
         auto setup = k_setup<0>;
         auto bin = k_bin<0>;
         auto bin16 = k_bin_small<0, 16>;
@@ -2019,8 +2025,8 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
             default: break;
         }
         uint32_t *big_n = counters + RF_CNT_LIVE_G + g, *mid_n = counters + RF_CNT_LIVE_MID_G + g;
-        const uint32_t blocks = min(groups[g].nblocks, (uint32_t)nsm * 32);
-        RF_NEXT(setup, blocks, RF_SETUP_THREADS, 0, s, draws, nd, jobs, nj, groups[g].block0, groups[g].nblocks, tile_w,
+        const uint32_t blocks = min(nblocks, (uint32_t)nsm * 32);
+        RF_NEXT(setup, blocks, RF_SETUP_THREADS, 0, s, draws, nd, jobs, nj, block0, nblocks, tile_w,
                                                   cpos, tcnt, toff, tpoly, pool, prims, rows_total, rows, rows_cap,
                                                   rprims, ent, mask, big, big_n, mid, mid_n, marks, stats, perm, ptri);
         cudaError_t e = cudaGetLastError();

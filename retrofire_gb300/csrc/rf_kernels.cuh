@@ -38,9 +38,9 @@
 #define RF_RASTER_MAX_THREADS 256
 // The jobs of a frame are laid out by raster group: one shader kind (or
 // RF_K_ANY: jobs that mix kinds) and one context (the default one on a depth
-// target, or any other).  Every group has setup, binning and raster launches
-// of its own, specialised for its kind, its own live lists and its own part
-// of the work list.
+// target, or any other).  Every group has a raster launch of its own,
+// specialised for both, and its own part of the work list; the groups of one
+// kind share setup and binning launches and live lists.
 #define RF_MAX_GROUPS (2 * (RF_K_ANY + 1))
 struct RasterGroup {
     int32_t kind;
@@ -62,7 +62,7 @@ struct RasterGroup {
 #define RF_CNT_CLIPQ 10   // triangles queued for clipping
 #define RF_CNT_QUEUE_G 16     // + g: work-list queue head of raster group g
 #define RF_CNT_ITEMS_G (RF_CNT_QUEUE_G + RF_MAX_GROUPS)  // + g: its heavy tiles and crowded tiles' slices
-#define RF_CNT_LIVE_G (RF_CNT_ITEMS_G + RF_MAX_GROUPS)   // + g: its live triangles, binned a warp each
+#define RF_CNT_LIVE_G (RF_CNT_ITEMS_G + RF_MAX_GROUPS)   // + g, a kind's first group: live triangles, binned a warp each
 #define RF_CNT_LIVE_MID_G (RF_CNT_LIVE_G + RF_MAX_GROUPS)  // + g: ... sixteen lanes each (at most 16 rows)
 #define RF_CNT_N (RF_CNT_LIVE_MID_G + RF_MAX_GROUPS)
 #define RF_SCAN_BLOCK_ITEMS 4096u  // values one scan block takes (one launch instead of three)
@@ -147,11 +147,11 @@ cudaError_t launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t 
                         uint32_t *total, cudaStream_t s);
 // Triangle setup (k_setup: also the row records and tile bits of triangles
 // of a few rows), then scanline statistics, row records and tile binning of
-// the others (k_bin_small for at most 16 rows, then k_bin), per raster group.
+// the others (k_bin_small for at most 16 rows, then k_bin), per shader kind.
 // rows holds rows_cap words; rows_total receives the words the frame asked
 // for, each triangle's records placed by k_setup from it (rows_total[1] is
 // the lists' cursor); live (room for twice every output triangle) receives
-// the index of each triangle left for the binning pass, group after group:
+// the index of each triangle left for the binning pass, kind after kind:
 // those for k_bin (counters[RF_CNT_LIVE_G + g]) in its first half, the regular
 // ones with at most 16 rows on the target (counters[RF_CNT_LIVE_MID_G + g])
 // in its second; *marks receives the (triangle, tile) bits set in all.

@@ -6,6 +6,8 @@
 // pass marks them, zero again once the list pass has read them.
 #include <sys/mman.h>
 
+#include <set>
+
 #include "../../retrofire_gb300/csrc/rf_api.cu"
 
 namespace {
@@ -28,6 +30,9 @@ uint64_t g_bad_draws = 0, g_seen_draws = 0;  // descriptors that reached the dev
 uint32_t g_tris = 1;                         // triangles of every draw
 const void *g_last_mask = nullptr;
 size_t g_last_size = 0;
+
+std::vector<RasterGroup> g_groups;   // of the last frame
+std::set<cudaStream_t> g_streams;    // ... that its groups are on
 
 // Words of the masks and summaries the jobs lay out.
 size_t job_words(const JobDev *jobs, uint32_t nj) {
@@ -103,7 +108,11 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t *, cudaGraph_t, unsigned long l
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorNotSupported; }
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { *s = reinterpret_cast<cudaStream_t>(1); return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
+    static uintptr_t n = 0;
+    *s = reinterpret_cast<cudaStream_t>(++n);
+    return cudaSuccess;
+}
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t e, unsigned) { return event_ok(e); }
@@ -171,10 +180,15 @@ cudaError_t launch_dsort(const DrawDev *, uint32_t, const JobDev *, uint32_t, ui
 cudaError_t launch_lines(const DrawDev *, const JobDev *, uint32_t, const float4 *, const uint8_t *, LineRec *, uint32_t *,
                          uint32_t, uint32_t *, StatsDev *, int, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_stamp(unsigned long long *, cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_raster(uint32_t, const RasterGroup *, uint32_t, const JobDev *, uint32_t, const DrawDev *,
+cudaError_t launch_raster(uint32_t, const RasterGroup *g, uint32_t ng, const JobDev *, uint32_t, const DrawDev *,
                           const PrimRec *, const RasterPrim *, const uint32_t *, const uint2 *, const uint32_t *,
                           const uint2 *, const uint2 *, uint32_t, const uint32_t *, uint32_t *, StatsDev *, uint32_t, int,
-                          const cudaStream_t *, uint32_t) { return cudaSuccess; }
+                          const cudaStream_t *st, uint32_t nst) {
+    g_groups.assign(g, g + ng);
+    g_streams.clear();
+    for (uint32_t i = 0; i < ng; ++i) g_streams.insert(st[i % nst]);
+    return cudaSuccess;
+}
 cudaError_t launch_mesh_bbox(const float *, uint32_t, uint32_t, float *, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_stats_fold(const StatsDev *, uint32_t, StatsDev *, cudaStream_t) { return cudaSuccess; }
 uint32_t dsort_scan_items(uint32_t) { return 0; }
@@ -317,5 +331,37 @@ int32_t shim_event_fails(uint32_t k, int32_t *out) {
     *out = rf_render_batch(ctx, j, 2, nullptr);
     rf_ctx_destroy(ctx);
     return st;
+}
+// A batch of n jobs (shader, 1 for the default context or 0, triangles): its raster
+// groups as (shader, default context, triangles), the streams they are on and
+// the kernels counted; returns the groups, or -1.
+int32_t shim_groups(const uint32_t *jobs, uint32_t n, uint32_t *out, uint32_t *streams, uint64_t *kernels) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return -1;
+    rf_ctx_set_tiling(ctx, 32, 4);
+    std::vector<rf_draw> d(n);
+    std::vector<rf_job> j(n);
+    const std::vector<float> v(3 * 7, 0.5f);
+    g_tris = 0;  // (descriptors not looked at)
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t *q = jobs + 3 * i;
+        std::vector<uint32_t> idx(3 * (size_t)q[2], 0u);
+        if (rf_mesh_upload(ctx, v.data(), 3, 4, q[0] == RF_SHADER_FLAT ? 0 : 3, idx.data(), q[2], &d[i].mesh)) return -1;
+        if (rf_target_create(ctx, 32, 32, RF_ARGB8888, 1, &j[i].target)) return -1;
+        d[i].shader = (int32_t)q[0];
+        j[i].ndraws = 1;
+        j[i].draws = &d[i];
+        j[i].flags = {q[1] ? RF_DEPTH_LESS : RF_DEPTH_GREATER, 1, 1, RF_CULL_BACK, 0};
+    }
+    if (rf_render_batch(ctx, j.data(), n, nullptr)) return -1;
+    rf_ctx_counts(ctx, kernels, nullptr, nullptr);
+    rf_ctx_destroy(ctx);
+    for (size_t g = 0; g < g_groups.size(); ++g) {
+        out[3 * g] = (uint32_t)g_groups[g].kind;
+        out[3 * g + 1] = g_groups[g].fast;
+        out[3 * g + 2] = g_groups[g].ntri;
+    }
+    *streams = (uint32_t)g_streams.size();
+    return (int32_t)g_groups.size();
 }
 }

@@ -28,6 +28,7 @@ def shim(tmp_path_factory):
     L.shim_draws.argtypes = [C.c_void_p, C.c_uint32, C.c_uint64, C.POINTER(C.c_uint64)]
     L.shim_alloc_fails.argtypes = [C.c_uint32, C.POINTER(C.c_uint64)]
     L.shim_event_fails.argtypes = [C.c_uint32, C.POINTER(C.c_int32)]
+    L.shim_groups.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)]
     L.shim_refused.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]
     return L
 
@@ -126,3 +127,28 @@ def test_frame_after_one_short_of_events(shim, k):
     out = C.c_int32()
     st = shim.shim_event_fails(k, C.byref(out))
     assert (st, out.value) in ((4, 0), (0, 0))  # RF_ERR_OOM; 0: the batch makes fewer
+
+
+FLAT, GOURAUD, SRGB, MIXED = 0, 1, 4, 5
+
+
+@pytest.mark.parametrize("jobs,groups", [  # (shader, default context, triangles)
+    ([(GOURAUD, 1, 100)], [(GOURAUD, 1, 100)]),
+    ([(FLAT, 1, 100), (GOURAUD, 1, 200)], [(MIXED, 1, 300)]),
+    ([(FLAT, 1, 5), (GOURAUD, 0, 7)], [(FLAT, 1, 5), (GOURAUD, 0, 7)]),
+    ([(k, c, 10) for k in (SRGB, FLAT, GOURAUD) for c in (0, 1)], [(MIXED, 1, 30), (MIXED, 0, 30)]),
+    ([(GOURAUD, 0, 40), (GOURAUD, 1, 40)], [(GOURAUD, 1, 40), (GOURAUD, 0, 40)]),
+    ([(FLAT, 1, 33000), (GOURAUD, 1, 10), (GOURAUD, 1, 20)], [(FLAT, 1, 33000), (GOURAUD, 1, 30)]),
+    ([(FLAT, 1, 9), (GOURAUD, 1, 20000), (GOURAUD, 1, 20000), (SRGB, 1, 9)], [(GOURAUD, 1, 40000), (MIXED, 1, 18)]),
+])
+def test_raster_groups(shim, jobs, groups):
+    """Groups of few triangles are one of mixed kinds, the others a group each,
+    on a stream each; the groups of one kind share their setup launches."""
+    a, out = np.array(jobs, np.uint32), np.zeros(64, np.uint32)
+    streams, k = C.c_uint32(), C.c_uint64()
+    n = shim.shim_groups(a.ctypes.data, len(a), out.ctypes.data, C.byref(streams), C.byref(k))
+    assert [tuple(r) for r in out[:3 * n].reshape(n, 3).tolist()] == groups
+    assert streams.value == n
+    kinds = len({g[0] for g in groups})
+    # a mesh's box two, zero, vertex, clip two, lists, the stats, three a kind, one a group
+    assert k.value == 2 * len(jobs) + 6 + 3 * kinds + n

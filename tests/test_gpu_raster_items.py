@@ -236,3 +236,40 @@ def test_tables_that_no_row_takes(tw, kind):
     assert o[2]["frags_o"] > 0
     for _ in range(3):
         assert_parity(gpu_render([d], vp, w, h, ctx=ctx, tile=(tw, 4)), o, what="width %d" % tw)
+
+
+@pytest.mark.parametrize("large", [(rf.GOURAUD, rf.TEX_GOURAUD), (rf.FLAT, rf.GOURAUD, rf.TEXTURED, rf.TEX_GOURAUD,
+                                                                  rf.GOURAUD_SRGB)])
+@pytest.mark.parametrize("graphs", [False, True])
+def test_large_and_small_groups_in_one_batch(graphs, large):
+    """Raster groups large enough for kernels of their own, of some kinds or of
+    every one, in both contexts, and small ones that go together: replayed too."""
+    dev = rf.Device()
+    dev.set_graphs(graphs)
+    w, h = 260, 130
+    vp = mat.viewport(0, 0, w, h)
+    jobs, keep = [], []
+    try:
+        kinds = [rf.FLAT, rf.GOURAUD, rf.TEXTURED, rf.TEX_GOURAUD, rf.GOURAUD_SRGB]
+        for i, (k, test, n) in enumerate([(k, t, n) for n in (60, 33000, 90) for t in (rf.DEPTH_LESS, rf.DEPTH_GREATER)
+                                          for k in kinds if n == 60 or k in large]):
+            ctx = rf.Context(face_cull=rf.CULL_NONE, depth_test=test,
+                             depth_clear=float("inf") if test == rf.DEPTH_LESS else 0.1)
+            d = tris(300 + i, n, w, h, (1, 6, 1, 6) if n > 1000 else (2, 60, 2, 60), k)
+            tg = rf.Framebuf(w, h, device=dev)
+            m = rf.Mesh(d.verts, d.faces, pos_dim=4, device=dev)
+            t = rf.Texture(d.tex, device=dev) if d.tex is not None else None
+            keep += [tg, m] + ([t] if t else [])
+            jobs.append((rf.Scene(tg, [(m, rf.Shader(d.shader, d.flat_rgba, t), None)], vp, ctx),
+                         oracle_render([d], vp, w, h, ctx=ctx), ctx, 1 if k == rf.GOURAUD_SRGB else 0))
+        for _ in range(3):
+            for sc, _, ctx, _ in jobs:
+                sc.target.clear(ctx.color_clear, ctx.depth_clear)
+            stats = rf.render_batch([j[0] for j in jobs], device=dev)
+            for (sc, ref, ctx, tol), st in zip(jobs, stats):
+                col, dep = sc.target.read()
+                assert_parity((col, dep, st), ref, color_tol=tol)
+    finally:
+        for x in keep:
+            x.close()
+        dev.close()
