@@ -7,11 +7,11 @@
 // k_line_setup: one thread per line; clips it, walks its pixels with the
 // reference's running sum (stats, and the tiles it touches: a per-tile
 // bitmask over the lines, bit order = submission order).
-// k_line_raster: a warp per quarter of a 32x32 tile (8 rows, its pixels in
-// shared memory) takes the tile's lines in order, 32 at a time, and their steps
-// inside its columns (a line that steps along x) or rows, 32 of any lines a
-// pass: a lane's pixel comes from the k-step running sum, and lanes that meet
-// in a pixel go in submission order.
+// k_line_raster: a warp per quarter or half of a 32x32 tile (8 or 16 rows, its
+// pixels in shared memory unless its lines are few) takes the tile's lines in
+// order, 32 at a time, and their steps inside its columns (a line that steps
+// along x) or rows, 32 of any lines a pass: a lane's pixel comes from the
+// running sum, and lanes that meet in a pixel go in submission order.
 #include "rf_raster.cuh"
 
 using namespace rfx;
@@ -197,8 +197,8 @@ __global__ void k_line_setup(const DrawDev *__restrict__ draws, const JobDev *__
 }
 
 // The k-step running sum from s: one add after the other up to RF_LINE_STEP
-// steps (4 cycles each; a wireframe's lines are mostly shorter), else the exact
-// jump.
+// steps (4 cycles each; a wireframe's lines are mostly shorter, and so are a
+// line's steps in a tile), else the exact jump.
 #define RF_LINE_STEP 64u
 __device__ __forceinline__ float line_step(float s, float d, uint32_t k) {
     if (k > RF_LINE_STEP) return jump(s, d, k);
@@ -210,27 +210,53 @@ __device__ __forceinline__ float line_step(float s, float d, uint32_t k) {
     return s;
 }
 
+// Leaves out steps of a line (n of them, the first at R.begin with the value
+// R.s0) whose pixels miss the rows (columns) [a0, a1): those the line, as one,
+// is more than a pixel away from.  |d| <= 1 and n <= 32, so 32 additions near
+// the target are off by far less; below 0 a step draws in row (column) 0.
+__device__ __forceinline__ void line_trim(LineRec &R, uint32_t &n, uint32_t a0, uint32_t a1) {
+    if (!(fabsf(R.s0) < 1e6f)) return;
+    const float lo = a0 ? (float)a0 - 1.0f : -1e7f, hi = (float)a1 + 1.0f, last = (float)n * R.d + R.s0;
+    if (fmaxf(R.s0, last) < lo || fminf(R.s0, last) > hi) {
+        n = 0;
+        return;
+    }
+    // the steps that enter and leave [lo, hi], moved apart by one
+    const float in = R.d > 0.0f ? lo : hi, out = R.d > 0.0f ? hi : lo, r = fdiv(1.0f, R.d);
+    const uint32_t k0 = (uint32_t)fminf(fmaxf((in - R.s0) * r - 1.0f, 0.0f), (float)n);
+    const uint32_t k1 = (uint32_t)fminf(fmaxf((out - R.s0) * r + 2.0f, 0.0f), (float)n);
+    if (!(fabsf(R.d) > 1e-6f) || (k0 == 0u && k1 == n)) return;  // (too flat to cross: every step)
+    R.s0 = line_step(R.s0, R.d, k0);
+    R.begin += k0;
+    n = k1 > k0 ? k1 - k0 : 0u;
+}
+
 #define RF_LINE_WARPS 4
-#define RF_LINE_ROWS 8u    // tile rows a warp draws
 #define RF_LINE_PITCH 33u  // words per tile row in shared memory (odd: steep lines hit different banks)
 // Bound by the latencies of the fullest tiles (up to 200 lines of a wireframe of
 // 12,416 at 1280x720): one line a pass, a lane per column or row, each line's
 // record and pixels waited for in turn, took 117 us there.  With a batch's
 // records loaded together, the pixels in shared memory and short lines sharing
-// a pass 65, with short lines stepped instead of jumped 60, and with four warps
-// a tile, RF_LINE_ROWS rows each, 31 (each reads all of the tile's mask, which
-// is in L2, but steps only the lines that can reach its rows).
+// a pass 65, and with four warps a tile, ROWS rows each, 31 (each reads all of
+// the tile's mask, which is in L2).  The running sum is worked out once a line
+// and part, at its first step there, and stepped on from that (with a jump a
+// pixel 30,000 lines of up to 3,000 px took 4.0 ms on 320 x 240, 2.7 ms one line
+// a pass; now 1.3), and only for the steps that can reach the part's rows.
+// Parts with few lines, which are most of a large target's, draw in place: moved
+// through shared memory 30,000 lines of up to 20 px on 3840 x 2160 took 210 us,
+// now 149.
+template <uint32_t ROWS>  // tile rows a warp draws
 __global__ void __launch_bounds__(RF_LINE_WARPS * 32)
 k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
               const uint32_t *mask, uint32_t ntiles, uint32_t *__restrict__ queue,
               StatsDev *__restrict__ stats) {
     rfd::grid_begin();
     constexpr uint32_t FULL = 0xFFFFFFFFu;
-    __shared__ uint32_t s_col[RF_LINE_WARPS][RF_LINE_ROWS * RF_LINE_PITCH];
-    __shared__ float s_dep[RF_LINE_WARPS][RF_LINE_ROWS * RF_LINE_PITCH];
+    __shared__ uint32_t s_col[RF_LINE_WARPS][ROWS * RF_LINE_PITCH];
+    __shared__ float s_dep[RF_LINE_WARPS][ROWS * RF_LINE_PITCH];
     __shared__ LineRec s_rec[RF_LINE_WARPS][32];
     __shared__ uint32_t s_pend[RF_LINE_WARPS][64];  // the tile's lines found, not drawn yet
-    __shared__ uint2 s_item[RF_LINE_WARPS][32];  // per line of the batch with steps here: first step, first item
+    __shared__ uint2 s_item[RF_LINE_WARPS][32];  // per line of the batch with steps here: its lane, first item
     const JobDev &J = jobs[0];
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t below = (1u << lane) - 1u, upto = below | (1u << lane);
@@ -244,13 +270,13 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
         uint32_t part = 0;
         if (lane == 0) part = atomicAdd(queue, 1u);
         part = __shfl_sync(FULL, part, 0);
-        const uint32_t tile = part / (RF_TILE_H / RF_LINE_ROWS);
+        const uint32_t tile = part / (RF_TILE_H / ROWS);
         if (tile >= ntiles) break;
         const uint32_t ty = tile / J.tiles_x, tx = tile - ty * J.tiles_x;
         const uint32_t tx0 = tx * RF_TILE_H, tx1 = min(tx0 + RF_TILE_H, J.w);
-        const uint32_t ty0 = ty * RF_TILE_H + part % (RF_TILE_H / RF_LINE_ROWS) * RF_LINE_ROWS;
+        const uint32_t ty0 = ty * RF_TILE_H + part % (RF_TILE_H / ROWS) * ROWS;
         if (ty0 >= J.h) continue;
-        const uint32_t ty1 = min(ty0 + RF_LINE_ROWS, J.h);
+        const uint32_t ty1 = min(ty0 + ROWS, J.h);
         const uint32_t *tm = mask + (size_t)tile * J.mask_words;
         bool loaded = false;
         // The tile's lines in order: 32 mask words at a time (the next four
@@ -261,6 +287,13 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
         uint32_t word = 0, incl = 0, nlines = 0, lb = 0, wb = 0, pend = 0;
         for (bool last = false; !last;) {
             if (lb >= nlines) {
+                while (wb < J.mask_words && !__any_sync(FULL, next[0] != 0u)) {  // (no lines in these)
+                    wb += 32u;
+                    next[0] = next[1];
+                    next[1] = next[2];
+                    next[2] = next[3];
+                    next[3] = words(wb + 96u);
+                }
                 last = wb >= J.mask_words;
                 word = last ? 0u : next[0];
                 incl = __popc(word);
@@ -296,10 +329,12 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
             __syncwarp();
             if (pend == 0u || (pend < 32u && !last)) continue;
             {
-                if (!loaded) {
+                // (the part's only batch: its pixels are drawn where they lie)
+                const bool direct = last && !loaded && pend <= 32u;
+                if (!loaded && !direct) {
                     loaded = true;
 #pragma unroll 8
-                    for (uint32_t r = 0; r < RF_LINE_ROWS; ++r)
+                    for (uint32_t r = 0; r < ROWS; ++r)
                         if (ty0 + r < ty1 && tx0 + lane < tx1) {
                             const size_t i = (size_t)(ty0 + r) * J.w + tx0 + lane;
                             col[r * RF_LINE_PITCH + lane] = J.color[i];
@@ -312,22 +347,17 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
                 __syncwarp();
                 s_pend[wib][lane] = left;
                 pend -= here;
-                uint32_t n = 0, first = 0;  // this line's steps in the tile's columns (rows)
+                uint32_t n = 0;  // this line's steps in the tile's columns (rows)
                 if (lane < here) {
-                    const LineRec R = recs[line];
-                    s_rec[wib][lane] = R;
+                    LineRec R = recs[line];
                     const uint64_t t0 = R.wide ? tx0 : ty0, t1 = R.wide ? tx1 : ty1;
                     const uint64_t a = max(R.begin, t0), b = min(R.begin + R.n, t1);
-                    // (a short line along x, a row or more above or below: skipped.
-                    // Its |d| <= 1, so RF_LINE_STEP additions near these rows are
-                    // off by far less than a row; below 0 it draws in row 0.)
-                    const float y0 = R.s0, y1 = fadd(R.s0, fmul(R.d, (float)R.n));
-                    const bool off = R.wide && R.n <= RF_LINE_STEP &&
-                                     (fmaxf(fmaxf(y0, y1), 0.0f) + 1.0f < (float)ty0 ||
-                                      fminf(y0, y1) - 1.0f > (float)ty1);
-                    if (a < b && !off) {
+                    if (a < b) {
                         n = (uint32_t)(b - a);
-                        first = (uint32_t)(a - R.begin);
+                        R.s0 = line_step(R.s0, R.d, (uint32_t)(a - R.begin));
+                        R.begin = a;
+                        line_trim(R, n, R.wide ? ty0 : tx0, R.wide ? ty1 : tx1);
+                        s_rec[wib][lane] = R;
                     }
                 }
                 uint32_t items = n;
@@ -339,7 +369,7 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
                 const uint32_t total = __shfl_sync(FULL, items, 31), at = items - n;
                 const uint32_t nz = __ballot_sync(FULL, n != 0u);
                 // (packed: the table's entries are the lines with steps here)
-                if (n) s_item[wib][__popc(nz & below)] = make_uint2(first << 5 | lane, at);
+                if (n) s_item[wib][__popc(nz & below)] = make_uint2(lane, at);
                 __syncwarp();
 #pragma unroll 1
                 for (uint32_t base = 0; base < total; base += 32u) {
@@ -349,8 +379,8 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
                     float z = 0.0f;
                     if (base + lane < total) {
                         const uint2 it = s_item[wib][before + __popc(starts & upto) - 1u];
-                        const LineRec &R = s_rec[wib][it.x & 31u];
-                        const uint32_t step = (it.x >> 5) + (base + lane - it.y);
+                        const LineRec &R = s_rec[wib][it.x];
+                        const uint32_t step = base + lane - it.y;
                         const uint64_t along = R.begin + step, across = as_usize(line_step(R.s0, R.d, step));
                         const uint64_t x = R.wide ? along : across, y = R.wide ? across : along;
                         if (x >= tx0 && x < tx1 && y >= ty0 && y < ty1) {
@@ -363,8 +393,12 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
                     const uint32_t rounds = __reduce_max_sync(FULL, rank);
                     for (uint32_t r = 0; r <= rounds; ++r) {
                         if (idx != 0xFFFFFFFFu && rank == r) {
+                            const uint32_t py = idx / RF_LINE_PITCH, px = idx - py * RF_LINE_PITCH;
+                            const size_t at = direct ? (size_t)(ty0 + py) * J.w + tx0 + px : idx;
+                            uint32_t *pc = direct ? J.color : col;
+                            float *pd = direct ? J.depth : dep;
                             bool pass = true;
-                            const float cur = has_depth ? dep[idx] : 0.0f;
+                            const float cur = has_depth ? pd[at] : 0.0f;
                             switch (test) {  // ctx.rs:86-89
                                 case RF_K_DEPTH_NONE: pass = true; break;
                                 case RF_K_DEPTH_LESS: pass = cur < z; break;
@@ -373,10 +407,10 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
                             }
                             if (pass) {
                                 if (color_write) {
-                                    col[idx] = color;
+                                    pc[at] = color;
                                     fo += 1;
                                 }
-                                if (depth_write) dep[idx] = z;
+                                if (depth_write) pd[at] = z;
                             }
                         }
                         __syncwarp();  // (these pixels before the next round's tests)
@@ -386,7 +420,7 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
         }
         if (loaded) {
 #pragma unroll 8
-            for (uint32_t r = 0; r < RF_LINE_ROWS; ++r)
+            for (uint32_t r = 0; r < ROWS; ++r)
                 if (ty0 + r < ty1 && tx0 + lane < tx1) {
                     const size_t i = (size_t)(ty0 + r) * J.w + tx0 + lane;
                     if (color_write) J.color[i] = col[r * RF_LINE_PITCH + lane];
@@ -408,8 +442,15 @@ cudaError_t launch_lines(const DrawDev *draws, const JobDev *jobs, uint32_t nl, 
     RF_NEXT(k_line_setup, blocks, 128, 0, s, draws, jobs, nl, cpos, coc, recs, mask, stats);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const uint32_t rblocks = min((ntiles * (RF_TILE_H / RF_LINE_ROWS) + RF_LINE_WARPS - 1) / RF_LINE_WARPS, (uint32_t)nsm * 8);
-    RF_NEXT(k_line_raster, rblocks, RF_LINE_WARPS * 32, 0, s, jobs, recs, mask, ntiles, queue, stats);
+    // Quarters of a tile while those of the target are about as many as the warps
+    // that are resident, else halves: lines of up to 3,000 px, 30,000 on 1280 x
+    // 720 (920 tiles) 669 us in quarters and 836 in halves, on 1920 x 1080 (2,040)
+    // 818 and 769, on 3840 x 2160 1,313 and 1,067.
+    const bool quarters = ntiles <= (uint32_t)nsm * 8;
+    auto raster = quarters ? k_line_raster<RF_TILE_H / 4> : k_line_raster<RF_TILE_H / 2>;
+    const uint32_t parts = ntiles * (quarters ? 4u : 2u);
+    const uint32_t rblocks = min((parts + RF_LINE_WARPS - 1) / RF_LINE_WARPS, (uint32_t)nsm * 8);
+    RF_NEXT(raster, rblocks, RF_LINE_WARPS * 32, 0, s, jobs, recs, mask, ntiles, queue, stats);
     return cudaGetLastError();
 }
 

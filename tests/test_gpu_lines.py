@@ -192,3 +192,27 @@ def test_tile_parts(size, shape):
     # (the viewport above the target: rows below 0 draw in row 0)
     g, o = both(v, li, rf.GOURAUD, mat.viewport(0, -20, w, h - 20), w, h, pos_dim=4)
     check(g, o, "%s %dx%d above" % (shape, w, h))
+
+
+@pytest.mark.parametrize("size", [(1500, 700), (64, 2500), (3000, 40), (1917, 1081)])
+def test_long_lines(size):
+    """Lines across many tiles at every slope, those along one axis and those at
+    45 degrees among them, some from far outside a viewport larger than the
+    target; a few lines on many tiles, and many."""
+    w, h = size
+    rng = np.random.default_rng(w + h)
+    for n, vw, vh in ((7, w, h), (600, w, h), (600, 4 * w, 4 * h)):
+        a = rng.uniform([-0.9, -0.9], [0.9, 0.9], (n, 2))
+        ang = rng.choice(np.concatenate([np.linspace(0, 2 * np.pi, 16, endpoint=False), rng.uniform(0, 2 * np.pi, 8),
+                                         [1e-3, -1e-3, np.pi / 2 + 1e-3]]), n)
+        r = rng.uniform(0.05, 3.0, n)
+        b = a + np.stack([r * np.cos(ang), r * np.sin(ang)], -1) * (1.0, vw / vh)
+        z = rng.choice([0.5, 0.75, 1.0], n).repeat(2)
+        p = np.zeros((2 * n, 4), np.float32)
+        p[0::2, :2], p[1::2, :2], p[:, 3] = a, b, 1.0
+        v = np.concatenate([p * z[:, None].astype(np.float32), rng.uniform(0, 1, (2 * n, 3))], 1).astype(np.float32)
+        li = np.arange(2 * n, dtype=np.uint32).reshape(n, 2)
+        for vp in (mat.viewport(0, 0, vw, vh), mat.viewport(-w, -h, vw - w, vh - h)):
+            for ctx, depth in ((rf.Context(), True), (rf.Context(depth_test=rf.DEPTH_NONE), False)):
+                g, o = both(v, li, rf.GOURAUD, vp, w, h, pos_dim=4, ctx=ctx, depth=depth)
+                check(g, o, "%d lines %dx%d in %dx%d" % (n, w, h, vw, vh))
