@@ -325,12 +325,13 @@ static __device__ __noinline__ float jump_far(float s, float d, uint32_t k) { re
 // The lane's scanline j of half H (raster.rs:84-113), clipped to the tile,
 // then its fragments (raster.rs:60-69) into the tile (target.rs:163-198).
 // FAST: the default context (depth test Less, colour and depth writes on).
+// rv: the row's quantities, where the lane walks them.
 template <int KIND, bool FAST>
 __device__ __forceinline__ void span(TileCtx &T, const Paint &d, const HalfRec *__restrict__ H,
-                                     const HalfRuns *__restrict__ U, uint32_t j) {
+                                     const HalfRuns *__restrict__ U, uint32_t j, bool walked, const float *rv) {
     constexpr int NC = Kind<KIND>::NC;
-    const float lx = row_value(H, U, RF_R_LX, j);
-    const float rx = row_value(H, U, RF_R_RX, j);
+    const float lx = walked ? rv[RF_R_LX] : row_value(H, U, RF_R_LX, j);
+    const float rx = walked ? rv[RF_R_RX] : row_value(H, U, RF_R_RX, j);
     const float x0r = round_up_to_half(lx), x1r = round_up_to_half(rx);
     // xs..xe as `as usize` (target.rs:259-262), zip-truncated to the
     // fragment count, clipped to the tile.  32-bit saturating casts give the
@@ -354,9 +355,9 @@ __device__ __forceinline__ void span(TileCtx &T, const Paint &d, const HalfRec *
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
         dv[c] = H->dvdx[c];
-        const float c0 = row_value(H, U, RF_R_C + c, j);
+        const float c0 = walked ? rv[RF_R_C + c] : row_value(H, U, RF_R_C + c, j);
         const float adj = fadd(c0, fmul(fsub(fadd(c0, dv[c]), c0), tshift));
-        v[c] = jump_far(adj, dv[c], k0);
+        v[c] = jump(adj, dv[c], k0);
     }
     constexpr int NP = PreNC<KIND>::NP;
     float2 v2[NP], dv2[NP];
@@ -367,7 +368,8 @@ __device__ __forceinline__ void span(TileCtx &T, const Paint &d, const HalfRec *
     }
     uint32_t idx = (a - T.tx0) * RF_TILE_H + T.row;
     const uint32_t end = (b - T.tx0) * RF_TILE_H + T.row;
-    while (idx < end) T.frags_o += px_group<KIND, FAST, 1>(T, d, (uint32_t)KIND, v2, dv2, idx, end);
+    constexpr int U_PX = FAST && !Kind<KIND>::TEXTURED ? 4 : 1;
+    while (idx < end) T.frags_o += px_group<KIND, FAST, U_PX>(T, d, (uint32_t)KIND, v2, dv2, idx, end);
 }
 
 // Which scanline of a half lands on row y: row(j) = (y0r + j) as usize =
@@ -406,6 +408,11 @@ __device__ __forceinline__ void raster_prim_k(TileCtx &T, const Paint &d, const 
     const HalfRuns *U = start1 ? &P->runs[1] : &P->runs[0];
     uint32_t j = start1 ? b0 : a0, jend = start1 ? b1 : a1;
     bool more = !start1 && b1 > b0;
+    // The rows above the buffer, all of them one lane's, are walked
+    // (ScanlineIter::next); a single row's quantities are worked out as asked.
+    constexpr int NQ = RF_R_C + Kind<KIND>::NC;
+    float rv[NQ];
+    bool walked = false;
     for (;;) {
         if (j >= jend) {
             if (!more) break;
@@ -414,10 +421,20 @@ __device__ __forceinline__ void raster_prim_k(TileCtx &T, const Paint &d, const 
             j = b0;
             jend = b1;
             more = false;
+            walked = false;
             continue;
         }
-        span<KIND, FAST>(T, d, H, U, j);
+        if (!walked && jend - j > 1u) {
+            walked = true;
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) rv[r] = row_value(H, U, r, j);
+        }
+        span<KIND, FAST>(T, d, H, U, j, walked, rv);
         ++j;
+        if (walked) {
+#pragma unroll
+            for (int r = 0; r < NQ; ++r) rv[r] = fadd(rv[r], H->d[r]);
+        }
     }
 }
 

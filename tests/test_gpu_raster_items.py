@@ -273,3 +273,20 @@ def test_large_and_small_groups_in_one_batch(graphs, large):
         for x in keep:
             x.close()
         dev.close()
+
+
+@pytest.mark.parametrize("tw", [8, 32])
+@pytest.mark.parametrize("kind", sorted(NATTR))
+def test_triangles_past_the_top(kind, tw):
+    """Triangles whose first rows lie above the target (all of them drawn in row
+    0, one lane's): of one such row and of hundreds, the two halves' both, in
+    both contexts."""
+    w, h = 210, 70
+    parts = [tris(60 + i, 60, w, 2 * h, (4, 80, y0, y1), kind) for i, (y0, y1) in enumerate(((1, 6), (20, 90), (200, 700)))]
+    v = np.concatenate([p.verts for p in parts])
+    d = DrawSpec(v, np.arange(len(v), dtype=np.uint32).reshape(-1, 3), kind, pos_dim=4, flat_rgba=0xFF336699,
+                 tex=parts[0].tex)
+    vp = mat.viewport(0, -h, w, h)
+    for ctx in (rf.Context(face_cull=rf.CULL_NONE), rf.Context(face_cull=rf.CULL_NONE, depth_test=rf.DEPTH_NONE)):
+        g, o = gpu_render([d], vp, w, h, ctx=ctx, tile=(tw, 4)), oracle_render([d], vp, w, h, ctx=ctx)
+        assert_parity(g, o, color_tol=1 if kind == rf.GOURAUD_SRGB else 0, what="kind %d" % kind)
