@@ -1064,11 +1064,15 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
         return RF_OK;
     };
 
-    if (tuned) CK(cudaEventRecord(tuned->e0, s));
+    // (a trial frame's events hold its GPU work and nothing that comes once a
+    // width: kernels are loaded before the first, a graph is made and uploaded)
+    if (tuned) CK(rfk::load_raster(TW, ctx->groups.data(), ng));
+    const bool replay = !sorted && ctx->graphs && !ctx->timing;
+    if (tuned && !replay) CK(cudaEventRecord(tuned->e0, s));
     ctx->mask_suspect = true;  // (until every launch is queued)
     if (sorted) {
         if ((st = enqueue_sorted())) return st;
-    } else if (ctx->graphs && !ctx->timing) {
+    } else if (replay) {
         GraphKey key{};
         const uint64_t kv[] = {ctx->gen, ndraws, nj, nv, nt, ntiles, mask_words, TW, ctx->warps,
                                pieces(hj), (any_cull ? 2u : 0u) | (per_job ? 1u : 0u), ctx->rows_cap, ctx->list_cap};
@@ -1108,6 +1112,10 @@ rf_status run_jobs(rf_ctx *ctx, const JobIn *in, uint32_t nin, bool per_job,
             hit = &ctx->gcache.back();
         }
         hit->used = ++ctx->gclock;
+        if (tuned) {
+            CK(cudaGraphUpload(hit->exec, s));
+            CK(cudaEventRecord(tuned->e0, s));
+        }
         CK(cudaGraphLaunch(hit->exec, s));
         ctx->graph_launches += 1;
     } else {

@@ -2060,6 +2060,25 @@ cudaError_t launch_lists(const JobDev *jobs, uint32_t nj, uint32_t *mask, uint32
     return cudaGetLastError();
 }
 
+static cudaError_t raster_of(uint32_t tile_w, bool one, int kind, RF_RASTER_PARAMS) {
+    switch (tile_w) {
+        case 8: return one ? launch_raster_tw8(kind, RF_RASTER_ARGS) : launch_raster_any_tw8(kind, RF_RASTER_ARGS);
+        case 16: return one ? launch_raster_tw16(kind, RF_RASTER_ARGS) : launch_raster_any_tw16(kind, RF_RASTER_ARGS);
+        case 64: return one ? launch_raster_tw64(kind, RF_RASTER_ARGS) : launch_raster_any_tw64(kind, RF_RASTER_ARGS);
+        default: return one ? launch_raster_tw32(kind, RF_RASTER_ARGS) : launch_raster_any_tw32(kind, RF_RASTER_ARGS);
+    }
+}
+
+cudaError_t load_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng) {
+    for (uint32_t g = 0; g < ng; ++g) {
+        const cudaError_t e = raster_of(tile_w, groups[g].fast, groups[g].kind, nullptr, 0, nullptr, nullptr, nullptr,
+                                        nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr,
+                                        nullptr, 0, 0, nullptr);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng, const JobDev *jobs, uint32_t nj,
                           const DrawDev *draws, const PrimRec *prims, const RasterPrim *rprims, const uint32_t *rows,
                           const uint2 *ent, const uint32_t *mask, const uint2 *segs,
@@ -2074,13 +2093,7 @@ cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t n
         const uint32_t *nfirst = counters + RF_CNT_ITEMS_G + g;
         uint32_t *queue = counters + RF_CNT_QUEUE_G + g;
         const cudaStream_t s = st[g % nst];
-        cudaError_t e;
-        switch (tile_w) {
-            case 8: e = one ? launch_raster_tw8(kind, RF_RASTER_ARGS) : launch_raster_any_tw8(kind, RF_RASTER_ARGS); break;
-            case 16: e = one ? launch_raster_tw16(kind, RF_RASTER_ARGS) : launch_raster_any_tw16(kind, RF_RASTER_ARGS); break;
-            case 64: e = one ? launch_raster_tw64(kind, RF_RASTER_ARGS) : launch_raster_any_tw64(kind, RF_RASTER_ARGS); break;
-            default: e = one ? launch_raster_tw32(kind, RF_RASTER_ARGS) : launch_raster_any_tw32(kind, RF_RASTER_ARGS); break;
-        }
+        const cudaError_t e = raster_of(tile_w, one, kind, RF_RASTER_ARGS);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

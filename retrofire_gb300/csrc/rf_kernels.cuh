@@ -223,6 +223,9 @@ cudaError_t launch_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t n
                           const uint2 *ent, const uint32_t *mask, const uint2 *segs,
                           const uint2 *list, uint32_t ntiles, const uint32_t *items, uint32_t *counters,
                           StatsDev *stats, uint32_t warps, int nsm, const cudaStream_t *st, uint32_t nst);
+// Loads the groups' raster kernels for a tile width: a kernel's first launch in a
+// process does so otherwise.
+cudaError_t load_raster(uint32_t tile_w, const RasterGroup *groups, uint32_t ng);
 cudaError_t launch_fill(uint32_t *color, float *depth, size_t n, uint32_t px, float z,
                         uint32_t flags, int nsm, cudaStream_t s);
 // Object culling of the draws with RF_DRAW_CULL_BBOX (sets DrawDev::culled

@@ -1554,6 +1554,7 @@ static cudaError_t launch_raster_k(RF_RASTER_PARAMS) {
     struct Tag {};  // one per (TW, KIND, FAST)
     cudaError_t e = opt_in_smem<Tag>(k_raster<TW, KIND, FAST>, (int)SMEM_MAX);
     if (e != cudaSuccess) return e;
+    if (ntiles == 0) return cudaSuccess;  // (loaded)
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_raster<TW, KIND, FAST>, warps * 32, smem);
     if (per_sm < 1) per_sm = 1;

@@ -7,6 +7,7 @@
 #include <sys/mman.h>
 
 #include <set>
+#include <string>
 
 #include "../../retrofire_gb300/csrc/rf_api.cu"
 
@@ -31,6 +32,9 @@ uint32_t g_tris = 1;                         // triangles of every draw
 const void *g_last_mask = nullptr;
 size_t g_last_size = 0;
 
+// The frames' calls: B(egin of a capture), I(nstantiate), U(pload), G(raph
+// launch), R(aster launch), L(oad of raster kernels), E(vent that times), a bar after each.
+std::string g_log;
 std::vector<RasterGroup> g_groups;   // of the last frame
 std::set<cudaStream_t> g_streams;    // ... that its groups are on
 
@@ -90,24 +94,36 @@ cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int *n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t) { return "error"; }
-cudaError_t cudaEventCreate(cudaEvent_t *e) {
+cudaError_t cudaEventCreate(cudaEvent_t *e) {  // (2: one that times)
     if (g_fail_event >= 0 && g_fail_event-- == 0) return cudaErrorMemoryAllocation;
-    *e = reinterpret_cast<cudaEvent_t>(1);
+    *e = reinterpret_cast<cudaEvent_t>(2);
     return cudaSuccess;
 }
 cudaError_t event_ok(cudaEvent_t e) { return e ? cudaSuccess : cudaErrorInvalidResourceHandle; }
-cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) {
+    const cudaError_t st = cudaEventCreate(e);
+    if (!st) *e = reinterpret_cast<cudaEvent_t>(1);
+    return st;
+}
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 1.0f; return cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t e) { return event_ok(e); }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return event_ok(e); }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) {
+    if (e == reinterpret_cast<cudaEvent_t>(2)) g_log += 'E';
+    return event_ok(e);
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t e) { return event_ok(e); }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t *, cudaGraph_t, unsigned long long) { return cudaErrorNotSupported; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorNotSupported; }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorNotSupported; }
-cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorNotSupported; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t, unsigned long long) {
+    g_log += 'I';
+    *x = reinterpret_cast<cudaGraphExec_t>(1);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphUpload(cudaGraphExec_t, cudaStream_t) { g_log += 'U'; return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { g_log += 'G'; return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { g_log += 'B'; return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { *g = nullptr; return cudaSuccess; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
     static uintptr_t n = 0;
     *s = reinterpret_cast<cudaStream_t>(++n);
@@ -184,11 +200,13 @@ cudaError_t launch_raster(uint32_t, const RasterGroup *g, uint32_t ng, const Job
                           const PrimRec *, const RasterPrim *, const uint32_t *, const uint2 *, const uint32_t *,
                           const uint2 *, const uint2 *, uint32_t, const uint32_t *, uint32_t *, StatsDev *, uint32_t, int,
                           const cudaStream_t *st, uint32_t nst) {
+    g_log += 'R';
     g_groups.assign(g, g + ng);
     g_streams.clear();
     for (uint32_t i = 0; i < ng; ++i) g_streams.insert(st[i % nst]);
     return cudaSuccess;
 }
+cudaError_t load_raster(uint32_t, const RasterGroup *, uint32_t) { g_log += 'L'; return cudaSuccess; }
 cudaError_t launch_mesh_bbox(const float *, uint32_t, uint32_t, float *, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_stats_fold(const StatsDev *, uint32_t, StatsDev *, cudaStream_t) { return cudaSuccess; }
 uint32_t dsort_scan_items(uint32_t) { return 0; }
@@ -363,5 +381,20 @@ int32_t shim_groups(const uint32_t *jobs, uint32_t n, uint32_t *out, uint32_t *s
     }
     *streams = (uint32_t)g_streams.size();
     return (int32_t)g_groups.size();
+}
+// n frames of one shape with the tile width picked online; log: their calls.
+int32_t shim_trials(uint32_t n, int graphs, int32_t sort, char *log, uint32_t room) {
+    rf_ctx *ctx = nullptr;
+    if (rf_ctx_create(nullptr, &ctx)) return -1;
+    rf_ctx_set_graphs(ctx, graphs);
+    g_log.clear();
+    rf_status st = RF_OK;
+    for (uint32_t i = 0; i < n && !st; ++i) {
+        st = frame(ctx, 20, 64, 64, sort);
+        g_log += '|';
+    }
+    rf_ctx_destroy(ctx);
+    snprintf(log, room, "%s", g_log.c_str());
+    return st;
 }
 }

@@ -29,6 +29,7 @@ def shim(tmp_path_factory):
     L.shim_alloc_fails.argtypes = [C.c_uint32, C.POINTER(C.c_uint64)]
     L.shim_event_fails.argtypes = [C.c_uint32, C.POINTER(C.c_int32)]
     L.shim_groups.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)]
+    L.shim_trials.argtypes = [C.c_uint32, C.c_int, C.c_int32, C.c_char_p, C.c_uint32]
     L.shim_refused.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]
     return L
 
@@ -152,3 +153,16 @@ def test_raster_groups(shim, jobs, groups):
     kinds = len({g[0] for g in groups})
     # a mesh's box two, zero, vertex, clip two, lists, the stats, three a kind, one a group
     assert k.value == 2 * len(jobs) + 6 + 3 * kinds + n
+
+
+@pytest.mark.parametrize("graphs,sort,timed", [(0, 0, "ERE"), (1, 0, "EGE"), (0, 1, "ERE"), (1, 1, "ERE")])
+def test_trials_time_the_frame_alone(shim, graphs, sort, timed):
+    """The frames that pick a tile width: loading its kernels, capturing,
+    instantiating and uploading its graph all come before the first event."""
+    log = C.create_string_buffer(4096)
+    assert shim.shim_trials(9, graphs, sort, log, len(log)) == 0
+    f = log.value.decode().split("|")
+    for trial in f[1:5]:
+        assert trial.count("E") == 2 and trial[trial.index("E"):] == timed, f
+        assert "L" in trial[:trial.index("E")]
+    assert not any("E" in x or "L" in x for x in f[:1] + f[5:])
