@@ -68,6 +68,33 @@ __device__ __forceinline__ uint32_t warp_upper_index(uint32_t n, uint32_t x, F k
     }
 }
 
+// Position of the r-th set bit of v (r >= 1, at most popc(v)): halving
+// search on popcounts.
+__device__ __forceinline__ uint32_t nth_bit(uint32_t v, uint32_t r) {
+    uint32_t pos = 0;
+#pragma unroll
+    for (uint32_t w = 16; w >= 1; w >>= 1) {
+        const uint32_t c = __popc(v & ((1u << w) - 1u));
+        if (c < r) {
+            r -= c;
+            v >>= w;
+            pos += w;
+        }
+    }
+    return pos;
+}
+// The lane whose bits hold the k-th of all (incl: the lanes' inclusive
+// counts; every lane calls).
+__device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t k) {
+    uint32_t L = 0;
+#pragma unroll
+    for (uint32_t step = 16; step >= 1; step >>= 1) {
+        const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, L + step - 1u);
+        if (v <= k) L += step;
+    }
+    return L & 31u;
+}
+
 // Warp-aggregated 64-bit counter add (all 32 lanes must call).
 __device__ __forceinline__ void warp_add_u64(unsigned long long *dst, unsigned long long v,
                                              bool same_dst) {

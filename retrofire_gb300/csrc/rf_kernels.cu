@@ -1214,7 +1214,7 @@ k_setup(const DrawDev *__restrict__ draws, uint32_t nd, const JobDev *__restrict
 // 0 when its draws mix shader kinds (taken per triangle).
 template <int NCT>
 __global__ void __launch_bounds__(256, 4)
-k_bin(const DrawDev *__restrict__ draws, const JobDev *__restrict__ jobs,
+k_bin(const JobDev *__restrict__ jobs,
       PrimRec *prims, const uint32_t *live, uint32_t tile_w,
       uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims,
       uint2 *__restrict__ ent, uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
@@ -1553,7 +1553,7 @@ __global__ void __launch_bounds__(256, 4)
 k_bin_small(const JobDev *__restrict__ jobs, PrimRec *prims,
             const uint32_t *live_small, uint32_t *__restrict__ live, uint32_t tile_w,
             uint32_t *__restrict__ rows, unsigned long long rows_cap, RasterPrim *__restrict__ rprims, uint2 *__restrict__ ent,
-            uint32_t *__restrict__ mask, StatsDev *__restrict__ stats, uint32_t *__restrict__ counters,
+            uint32_t *__restrict__ mask, StatsDev *__restrict__ stats,
             unsigned long long *__restrict__ marks, const uint32_t *small_n,
             uint32_t *__restrict__ live_n) {
     grid_begin();
@@ -1766,21 +1766,6 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *prims,
 // registers and 5 us more.
 #define RF_LIST_WARPS 4u
 namespace {
-// Position of the r-th set bit of v (r >= 1, at most popc(v)): halving
-// search on popcounts.
-__device__ __forceinline__ uint32_t nth_bit(uint32_t v, uint32_t r) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (uint32_t w = 16; w >= 1; w >>= 1) {
-        const uint32_t c = __popc(v & ((1u << w) - 1u));
-        if (c < r) {
-            r -= c;
-            v >>= w;
-            pos += w;
-        }
-    }
-    return pos;
-}
 __device__ __forceinline__ uint32_t warp_incl(uint32_t v, uint32_t lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1788,17 +1773,6 @@ __device__ __forceinline__ uint32_t warp_incl(uint32_t v, uint32_t lane) {
         if (lane >= (uint32_t)o) v += y;
     }
     return v;
-}
-// The lane whose bits hold the k-th of all (incl: the lanes' inclusive
-// counts; every lane calls).
-__device__ __forceinline__ uint32_t lane_of(uint32_t incl, uint32_t k) {
-    uint32_t L = 0;
-#pragma unroll
-    for (uint32_t step = 16; step >= 1; step >>= 1) {
-        const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, L + step - 1u);
-        if (v <= k) L += step;
-    }
-    return L & 31u;
 }
 }  // namespace
 
@@ -2036,10 +2010,10 @@ cudaError_t launch_setup(const DrawDev *draws, uint32_t nd, const JobDev *jobs, 
         // smaller ones that found no room for their records); the counts are
         // only known on the device.
         const uint32_t sblocks = min((gt + 31) / 32, (uint32_t)nsm * 4);
-        RF_NEXT(bin16, sblocks, 256, 0, s, jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
-                                      counters, marks, mid_n, big_n);
+        RF_NEXT(bin16, sblocks, 256, 0, s, jobs, prims, mid, big, tile_w, rows, rows_cap, rprims, ent, mask, stats, marks,
+                mid_n, big_n);
         const uint32_t wblocks = min(gt, (uint32_t)nsm * 16);
-        RF_NEXT(bin, wblocks, 256, 0, s, draws, jobs, prims, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
+        RF_NEXT(bin, wblocks, 256, 0, s, jobs, prims, big, tile_w, rows, rows_cap, rprims, ent, mask, stats,
                                     counters, marks, big_n);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         big += (size_t)gt * fan;

@@ -312,17 +312,11 @@ k_line_raster(const JobDev *__restrict__ jobs, const LineRec *recs,
             }
             if (lb < nlines) {
                 const uint32_t k = lb + lane;
-                uint32_t L = 0;
-#pragma unroll
-                for (uint32_t step = 16; step >= 1; step >>= 1) {
-                    const uint32_t v = __shfl_sync(FULL, incl, L + step - 1u);
-                    if (v <= k) L += step;
-                }
-                L &= 31u;
+                const uint32_t L = lane_of(incl, k);
                 const uint32_t wl = __shfl_sync(FULL, word, L);
                 const uint32_t ex = __shfl_sync(FULL, incl - __popc(word), L);
                 if (k < nlines)
-                    s_pend[wib][pend + lane] = (wb - 32u + L) * 32u + rfr::nth_set_bit(wl, k - ex + 1u);
+                    s_pend[wib][pend + lane] = (wb - 32u + L) * 32u + nth_bit(wl, k - ex + 1u);
                 pend += min(nlines - lb, 32u);
                 lb += 32u;
             }

@@ -547,21 +547,6 @@ __device__ __forceinline__ float tile_depth_min(const TileCtx &T) {
 struct WarpTake {
     uint32_t take, total, src, pos, end_lane, end_rest;
 };
-// Position of the r-th set bit of v (r >= 1, at most popc(v)): halving
-// search on popcounts.
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t v, uint32_t r) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (uint32_t w = 16; w >= 1; w >>= 1) {
-        const uint32_t c = __popc(v & ((1u << w) - 1u));
-        if (c < r) {
-            r -= c;
-            v >>= w;
-            pos += w;
-        }
-    }
-    return pos;
-}
 // (Out of line: it runs once per 32 triangles, and the kernels that switch
 // on the shader kind per triangle are large already.)
 static __device__ __noinline__ WarpTake warp_take(uint32_t b, uint32_t want, uint32_t first, uint32_t lane) {
@@ -588,14 +573,14 @@ static __device__ __noinline__ WarpTake warp_take(uint32_t b, uint32_t want, uin
     const uint32_t exL = __shfl_sync(0xFFFFFFFFu, ex, L);
     const uint32_t bL = __shfl_sync(0xFFFFFFFFu, b, L);
     t.src = L;
-    t.pos = nth_set_bit(bL, k - exL + 1u);  // (meaningless on lanes outside the take)
+    t.pos = nth_bit(bL, k - exL + 1u);  // (meaningless on lanes outside the take)
     // Where the take stopped: the source of slot take - 1.
     const uint32_t last = first + (t.take ? t.take : 1u) - 1u;
     t.end_lane = __shfl_sync(0xFFFFFFFFu, L, last & 31u);
     const uint32_t end_ex = __shfl_sync(0xFFFFFFFFu, exL, last & 31u);
     const uint32_t end_b = __shfl_sync(0xFFFFFFFFu, bL, last & 31u);
     const uint32_t used = t.take - end_ex;  // bits of end_lane taken
-    const uint32_t lastpos = nth_set_bit(end_b, used ? used : 1u);
+    const uint32_t lastpos = nth_bit(end_b, used ? used : 1u);
     t.end_rest = used ? (end_b & ~((2u << lastpos) - 1u)) : end_b;
     return t;
 }
@@ -1402,7 +1387,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
                         pend &= ~gm;
                         if (SPLIT && pend == 0u && cnt <= 8u) {
                             // The last ones, and few: four lanes a span.
-                            const uint32_t src = nth_set_bit(gm, min(lane >> 2, cnt - 1u) + 1u);
+                            const uint32_t src = nth_bit(gm, min(lane >> 2, cnt - 1u) + 1u);
                             go = lane >> 2 < cnt;
                             row = __shfl_sync(FULL, row, src);
                             ki = __shfl_sync(FULL, ki, src);
