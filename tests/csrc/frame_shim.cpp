@@ -403,9 +403,10 @@ int32_t shim_trials(uint32_t n, int graphs, int32_t sort, char *log, uint32_t ro
     return st;
 }
 // The tile width picked for a frame whose trials take ms[0..4).
-uint32_t shim_pick(const float *ms) {
+uint32_t shim_pick(const float *ms, int graphs) {
     rf_ctx *ctx = nullptr;
     if (rf_ctx_create(nullptr, &ctx)) return 0;
+    rf_ctx_set_graphs(ctx, graphs);
     memcpy(g_trial_ms, ms, sizeof g_trial_ms);
     g_trial = 0;
     for (int i = 0; i < 6; ++i)

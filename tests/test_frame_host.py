@@ -30,7 +30,7 @@ def shim(tmp_path_factory):
     L.shim_event_fails.argtypes = [C.c_uint32, C.POINTER(C.c_int32)]
     L.shim_groups.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint64)]
     L.shim_trials.argtypes = [C.c_uint32, C.c_int, C.c_int32, C.c_char_p, C.c_uint32]
-    L.shim_pick.argtypes = [C.c_void_p]
+    L.shim_pick.argtypes = [C.c_void_p, C.c_int]
     L.shim_refused.argtypes = [C.c_uint32, C.c_uint32, C.POINTER(C.c_uint64)]
     return L
 
@@ -169,8 +169,9 @@ def test_trials_time_the_frame_alone(shim, graphs, sort, timed):
     assert not any("E" in x or "L" in x for x in f[:1] + f[5:])
 
 
-@pytest.mark.parametrize("ms,width", [((10, 10, 10, 10), 8), ((10, 9.8, 9.6, 11), 8), ((10, 9, 8.8, 12), 16),
-                                      ((10, 9.7, 9, 8.9), 32), ((10, 9, 8, 7), 64), ((1, 2, 3, 4), 8)])
-def test_a_wider_tile_has_to_be_clearly_faster(shim, ms, width):
-    a = np.array(ms, np.float32)
-    assert shim.shim_pick(a.ctypes.data) == width
+@pytest.mark.parametrize("us,replayed,launched", [
+    ((100, 100, 100, 100), 8, 8), ((100, 98, 96, 110), 32, 8), ((59.5, 54.8, 62.2, 70), 16, 8), ((140, 120, 118, 150), 16, 16),
+    ((1000, 975, 960, 970), 32, 32), ((100, 90, 80, 68), 64, 64), ((100, 200, 300, 400), 8, 8)])
+def test_a_wider_tile_has_to_be_clearly_faster(shim, us, replayed, launched):
+    a = np.array(us, np.float32) / 1000
+    assert (shim.shim_pick(a.ctypes.data, 1), shim.shim_pick(a.ctypes.data, 0)) == (replayed, launched)
