@@ -1205,7 +1205,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
             if (TRIM) full += __reduce_add_sync(FULL, put ? rows0 : 0u);
             todo &= ~took;
         }
-        const bool slow_now = todo && ((slows >> (__ffs(todo) - 1)) & 1u);  // (the next one has no records)
+        const uint32_t slow_now = todo && ((slows >> (__ffs(todo) - 1)) & 1u) ? todo & (0u - todo) : 0u;
         if (!todo && !done) continue;  // the table has room left
 
         // The table's triangles, scanline by scanline.  (Their steps arrive
@@ -1436,14 +1436,12 @@ __device__ __forceinline__ void raster_tile(const RasterArgs &A, const JobDev &J
             nt = full = 0;
             if constexpr (FAST) tzmin = tile_depth_min<TW>(T);
         }
-        if (slow_now) {  // (and those right behind it)
-            do {
-                const uint32_t l = __ffs(todo) - 1u;
-                const uint32_t ps = __shfl_sync(FULL, p, l), ds = __shfl_sync(FULL, hdraw, l);
-                T.frags_o += raster_prim_slow<KIND, FAST>(T, (uint32_t)A.draws[ds].shader, A.draws + ds, A.prims + ps);
-                __syncwarp();
-                todo &= todo - 1u;
-            } while (todo && ((slows >> (__ffs(todo) - 1)) & 1u));
+        if (slow_now) {
+            const uint32_t l = __ffs(slow_now) - 1u;
+            const uint32_t ps = __shfl_sync(FULL, p, l), ds = __shfl_sync(FULL, hdraw, l);
+            T.frags_o += raster_prim_slow<KIND, FAST>(T, (uint32_t)A.draws[ds].shader, A.draws + ds, A.prims + ps);
+            __syncwarp();
+            todo &= ~slow_now;
         }
         if (done) break;
     }
