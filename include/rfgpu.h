@@ -145,8 +145,9 @@ rf_status rf_ctx_set_tiling(rf_ctx *ctx, uint32_t tile_w, uint32_t warps_per_blo
  * for each frame shape (draw, scene, vertex and triangle counts, target
  * pixels) the first frame is a warm-up, the next four run with tile widths
  * 8, 16, 32 and 64 while CUDA events time their GPU work, and every later
- * frame of that shape uses the fastest.  Results do not depend on the
- * width.  rf_ctx_last_tiling reports the last frame's width and warps. */
+ * frame of that shape uses the fastest (a wider one where it is clearly
+ * faster).  Results do not depend on the width.  rf_ctx_last_tiling reports
+ * the last frame's width and warps. */
 rf_status rf_ctx_set_online_tuning(rf_ctx *ctx, int32_t enable);
 rf_status rf_ctx_last_tiling(rf_ctx *ctx, uint32_t *tile_w, uint32_t *warps);
 

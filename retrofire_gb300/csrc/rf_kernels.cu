@@ -821,9 +821,9 @@ __device__ __forceinline__ void row_record(float lx, float rx, const float *cv, 
 static_assert(RF_SETUP_WORDS % 2 == 1 && RF_SETUP_WORDS * 4 >= sizeof(RasterPrim), "setup slots");
 // Triangles of at most RF_INLINE_ROWS rows on the target, no wider than
 // RF_INLINE_WIDTH px, are binned by the thread that sets them up (500 k-triangle
-// grid: setup stage 200 us, 245 with eight lanes a triangle in a launch of their
-// own; 100,000 triangles 224 and 235).  Larger ones leave a warp waiting for the
-// longest.
+// grid at width 8: setup stage 160 us, 231 with sixteen lanes a triangle in
+// k_bin_small; 64 uneven scenes 798 and 951; 100,000 triangles 233 both ways).
+// Larger ones leave a warp waiting for the longest.
 #define RF_INLINE_ROWS 8u
 #define RF_INLINE_WIDTH 128.0f
 // Bound by the instructions and their latencies of a warp's 32 triangles, not
@@ -1761,9 +1761,9 @@ k_bin_small(const JobDev *__restrict__ jobs, PrimRec *prims,
 #define RF_HEAVY_MIN 16u  // ... nor taken early
 // Warps a block, which takes its lists' place with one atomic: its warps wait
 // for the longest of them, and all wait for memory, so small blocks and as many
-// as 42 registers allow.  Setup stage of the 500 k-triangle grid 148 us with 8
-// warps and 48 registers, 142 so; loading 64 summary words ahead took 62
-// registers and 5 us more.
+// as 42 registers allow.  Setup stage of the 500 k-triangle grid 167 us with 8
+// warps and 48 registers, 160 so (width 8); loading 64 summary words ahead took
+// 62 registers and 5 us more.
 #define RF_LIST_WARPS 4u
 namespace {
 __device__ __forceinline__ uint32_t warp_incl(uint32_t v, uint32_t lane) {

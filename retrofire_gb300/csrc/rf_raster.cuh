@@ -32,9 +32,9 @@
 // What bounds it: the chain of dependent instructions of each warp (16 warps
 // per SM, 38 % of issue slots), so what counts is instructions per triangle:
 // one warp pass per triangle -- lane = row, most lanes idle on small
-// triangles -- measured 478 us on the 500 k-triangle grid at 1080p (now 90),
-// 337 us on 10 k instanced cubes (81), 2.40 ms on 64 uneven scenes (0.51)
-// and 236 us on 100 k triangles of 1..10^4 px^2 (163).
+// triangles -- measured 478 us on the 500 k-triangle grid at 1080p (now 80 at
+// width 8), 337 us on 10 k instanced cubes (85), 2.40 ms on 64 uneven scenes
+// (0.52) and 236 us on 100 k triangles of 1..10^4 px^2 (163 at width 16).
 // The loop's code has to stay small: with every helper inlined (8,000
 // instructions) warps waited on instruction fetch as long as they worked.
 // A tile of whole 32-column blocks goes back to HBM through the copy engine
@@ -745,8 +745,9 @@ constexpr uint32_t RF_CAND_WORDS = 256u;  // 31 left over and a batch of 32 fans
 static_assert(31 + 32 * RF_MAX_FAN <= RF_CAND_WORDS, "ring size");
 constexpr uint32_t RF_TAB_WORDS = (4u + 2u * RF_NC + 2u) * 32u;
 // By row from this many scanlines a triangle in the tile: at 6 the grid's
-// raster takes 158 us and the crates' 77, at 10 and 16 139 and 57; the fill
-// frame's triangles (18) are even at all three.
+// raster takes 107 us and the crates' 63, at 10 and at 16 84 and 51 (width 8);
+// 64 uneven scenes 530 at 6 and 10, 545 at 16; the fill frame's triangles (18
+// rows) are even at all three.
 constexpr uint32_t RF_ROW_MEAN = 10u;
 template <int TW, int KIND>
 struct Region {
